@@ -35,11 +35,8 @@ sys.path.insert(0, ROOT)
 WORKLOAD = dict(N=192, coils=32, spokes=50000, samples=384, width=4, oversamp=1.25)
 FALLBACK_HBM_GBS = 6650.0
 METRIC = "NUFFT fwd+adj k-space samples/s (3D kooshball)"
-# kernels that run the workload's interpolation / gridding (3D, width 4, 32 coils):
-# tensor-core gridding (grid_tmem_kernel) unless DMR_NO_TC selects the cell-cube kernel
-KERNELS = {"interp": "interp_cube_kernel",
-           "grid": "grid_cube_kernel" if os.environ.get("DMR_NO_TC", "0") not in ("", "0") else "grid_tmem_kernel",
-           "grid_det": "grid_tmem_kernel"}
+# kernels that run the workload's interpolation / gridding (3D, width 4, 32 coils)
+KERNELS = {"interp": "interp_march_kernel", "grid": "grid_planes_kernel", "grid_det": "grid_planes_kernel"}
 UNIT = "samples/s"
 
 
@@ -221,7 +218,7 @@ class CpuBaseline:
 def parity_check(F, cb, plan, img, ksp, dcf, coils=(0, 1)):
     """Relative L2 error of the timed GPU path against the oracle at the full
     workload size, on two of its coils (coils are independent): forward,
-    atomic (tensor-core) adjoint and deterministic adjoint."""
+    atomic adjoint and deterministic adjoint."""
     R, sel = cb.R, list(coils)
 
     def rel(a, b):

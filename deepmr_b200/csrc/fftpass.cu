@@ -293,6 +293,11 @@ struct FftGeom {
     int64_t gsize, isize; // points per grid / image
     const float *apod[3]; // per-axis apodisation by image index (nullptr: 1)
     float scale;
+    // coil-interleaved grids (row passes with IL): the line set of a (chunk,
+    // frame) is (z, y, coil), element stride CS; images stay (batch, frame, z, y, x)
+    int CS = 1;
+    int nframes = 1;
+    int64_t batch = 0;
 };
 
 __host__ __device__ __forceinline__ int wrapi(int v, int n)
@@ -334,11 +339,14 @@ struct RowLine {
     float s;
 };
 
+// With IL line `row` is coil row % CS of image row row / CS of a (chunk, frame);
+// coils past the batch have no image row (offset -1) but a grid row.
+template <bool IL>
 __device__ __forceinline__ void row_lines(const FftGeom &g, int64_t row0, int64_t nrows, RowLine *lines)
 {
     const int c = threadIdx.x;
     if (c >= kFftLines) return;
-    const int64_t row = row0 + c;
+    int64_t row = row0 + c;
     RowLine ln;
     ln.img = -1;
     ln.grid = -1;
@@ -346,12 +354,23 @@ __device__ __forceinline__ void row_lines(const FftGeom &g, int64_t row0, int64_
     if (row < nrows) {
         const int N1 = g.N[1], N2 = g.N[2];
         const int64_t plane = (int64_t)N2 * N1;
+        int coil = 0;
+        if (IL) {
+            const int64_t r = row / g.CS;
+            coil = (int)(row - r * g.CS);
+            row = r;
+        }
         const int64_t bf = row / plane;
         const int rr = (int)(row - bf * plane);
         const int y = rr % N1, z = rr / N1;
         const int qy = wrapi(y + g.off[1], g.G[1]), qz = wrapi(z + g.off[2], g.G[2]);
         ln.img = bf * g.isize + (int64_t)rr * g.N[0];
         ln.grid = bf * g.gsize + ((int64_t)qz * g.G[1] + qy) * g.G[0];
+        if (IL) {
+            const int64_t chunk = bf / g.nframes, f = bf - chunk * g.nframes, b = chunk * g.CS + coil;
+            ln.img = b < g.batch ? (b * g.nframes + f) * g.isize + (int64_t)rr * g.N[0] : -1;
+            ln.grid = ln.grid * g.CS + coil;
+        }
         float s = g.scale;
         if (g.apod[1]) s *= g.apod[1][y];
         if (g.apod[2]) s *= g.apod[2][z];
@@ -368,7 +387,9 @@ __device__ __forceinline__ void row_lines(const FftGeom &g, int64_t row0, int64_
 //   as full grid rows;
 //   adjoint (CROP true): grid rows are inverse-transformed and the kept x,
 //   scaled and apodised, written to the image.
-template <class F, bool CROP>
+// With IL the lines are 16 neighbouring (row, coil) pairs and the grid is
+// interleaved, so its accesses run along the lines; the image's along x.
+template <class F, bool CROP, bool IL>
 __global__ void __launch_bounds__(F::T, F::MINB) fft_rows_kernel(FftGeom g, const float2 *__restrict__ tw,
                                                         const void *__restrict__ src, int src_real,
                                                         float2 *__restrict__ dst)
@@ -394,14 +415,39 @@ __global__ void __launch_bounds__(F::T, F::MINB) fft_rows_kernel(FftGeom g, cons
             apx[i] = ii < N0 ? (g.apod[0] ? g.apod[0][ii] : 1.0f) : 0.0f;
         }
     }
-    const int64_t nrows = g.nbf * g.N[2] * g.N[1];
+    const int64_t nrows = g.nbf * g.N[2] * g.N[1] * (IL ? g.CS : 1);
     const int64_t ntiles = (nrows + kFftLines - 1) / kFftLines;
     // loads of tile t into buffer `slot` (line data first, so a barrier)
     auto prefetch = [&](int64_t t, int slot) {
-        row_lines(g, t * kFftLines, nrows, lines[slot]);
+        row_lines<IL>(g, t * kFftLines, nrows, lines[slot]);
         __syncthreads();
         if (threadIdx.x < kFftLines) line_s[slot][threadIdx.x] = lines[slot][threadIdx.x].s;
         float2 *buf = bufs + slot * L * kFftLP;
+        if (IL && CROP) {
+            if ((g.CS & 1) == 0) {
+                // pairs of coils (16 bytes): a pair never straddles two rows
+                constexpr int P = kFftLines / 2;
+                const int c = 2 * (threadIdx.x % P);
+                const int64_t go = lines[slot][c].grid;
+                const float2 *sp = reinterpret_cast<const float2 *>(src) + (go >= 0 ? go : 0);
+                const int64_t st = go >= 0 ? g.CS : 0;
+                for (int q = threadIdx.x / P; q < L; q += T / P) {
+                    const unsigned d = (unsigned)__cvta_generic_to_shared(buf + q * kFftLP + c);
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(sp + q * st),
+                                 "r"(go >= 0 ? 16 : 0)
+                                 : "memory");
+                }
+            } else {
+                const int c = threadIdx.x & (kFftLines - 1);
+                const int64_t go = lines[slot][c].grid;
+                for (int q = threadIdx.x >> kFftShift; q < L; q += T / kFftLines)
+                    cp_async_fill(buf + q * kFftLP + c,
+                                  reinterpret_cast<const float2 *>(src) + (go >= 0 ? go + (int64_t)q * g.CS : 0), 8,
+                                  go >= 0);
+            }
+            cp_async_commit();
+            return;
+        }
         for (int e = threadIdx.x; e < kFftLines * L; e += T) {
             const int c = e / L, q = e - c * L;
             const RowLine ln = lines[slot][c];
@@ -444,6 +490,16 @@ __global__ void __launch_bounds__(F::T, F::MINB) fft_rows_kernel(FftGeom g, cons
         const int c = w & (kFftLines - 1), k1 = w >> kFftShift;
         float2 b[L2];
         if (k1 < L1) step_b<F>(buf, tws, CROP, c, k1, b);
+        if (IL && !CROP) {
+            // straight to the grid: the 16 lines are neighbours there
+            const int64_t go = lines[cur][c].grid;
+            if (k1 < L1 && go >= 0) {
+#pragma unroll
+                for (int k2 = 0; k2 < L2; k2++) dst[go + (int64_t)(k1 + L1 * k2) * g.CS] = b[k2];
+            }
+            __syncthreads();
+            continue;
+        }
         __syncthreads();
         if (k1 < L1) {
 #pragma unroll
@@ -737,15 +793,15 @@ int launch_cols_t(const FftGeom &g, const ColArgs &a, const float2 *tw, float2 *
     return launch_cols_tt<F, false, false>(g, a, tw, grid, st);
 }
 
-template <class F, bool CROP>
+template <class F, bool CROP, bool IL>
 int launch_rows_t(const FftGeom &g, const float2 *tw, const void *src, int src_real, float2 *dst, cudaStream_t st)
 {
     const size_t smem = smem_bytes(F::L);
-    const int64_t ntiles = (g.nbf * g.N[2] * g.N[1] + kFftLines - 1) / kFftLines;
+    const int64_t ntiles = (g.nbf * g.N[2] * g.N[1] * (IL ? g.CS : 1) + kFftLines - 1) / kFftLines;
     if (ntiles == 0) return DMR_OK;
     int blocks = 0;
-    DMR_TRY(blocks_for((const void *)fft_rows_kernel<F, CROP>, F::T, smem, ntiles, &blocks));
-    fft_rows_kernel<F, CROP><<<blocks, F::T, smem, st>>>(g, tw, src, src_real, dst);
+    DMR_TRY(blocks_for((const void *)fft_rows_kernel<F, CROP, IL>, F::T, smem, ntiles, &blocks));
+    fft_rows_kernel<F, CROP, IL><<<blocks, F::T, smem, st>>>(g, tw, src, src_real, dst);
     DMR_LAUNCHED(CROP ? "fft_crop_rows_kernel" : "fft_pad_rows_kernel");
     return DMR_OK;
 }
@@ -785,14 +841,15 @@ int launch_cols(int L, const FftGeom &g, const ColArgs &a, const float2 *tw, flo
     }
 }
 
+template <bool IL = false>
 int launch_rows(int L, bool crop, const FftGeom &g, const float2 *tw, const void *src, int src_real, float2 *dst,
                 cudaStream_t st)
 {
     switch (L) {
 #define DMR_FFT_CASE(L, L1, L2)                                                                     \
     case L:                                                                                         \
-        return crop ? launch_rows_t<Len<L, L1, L2>, true>(g, tw, src, src_real, dst, st)            \
-                    : launch_rows_t<Len<L, L1, L2>, false>(g, tw, src, src_real, dst, st);
+        return crop ? launch_rows_t<Len<L, L1, L2>, true, IL>(g, tw, src, src_real, dst, st)        \
+                    : launch_rows_t<Len<L, L1, L2>, false, IL>(g, tw, src, src_real, dst, st);
         DMR_FFT_LENGTHS(DMR_FFT_CASE)
 #undef DMR_FFT_CASE
     default: return DMR_ERR_UNSUPPORTED;
@@ -889,6 +946,51 @@ int fft3_adjoint(const dmr_plan *p, float2 *grid, int64_t batch, float2 *image, 
     if (g.G[2] > 1) DMR_TRY(launch_cols(g.G[2], g, z_pass(g, true), tw[2], grid, st));
     DMR_TRY(launch_cols(g.G[1], g, y_pass(g, true), tw[1], grid, st));
     return launch_rows(g.G[0], true, g, tw[0], grid, 0, image, st);
+}
+
+namespace {
+
+// geometry of the column passes on an interleaved grid: x and coil are one
+// contiguous axis
+FftGeom il_cols(const FftGeom &g)
+{
+    FftGeom c = g;
+    c.G[0] *= g.CS;
+    c.gsize *= g.CS;
+    return c;
+}
+
+FftGeom il_geom(const dmr_plan *p, int64_t batch, int64_t nchunks, int CS, float scale)
+{
+    FftGeom g = make_geom(p, nchunks, scale);  // nbf: (chunk, frame) sets
+    g.CS = CS;
+    g.nframes = p->g.nframes;
+    g.batch = batch;
+    return g;
+}
+
+}  // namespace
+
+int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nchunks, int CS,
+                    float2 *grid, cudaStream_t st)
+{
+    const FftGeom g = il_geom(p, batch, nchunks, CS, 1.0f), c = il_cols(g);
+    const float2 *tw[3] = {nullptr, nullptr, nullptr};
+    for (int a = 0; a < 3; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    DMR_TRY(launch_rows<true>(g.G[0], false, g, tw[0], image, image_real, grid, st));
+    DMR_TRY(launch_cols(g.G[1], c, y_pass(c, false), tw[1], grid, st));
+    return launch_cols(g.G[2], c, z_pass(c, false), tw[2], grid, st);
+}
+
+int fft3_adjoint_il(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nchunks, int CS, float2 *image,
+                    cudaStream_t st)
+{
+    const FftGeom g = il_geom(p, batch, nchunks, CS, (float)(1.0 / (double)p->g.gsize)), c = il_cols(g);
+    const float2 *tw[3] = {nullptr, nullptr, nullptr};
+    for (int a = 0; a < 3; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    DMR_TRY(launch_cols(g.G[2], c, z_pass(c, true), tw[2], grid, st));
+    DMR_TRY(launch_cols(g.G[1], c, y_pass(c, true), tw[1], grid, st));
+    return launch_rows<true>(g.G[0], true, g, tw[0], grid, 0, image, st);
 }
 
 bool toep3_applies(int ndim, const int32_t *kshape, const int32_t *ishape)

@@ -1,0 +1,48 @@
+// 3D interpolation and gridding on a coil-interleaved grid (march.cu): plan
+// structures and the calls of the pipelines.
+//
+// A batch of coils is cut into `n` chunks of `CS` coils (at most 32; the last
+// chunk may hold fewer, its grid keeps the stride CS). The grid of a chunk is
+// (frame, z, y, x, coil) in FFT order; rows are (sample in sorted order, coil)
+// with the coil stride rounded up to even.
+#pragma once
+
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+struct dmr_plan;
+
+namespace dmr {
+
+struct MarchChunks {
+    int64_t n;
+    int CS;
+};
+
+// sorts the samples and builds the work lists (no-op, mp_W stays 0, where the
+// kernels do not apply: not 3D, mixed widths or widths outside 2..6, or a grid
+// huge for its samples). keys / keys_s / vals: total int32 each, vals = 0..total-1
+int march_build(::dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
+                cudaStream_t st);
+
+MarchChunks march_chunks(const ::dmr_plan *p, int64_t batch);
+size_t march_rows_bytes(const ::dmr_plan *p, int CS);
+size_t march_il_bytes(const ::dmr_plan *p, int CS);
+
+// grid -> k-space, k-space -> grid for a batch. The grid is interleaved by
+// chunks, or planar (coil, frame, z, y, x) with `il` the interleaved grid of one
+// chunk; `rows`: the rows of one chunk. Deterministic gridding takes its
+// scratch (every unit's plane of a chunk) from the library pool;
+// DMR_ERR_UNSUPPORTED, before any launch, when that exceeds det_limit (> 0) or
+// the pool has no memory.
+int march_interp(const ::dmr_plan *p, const float2 *grid, bool planar, float2 *ksp, int64_t batch, const float *weight,
+                 int wpb, float2 *rows, float2 *il, cudaStream_t st);
+int march_grid(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool planar, int64_t batch,
+               const float *weight, int wpb, int det, int64_t det_limit, float2 *rows, float2 *il, cudaStream_t st);
+// the same on planar grids with rows and il from the library pool
+int march_interp_pool(const ::dmr_plan *p, const float2 *grid, float2 *ksp, int64_t batch, const float *weight,
+                      int wpb, cudaStream_t st);
+int march_grid_pool(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch, const float *weight,
+                    int wpb, int det, int64_t det_limit, cudaStream_t st);
+
+}  // namespace dmr

@@ -13,6 +13,7 @@
 #include <map>
 #include <tuple>
 
+#include "march.cuh"
 #include "plan.cuh"
 
 namespace dmr {
@@ -176,6 +177,9 @@ struct NufftWs {
     void *fft_work;
     void *rt_scratch;  // register-tile gridding partial sums (split regions)
     size_t rt_bytes;
+    float2 *rows;      // 3D march kernels: rows of one chunk of coils
+    float2 *il;        // and its interleaved grid, when the grid itself is planar (cuFFT)
+    MarchChunks march;
     std::shared_ptr<FftPlan> fft;
 };
 
@@ -191,10 +195,20 @@ static int nufft_ws(dmr_plan *p, int64_t batch, void *ws, size_t ws_bytes, Nufft
         fp = get_fft_plan(g.ndim, dims, batch * g.nframes, &err);
         if (!fp) return err;
     }
-    const size_t grid_bytes = align_up((size_t)batch * g.nframes * g.gsize * sizeof(float2), 256);
+    int64_t slots = batch;  // coil slots of the grid
+    size_t rows_bytes = 0, il_bytes = 0;
+    out.march = MarchChunks{0, 0};
+    if (p->mp_W) {
+        out.march = march_chunks(p, batch);
+        rows_bytes = march_rows_bytes(p, out.march.CS);
+        if (fp) il_bytes = march_il_bytes(p, out.march.CS);
+        else slots = out.march.n * out.march.CS;  // interleaved chunks, the last one padded
+    }
+    const size_t grid_bytes = align_up((size_t)slots * g.nframes * g.gsize * sizeof(float2), 256);
     const size_t fft_bytes = fp ? align_up(fp->work_bytes, 256) : 0;
     const size_t rt_bytes = align_up(grid_scratch_bytes(p, batch), 256);
-    const size_t total = grid_bytes + fft_bytes + rt_bytes;
+    // the register-tile scratch and the march buffers are never in use together
+    const size_t total = grid_bytes + fft_bytes + std::max(rt_bytes, rows_bytes + il_bytes);
     if (need) *need = total;
     if (!ws) return DMR_OK;
     DMR_CHECK(ws_bytes >= total, DMR_ERR_WORKSPACE, "workspace too small: %zu < %zu", ws_bytes, total);
@@ -203,6 +217,8 @@ static int nufft_ws(dmr_plan *p, int64_t batch, void *ws, size_t ws_bytes, Nufft
     out.fft_work = fp && fp->work_bytes ? (char *)ws + grid_bytes : nullptr;
     out.rt_scratch = rt_bytes ? (char *)ws + grid_bytes + fft_bytes : nullptr;
     out.rt_bytes = rt_bytes;
+    out.rows = (float2 *)((char *)ws + grid_bytes + fft_bytes);
+    out.il = (float2 *)((char *)ws + grid_bytes + fft_bytes + rows_bytes);
     out.fft = fp;
     return DMR_OK;
 }
@@ -371,6 +387,14 @@ extern "C" int dmr_nufft_forward(dmr_plan *p, const void *image, int image_real,
     DMR_CHECK(p && image && kspace && batch >= 1, DMR_ERR_INVALID, "bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     float2 *grid = nullptr;
+    if (p->mp_W) {
+        NufftWs w;
+        DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
+        if (w.fft) DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));
+        else DMR_TRY(fft3_forward_il(p, image, image_real, batch, w.march.n, w.march.CS, w.grid, st));
+        return march_interp(p, w.grid, w.fft != nullptr, (float2 *)kspace, batch, weight, weight_per_batch, w.rows,
+                            w.il, st);
+    }
     DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));
     return interp_dispatch(p, grid, (float2 *)kspace, batch, weight, weight_per_batch, st);
 }
@@ -385,8 +409,17 @@ extern "C" int dmr_nufft_adjoint(dmr_plan *p, const void *kspace, int kspace_rea
     const Geom &g = p->g;
     NufftWs w;
     DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
-    DMR_TRY(grid_dispatch(p, kspace, kspace_real, w.grid, batch, weight, weight_per_batch,
-                          deterministic, w.rt_scratch, w.rt_bytes, st));
+    int rc = DMR_ERR_UNSUPPORTED;
+    if (grid_march_applies(p, batch, deterministic)) {
+        rc = march_grid(p, kspace, kspace_real, w.grid, w.fft != nullptr, batch, weight, weight_per_batch,
+                        deterministic, det_scratch_limit(), w.rows, w.il, st);
+        if (rc == DMR_OK && !w.fft)
+            return fft3_adjoint_il(p, w.grid, batch, w.march.n, w.march.CS, (float2 *)image, st);
+    }
+    if (rc == DMR_ERR_UNSUPPORTED)
+        rc = grid_dispatch(p, kspace, kspace_real, w.grid, batch, weight, weight_per_batch, deterministic,
+                           w.rt_scratch, w.rt_bytes, st);
+    DMR_TRY(rc);
     if (!w.fft) return fft3_adjoint(p, w.grid, batch, (float2 *)image, st);
     DMR_TRY(fft_exec(*w.fft, w.grid, CUFFT_INVERSE, w.fft_work, st));
     ResizeArgs r;

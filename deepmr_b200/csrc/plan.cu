@@ -9,6 +9,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -16,6 +17,7 @@
 #include <string>
 
 #include "kb.cuh"
+#include "march.cuh"
 #include "plan.cuh"
 
 namespace dmr {
@@ -466,8 +468,13 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     for (int64_t i = 0; i < nkeys; i++) h_start[i + 1] = h_start[i] + h_counts[i];
 
     // bins of the 3D tensor-core gridding: region (T + W - 1) of 7 x 6 x 6
-    // points (x, y, z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..5
-    if (ndim == 3 && total > 0 && g.W[0] == g.W[1] && g.W[1] == g.W[2] && g.W[0] >= 2 && g.W[0] <= 5) {
+    // points (x, y, z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..4 (at width
+    // 5 with 32 coils the kernel's bounded waits ran out)
+    // (only where dmr_tc_min_coils was set: 1.3 GB and a second sort for the
+    // 192^3 kooshball)
+    if (total > 0) DMR_TRY(march_build(p.get(), rk, keys, keys_s, vals, st));
+    if (tc_min_coils() < INT_MAX && ndim == 3 && total > 0 && g.W[0] == g.W[1] && g.W[1] == g.W[2] &&
+        g.W[0] >= 2 && g.W[0] <= 4) {
         const int W = g.W[0];
         int tT[3] = {8 - W, 7 - W, 7 - W}, tnb[3];
         for (int a = 0; a < 3; a++) {

@@ -90,6 +90,12 @@ bool fft3_applies(const ::dmr_plan *p);
 int fft3_forward(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, float2 *grid,
                  cudaStream_t st);
 int fft3_adjoint(const ::dmr_plan *p, float2 *grid, int64_t batch, float2 *image, cudaStream_t st);
+// the same with the coil-interleaved grid of march.cuh: nchunks chunks of CS
+// coils, (chunk, frame, z, y, x, coil)
+int fft3_forward_il(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nchunks, int CS,
+                    float2 *grid, cudaStream_t st);
+int fft3_adjoint_il(const ::dmr_plan *p, float2 *grid, int64_t batch, int64_t nchunks, int CS, float2 *image,
+                    cudaStream_t st);
 // the same passes for the 3D Toeplitz self-adjoint: whether they apply
 // (kernel extents at least the image's and with a compiled transform), and
 // pad + FFT + kernel multiply + inverse FFT + crop (data: batch kernel grids)
@@ -101,6 +107,13 @@ int fft3_toeplitz(int ndim, const int32_t *kshape_zyx, const int32_t *ishape_zyx
 int grid_tc_dispatch(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
                      const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes,
                      cudaStream_t st);
+// smallest batch of atomic tensor-core gridding (dmr_tc_min_coils), DMR_NO_TC,
+// and the deterministic scratch limit (dmr_det_scratch_limit)
+int tc_min_coils();
+bool tc_disabled();
+int64_t det_scratch_limit();
+// whether gridding of `batch` coils runs on the plane kernel (march.cuh)
+bool grid_march_applies(const ::dmr_plan *p, int64_t batch, int det);
 // tensor-core gridding with the plan's gridding bins (tmgrid.cu), atomic or
 // deterministic (partial sums per work item, then a gather per grid point;
 // scratch from the caller when it holds tm_scratch_bytes, else from the
@@ -166,6 +179,23 @@ struct dmr_plan {
     dmr::RtItem *rt_reduce = nullptr;
     int nrt_reduce = 0;
     int rt_slots = 0;
+    // 3D march order (march.cu; mp_W == 0: not planned): tiles along x and y,
+    // CSR offsets per cell, sorted position -> sample and back, per sorted
+    // sample the tap weights and z cell, gridding units for 1, 2, 4 and 8
+    // planes per warp (int4), the first unit of each (frame tile, plane), and
+    // interpolation items (int4)
+    int mp_W = 0;
+    int mp_nt[2] = {0, 0};
+    int32_t *mp_cstart = nullptr;
+    int32_t *mp_sidx = nullptr;
+    int32_t *mp_inv = nullptr;
+    int32_t *mp_zc = nullptr;
+    float *mp_rec = nullptr;
+    void *mp_units[4] = {nullptr, nullptr, nullptr, nullptr};
+    int mp_nunits[4] = {0, 0, 0, 0};
+    int32_t *mp_ustart = nullptr;
+    void *mp_items = nullptr;
+    int mp_nitems = 0;
     // device status word: blocks of this plan's calls whose bounded wait ran out
     // (dmr_plan_status; 0 while every result is valid)
     int32_t *status = nullptr;
@@ -193,5 +223,13 @@ struct dmr_plan {
         cudaFree(rt_items);
         cudaFree(rt_reduce);
         cudaFree(status);
+        cudaFree(mp_cstart);
+        cudaFree(mp_sidx);
+        cudaFree(mp_inv);
+        cudaFree(mp_zc);
+        cudaFree(mp_rec);
+        for (void *u : mp_units) cudaFree(u);
+        cudaFree(mp_ustart);
+        cudaFree(mp_items);
     }
 };

@@ -15,9 +15,11 @@
 // centred index c of an axis is stored at (c - G//2) mod G — so the fftshift
 // of the reference's centred FFT (src/deepmr/fft/fft.py:77-80) costs nothing.
 #include <algorithm>
+#include <climits>
 #include <cstdlib>
 
 #include "kb.cuh"
+#include "march.cuh"
 #include "plan.cuh"
 
 namespace dmr {
@@ -1364,6 +1366,10 @@ int interp_dispatch(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_t 
                     const float *weight, int wpb, cudaStream_t st)
 {
     if (p->nwork == 0) return DMR_OK;
+    if (p->mp_W) {
+        const int rc = march_interp_pool(p, grid, ksp, batch, weight, wpb, st);
+        if (rc != DMR_ERR_UNSUPPORTED) return rc;
+    }
     const int cw = cube_width(p->g);
     if (cw > 0) {
         switch (p->g.ndim * 100 + cw) {
@@ -1401,22 +1407,30 @@ size_t grid_scratch_bytes(const dmr_plan *p, int64_t batch)
     return rt_scratch_bytes(p, batch);
 }
 
-// minimum coil count of atomic tensor-core gridding (dmr_tc_min_coils)
-static std::atomic<int> g_tc_min_coils{20};
+// minimum coil count of atomic tensor-core gridding (dmr_tc_min_coils); the
+// plane kernel of march.cu is faster at every batch, so by default none
+static std::atomic<int> g_tc_min_coils{INT_MAX};
+
+int tc_min_coils() { return g_tc_min_coils.load(); }
+
+bool grid_march_applies(const dmr_plan *p, int64_t batch, int det)
+{
+    if (p->mp_W == 0 || grid_variant() != 0) return false;
+    if (det) return !tc_disabled();
+    return p->tg_T[0] == 0 || batch < tc_min_coils();
+}
 
 int grid_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
                   const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes,
                   cudaStream_t st)
 {
-    // 3D gridding on the tensor cores: atomic, or deterministic (per-item
-    // partial sums gathered per grid point in a fixed order, bitwise
-    // reproducible), when the plan's gridding bins apply.
-    // Its cost is mostly per sample (the spreading operand and the region
-    // read-back are built for all 32 coil slots), so atomic gridding of fewer
-    // coils runs on the CUDA cores, whose cost scales with the coil count
-    // (192^3 kooshball: 12.1 vs 13.6 ms for 16 coils, 6.0 vs 13.0 for 8,
-    // 24.1 vs 16.8 for 32).
-    if (p->g.ndim == 3 && grid_variant() == 0 && (det || batch >= g_tc_min_coils.load())) {
+    if (grid_march_applies(p, batch, det)) {
+        const int rc = march_grid_pool(p, ksp, kreal, grid, batch, weight, wpb, det, det_scratch_limit(), st);
+        if (rc != DMR_ERR_UNSUPPORTED) return rc;
+    }
+    // atomic 3D gridding on the tensor cores where dmr_tc_min_coils asks for it
+    // (plans made under that setting have its gridding bins)
+    if (p->g.ndim == 3 && grid_variant() == 0 && !det && batch >= tc_min_coils()) {
         const int rc = grid_tc_dispatch(p, ksp, kreal, grid, batch, weight, wpb, det, scratch, scratch_bytes, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }

@@ -23,11 +23,11 @@ namespace dmr {
 
 __device__ int g_tc_timeouts = 0;  // blocks whose wait ran out, all plans (should stay 0)
 
-static int tc_disabled()
+bool tc_disabled()
 {
-    static const int v = [] {
+    static const bool v = [] {
         const char *e = getenv("DMR_NO_TC");
-        return e && atoi(e) ? 1 : 0;
+        return e && atoi(e);
     }();
     return v;
 }
@@ -36,6 +36,8 @@ static std::atomic<int> g_tc_stall{0};  // test hook (dmr_tc_test_stall)
 // largest scratch (bytes) deterministic tensor-core gridding may take, 0: no
 // limit (dmr_det_scratch_limit)
 static std::atomic<int64_t> g_det_scratch_max{0};
+
+int64_t det_scratch_limit() { return g_det_scratch_max.load(); }
 
 // device address of g_tc_timeouts, looked up once per device (that device current)
 static int timeouts_ptr(int dev, int **out)

@@ -66,12 +66,11 @@ __all__ = [
 def set_deterministic_gridding(flag=True):
     """Select the gridding kernel used by the adjoint NUFFT.
 
-    True: bitwise reproducible — 3D plans grid on the tensor cores with
-    every work item (a bin, or 2048 samples of a heavier one) storing its
-    region's partial sums, which a gather then adds per grid point in a fixed
-    order (the partial sums take 2 KB per work item and coil in the library's
-    scratch pool: see release_scratch); other plans with one owner per grid
-    point or per tile.
+    True: bitwise reproducible — 3D plans store the plane of every gridding
+    unit (a tile's plane, or 512 samples of a heavier one), and a gather then
+    adds the planes per grid point in a fixed order (they take 392 bytes per
+    unit and coil at width 4 in the library's scratch pool: see
+    release_scratch); other plans with one owner per grid point or per tile.
     False (default): grid-point additions with atomics (summation order may
     vary between runs, results agree to float32 rounding).
     Returns the previous setting.
@@ -98,8 +97,8 @@ def release_scratch(device=None):
 
 
 def set_deterministic_scratch_limit(nbytes):
-    """Largest scratch (bytes) that deterministic 3D tensor-core gridding may
-    take (2 KB per gridding work item and coil); a call that would need more,
+    """Largest scratch (bytes) that deterministic 3D plane gridding may take
+    (392 bytes per gridding unit and coil at width 4); a call that would need more,
     or for which the device has no memory left, runs on the register-tile
     kernel instead (deterministic, slower, small scratch). 0 removes the
     limit (the default). Process-wide; returns the previous limit."""

@@ -384,8 +384,8 @@ def _as_cfloat(x):
     return x.to(torch.complex64)
 
 
-# Gridding kernel of the adjoint: False (default) = shared-memory tiles flushed
-# with global atomics; True = fixed-order owner tiles (bitwise reproducible).
+# Gridding kernel of the adjoint: False (default) = tiles flushed with global
+# atomics; True = fixed-order sums (bitwise reproducible).
 DETERMINISTIC_GRIDDING = False
 
 # Device status of the gridding (a bounded wait that ran out, DMR_ERR_TIMEOUT)
@@ -445,10 +445,9 @@ def _weight_arg(weight, batch_shape, interp, frames_shape, dev):
 # separate copy engines), instead of copy in -> compute -> copy out in series.
 PIPELINE_MIN_BYTES = 64 << 20
 PIPELINE_CHUNKS = 16
-# batch items per chunk of a host-pipelined 3D adjoint, at least: atomic
-# gridding of a few coils runs on the CUDA cores at a cost proportional to the
-# coils; the deterministic tensor-core gridding costs about the same for 8
-# coils as for 32
+# batch items per chunk of a host-pipelined 3D adjoint, at least: small chunks
+# overlap best with the copies, which bound the call; the deterministic mode's
+# cost per chunk is mostly per sample, so its chunks are larger
 ADJOINT_MIN_CHUNK_3D = 2
 ADJOINT_MIN_CHUNK_3D_DET = 8
 

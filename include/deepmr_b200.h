@@ -97,11 +97,13 @@ int dmr_tc_test_stall(int enable);
 int dmr_fft3_fused(dmr_plan *plan);
 
 /*
- * Tuning knob, no reference counterpart: atomic gridding of a 3D plan runs on
- * the tensor cores for batches of at least `coils` coils (default 20; below,
- * the CUDA-core kernel, whose cost scales with the coil count, is faster) and
- * on the CUDA cores otherwise. coils <= 0 only queries. Returns the previous
- * value. Process-wide; deterministic gridding is not affected.
+ * Tuning knob, no reference counterpart: atomic gridding of 3D plans of widths
+ * 2..4 that are made while it is set runs on the tensor cores for batches of
+ * at least `coils` coils and on the CUDA cores otherwise. By default
+ * (INT32_MAX) none does: the CUDA-core plane kernel is faster at every batch
+ * (192^3 kooshball, 32 coils: 8.1 ms with its row transposition, tensor cores
+ * 16.2 ms) and closer to the exact sums. coils <= 0 only queries. Returns the
+ * previous value. Process-wide; deterministic gridding is not affected.
  */
 int dmr_tc_min_coils(int coils);
 
@@ -109,17 +111,17 @@ int dmr_tc_min_coils(int coils);
  * Housekeeping, no reference counterpart: gives back to `device` the memory
  * that the library's scratch pool holds beyond what is in use. Calls without
  * a large enough workspace take their gridding scratch from this pool, which
- * keeps it for the next call; deterministic 3D gridding keeps every work
- * item's partial sums there (2 KB per gridding work item and coil: 13.6 GB
- * for 32 coils of the 192^3, 19.2 M-sample kooshball). Synchronises the
- * device first. Returns 0 or a DMR_ERR_* code.
+ * keeps it for the next call; deterministic 3D gridding keeps every gridding
+ * unit's plane there (392 bytes per unit and coil at width 4: 10.9 GB for 32
+ * coils of the 192^3, 19.2 M-sample kooshball), and dmr_interp / dmr_grid of
+ * 3D plans a chunk's rows and interleaved grid. Synchronises the device first. Returns 0 or a DMR_ERR_* code.
  */
 int dmr_scratch_release(int device);
 
 /*
  * Memory control, no reference counterpart: the largest scratch, in bytes,
- * that deterministic 3D tensor-core gridding may take (its per-item partial
- * sums, 2 KB per gridding work item and coil). A call that would need more,
+ * that deterministic 3D plane gridding may take for the planes of its units
+ * (392 bytes per unit and coil at width 4). A call that would need more,
  * or for which the pool has no memory, runs on the register-tile kernel (or
  * the colour passes) instead: deterministic as well, slower, with a small
  * scratch. bytes > 0 sets the limit, 0 removes it (the default), < 0 only
@@ -198,12 +200,11 @@ int dmr_interp(const dmr_plan *plan, const void *grid, void *kspace,
  *  deterministic: 0 = shared-memory tiles flushed with global atomics
  *     (summation order may vary between runs);
  *     1 = every grid point is summed by one owner in a fixed order (bitwise
- *     reproducible, no float atomics): 3D grids of 8 or more coils keep
- *     8^3-point block regions in registers (regions too dense for one block
- *     are split into partial sums added in a fixed order; without a caller
- *     workspace this call takes their scratch from a library-owned
- *     stream-ordered memory pool); other grids run the bins in colour passes
- *     of disjoint tiles.
+ *     reproducible, no float atomics): 3D grids store every unit's plane in
+ *     scratch and add the planes per grid point in a fixed order (scratch from
+ *     a library-owned stream-ordered memory pool); where that does not apply,
+ *     3D grids of 8 or more coils keep 8^3-point block regions in registers,
+ *     and other grids run the bins in colour passes of disjoint tiles.
  */
 int dmr_grid(const dmr_plan *plan, const void *kspace, int kspace_real,
              void *grid, int64_t batch, const float *weight,
