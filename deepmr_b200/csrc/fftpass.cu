@@ -974,21 +974,24 @@ FftGeom il_geom(const dmr_plan *p, int64_t batch, int64_t nchunks, int CS, float
 int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nchunks, int CS,
                     float2 *grid, cudaStream_t st)
 {
+    if (CS == 1) return fft3_forward(p, image, image_real, batch, grid, st);  // the same layout
     const FftGeom g = il_geom(p, batch, nchunks, CS, 1.0f), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < 3; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
     DMR_TRY(launch_rows<true>(g.G[0], false, g, tw[0], image, image_real, grid, st));
     DMR_TRY(launch_cols(g.G[1], c, y_pass(c, false), tw[1], grid, st));
+    if (g.G[2] == 1) return DMR_OK;  // 2D
     return launch_cols(g.G[2], c, z_pass(c, false), tw[2], grid, st);
 }
 
 int fft3_adjoint_il(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nchunks, int CS, float2 *image,
                     cudaStream_t st)
 {
+    if (CS == 1) return fft3_adjoint(p, grid, batch, image, st);
     const FftGeom g = il_geom(p, batch, nchunks, CS, (float)(1.0 / (double)p->g.gsize)), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < 3; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
-    DMR_TRY(launch_cols(g.G[2], c, z_pass(c, true), tw[2], grid, st));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    if (g.G[2] > 1) DMR_TRY(launch_cols(g.G[2], c, z_pass(c, true), tw[2], grid, st));
     DMR_TRY(launch_cols(g.G[1], c, y_pass(c, true), tw[1], grid, st));
     return launch_rows<true>(g.G[0], true, g, tw[0], grid, 0, image, st);
 }

@@ -40,11 +40,12 @@ namespace {
 // tile extent by kernel width: the tile plus its halo is at most 8 x 8 points,
 // which a lane of the gridding kernel holds in registers
 __host__ __device__ constexpr int march_tile(int W) { return W <= 4 ? 4 : 3; }
-__host__ __device__ constexpr int march_rec(int W) { return (3 * W + 3) / 4 * 4; }
+__host__ __device__ constexpr int march_rec(int W, int ndim = 3) { return (ndim * W + 3) / 4 * 4; }
 
 // visits of a gridding unit / samples of an interpolation item, at most: heavier
 // ones (the centre of k-space) are split so that no warp runs far behind
 constexpr int kUnitVisits = 512;
+constexpr int kUnitVisits2 = 128;  // 2D: few tiles, and no z axis to spread a dense one over
 constexpr int kItemSamples = 144;
 constexpr int kItemZ = 8;  // z cells of an interpolation item
 // rows of cell columns of an interpolation item (a tile has T / march_rows items per z block)
@@ -104,7 +105,7 @@ __global__ void march_key_kernel(Geom g, int T, int nt0, int nt1, const int64_t 
         }
         const int x = pmod(first_tap_dev(rk0[i], g.W[0]), g.G[0]);
         const int y = pmod(first_tap_dev(rk1[i], g.W[1]), g.G[1]);
-        const int z = pmod(first_tap_dev(rk2[i], g.W[2]), g.G[2]);
+        const int z = g.ndim == 3 ? pmod(first_tap_dev(rk2[i], g.W[2]), g.G[2]) : 0;
         const int tx = x / T, ty = y / T;
         const int col = ((lo * nt1 + ty) * nt0 + tx) * (T * T) + (y - ty * T) * T + (x - tx * T);
         const int key = col * g.G[2] + z;
@@ -118,14 +119,14 @@ __global__ void march_rec_kernel(Geom g, const int32_t *__restrict__ sidx, const
                                  const float *__restrict__ rk1, const float *__restrict__ rk2,
                                  float *__restrict__ rec, int32_t *__restrict__ zc, int32_t *__restrict__ inv)
 {
-    const int W = g.W[0], R = march_rec(W);
+    const int W = g.W[0], R = march_rec(W, g.ndim);
     for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < g.total;
          j += (int64_t)gridDim.x * blockDim.x) {
         const int32_t i = sidx[j];
         inv[i] = (int32_t)j;
-        const float k[3] = {rk0[i], rk1[i], rk2[i]};
+        const float k[3] = {rk0[i], rk1[i], g.ndim == 3 ? rk2[i] : 0.0f};
         float *r = rec + j * R;
-        for (int a = 0; a < 3; a++) {
+        for (int a = 0; a < g.ndim; a++) {
             const int x0 = first_tap_dev(k[a], W);
             for (int t = 0; t < W; t++) {
                 const float w = tap_weight(x0, t, k[a], W, g.inv_hw[a], g.beta[a]);
@@ -147,7 +148,7 @@ __device__ __forceinline__ void plane_cells(int z0, int z1, int W, int G, int &a
 
 // gridding units of np planes: number of pieces of each (frame tile, plane group)
 __global__ void march_unit_count_kernel(const int32_t *__restrict__ cstart, int64_t nft, int TT, int G2, int W, int np,
-                                        int nzu, int32_t *__restrict__ counts)
+                                        int nzu, int most, int32_t *__restrict__ counts)
 {
     const int64_t n = nft * nzu;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -165,19 +166,20 @@ __global__ void march_unit_count_kernel(const int32_t *__restrict__ cstart, int6
             const int32_t *cs = cstart + (ft * TT + c) * G2;
             visits += cs[b] - cs[a] + (cs[G2] - cs[wa]);
         }
-        counts[i] = (visits + kUnitVisits - 1) / kUnitVisits;
+        counts[i] = (visits + most - 1) / most;
     }
 }
 
 // (frame tile, plane group, first visit, end visit) of every unit
-__global__ void march_unit_fill_kernel(const int32_t *__restrict__ start, int64_t nft, int nzu, int4 *__restrict__ units)
+__global__ void march_unit_fill_kernel(const int32_t *__restrict__ start, int64_t nft, int nzu, int most,
+                                       int4 *__restrict__ units)
 {
     const int64_t n = nft * nzu;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int s = start[i], e = start[i + 1];
         const int ft = (int)(i / nzu), zu = (int)(i - (int64_t)ft * nzu);
         for (int u = s; u < e; u++)
-            units[u] = make_int4(ft, zu, (u - s) * kUnitVisits, u + 1 == e ? 0x7fffffff : (u - s + 1) * kUnitVisits);
+            units[u] = make_int4(ft, zu, (u - s) * most, u + 1 == e ? 0x7fffffff : (u - s + 1) * most);
     }
 }
 
@@ -358,9 +360,9 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float2 *__restrict
 constexpr int kGridWarps = 4;
 constexpr int kVisitBatch = 16;
 
-template <int W, int NP>
+template <int W, int NP, int ND>
 struct PlaneShape {
-    static constexpr int T = march_tile(W), R = T + W - 1, REC = march_rec(W);
+    static constexpr int T = march_tile(W), R = T + W - 1, REC = march_rec(W, ND);
     static constexpr int CC = 32 / NP;     // coil lanes
     static constexpr int ROWB = CC * 8;    // bytes of a staged row
     static constexpr int RECS = kVisitBatch * ROWB, ZCS = RECS + kVisitBatch * REC * 4;
@@ -368,13 +370,13 @@ struct PlaneShape {
     static constexpr int SMEM = kGridWarps * 2 * BUF;
 };
 
-template <int W, int NP>
+template <int W, int NP, int ND>
 __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
     grid_planes_kernel(MarchGeom g, const int4 *__restrict__ units, int nunits, const int32_t *__restrict__ cstart,
                        const float *__restrict__ rec, const int32_t *__restrict__ zc, const float2 *__restrict__ rows,
                        float2 *__restrict__ grid, float2 *__restrict__ scratch)
 {
-    using S = PlaneShape<W, NP>;
+    using S = PlaneShape<W, NP, ND>;
     constexpr int T = S::T, R = S::R, REC = S::REC, CC = S::CC, TT = T * T;
     extern __shared__ __align__(16) unsigned char msm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -391,7 +393,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
         const int col = lane & 15, wrapped = lane >> 4;
         if (col < TT) {
             int a, b, wa;
-            plane_cells(z0, z1, W, g.G[2], a, b, wa);
+            plane_cells(z0, z1, ND == 3 ? W : 1, g.G[2], a, b, wa);
             const int32_t *cs = cstart + ((int64_t)ft * TT + col) * g.G[2];
             beg = cs[wrapped ? wa : a];
             cnt = cs[wrapped ? g.G[2] : b] - beg;
@@ -440,7 +442,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
             const int jr = __shfl_sync(0xffffffffu, j, r & (kVisitBatch - 1));
             if (r < kVisitBatch) cp16(dst + S::RECS + p * 16, rec + (int64_t)jr * REC + 4 * piece);
         }
-        if (lane < kVisitBatch) cp4(dst + S::ZCS + lane * 4, zc + j);
+        if (ND == 3 && lane < kVisitBatch) cp4(dst + S::ZCS + lane * 4, zc + j);
     };
 
     float2 acc[R][R];
@@ -458,10 +460,13 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
 #pragma unroll
         for (int q = 0; q < (2 * W + 3) / 4; q++)
             *reinterpret_cast<float4 *>(w + 4 * q) = *reinterpret_cast<const float4 *>(wp + 4 * q);
-        const int iz = zoff - *reinterpret_cast<const int *>(msm + buf + S::ZCS + i * 4);  // this lane's plane is tap iz
-        float2 t = make_float2(0.0f, 0.0f);
-        // (a select, not a zero weight: values that are not finite stay in their W planes)
-        if (NP == 1 || (unsigned)iz < (unsigned)W) t = __fmul2_rn(dup(wp[2 * W + iz]), v);
+        float2 t = v;
+        if constexpr (ND == 3) {
+            const int iz = zoff - *reinterpret_cast<const int *>(msm + buf + S::ZCS + i * 4);  // this lane's plane is tap iz
+            t = make_float2(0.0f, 0.0f);
+            // (a select, not a zero weight: values that are not finite stay in their W planes)
+            if (NP == 1 || (unsigned)iz < (unsigned)W) t = __fmul2_rn(dup(wp[2 * W + iz]), v);
+        }
 #pragma unroll
         for (int jy = 0; jy < W; jy++) {
             const float2 ty = __fmul2_rn(dup(w[W + jy]), t);
@@ -921,15 +926,15 @@ MarchGeom march_geom(const dmr_plan *p, int CS)
     return m;
 }
 
-template <int W, int NP>
+template <int W, int NP, int ND>
 int launch_planes_np(const dmr_plan *p, const MarchGeom &m, const float2 *rows, float2 *grid, float2 *scratch,
                      cudaStream_t st)
 {
-    using S = PlaneShape<W, NP>;
+    using S = PlaneShape<W, NP, ND>;
     constexpr int L = NP == 1 ? 0 : (NP == 2 ? 1 : (NP == 4 ? 2 : 3));
     const int n = p->mp_nunits[L];
     if (n == 0) return DMR_OK;
-    auto kern = grid_planes_kernel<W, NP>;
+    auto kern = grid_planes_kernel<W, NP, ND>;
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
     kern<<<(unsigned)ceil_div(n, kGridWarps), 32 * kGridWarps, S::SMEM, st>>>(m, (const int4 *)p->mp_units[L], n,
                                                                              p->mp_cstart, p->mp_rec, p->mp_zc, rows,
@@ -947,10 +952,11 @@ int launch_planes(const dmr_plan *p, const MarchGeom &m, const float2 *rows, flo
 {
     // deterministic units are always single planes, so that a coil's sums do
     // not depend on how many coils it is gridded with
-    if (scratch || m.CS > 16) return launch_planes_np<W, 1>(p, m, rows, grid, scratch, st);
-    if (m.CS > 8) return launch_planes_np<W, 2>(p, m, rows, grid, scratch, st);
-    if (m.CS > 4) return launch_planes_np<W, 4>(p, m, rows, grid, scratch, st);
-    return launch_planes_np<W, 8>(p, m, rows, grid, scratch, st);
+    if (p->g.ndim == 2) return launch_planes_np<W, 1, 2>(p, m, rows, grid, scratch, st);
+    if (scratch || m.CS > 16) return launch_planes_np<W, 1, 3>(p, m, rows, grid, scratch, st);
+    if (m.CS > 8) return launch_planes_np<W, 2, 3>(p, m, rows, grid, scratch, st);
+    if (m.CS > 4) return launch_planes_np<W, 4, 3>(p, m, rows, grid, scratch, st);
+    return launch_planes_np<W, 8, 3>(p, m, rows, grid, scratch, st);
 }
 
 template <int W>
@@ -1009,13 +1015,18 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
 {
     const Geom &g = p->g;
     const int W = g.W[0];
-    if (g.ndim != 3 || g.total == 0 || W < 2 || W > 6 || g.W[1] != W || g.W[2] != W) return DMR_OK;
+    if (g.ndim < 2 || g.total == 0 || W < 2 || W > 6 || g.W[1] != W || (g.ndim == 3 && g.W[2] != W)) return DMR_OK;
     const int T = march_tile(W), TT = T * T;
     const int nt0 = (int)ceil_div(g.G[0], T), nt1 = (int)ceil_div(g.G[1], T);
     const int64_t nft = (int64_t)g.nframes * nt0 * nt1, ncells = nft * TT * g.G[2];
     // the CSR offsets take 4 bytes per cell: not for grids that are huge for
     // their samples (their plans keep the bin kernels)
     if (ncells >= INT32_MAX || ncells > 16 * g.total + (1 << 24)) return DMR_OK;
+    // 2D tiles pay from a few samples per tile on (below, a tile's flush costs
+    // more than its samples' own additions: direct2d.cu)
+    if (g.ndim == 2 && g.total < 4 * nft) return DMR_OK;
+    const bool d3 = g.ndim == 3;
+    const int most = d3 ? kUnitVisits : kUnitVisits2, nl = d3 ? 5 : 1;  // lists: units of 1, 2, 4, 8 planes, items
     struct Temp {
         void *ptr[3] = {};
         ~Temp()
@@ -1050,7 +1061,7 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     g_launches.fetch_add(2);
     DMR_TRY(march_alloc(&p->mp_inv, g.total));
     DMR_TRY(march_alloc(&p->mp_zc, g.total));
-    DMR_TRY(march_alloc(&p->mp_rec, (size_t)g.total * march_rec(W)));
+    DMR_TRY(march_alloc(&p->mp_rec, (size_t)g.total * march_rec(W, g.ndim)));
     march_rec_kernel<<<march_blocks(g.total), 256, 0, st>>>(g, p->mp_sidx, rk[0], rk[1], rk[2], p->mp_rec, p->mp_zc,
                                                            p->mp_inv);
     DMR_LAUNCHED("march_rec_kernel");
@@ -1062,11 +1073,11 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     off[5] = off[4] + nft * nzbh + 1;
     DMR_TRY(march_alloc(&starts, off[5]));
     tmp.ptr[2] = starts;
-    for (int l = 0; l < 5; l++) {
+    for (int l = 0; l < nl; l++) {
         const int64_t n = off[l + 1] - off[l];
         if (l < 4)
-            march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], W, np[l], nzu[l],
-                                                                    counts);
+            march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], d3 ? W : 1, np[l],
+                                                                    nzu[l], most, counts);
         else
             march_item_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, cols, g.G[2], nzb,
                                                                     counts);
@@ -1074,17 +1085,17 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
         DMR_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb, counts, starts + off[l], (int)n, st));
         g_launches.fetch_add(1);
     }
-    int32_t total[5];
-    for (int l = 0; l < 5; l++)
+    int32_t total[5] = {0};
+    for (int l = 0; l < nl; l++)
         DMR_CUDA(cudaMemcpyAsync(&total[l], starts + off[l + 1] - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    for (int l = 0; l < 5; l++) {
+    for (int l = 0; l < nl; l++) {
         int4 *list = nullptr;
         DMR_TRY(march_alloc(&list, total[l]));
         if (l < 4) {
             p->mp_units[l] = list;
             p->mp_nunits[l] = total[l];
-            march_unit_fill_kernel<<<march_blocks(nft * nzu[l]), 256, 0, st>>>(starts + off[l], nft, nzu[l], list);
+            march_unit_fill_kernel<<<march_blocks(nft * nzu[l]), 256, 0, st>>>(starts + off[l], nft, nzu[l], most, list);
         } else {
             p->mp_items = list;
             p->mp_nitems = total[l];
@@ -1106,7 +1117,7 @@ MarchChunks march_chunks(const dmr_plan *p, int64_t batch)
 {
     // up to 32 coils at a time, fewer when the rows would take over 8 GB
     int64_t most = 32;
-    while (most > 4 && p->g.total * most * (int64_t)sizeof(float2) > (8ll << 30)) most /= 2;
+    if (p->mp_W) while (most > 4 && p->g.total * most * (int64_t)sizeof(float2) > (8ll << 30)) most /= 2;
     MarchChunks c;
     c.n = ceil_div(batch, most);
     c.CS = (int)ceil_div(batch, c.n);
@@ -1115,6 +1126,7 @@ MarchChunks march_chunks(const dmr_plan *p, int64_t batch)
 
 size_t march_rows_bytes(const dmr_plan *p, int CS)
 {
+    if (!p->mp_W) return 0;  // 2D without tiles: no rows
     return align_up((size_t)p->g.total * ((CS + 1) & ~1) * sizeof(float2), 256);
 }
 
@@ -1194,13 +1206,19 @@ int march_interp(const dmr_plan *p, const float2 *grid, bool planar, float2 *ksp
     const MarchChunks ch = march_chunks(p, batch);
     const MarchGeom m = march_geom(p, ch.CS);
     const int64_t npts = (int64_t)p->g.nframes * p->g.gsize;
+    DMR_CHECK(ch.n < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
+    if (p->d2_W && !planar) return d2_interp(p, grid, ksp, 0, ch.n, ch.CS, batch, weight, wpb, st);
     for (int64_t k = 0; k < ch.n; k++) {
         const int64_t b0 = k * ch.CS;
         const int cact = (int)std::min<int64_t>(ch.CS, batch - b0);
         const float2 *src = grid + b0 * npts;
-        if (planar) {
+        if (planar && ch.CS > 1) {
             DMR_TRY(transpose<false>(src, il, npts, cact, ch.CS, st));
             src = il;
+        }
+        if (p->d2_W) {
+            DMR_TRY(d2_interp(p, src, ksp, b0, 1, ch.CS, batch, weight, wpb, st));
+            continue;
         }
         DMR_TRY(interp_chunk(p, m, src, rows, st));
         DMR_TRY(rows_out(p, m, rows, b0, cact, weight, wpb, ksp, st));
@@ -1216,6 +1234,22 @@ int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool
     const int64_t npts = (int64_t)p->g.nframes * p->g.gsize;
     const size_t chunk_bytes = (size_t)npts * ch.CS * sizeof(float2);
     float2 *scratch = nullptr;
+    DMR_CHECK(ch.n < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
+    if (!p->mp_W) {
+        // 2D, too sparse for tiles
+        if (det) return DMR_ERR_UNSUPPORTED;
+        if (!planar || ch.CS == 1) {
+            DMR_CUDA(cudaMemsetAsync(grid, 0, chunk_bytes * ch.n, st));
+            return d2_grid(p, ksp, kreal, grid, 0, ch.n, ch.CS, batch, weight, wpb, st);
+        }
+        for (int64_t k = 0; k < ch.n; k++) {
+            const int64_t b0 = k * ch.CS;
+            DMR_CUDA(cudaMemsetAsync(il, 0, chunk_bytes, st));
+            DMR_TRY(d2_grid(p, ksp, kreal, il, b0, 1, ch.CS, batch, weight, wpb, st));
+            DMR_TRY(transpose<true>(il, grid + b0 * npts, npts, (int)std::min<int64_t>(ch.CS, batch - b0), ch.CS, st));
+        }
+        return DMR_OK;
+    }
     if (det) {
         // every unit's plane of one chunk of coils; over the caller's limit, or
         // no memory for it: another deterministic kernel takes the call
@@ -1237,12 +1271,12 @@ int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool
         for (int64_t k = 0; k < ch.n; k++) {
             const int64_t b0 = k * ch.CS;
             const int cact = (int)std::min<int64_t>(ch.CS, batch - b0);
-            float2 *dst = planar ? il : grid + b0 * npts;
+            float2 *dst = planar && ch.CS > 1 ? il : grid + b0 * npts;
             DMR_TRY(rows_in(p, m, ksp, kreal, b0, cact, weight, wpb, rows, st));
             if (!det) DMR_CUDA(cudaMemsetAsync(dst, 0, chunk_bytes, st));
             DMR_TRY(grid_chunk(p, m, rows, dst, scratch, st));
             if (det) DMR_TRY(gather_chunk(p, m, scratch, dst, st));
-            if (planar) DMR_TRY(transpose<true>(il, grid + b0 * npts, npts, cact, ch.CS, st));
+            if (planar && ch.CS > 1) DMR_TRY(transpose<true>(il, grid + b0 * npts, npts, cact, ch.CS, st));
         }
         return DMR_OK;
     };
@@ -1255,22 +1289,23 @@ int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool
 struct MarchPool {
     float2 *rows = nullptr, *il = nullptr;
     cudaStream_t st;
+    void *owned = nullptr;
     MarchPool(const dmr_plan *p, int64_t batch, cudaStream_t s) : st(s)
     {
         const int CS = march_chunks(p, batch).CS;
         const size_t a = march_rows_bytes(p, CS), b = march_il_bytes(p, CS);
         cudaMemPool_t pool = scratch_pool(p->device);
-        void *q = nullptr;
-        if (pool && cudaMallocFromPoolAsync(&q, a + b, pool, st) == cudaSuccess) {
-            rows = (float2 *)q;
-            il = (float2 *)((char *)q + a);
+        if (pool && cudaMallocFromPoolAsync(&owned, a + b, pool, st) == cudaSuccess) {
+            rows = (float2 *)owned;
+            il = (float2 *)((char *)owned + a);
         } else {
+            owned = nullptr;
             cudaGetLastError();
         }
     }
     ~MarchPool()
     {
-        if (rows) cudaFreeAsync(rows, st);
+        if (owned) cudaFreeAsync(owned, st);
     }
 };
 
@@ -1278,7 +1313,7 @@ int march_interp_pool(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_
                       cudaStream_t st)
 {
     MarchPool b(p, batch, st);
-    if (!b.rows) return DMR_ERR_UNSUPPORTED;
+    if (!b.owned) return DMR_ERR_UNSUPPORTED;
     return march_interp(p, grid, true, ksp, batch, weight, wpb, b.rows, b.il, st);
 }
 
@@ -1286,7 +1321,7 @@ int march_grid_pool(const dmr_plan *p, const void *ksp, int kreal, float2 *grid,
                     int wpb, int det, int64_t det_limit, cudaStream_t st)
 {
     MarchPool b(p, batch, st);
-    if (!b.rows) return DMR_ERR_UNSUPPORTED;
+    if (!b.owned) return DMR_ERR_UNSUPPORTED;
     return march_grid(p, ksp, kreal, grid, true, batch, weight, wpb, det, det_limit, b.rows, b.il, st);
 }
 

@@ -25,6 +25,15 @@ struct MarchChunks {
 int march_build(::dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
                 cudaStream_t st);
 
+// 2D: per-sample records in acquisition order, interpolation, and gridding by
+// direct additions to the (zeroed) grid, for `nch` chunks of CS coils from coil
+// b0 on, interleaved (direct2d.cu)
+int d2_build(::dmr_plan *p, float *const rk[3], cudaStream_t st);
+int d2_interp(const ::dmr_plan *p, const float2 *grid, float2 *ksp, int64_t b0, int64_t nch, int CS, int64_t batch,
+              const float *weight, int wpb, cudaStream_t st);
+int d2_grid(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t b0, int64_t nch, int CS,
+            int64_t batch, const float *weight, int wpb, cudaStream_t st);
+
 MarchChunks march_chunks(const ::dmr_plan *p, int64_t batch);
 size_t march_rows_bytes(const ::dmr_plan *p, int CS);
 size_t march_il_bytes(const ::dmr_plan *p, int CS);

@@ -198,7 +198,7 @@ static int nufft_ws(dmr_plan *p, int64_t batch, void *ws, size_t ws_bytes, Nufft
     int64_t slots = batch;  // coil slots of the grid
     size_t rows_bytes = 0, il_bytes = 0;
     out.march = MarchChunks{0, 0};
-    if (p->mp_W) {
+    if (p->il_forward()) {
         out.march = march_chunks(p, batch);
         rows_bytes = march_rows_bytes(p, out.march.CS);
         if (fp) il_bytes = march_il_bytes(p, out.march.CS);
@@ -387,7 +387,7 @@ extern "C" int dmr_nufft_forward(dmr_plan *p, const void *image, int image_real,
     DMR_CHECK(p && image && kspace && batch >= 1, DMR_ERR_INVALID, "bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     float2 *grid = nullptr;
-    if (p->mp_W) {
+    if (p->il_forward()) {
         NufftWs w;
         DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
         if (w.fft) DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));

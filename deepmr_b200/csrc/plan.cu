@@ -472,7 +472,10 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     // 5 with 32 coils the kernel's bounded waits ran out)
     // (only where dmr_tc_min_coils was set: 1.3 GB and a second sort for the
     // 192^3 kooshball)
-    if (total > 0) DMR_TRY(march_build(p.get(), rk, keys, keys_s, vals, st));
+    if (total > 0) {
+        DMR_TRY(d2_build(p.get(), rk, st));
+        DMR_TRY(march_build(p.get(), rk, keys, keys_s, vals, st));
+    }
     if (tc_min_coils() < INT_MAX && ndim == 3 && total > 0 && g.W[0] == g.W[1] && g.W[1] == g.W[2] &&
         g.W[0] >= 2 && g.W[0] <= 4) {
         const int W = g.W[0];

@@ -179,7 +179,8 @@ struct dmr_plan {
     dmr::RtItem *rt_reduce = nullptr;
     int nrt_reduce = 0;
     int rt_slots = 0;
-    // 3D march order (march.cu; mp_W == 0: not planned): tiles along x and y,
+    // march order (march.cu; mp_W == 0: not planned; 3D, and 2D plans dense enough
+    // for tiles, which have gridding units only): tiles along x and y,
     // CSR offsets per cell, sorted position -> sample and back, per sorted
     // sample the tap weights and z cell, gridding units for 1, 2, 4 and 8
     // planes per warp (int4), the first unit of each (frame tile, plane), and
@@ -196,6 +197,13 @@ struct dmr_plan {
     int32_t *mp_ustart = nullptr;
     void *mp_items = nullptr;
     int mp_nitems = 0;
+    // 2D, acquisition order (direct2d.cu; d2_W == 0: not planned): tap weights
+    // and (first tap position, frame) per sample (int2)
+    int d2_W = 0;
+    float *d2_rec = nullptr;
+    void *d2_base = nullptr;
+    // whether forward transforms run on the interleaved grid
+    bool il_forward() const { return (g.ndim == 3 && mp_W) || d2_W; }
     // device status word: blocks of this plan's calls whose bounded wait ran out
     // (dmr_plan_status; 0 while every result is valid)
     int32_t *status = nullptr;
@@ -231,5 +239,7 @@ struct dmr_plan {
         for (void *u : mp_units) cudaFree(u);
         cudaFree(mp_ustart);
         cudaFree(mp_items);
+        cudaFree(d2_rec);
+        cudaFree(d2_base);
     }
 };

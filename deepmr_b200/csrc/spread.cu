@@ -1366,7 +1366,7 @@ int interp_dispatch(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_t 
                     const float *weight, int wpb, cudaStream_t st)
 {
     if (p->nwork == 0) return DMR_OK;
-    if (p->mp_W) {
+    if (p->il_forward()) {
         const int rc = march_interp_pool(p, grid, ksp, batch, weight, wpb, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }
@@ -1415,8 +1415,8 @@ int tc_min_coils() { return g_tc_min_coils.load(); }
 
 bool grid_march_applies(const dmr_plan *p, int64_t batch, int det)
 {
-    if (p->mp_W == 0 || grid_variant() != 0) return false;
-    if (det) return !tc_disabled();
+    if ((p->mp_W == 0 && p->d2_W == 0) || grid_variant() != 0) return false;
+    if (det) return p->mp_W && !(p->g.ndim == 3 && tc_disabled());
     return p->tg_T[0] == 0 || batch < tc_min_coils();
 }
 

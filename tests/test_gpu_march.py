@@ -128,3 +128,39 @@ def test_march_nan_stays_in_its_taps():
             _lib.check(L.dmr_grid(ip.handle, _lib.ptr(y), 0, _lib.ptr(grid), k, None, 0, det, st))
             bad = torch.isnan(grid.real)
             assert int(bad[0].sum()) == 64 and int(bad[1:].sum()) == 0, (k, det)
+
+
+@pytest.mark.parametrize("shape,width,os", [((18, 23), 4, 1.25), ((17, 12), 3, 2.0), ((9, 14), 5, 1.5), ((10, 8), 2, 2.0),
+                                            ((11, 9), 6, 2.0), ((32, 32), 4, 1.25), ((4, 5), 4, 1.25)])
+@pytest.mark.parametrize("nsamples", [40, 1200], ids=["sparse", "dense"])
+def test_2d_vs_oracle(shape, width, os, nsamples):
+    """2D: direct interpolation, direct (sparse) and tiled (dense) gridding, both
+    modes, around the coil-lane boundaries; samples on the band's edges wrap."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+    from oracle import nufft_ref as R
+
+    rng = np.random.default_rng(width)
+    n = np.asarray(shape[::-1], dtype=np.float64)
+    c = rng.uniform(-0.5, 0.5, (1, nsamples, 2)) * n
+    c[:, : nsamples // 2] *= 0.05
+    c[:, -8:] = np.sign(c[:, -8:]) * n * 0.4999
+    c = torch.as_tensor(c.astype(np.float32))
+    plan = F.plan_nufft(c, shape, width, os, device="cuda")
+    oplan = R.plan_nufft(c, shape, width, os)
+    img = synth.complex_gaussian((34,) + shape, seed=1)
+    ksp = synth.complex_gaussian((34,) + tuple(c.shape[:-1]), seed=2)
+    w = torch.rand(tuple(c.shape[:-1]), generator=torch.Generator().manual_seed(3))
+    y_ref = R.apply_nufft(img, oplan)
+    x_ref = R.apply_nufft_adj(ksp, oplan, weight=w)
+    for k in (1, 2, 3, 5, 8, 9, 17, 32, 34):
+        assert rel(F.apply_nufft(img[:k].cuda(), plan), y_ref[:k]) < TOL, k
+        for det in (False, True):
+            old = F.set_deterministic_gridding(det)
+            try:
+                x = F.apply_nufft_adj(ksp[:k].cuda(), plan, weight=w.cuda())
+                x2 = F.apply_nufft_adj(ksp[:k].cuda(), plan, weight=w.cuda())
+            finally:
+                F.set_deterministic_gridding(old)
+            assert rel(x, x_ref[:k]) < TOL, (k, det)
+            assert not det or torch.equal(x, x2), k
