@@ -205,13 +205,14 @@ __device__ __forceinline__ void reg_dft(float2 *v, const float2 *tw, bool inv)
     }
 }
 
-// A transform length L = L1 L2 (both at most 24, products of 2, 3, 4, 5, 7).
+// A transform length L = L1 L2 (both at most 32, products of 2, 3, 4, 5, 7).
 template <int L_, int L1_, int L2_>
 struct Len {
     static constexpr int L = L_, L1 = L1_, L2 = L2_;
     // one thread per (line, column) of step A and per (line, row) of step B
     static constexpr int T = kFftLines * (L1 > L2 ? L1 : L2);
-    static constexpr int MINB = T <= 256 ? DMR_FFT_MINB : 2;
+    static constexpr int MINB = T <= 256 ? DMR_FFT_MINB : (T <= 384 ? 2 : 1);
+    static constexpr int TOEP_MINB = T <= 384 ? DMR_FFT_TOEP_MINB : 1;
     static_assert(L1 * L2 == L, "factors");
 };
 
@@ -274,7 +275,7 @@ __device__ __forceinline__ void step_b(const float2 *buf, const float2 *tw, bool
     X(112, 16, 7) X(120, 12, 10) X(128, 16, 8) X(140, 20, 7) X(144, 12, 12) X(160, 16, 10)               \
     X(168, 12, 14) X(192, 16, 12) X(200, 20, 10) X(224, 16, 14) X(240, 16, 15) X(256, 16, 16)            \
     X(280, 20, 14) X(288, 18, 16) X(320, 20, 16) X(336, 24, 14) X(384, 24, 16) X(400, 20, 20)            \
-    X(480, 24, 20)
+    X(480, 24, 20) X(512, 32, 16) X(640, 32, 20)
 
 bool has_len(int L)
 {
@@ -623,7 +624,7 @@ __global__ void __launch_bounds__(F::T, F::MINB) fft_cols_kernel(FftGeom g, ColA
 // memory between the two transforms. Tiles run batch-fastest, so the blocks
 // that read one kernel tile run together and share it in L2.
 template <class F>
-__global__ void __launch_bounds__(F::T, DMR_FFT_TOEP_MINB) fft_toep_z_kernel(FftGeom g, ColArgs a, int64_t nk,
+__global__ void __launch_bounds__(F::T, F::TOEP_MINB) fft_toep_z_kernel(FftGeom g, ColArgs a, int64_t nk,
                                                           const float2 *__restrict__ kern, float kscale,
                                                           const float2 *__restrict__ tw, float2 *grid)
 {
@@ -1002,6 +1003,13 @@ bool toep3_applies(int ndim, const int32_t *kshape, const int32_t *ishape)
     for (int a = 0; a < ndim; a++)
         if (kshape[a] < ishape[a] || !has_len(kshape[a])) return false;
     return true;
+}
+
+size_t toep_extra_bytes(int ndim, const int32_t *kshape, size_t data_bytes, size_t work_bytes)
+{
+    size_t b = align_up(work_bytes, 256);
+    if (toep3_applies(ndim, kshape, kshape)) b = std::max(b, align_up(data_bytes / 4, 256));
+    return b;
 }
 
 // Toeplitz self-adjoint of a 3D image batch (src/deepmr/fft/nufft.py:609-669,

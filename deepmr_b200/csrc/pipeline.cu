@@ -668,7 +668,8 @@ extern "C" int dmr_toeplitz_workspace_bytes(int ndim, const int32_t *kshape, int
     int err = DMR_OK;
     auto fp = get_fft_plan(ndim, dims, batch, &err);
     if (!fp) return err;
-    *bytes = align_up((size_t)batch * ksize * sizeof(float2), 256) + align_up(fp->work_bytes, 256) +
+    const size_t data_bytes = align_up((size_t)batch * ksize * sizeof(float2), 256);
+    *bytes = data_bytes + toep_extra_bytes(ndim, kshape, data_bytes, fp->work_bytes) +
              align_up(kReduceBlocks * (sizeof(double) + sizeof(unsigned long long)), 256);
     return DMR_OK;
 }
@@ -685,7 +686,7 @@ static int toep_ws(int ndim, const int32_t *kshape, int64_t batch, void *ws, siz
     fp = get_fft_plan(ndim, dims, batch, &err);
     if (!fp) return err;
     const size_t a = align_up((size_t)batch * ksize * sizeof(float2), 256);
-    const size_t b = align_up(fp->work_bytes, 256);
+    const size_t b = toep_extra_bytes(ndim, kshape, a, fp->work_bytes);
     const size_t c = align_up(kReduceBlocks * (sizeof(double) + sizeof(unsigned long long)), 256);
     DMR_CHECK(ws && ws_bytes >= a + b + c, DMR_ERR_WORKSPACE, "workspace too small: %zu < %zu",
               ws_bytes, a + b + c);

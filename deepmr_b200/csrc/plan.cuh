@@ -100,6 +100,10 @@ int fft3_adjoint_il(const ::dmr_plan *p, float2 *grid, int64_t batch, int64_t nc
 // (kernel extents at least the image's and with a compiled transform), and
 // pad + FFT + kernel multiply + inverse FFT + crop (data: batch kernel grids)
 bool toep3_applies(int ndim, const int32_t *kshape, const int32_t *ishape);
+// bytes after the `data_bytes` of kernel grids in a Toeplitz workspace: cuFFT's
+// work area, or, where the passes apply, room for the batch's images (a quarter
+// of the grids holds them whenever the grids are twice the images on two axes)
+size_t toep_extra_bytes(int ndim, const int32_t *kshape, size_t data_bytes, size_t work_bytes);
 int fft3_toeplitz(int ndim, const int32_t *kshape_zyx, const int32_t *ishape_zyx, const float2 *kernel, int64_t nk,
                   const void *image, int image_real, float2 *out, int64_t batch, float2 *data, cudaStream_t st);
 // tensor-core gridding of 3D plans (tcgrid.cu: dispatch and health state,

@@ -128,115 +128,179 @@ __global__ void toep_mul_kernel(float2 *__restrict__ data, const float2 *__restr
 // ---------------------------------------------------------------------------
 // conjugate gradient (cg.py:150-221) with float64 inner products
 // ---------------------------------------------------------------------------
-constexpr int kCgParts = 512;  // fixed partition of every reduction (deterministic)
+// Every reduction runs over a fixed partition of at most kCgParts blocks, and
+// the last block to finish adds the blocks' sums in a fixed tree and derives
+// the scalar of the step: no separate scalar launches (one thread adding 512
+// sums took 24 us twice an iteration), results independent of block order.
+constexpr int kCgParts = 512;
+constexpr int kCgThreads = 256;
 
 struct CgState {
     double rsold[2];  // complex, as the reference's first dot(r, r)
     double rsnew;
     double alpha[2];
-    double beta;
-    double pad[2];
+    double beta[2];   // imaginary part zero in exact arithmetic
+    unsigned int done;  // blocks of the running reduction that have finished
+    unsigned int pad;
     double parts[2 * kCgParts];
 };
 
-// per-block partial of sum conj(a) b (or |a|^2 when b == a), fixed grid kCgParts
-__global__ void cdot_partial_kernel(const float2 *__restrict__ a, const float2 *__restrict__ b, int64_t n,
-                                    double *__restrict__ parts)
+// sum over the block of (re, im), in thread 0 (fixed order)
+__device__ __forceinline__ void block_sum(double &re, double &im)
 {
-    double re = 0.0, im = 0.0;
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const float2 u = a[e], v = b[e];
-        re += (double)u.x * v.x + (double)u.y * v.y;
-        im += (double)u.x * v.y - (double)u.y * v.x;
+    __shared__ double sr[kCgThreads / 32], si[kCgThreads / 32];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        re += __shfl_down_sync(0xffffffffu, re, d);
+        im += __shfl_down_sync(0xffffffffu, im, d);
     }
-    __shared__ double sr[256], si[256];
-    sr[threadIdx.x] = re;
-    si[threadIdx.x] = im;
+    if ((threadIdx.x & 31) == 0) {
+        sr[threadIdx.x >> 5] = re;
+        si[threadIdx.x >> 5] = im;
+    }
     __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) {
-            sr[threadIdx.x] += sr[threadIdx.x + h];
-            si[threadIdx.x] += si[threadIdx.x + h];
-        }
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
-        parts[2 * blockIdx.x] = sr[0];
-        parts[2 * blockIdx.x + 1] = si[0];
+        for (int w = 1; w < kCgThreads / 32; w++) {
+            re += sr[w];
+            im += si[w];
+        }
     }
+    __syncthreads();
 }
 
-__device__ __forceinline__ void sum_parts(const double *parts, double &re, double &im)
+// Ends a reduction kernel: the block's sum to its part, and in the last block
+// the total and the step's scalars. mode 0: rsold = <r, r> (initialisation);
+// 1: alpha = rsold / <p, AHAp>; 2: rsnew = Re<r, r>, beta = rsnew / rsold, rsold = rsnew
+__device__ __forceinline__ void cg_finish(CgState *s, double re, double im, int mode)
 {
-    re = 0.0;
-    im = 0.0;
-    for (int i = 0; i < kCgParts; i++) {
-        re += parts[2 * i];
-        im += parts[2 * i + 1];
+    __shared__ bool last;
+    block_sum(re, im);
+    if (threadIdx.x == 0) {
+        s->parts[2 * blockIdx.x] = re;
+        s->parts[2 * blockIdx.x + 1] = im;
+        __threadfence();
+        last = atomicAdd(&s->done, 1u) == gridDim.x - 1;
     }
-}
-
-// mode 0: rsold = <r, r> (initialisation); 1: alpha = rsold / <p, AHAp>;
-// 2: rsnew = Re<r, r>, beta = rsnew / rsold, rsold = rsnew
-__global__ void cg_scalar_kernel(CgState *__restrict__ s, int mode)
-{
-    double re, im;
-    sum_parts(s->parts, re, im);
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    re = im = 0.0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += kCgThreads) {
+        re += __ldcg(&s->parts[2 * i]);
+        im += __ldcg(&s->parts[2 * i + 1]);
+    }
+    block_sum(re, im);
+    if (threadIdx.x != 0) return;
+    s->done = 0;
+    const double o0 = s->rsold[0], o1 = s->rsold[1];
     if (mode == 0) {
         s->rsold[0] = re;
         s->rsold[1] = im;
         s->rsnew = re;
     } else if (mode == 1) {
         const double den = re * re + im * im;  // rsold / (re + i im)
-        s->alpha[0] = (s->rsold[0] * re + s->rsold[1] * im) / den;
-        s->alpha[1] = (s->rsold[1] * re - s->rsold[0] * im) / den;
+        s->alpha[0] = (o0 * re + o1 * im) / den;
+        s->alpha[1] = (o1 * re - o0 * im) / den;
     } else {
         s->rsnew = re;
         // beta = rsnew / rsold with rsold complex (real after the first step)
-        const double d = s->rsold[0] * s->rsold[0] + s->rsold[1] * s->rsold[1];
-        s->beta = re * s->rsold[0] / d;
-        s->pad[0] = -re * s->rsold[1] / d;  // imaginary part of beta (zero in exact arithmetic)
+        const double d = o0 * o0 + o1 * o1;
+        s->beta[0] = re * o0 / d;
+        s->beta[1] = -re * o1 / d;
         s->rsold[0] = re;
         s->rsold[1] = 0.0;
     }
 }
 
-__global__ void cg_init_kernel(const float2 *__restrict__ ahy, float2 *__restrict__ x, float2 *__restrict__ r,
-                               float2 *__restrict__ p, int64_t n)
+// x = 0, r = p = ahy, rsold = <r, r>
+__global__ void __launch_bounds__(kCgThreads) cg_init_kernel(const float2 *__restrict__ ahy, float2 *__restrict__ x,
+                                                            float2 *__restrict__ r, float2 *__restrict__ p, int64_t n,
+                                                            CgState *s)
 {
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-         e += (int64_t)gridDim.x * blockDim.x) {
+    double re = 0.0;
+    for (int64_t e = blockIdx.x * (int64_t)kCgThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kCgThreads) {
         const float2 v = ahy[e];
         x[e] = make_float2(0.0f, 0.0f);
         r[e] = v;
         p[e] = v;
+        re += (double)v.x * v.x + (double)v.y * v.y;
     }
+    cg_finish(s, re, 0.0, 0);
 }
 
-// x += alpha p; r -= alpha q  (complex64 arithmetic like the reference)
-__global__ void cg_update_xr_kernel(float2 *__restrict__ x, float2 *__restrict__ r, const float2 *__restrict__ p,
-                                    const float2 *__restrict__ q, int64_t n, const CgState *__restrict__ s)
+// alpha = rsold / <p, q>
+__global__ void __launch_bounds__(kCgThreads) cg_alpha_kernel(const float2 *__restrict__ p, const float2 *__restrict__ q,
+                                                             int64_t n, CgState *s)
+{
+    double re = 0.0, im = 0.0;
+    for (int64_t e = blockIdx.x * (int64_t)kCgThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kCgThreads) {
+        const float2 u = p[e], v = q[e];
+        re += (double)u.x * v.x + (double)u.y * v.y;
+        im += (double)u.x * v.y - (double)u.y * v.x;
+    }
+    cg_finish(s, re, im, 1);
+}
+
+// x += alpha p; r -= alpha q  (complex64 arithmetic like the reference); beta from <r, r>
+__global__ void __launch_bounds__(kCgThreads) cg_update_xr_kernel(float2 *__restrict__ x, float2 *__restrict__ r,
+                                                                 const float2 *__restrict__ p,
+                                                                 const float2 *__restrict__ q, int64_t n, CgState *s)
 {
     const float2 a = make_float2((float)s->alpha[0], (float)s->alpha[1]);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const float2 ap = cmul(p[e], a);
-        const float2 aq = cmul(q[e], a);
-        x[e] = make_float2(x[e].x + ap.x, x[e].y + ap.y);
-        r[e] = make_float2(r[e].x - aq.x, r[e].y - aq.y);
+    double re = 0.0;
+    for (int64_t e = blockIdx.x * (int64_t)kCgThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kCgThreads) {
+        const float2 ap = cmul(p[e], a), aq = cmul(q[e], a), xo = x[e], ro = r[e];
+        const float2 rn = make_float2(ro.x - aq.x, ro.y - aq.y);
+        x[e] = make_float2(xo.x + ap.x, xo.y + ap.y);
+        r[e] = rn;
+        re += (double)rn.x * rn.x + (double)rn.y * rn.y;
     }
+    cg_finish(s, re, 0.0, 2);
 }
 
 // p = r + beta p
-__global__ void cg_update_p_kernel(float2 *__restrict__ p, const float2 *__restrict__ r, int64_t n,
-                                   const CgState *__restrict__ s)
+__global__ void __launch_bounds__(kCgThreads) cg_update_p_kernel(float2 *__restrict__ p, const float2 *__restrict__ r,
+                                                                int64_t n, const CgState *__restrict__ s)
 {
-    const float2 bt = make_float2((float)s->beta, (float)s->pad[0]);
-    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
-         e += (int64_t)gridDim.x * blockDim.x) {
-        const float2 bp = cmul(p[e], bt);
-        p[e] = make_float2(r[e].x + bp.x, r[e].y + bp.y);
+    const float2 bt = make_float2((float)s->beta[0], (float)s->beta[1]);
+    for (int64_t e = blockIdx.x * (int64_t)kCgThreads + threadIdx.x; e < n; e += (int64_t)gridDim.x * kCgThreads) {
+        const float2 bp = cmul(p[e], bt), v = r[e];
+        p[e] = make_float2(v.x + bp.x, v.y + bp.y);
+    }
+}
+
+static int cg_blocks(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, kCgThreads), kCgParts)); }
+
+// img[c, i] = S_c[i] * x[i]
+__global__ void __launch_bounds__(256) sense_expand_kernel(int64_t isize, const float2 *__restrict__ maps,
+                                                          const float2 *__restrict__ x, float2 *__restrict__ img)
+{
+    const int64_t o = blockIdx.y * isize;
+    for (int64_t i = blockIdx.x * (int64_t)256 + threadIdx.x; i < isize; i += (int64_t)gridDim.x * 256)
+        img[o + i] = cmul(maps[o + i], x[i]);
+}
+
+// out[i] = sum_c conj(S_c[i]) * img[c, i] + lamda * x[i], coils summed in order
+__global__ void __launch_bounds__(128) sense_combine_kernel(int64_t isize, int64_t ncoils,
+                                                           const float2 *__restrict__ maps,
+                                                           const float2 *__restrict__ img,
+                                                           const float2 *__restrict__ x, float lamda,
+                                                           float2 *__restrict__ out)
+{
+    for (int64_t i = blockIdx.x * (int64_t)128 + threadIdx.x; i < isize; i += (int64_t)gridDim.x * 128) {
+        float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll 8
+        for (int64_t c = 0; c < ncoils; c++) {
+            const float2 v = cmulc(maps[c * isize + i], img[c * isize + i]);
+            acc.x += v.x;
+            acc.y += v.y;
+        }
+        if (lamda != 0.0f) {
+            const float2 xv = x[i];
+            acc.x += lamda * xv.x;
+            acc.y += lamda * xv.y;
+        }
+        out[i] = acc;
     }
 }
 
@@ -283,11 +347,28 @@ extern "C" int dmr_sense_normal(int ndim, const int32_t *kshape, const int32_t *
     auto fp = get_fft_plan(ndim, dims, ncoils, &err);
     if (!fp) return err;
     const size_t a = align_up((size_t)ncoils * g.ksize * sizeof(float2), 256);
-    const size_t b = align_up(fp->work_bytes, 256);
+    const size_t b = toep_extra_bytes(ndim, kshape, a, fp->work_bytes);
     DMR_CHECK(workspace && workspace_bytes >= a + b, DMR_ERR_WORKSPACE, "workspace too small: %zu < %zu",
               workspace_bytes, a + b);
     float2 *data = (float2 *)workspace;
     void *work = fp->work_bytes ? (char *)workspace + a : nullptr;
+    // compiled lengths: coil images through the fused, pruned passes of the
+    // Toeplitz self-adjoint (256^2, 16 coils: 46 us where pad, cuFFT, multiply,
+    // cuFFT and crop on the 512^2 grids took 89 us)
+    const size_t image_bytes = (size_t)ncoils * g.isize * sizeof(float2);
+    if (toep3_applies(ndim, kshape, ishape) && image_bytes <= b && ncoils < 65536) {
+        float2 *img = (float2 *)((char *)workspace + a);
+        const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(g.isize, 256), 148 * 8));
+        sense_expand_kernel<<<dim3(gx, (unsigned)ncoils), 256, 0, st>>>(g.isize, (const float2 *)maps, (const float2 *)x,
+                                                                       img);
+        DMR_LAUNCHED("sense_expand_kernel");
+        DMR_TRY(fft3_toeplitz(ndim, kshape, ishape, (const float2 *)kernel, 1, img, 0, img, ncoils, data, st));
+        sense_combine_kernel<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(g.isize, 128), 148 * 16)), 128,
+                               0, st>>>(g.isize, ncoils, (const float2 *)maps, img, (const float2 *)x, lamda,
+                                        (float2 *)out);
+        DMR_LAUNCHED("sense_combine_kernel");
+        return DMR_OK;
+    }
     const int64_t n = ncoils * g.ksize;
     sense_pad_kernel<<<blocks_for(n), 256, 0, st>>>(g, ncoils, (const float2 *)maps, (const float2 *)x, data);
     DMR_LAUNCHED("sense_pad_kernel");
@@ -314,12 +395,9 @@ extern "C" int dmr_cg_init(const void *ahy, void *x, void *r, void *p, int64_t n
     DMR_CHECK(ahy && x && r && p && state && n >= 1, DMR_ERR_INVALID, "bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     CgState *s = (CgState *)state;
-    cg_init_kernel<<<blocks_for(n), 256, 0, st>>>((const float2 *)ahy, (float2 *)x, (float2 *)r, (float2 *)p, n);
+    DMR_CUDA(cudaMemsetAsync(&s->done, 0, sizeof(s->done), st));
+    cg_init_kernel<<<cg_blocks(n), kCgThreads, 0, st>>>((const float2 *)ahy, (float2 *)x, (float2 *)r, (float2 *)p, n, s);
     DMR_LAUNCHED("cg_init_kernel");
-    cdot_partial_kernel<<<kCgParts, 256, 0, st>>>((const float2 *)r, (const float2 *)r, n, s->parts);
-    DMR_LAUNCHED("cdot_partial_kernel");
-    cg_scalar_kernel<<<1, 1, 0, st>>>(s, 0);
-    DMR_LAUNCHED("cg_scalar_kernel");
     return DMR_OK;
 }
 
@@ -328,18 +406,13 @@ extern "C" int dmr_cg_step(void *x, void *r, void *p, const void *q, int64_t n, 
     DMR_CHECK(x && r && p && q && state && n >= 1, DMR_ERR_INVALID, "bad argument");
     cudaStream_t st = (cudaStream_t)stream;
     CgState *s = (CgState *)state;
-    cdot_partial_kernel<<<kCgParts, 256, 0, st>>>((const float2 *)p, (const float2 *)q, n, s->parts);
-    DMR_LAUNCHED("cdot_partial_kernel");
-    cg_scalar_kernel<<<1, 1, 0, st>>>(s, 1);
-    DMR_LAUNCHED("cg_scalar_kernel");
-    cg_update_xr_kernel<<<blocks_for(n), 256, 0, st>>>((float2 *)x, (float2 *)r, (const float2 *)p,
-                                                       (const float2 *)q, n, s);
+    const int blocks = cg_blocks(n);
+    cg_alpha_kernel<<<blocks, kCgThreads, 0, st>>>((const float2 *)p, (const float2 *)q, n, s);
+    DMR_LAUNCHED("cg_alpha_kernel");
+    cg_update_xr_kernel<<<blocks, kCgThreads, 0, st>>>((float2 *)x, (float2 *)r, (const float2 *)p, (const float2 *)q, n,
+                                                       s);
     DMR_LAUNCHED("cg_update_xr_kernel");
-    cdot_partial_kernel<<<kCgParts, 256, 0, st>>>((const float2 *)r, (const float2 *)r, n, s->parts);
-    DMR_LAUNCHED("cdot_partial_kernel");
-    cg_scalar_kernel<<<1, 1, 0, st>>>(s, 2);
-    DMR_LAUNCHED("cg_scalar_kernel");
-    cg_update_p_kernel<<<blocks_for(n), 256, 0, st>>>((float2 *)p, (const float2 *)r, n, s);
+    cg_update_p_kernel<<<cg_blocks(n), kCgThreads, 0, st>>>((float2 *)p, (const float2 *)r, n, s);
     DMR_LAUNCHED("cg_update_p_kernel");
     return DMR_OK;
 }
