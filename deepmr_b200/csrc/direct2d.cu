@@ -221,10 +221,12 @@ int d2_build(dmr_plan *p, float *const rk[3], cudaStream_t st)
     const Geom &g = p->g;
     const int W = g.W[0];
     if (g.ndim != 2 || g.total == 0 || W < 2 || W > 6 || g.W[1] != W) return DMR_OK;
-    DMR_CUDA(cudaMalloc((void **)&p->d2_rec, (size_t)g.total * d2_rec(W) * sizeof(float)));
-    DMR_CUDA(cudaMalloc((void **)&p->d2_base, (size_t)g.total * sizeof(int2)));
+    DMR_TRY(plan_alloc(p->device, &p->d2_rec, (size_t)g.total * d2_rec(W), st));
+    int2 *base = nullptr;
+    DMR_TRY(plan_alloc(p->device, &base, g.total, st));
+    p->d2_base = base;
     const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(g.total, 256), 148 * 16);
-    d2_rec_kernel<<<blocks, 256, 0, st>>>(g, p->foff_dev, rk[0], rk[1], p->d2_rec, (int2 *)p->d2_base);
+    d2_rec_kernel<<<blocks, 256, 0, st>>>(g, p->foff_dev, rk[0], rk[1], p->d2_rec, base);
     DMR_LAUNCHED("d2_rec_kernel");
     p->d2_W = W;
     return DMR_OK;

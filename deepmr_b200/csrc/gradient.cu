@@ -170,6 +170,7 @@ extern "C" int dmr_nufft_traj_grad(dmr_plan *p, const void *image, int image_rea
     float2 *grid = nullptr;
     DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));
     if (g.total == 0) return DMR_OK;
+    DMR_TRY(plan_bins(p, st));
     float rs[3] = {1.0f, 1.0f, 1.0f};
     for (int a = 0; a < g.ndim; a++) rs[a] = std::ceil(p->os[a] * (float)g.N[a]) / (float)g.N[a];
     const int64_t *d_foff = p->foff_dev;

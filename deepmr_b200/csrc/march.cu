@@ -901,13 +901,6 @@ int march_blocks(int64_t n)
     return (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(n, 256), (int64_t)sms * 16));
 }
 
-template <typename T>
-int march_alloc(T **p, size_t n)
-{
-    DMR_CUDA(cudaMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)));
-    return DMR_OK;
-}
-
 MarchGeom march_geom(const dmr_plan *p, int CS)
 {
     const Geom &g = p->g;
@@ -1011,10 +1004,11 @@ int launch_interp(const dmr_plan *p, const MarchGeom &m, const float2 *grid, flo
 // ---------------------------------------------------------------------------
 // plan building and entry points (march.cuh)
 // ---------------------------------------------------------------------------
-int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals, cudaStream_t st)
+int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
+                MarchTotals &totals, cudaStream_t st)
 {
     const Geom &g = p->g;
-    const int W = g.W[0];
+    const int W = g.W[0], dev = p->device;
     if (g.ndim < 2 || g.total == 0 || W < 2 || W > 6 || g.W[1] != W || (g.ndim == 3 && g.W[2] != W)) return DMR_OK;
     const int T = march_tile(W), TT = T * T;
     const int nt0 = (int)ceil_div(g.G[0], T), nt1 = (int)ceil_div(g.G[1], T);
@@ -1026,91 +1020,83 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     // more than its samples' own additions: direct2d.cu)
     if (g.ndim == 2 && g.total < 4 * nft) return DMR_OK;
     const bool d3 = g.ndim == 3;
-    const int most = d3 ? kUnitVisits : kUnitVisits2, nl = d3 ? 5 : 1;  // lists: units of 1, 2, 4, 8 planes, items
-    struct Temp {
-        void *ptr[3] = {};
-        ~Temp()
-        {
-            for (void *q : ptr) cudaFree(q);
-        }
-    } tmp;
-    int32_t *counts = nullptr;
-    DMR_TRY(march_alloc(&counts, ncells + 1));
-    tmp.ptr[0] = counts;
-    DMR_TRY(march_alloc(&p->mp_cstart, ncells + 1));
+    // lists: gridding units of 1, 2, 4, 8 planes (2D: 1), interpolation items (3D)
+    const int most = d3 ? kUnitVisits : kUnitVisits2, nl = d3 ? 5 : 1;
+    const int np[4] = {1, 2, 4, 8};
+    const int nzb = (int)ceil_div(g.G[2], kItemZ), cols = T * march_rows(W), nzbh = nzb * (TT / cols);
+    int per[5];           // entries per frame tile before splitting
+    int64_t off[6] = {0};
+    for (int l = 0; l < nl; l++) {
+        per[l] = l < 4 ? (int)ceil_div(g.G[2], np[l]) : nzbh;
+        off[l + 1] = off[l] + nft * per[l] + 1;
+    }
+    PlanTemp tmp(dev, st);
+    int32_t *counts = nullptr, *starts = nullptr;
+    DMR_TRY(tmp.alloc(&counts, ncells + 1));
+    DMR_TRY(tmp.alloc(&starts, off[nl]));
+    DMR_TRY(plan_alloc(dev, &p->mp_cstart, ncells + 1, st));
+    DMR_TRY(plan_alloc(dev, &p->mp_sidx, g.total, st));
+    DMR_TRY(plan_alloc(dev, &p->mp_inv, g.total, st));
+    DMR_TRY(plan_alloc(dev, &p->mp_zc, d3 ? g.total : 1, st));
+    DMR_TRY(plan_alloc(dev, &p->mp_rec, (size_t)g.total * march_rec(W, g.ndim), st));
+    DMR_TRY(plan_alloc(dev, &p->mp_ustart, off[1], st));
     DMR_CUDA(cudaMemsetAsync(counts, 0, (ncells + 1) * sizeof(int32_t), st));
     march_key_kernel<<<march_blocks(g.total), 256, 0, st>>>(g, T, nt0, nt1, p->foff_dev, rk[0], rk[1], rk[2], keys,
                                                             counts);
     DMR_LAUNCHED("march_key_kernel");
     int bits = 1;
     while ((1ll << bits) < ncells) bits++;
-    const int np[4] = {1, 2, 4, 8};
-    int nzu[4];
-    for (int l = 0; l < 4; l++) nzu[l] = (int)ceil_div(g.G[2], np[l]);
-    const int nzb = (int)ceil_div(g.G[2], kItemZ), cols = T * march_rows(W), nzbh = nzb * (TT / cols);
     size_t tb = 0, t1 = 0;
-    DMR_TRY(march_alloc(&p->mp_sidx, g.total));
     DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_s, vals, p->mp_sidx, (int)g.total, 0, bits, st));
     DMR_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, t1, counts, p->mp_cstart, (int)(ncells + 1), st));
     tb = std::max(tb, t1);
-    void *temp = nullptr;
-    DMR_CUDA(cudaMalloc(&temp, std::max<size_t>(tb, 1)));
-    tmp.ptr[1] = temp;
+    char *temp = nullptr;
+    DMR_TRY(tmp.alloc(&temp, tb));
     DMR_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys_s, vals, p->mp_sidx, (int)g.total, 0, bits, st));
     DMR_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb, counts, p->mp_cstart, (int)(ncells + 1), st));
     g_launches.fetch_add(2);
-    DMR_TRY(march_alloc(&p->mp_inv, g.total));
-    DMR_TRY(march_alloc(&p->mp_zc, g.total));
-    DMR_TRY(march_alloc(&p->mp_rec, (size_t)g.total * march_rec(W, g.ndim)));
     march_rec_kernel<<<march_blocks(g.total), 256, 0, st>>>(g, p->mp_sidx, rk[0], rk[1], rk[2], p->mp_rec, p->mp_zc,
                                                            p->mp_inv);
     DMR_LAUNCHED("march_rec_kernel");
-    // unit and item lists: counts -> offsets -> lists (`counts` has room: every
-    // list has at most one entry per (frame tile, z) plus one)
-    int32_t *starts = nullptr;
-    int64_t off[6] = {0};
-    for (int l = 0; l < 4; l++) off[l + 1] = off[l] + nft * nzu[l] + 1;
-    off[5] = off[4] + nft * nzbh + 1;
-    DMR_TRY(march_alloc(&starts, off[5]));
-    tmp.ptr[2] = starts;
+    // counts -> offsets -> lists (`counts` has room: every list has at most one
+    // entry per (frame tile, z) plus one). A list holds at most one entry per
+    // non-empty group and one per `most` samples or visits, so it is allocated
+    // before its length is known
     for (int l = 0; l < nl; l++) {
         const int64_t n = off[l + 1] - off[l];
-        if (l < 4)
+        int4 *list = nullptr;
+        if (l < 4) {
+            const int64_t visits = g.total * (d3 ? ceil_div(np[l] + W - 1, np[l]) + 1 : 1);
+            DMR_TRY(plan_alloc(dev, &list, std::min(n, visits) + visits / most + 1, st));
             march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], d3 ? W : 1, np[l],
-                                                                    nzu[l], most, counts);
-        else
-            march_item_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, cols, g.G[2], nzb,
-                                                                    counts);
+                                                                    per[l], most, counts);
+        } else {
+            DMR_TRY(plan_alloc(dev, &list, std::min(n, g.total) + g.total / kItemSamples + 1, st));
+            march_item_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, cols, g.G[2], nzb, counts);
+        }
+        (l < 4 ? p->mp_units[l] : p->mp_items) = list;
         DMR_LAUNCHED("march_count_kernel");
         DMR_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb, counts, starts + off[l], (int)n, st));
         g_launches.fetch_add(1);
-    }
-    int32_t total[5] = {0};
-    for (int l = 0; l < nl; l++)
-        DMR_CUDA(cudaMemcpyAsync(&total[l], starts + off[l + 1] - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    DMR_CUDA(cudaStreamSynchronize(st));
-    for (int l = 0; l < nl; l++) {
-        int4 *list = nullptr;
-        DMR_TRY(march_alloc(&list, total[l]));
-        if (l < 4) {
-            p->mp_units[l] = list;
-            p->mp_nunits[l] = total[l];
-            march_unit_fill_kernel<<<march_blocks(nft * nzu[l]), 256, 0, st>>>(starts + off[l], nft, nzu[l], most, list);
-        } else {
-            p->mp_items = list;
-            p->mp_nitems = total[l];
-            march_item_fill_kernel<<<march_blocks(nft * nzbh), 256, 0, st>>>(starts + off[l], nft, nzbh, list);
-        }
+        if (l < 4)
+            march_unit_fill_kernel<<<march_blocks(n), 256, 0, st>>>(starts + off[l], nft, per[l], most, list);
+        else
+            march_item_fill_kernel<<<march_blocks(n), 256, 0, st>>>(starts + off[l], nft, per[l], list);
         DMR_LAUNCHED("march_fill_kernel");
+        DMR_CUDA(cudaMemcpyAsync(&totals.v[l], starts + off[l + 1] - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     }
     // the gather finds the units of a (frame tile, plane) by their offsets
-    DMR_TRY(march_alloc(&p->mp_ustart, off[1]));
     DMR_CUDA(cudaMemcpyAsync(p->mp_ustart, starts, off[1] * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    DMR_CUDA(cudaStreamSynchronize(st));
+    totals.n = nl;
     p->mp_nt[0] = nt0;
     p->mp_nt[1] = nt1;
     p->mp_W = W;
     return DMR_OK;
+}
+
+void march_lists(dmr_plan *p, const MarchTotals &totals)
+{
+    for (int l = 0; l < totals.n; l++) (l < 4 ? p->mp_nunits[l] : p->mp_nitems) = totals.v[l];
 }
 
 MarchChunks march_chunks(const dmr_plan *p, int64_t batch)

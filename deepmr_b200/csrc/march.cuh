@@ -22,8 +22,15 @@ struct MarchChunks {
 // sorts the samples and builds the work lists (no-op, mp_W stays 0, where the
 // kernels do not apply: not 3D, mixed widths or widths outside 2..6, or a grid
 // huge for its samples). keys / keys_s / vals: total int32 each, vals = 0..total-1
+// The lists' lengths are on their way to `totals` when it returns: march_lists
+// takes them once the stream has been synchronised
+struct MarchTotals {
+    int n = 0;
+    int32_t v[5] = {0};
+};
 int march_build(::dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
-                cudaStream_t st);
+                MarchTotals &totals, cudaStream_t st);
+void march_lists(::dmr_plan *p, const MarchTotals &totals);
 
 // 2D: per-sample records in acquisition order, interpolation, and gridding by
 // direct additions to the (zeroed) grid, for `nch` chunks of CS coils from coil

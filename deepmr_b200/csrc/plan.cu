@@ -11,6 +11,7 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
+#include <map>
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
@@ -64,16 +65,35 @@ __device__ __forceinline__ int first_tap(float k, int W)
     return (int)ceil((double)k - 0.5 * (double)W);
 }
 
-__global__ void preprocess_kernel(Geom g, const float *__restrict__ coord,
-                                  const int64_t *__restrict__ foff, float s0, float s1, float s2,
-                                  float h0, float h1, float h2, float *__restrict__ rk0,
-                                  float *__restrict__ rk1, float *__restrict__ rk2,
-                                  int32_t *__restrict__ keys, int32_t *__restrict__ vals,
-                                  int32_t *__restrict__ counts, int *__restrict__ err, int cell_order)
+__global__ void rescale_kernel(Geom g, const float *__restrict__ coord, float s0, float s1, float s2, float h0,
+                               float h1, float h2, float *__restrict__ rk0, float *__restrict__ rk1,
+                               float *__restrict__ rk2, int32_t *__restrict__ vals, int *__restrict__ err)
 {
     const float sc[3] = {s0, s1, s2};
     const float sh[3] = {h0, h1, h2};
     float *rk[3] = {rk0, rk1, rk2};
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.total;
+         i += (int64_t)gridDim.x * blockDim.x) {
+        for (int a = 0; a < g.ndim; a++) {
+            float k = __fadd_rn(__fmul_rn(coord[i * g.ndim + a], sc[a]), sh[a]);
+            if (!(fabsf(k) < 1.0e8f)) {  // non-finite or absurd coordinate
+                atomicOr(err, 1);
+                k = 0.0f;
+            }
+            rk[a][i] = k;
+        }
+        vals[i] = (int32_t)i;
+    }
+}
+
+// sort key of the bin kernels: (frame, bin, cell of the first tap inside the
+// bin), or (frame, bin) with the samples of a bin in acquisition order
+__global__ void bin_key_kernel(Geom g, const int64_t *__restrict__ foff, const float *__restrict__ rk0,
+                               const float *__restrict__ rk1, const float *__restrict__ rk2,
+                               int32_t *__restrict__ keys, int32_t *__restrict__ vals, int32_t *__restrict__ counts,
+                               int cell_order)
+{
+    const float *rk[3] = {rk0, rk1, rk2};
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.total;
          i += (int64_t)gridDim.x * blockDim.x) {
         // frame of sample i: last f with foff[f] <= i
@@ -84,18 +104,10 @@ __global__ void preprocess_kernel(Geom g, const float *__restrict__ coord,
         }
         int b[3] = {0, 0, 0}, l[3] = {0, 0, 0};
         for (int a = 0; a < g.ndim; a++) {
-            float k = __fadd_rn(__fmul_rn(coord[i * g.ndim + a], sc[a]), sh[a]);
-            if (!(fabsf(k) < 1.0e8f)) {  // non-finite or absurd coordinate
-                atomicOr(err, 1);
-                k = 0.0f;
-            }
-            rk[a][i] = k;
-            const int x0m = pmod(first_tap(k, g.W[a]), g.G[a]);
+            const int x0m = pmod(first_tap(rk[a][i], g.W[a]), g.G[a]);
             b[a] = x0m / g.T[a];
             l[a] = x0m - b[a] * g.T[a];
         }
-        // sort key: (frame, bin, cell of the first tap inside the bin), or
-        // (frame, bin) with the samples of a bin in acquisition order
         const int bin = lo * g.nbins + (b[2] * g.nb[1] + b[1]) * g.nb[0] + b[0];
         const int cell = (l[2] * g.T[1] + l[1]) * g.T[0] + l[0];
         keys[i] = cell_order ? bin * (g.T[0] * g.T[1] * g.T[2]) + cell : bin;
@@ -241,11 +253,36 @@ static void default_tile(int ndim, int T[3])
     else { T[0] = 4; T[1] = 4; T[2] = 4; }
 }
 
-template <typename T>
-static int dev_alloc(T **p, size_t n)
+// Plan memory comes from a pool of its own (stream-ordered, so that a plan
+// costs no device-wide allocator calls: 20 cudaMalloc / cudaFree pairs took
+// over 2 ms); the pool keeps at most 256 MB for the next plan.
+cudaMemPool_t plan_pool(int dev)
 {
-    if (n == 0) n = 1;
-    DMR_CUDA(cudaMalloc((void **)p, n * sizeof(T)));
+    static std::mutex mu;
+    static std::map<int, cudaMemPool_t> pools;
+    std::lock_guard<std::mutex> lk(mu);
+    auto it = pools.find(dev);
+    if (it != pools.end()) return it->second;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    uint64_t keep = 256ull << 20;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    pools[dev] = pool;
+    return pool;
+}
+
+int plan_alloc_bytes(int dev, void **p, size_t bytes, cudaStream_t st)
+{
+    cudaMemPool_t pool = plan_pool(dev);
+    DMR_CHECK(pool, DMR_ERR_CUDA, "no memory pool on device %d", dev);
+    DMR_CUDA(cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st));
     return DMR_OK;
 }
 
@@ -305,129 +342,35 @@ extern "C" int dmr_plan_destroy(dmr_plan *p)
     return DMR_OK;
 }
 
-namespace {
+namespace dmr {
 
-struct TempBuffers {
-    void *ptr[12] = {};
-    ~TempBuffers()
-    {
-        for (void *p : ptr) cudaFree(p);
-    }
-};
-
-}  // namespace
-
-extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os_shape,
-                               const int32_t *width, const float *beta, const float *oversamp,
-                               const float *coord, const int64_t *frame_offsets, int64_t nframes,
-                               const int32_t *tile, void *stream, dmr_plan **out)
+// Bins, work lists and the (bin, cell) sample order of the bin kernels. Plans
+// whose calls run on the interleaved kernels build them on the first call that
+// needs them (trajectory gradients in 3D, deterministic gridding over its
+// scratch limit, no pool memory): a host loop over all bins, milliseconds.
+int plan_bins(const dmr_plan *cp, cudaStream_t st)
 {
-    DMR_CHECK(out, DMR_ERR_INVALID, "out is NULL");
-    *out = nullptr;
-    DMR_CHECK(ndim >= 1 && ndim <= 3, DMR_ERR_INVALID, "ndim must be 1, 2 or 3 (got %d)", ndim);
-    DMR_CHECK(shape && os_shape && width && beta && oversamp && frame_offsets, DMR_ERR_INVALID,
-              "NULL parameter array");
-    DMR_CHECK(nframes >= 1 && nframes < (1 << 20), DMR_ERR_INVALID, "bad nframes %lld",
-              (long long)nframes);
-    const int64_t total = frame_offsets[nframes];
-    DMR_CHECK(frame_offsets[0] == 0 && total >= 0 && total < INT32_MAX, DMR_ERR_INVALID,
-              "frame offsets must start at 0 and total samples must fit in int32");
-    for (int64_t f = 0; f < nframes; f++)
-        DMR_CHECK(frame_offsets[f + 1] >= frame_offsets[f], DMR_ERR_INVALID,
-                  "frame offsets must be non-decreasing");
-    DMR_CHECK(coord || total == 0, DMR_ERR_INVALID, "coord is NULL");
-
-    cudaStream_t st = (cudaStream_t)stream;
-    std::unique_ptr<dmr_plan> p(new dmr_plan());
-    DMR_CUDA(cudaGetDevice(&p->device));
+    dmr_plan *p = const_cast<dmr_plan *>(cp);
+    std::lock_guard<std::mutex> lock(p->bins_mu);
+    if (p->bins_ready) return DMR_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    DMR_CUDA(cudaStreamIsCapturing(st, &cap));
+    DMR_CHECK(cap == cudaStreamCaptureStatusNone, DMR_ERR_UNSUPPORTED,
+              "this call builds bin structures on its first use: run it once before capturing it");
     Geom &g = p->g;
-    memset(&g, 0, sizeof(g));
-    g.ndim = ndim;
-    g.nframes = (int)nframes;
-    g.total = total;
-    int T[3];
-    default_tile(ndim, T);
-    for (int a = 0; a < 3; a++) {
-        g.G[a] = g.N[a] = g.W[a] = g.T[a] = g.nb[a] = 1;
-        g.half[a] = 0;
-        g.beta[a] = 0.0f;
-        g.inv_hw[a] = 1.0;
-        p->os[a] = 1.0f;
-    }
-    for (int i = 0; i < ndim; i++) {
-        const int a = ndim - 1 - i;  // (z, y, x) input -> x = 0
-        g.N[a] = shape[i];
-        g.G[a] = os_shape[i];
-        g.W[a] = width[i];
-        g.beta[a] = beta[i];
-        p->os[a] = oversamp[i];
-        DMR_CHECK(g.N[a] >= 1 && g.G[a] >= 1 && g.W[a] >= 1 && g.W[a] <= 16, DMR_ERR_INVALID,
-                  "bad axis %d: shape %d os_shape %d width %d (widths up to 16)", i, g.N[a],
-                  g.G[a], g.W[a]);
-        DMR_CHECK(g.W[a] == 1 || g.G[a] >= g.W[a], DMR_ERR_UNSUPPORTED,
-                  "oversampled grid %d smaller than kernel width %d on axis %d", g.G[a], g.W[a], i);
-        g.half[a] = g.G[a] / 2;
-        g.inv_hw[a] = 1.0 / (g.W[a] / 2.0);
-        const int t = tile ? tile[i] : T[a];
-        DMR_CHECK(t >= 1, DMR_ERR_INVALID, "bad tile");
-        g.T[a] = std::min(t, g.G[a]);
-        g.nb[a] = (int)ceil_div(g.G[a], g.T[a]);
-    }
-    g.nbins = g.nb[0] * g.nb[1] * g.nb[2];
-    g.gsize = (int64_t)g.G[0] * g.G[1] * g.G[2];
-    g.isize = (int64_t)g.N[0] * g.N[1] * g.N[2];
-    DMR_CHECK((int64_t)g.nbins * nframes * g.T[0] * g.T[1] * g.T[2] < INT32_MAX, DMR_ERR_UNSUPPORTED,
-              "too many bins x cells for 32-bit sort keys");
-    p->scale = kernel_scale(g);
-    p->frame_offsets.assign(frame_offsets, frame_offsets + nframes + 1);
-
-    // apodisation tables (image index), per axis
-    for (int a = 0; a < 3; a++) {
-        std::vector<float> ap = apod_table(g.N[a], a < ndim ? g.W[a] : 1, p->os[a], g.beta[a]);
-        DMR_TRY(dev_alloc(&p->apod[a], ap.size()));
-        DMR_CUDA(cudaMemcpyAsync(p->apod[a], ap.data(), ap.size() * sizeof(float),
-                                 cudaMemcpyHostToDevice, st));
-        DMR_CUDA(cudaStreamSynchronize(st));
-    }
-
-    // rescale constants (nufft.py:415-418), float32 like numpy
-    float sc[3] = {1, 1, 1}, sh[3] = {0, 0, 0};
-    for (int a = 0; a < ndim; a++) {
-        const float gos = std::ceil(p->os[a] * (float)g.N[a]);
-        sc[a] = gos / (float)g.N[a];
-        sh[a] = std::floor(gos / 2.0f);
-    }
-
-    const int64_t nkeys = (int64_t)nframes * g.nbins;
-    TempBuffers tmp;
+    const int ndim = g.ndim, dev = p->device;
+    const int64_t total = g.total, nframes = g.nframes;
+    float *const *rk = p->rk;
+    const int64_t nkeys = nframes * g.nbins;
+    PlanTemp tmp(dev, st);
     int32_t *keys = nullptr, *keys_s = nullptr, *vals = nullptr, *counts = nullptr;
-    int64_t *d_foff = nullptr;
-    int *d_err = nullptr;
-    float *rk[3] = {nullptr, nullptr, nullptr};
-    DMR_TRY(dev_alloc(&keys, total));
-    tmp.ptr[0] = keys;
-    DMR_TRY(dev_alloc(&keys_s, total));
-    tmp.ptr[1] = keys_s;
-    DMR_TRY(dev_alloc(&vals, total));
-    tmp.ptr[2] = vals;
-    DMR_TRY(dev_alloc(&counts, nkeys));
-    tmp.ptr[3] = counts;
-    DMR_TRY(dev_alloc(&d_foff, nframes + 1));
-    p->foff_dev = d_foff;  // kept by the plan
-    DMR_TRY(dev_alloc(&d_err, 1));
-    tmp.ptr[5] = d_err;
-    for (int a = 0; a < ndim; a++) {
-        DMR_TRY(dev_alloc(&rk[a], total));
-        tmp.ptr[6 + a] = rk[a];
-        DMR_TRY(dev_alloc(&p->scoord[a], total));
-    }
-    DMR_TRY(dev_alloc(&p->sidx, total));
-    DMR_TRY(dev_alloc(&p->status, 1));
-    DMR_CUDA(cudaMemsetAsync(p->status, 0, sizeof(int32_t), st));
+    DMR_TRY(tmp.alloc(&keys, total));
+    DMR_TRY(tmp.alloc(&keys_s, total));
+    DMR_TRY(tmp.alloc(&vals, total));
+    DMR_TRY(tmp.alloc(&counts, nkeys));
+    for (int a = 0; a < ndim; a++) DMR_TRY(plan_alloc(dev, &p->scoord[a], total, st));
+    DMR_TRY(plan_alloc(dev, &p->sidx, total, st));
     DMR_CUDA(cudaMemsetAsync(counts, 0, nkeys * sizeof(int32_t), st));
-    DMR_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), st));
-    DMR_CUDA(cudaMemcpyAsync(d_foff, frame_offsets, (nframes + 1) * sizeof(int64_t),
-                             cudaMemcpyHostToDevice, st));
 
     // Within a bin, samples are sorted by the cell of their first tap (register
     // reuse of the cube kernels); DMR_SORT_CELL=0 keeps them in acquisition
@@ -435,19 +378,17 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     const char *env_order = getenv("DMR_SORT_CELL");
     const int cell_order = env_order ? atoi(env_order) != 0 : 1;
     if (total > 0) {
-        preprocess_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(
-            g, coord, d_foff, sc[0], sc[1], sc[2], sh[0], sh[1], sh[2], rk[0], rk[1], rk[2],
-            keys, vals, counts, d_err, cell_order);
-        DMR_LAUNCHED("preprocess_kernel");
+        bin_key_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, p->foff_dev, rk[0], rk[1], rk[2], keys, vals, counts,
+                                                                cell_order);
+        DMR_LAUNCHED("bin_key_kernel");
         const int64_t nsort = nkeys * (cell_order ? (int64_t)g.T[0] * g.T[1] * g.T[2] : 1);
         int end_bit = 1;
         while ((1ll << end_bit) < nsort) end_bit++;
         size_t temp_bytes = 0;
         DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_s, vals, p->sidx,
                                                  (int)total, 0, end_bit, st));
-        void *temp = nullptr;
-        DMR_CUDA(cudaMalloc(&temp, std::max<size_t>(temp_bytes, 1)));
-        tmp.ptr[9] = temp;
+        char *temp = nullptr;
+        DMR_TRY(tmp.alloc(&temp, temp_bytes));
         DMR_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_s, vals, p->sidx,
                                                  (int)total, 0, end_bit, st));
         g_launches.fetch_add(1);
@@ -456,101 +397,12 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
         DMR_LAUNCHED("gather_sorted_kernel");
     }
     std::vector<int32_t> h_counts(nkeys);
-    int h_err = 0;
-    DMR_CUDA(cudaMemcpyAsync(h_counts.data(), counts, nkeys * sizeof(int32_t),
-                             cudaMemcpyDeviceToHost, st));
-    DMR_CUDA(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    DMR_CUDA(cudaMemcpyAsync(h_counts.data(), counts, nkeys * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    DMR_CHECK(h_err == 0, DMR_ERR_COORD, "non-finite (or |k| >= 1e8) k-space coordinate");
 
     // bin offsets
     std::vector<int32_t> h_start(nkeys + 1, 0);
     for (int64_t i = 0; i < nkeys; i++) h_start[i + 1] = h_start[i] + h_counts[i];
-
-    // bins of the 3D tensor-core gridding: region (T + W - 1) of 7 x 6 x 6
-    // points (x, y, z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..4 (at width
-    // 5 with 32 coils the kernel's bounded waits ran out)
-    // (only where dmr_tc_min_coils was set: 1.3 GB and a second sort for the
-    // 192^3 kooshball)
-    if (total > 0) {
-        DMR_TRY(d2_build(p.get(), rk, st));
-        DMR_TRY(march_build(p.get(), rk, keys, keys_s, vals, st));
-    }
-    if (tc_min_coils() < INT_MAX && ndim == 3 && total > 0 && g.W[0] == g.W[1] && g.W[1] == g.W[2] &&
-        g.W[0] >= 2 && g.W[0] <= 4) {
-        const int W = g.W[0];
-        int tT[3] = {8 - W, 7 - W, 7 - W}, tnb[3];
-        for (int a = 0; a < 3; a++) {
-            tT[a] = std::min(tT[a], g.G[a]);
-            tnb[a] = (int)ceil_div(g.G[a], tT[a]);
-        }
-        const int tbins = tnb[0] * tnb[1] * tnb[2];
-        const int64_t tkeys = (int64_t)nframes * tbins;
-        if (tkeys < INT32_MAX) {
-            int32_t *tcounts = nullptr;
-            DMR_TRY(dev_alloc(&tcounts, tkeys));
-            tmp.ptr[10] = tcounts;
-            DMR_CUDA(cudaMemsetAsync(tcounts, 0, tkeys * sizeof(int32_t), st));
-            tg_key_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], tnb[0], tnb[1], tnb[2],
-                                                                   tbins, d_foff, rk[0], rk[1], rk[2], keys, tcounts);
-            DMR_LAUNCHED("tg_key_kernel");
-            int tbit = 1;
-            while ((1ll << tbit) < tkeys) tbit++;
-            for (int a = 0; a < 3; a++) DMR_TRY(dev_alloc(&p->tg_scoord[a], total));
-            DMR_TRY(dev_alloc(&p->tg_sidx, total));
-            size_t tb = 0;
-            DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
-                                                     tbit, st));
-            void *ttemp = nullptr;
-            DMR_CUDA(cudaMalloc(&ttemp, std::max<size_t>(tb, 1)));
-            tmp.ptr[11] = ttemp;
-            DMR_CUDA(cub::DeviceRadixSort::SortPairs(ttemp, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
-                                                     tbit, st));
-            g_launches.fetch_add(1);
-            gather_sorted_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(
-                total, ndim, p->tg_sidx, rk[0], rk[1], rk[2], p->tg_scoord[0], p->tg_scoord[1], p->tg_scoord[2]);
-            DMR_LAUNCHED("gather_sorted_kernel");
-            p->tg_wp = W <= 4 ? 4 : 8;
-            DMR_TRY(dev_alloc(&p->tg_w, (size_t)total * 3 * p->tg_wp));
-            DMR_TRY(dev_alloc(&p->tg_l, total));
-            tg_weights_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], p->tg_wp,
-                                                                       p->tg_scoord[0], p->tg_scoord[1],
-                                                                       p->tg_scoord[2], p->tg_w, p->tg_l);
-            DMR_LAUNCHED("tg_weights_kernel");
-            std::vector<int32_t> hc(tkeys);
-            DMR_CUDA(cudaMemcpyAsync(hc.data(), tcounts, tkeys * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-            DMR_CUDA(cudaStreamSynchronize(st));
-            std::vector<int32_t> ts(tkeys + 1, 0);
-            for (int64_t i = 0; i < tkeys; i++) ts[i + 1] = ts[i] + hc[i];
-            std::vector<WorkItem> titems;
-            std::vector<int32_t> torder;
-            make_items(ts, tbins, tnb, kTgSegment, titems, torder);
-            DMR_TRY(dev_alloc(&p->tg_work, titems.size()));
-            DMR_TRY(dev_alloc(&p->tg_order, torder.size()));
-            if (!titems.empty()) {
-                DMR_CUDA(cudaMemcpyAsync(p->tg_work, titems.data(), titems.size() * sizeof(WorkItem),
-                                         cudaMemcpyHostToDevice, st));
-                DMR_CUDA(cudaMemcpyAsync(p->tg_order, torder.data(), torder.size() * sizeof(int32_t),
-                                         cudaMemcpyHostToDevice, st));
-            }
-            // deterministic mode: the items of each bin (make_items numbers
-            // them in key order, kTgSegment samples each)
-            std::vector<int32_t> istart(tkeys + 1, 0);
-            for (int64_t k = 0; k < tkeys; k++)
-                istart[k + 1] = istart[k] + (int32_t)ceil_div(ts[k + 1] - ts[k], kTgSegment);
-            DMR_CHECK(istart[tkeys] == (int64_t)titems.size(), DMR_ERR_UNSUPPORTED, "gridding item count mismatch");
-            DMR_TRY(dev_alloc(&p->tg_item_start, istart.size()));
-            DMR_CUDA(cudaMemcpyAsync(p->tg_item_start, istart.data(), istart.size() * sizeof(int32_t),
-                                     cudaMemcpyHostToDevice, st));
-            DMR_CUDA(cudaStreamSynchronize(st));
-            p->tg_nwork = (int)titems.size();
-            p->tg_nbins = tbins;
-            for (int a = 0; a < 3; a++) {
-                p->tg_T[a] = tT[a];
-                p->tg_nb[a] = tnb[a];
-            }
-        }
-    }
 
     // interpolation / atomic-gridding items: non-empty bins in chunks of at most
     // kChunk samples (bounded work per block), in spatial order so that blocks
@@ -638,7 +490,7 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
         det.insert(det.end(), by_color[c].begin(), by_color[c].end());
         p->det_color_start.push_back((int)det.size());
     }
-    DMR_TRY(dev_alloc(&p->det_work, det.size()));
+    DMR_TRY(plan_alloc(dev, &p->det_work, det.size(), st));
     if (!det.empty())
         DMR_CUDA(cudaMemcpyAsync(p->det_work, det.data(), det.size() * sizeof(WorkItem),
                                  cudaMemcpyHostToDevice, st));
@@ -666,12 +518,12 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     }
     p->nwork = (int)items.size();
     p->ntiles = (int)order.size();
-    DMR_TRY(dev_alloc(&p->bin_start, nkeys + 1));
-    DMR_TRY(dev_alloc(&p->work, items.size()));
-    DMR_TRY(dev_alloc(&p->tiles, order.size()));
+    DMR_TRY(plan_alloc(dev, &p->bin_start, nkeys + 1, st));
+    DMR_TRY(plan_alloc(dev, &p->work, items.size(), st));
+    DMR_TRY(plan_alloc(dev, &p->tiles, order.size(), st));
     DMR_CUDA(cudaMemcpyAsync(p->bin_start, h_start.data(), (nkeys + 1) * sizeof(int32_t),
                              cudaMemcpyHostToDevice, st));
-    DMR_TRY(dev_alloc(&p->work_order, items.size()));
+    DMR_TRY(plan_alloc(dev, &p->work_order, items.size(), st));
     if (!items.empty()) {
         DMR_CUDA(cudaMemcpyAsync(p->work, items.data(), items.size() * sizeof(WorkItem),
                                  cudaMemcpyHostToDevice, st));
@@ -681,7 +533,223 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     DMR_CUDA(cudaMemcpyAsync(p->tiles, order.data(), order.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    DMR_TRY(rt_build(p.get(), h_start, st));
+    DMR_TRY(rt_build(p, h_start, st));
+    DMR_CUDA(cudaStreamSynchronize(st));
+    p->bins_ready = true;
+    return DMR_OK;
+}
+
+// Tensor-core gridding order of 3D plans made while dmr_tc_min_coils is set
+static int tg_build(dmr_plan *p, int32_t *keys, int32_t *keys_s, int32_t *vals, cudaStream_t st)
+{
+    const Geom &g = p->g;
+    const int64_t total = g.total, nframes = g.nframes;
+    float *const *rk = p->rk;
+    const int dev = p->device;
+    PlanTemp tmp(dev, st);
+    // bins of the 3D tensor-core gridding: region (T + W - 1) of 7 x 6 x 6
+    // points (x, y, z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..4 (at width
+    // 5 with 32 coils the kernel's bounded waits ran out)
+    // (only where dmr_tc_min_coils was set: 1.3 GB and a second sort for the
+    // 192^3 kooshball)
+    if (tc_min_coils() == INT_MAX || g.ndim != 3 || total == 0 || g.W[0] != g.W[1] || g.W[1] != g.W[2] || g.W[0] < 2 ||
+        g.W[0] > 4)
+        return DMR_OK;
+    {
+        const int W = g.W[0];
+        int tT[3] = {8 - W, 7 - W, 7 - W}, tnb[3];
+        for (int a = 0; a < 3; a++) {
+            tT[a] = std::min(tT[a], g.G[a]);
+            tnb[a] = (int)ceil_div(g.G[a], tT[a]);
+        }
+        const int tbins = tnb[0] * tnb[1] * tnb[2];
+        const int64_t tkeys = (int64_t)nframes * tbins;
+        if (tkeys < INT32_MAX) {
+            int32_t *tcounts = nullptr;
+            DMR_TRY(tmp.alloc(&tcounts, tkeys));
+            DMR_CUDA(cudaMemsetAsync(tcounts, 0, tkeys * sizeof(int32_t), st));
+            tg_key_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], tnb[0], tnb[1], tnb[2],
+                                                                   tbins, p->foff_dev, rk[0], rk[1], rk[2], keys, tcounts);
+            DMR_LAUNCHED("tg_key_kernel");
+            int tbit = 1;
+            while ((1ll << tbit) < tkeys) tbit++;
+            for (int a = 0; a < 3; a++) DMR_TRY(plan_alloc(dev, &p->tg_scoord[a], total, st));
+            DMR_TRY(plan_alloc(dev, &p->tg_sidx, total, st));
+            size_t tb = 0;
+            DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
+                                                     tbit, st));
+            char *ttemp = nullptr;
+            DMR_TRY(tmp.alloc(&ttemp, tb));
+            DMR_CUDA(cub::DeviceRadixSort::SortPairs(ttemp, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
+                                                     tbit, st));
+            g_launches.fetch_add(1);
+            gather_sorted_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(
+                total, 3, p->tg_sidx, rk[0], rk[1], rk[2], p->tg_scoord[0], p->tg_scoord[1], p->tg_scoord[2]);
+            DMR_LAUNCHED("gather_sorted_kernel");
+            p->tg_wp = W <= 4 ? 4 : 8;
+            DMR_TRY(plan_alloc(dev, &p->tg_w, (size_t)total * 3 * p->tg_wp, st));
+            DMR_TRY(plan_alloc(dev, &p->tg_l, total, st));
+            tg_weights_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], p->tg_wp,
+                                                                       p->tg_scoord[0], p->tg_scoord[1],
+                                                                       p->tg_scoord[2], p->tg_w, p->tg_l);
+            DMR_LAUNCHED("tg_weights_kernel");
+            std::vector<int32_t> hc(tkeys);
+            DMR_CUDA(cudaMemcpyAsync(hc.data(), tcounts, tkeys * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+            DMR_CUDA(cudaStreamSynchronize(st));
+            std::vector<int32_t> ts(tkeys + 1, 0);
+            for (int64_t i = 0; i < tkeys; i++) ts[i + 1] = ts[i] + hc[i];
+            std::vector<WorkItem> titems;
+            std::vector<int32_t> torder;
+            make_items(ts, tbins, tnb, kTgSegment, titems, torder);
+            DMR_TRY(plan_alloc(dev, &p->tg_work, titems.size(), st));
+            DMR_TRY(plan_alloc(dev, &p->tg_order, torder.size(), st));
+            if (!titems.empty()) {
+                DMR_CUDA(cudaMemcpyAsync(p->tg_work, titems.data(), titems.size() * sizeof(WorkItem),
+                                         cudaMemcpyHostToDevice, st));
+                DMR_CUDA(cudaMemcpyAsync(p->tg_order, torder.data(), torder.size() * sizeof(int32_t),
+                                         cudaMemcpyHostToDevice, st));
+            }
+            // deterministic mode: the items of each bin (make_items numbers
+            // them in key order, kTgSegment samples each)
+            std::vector<int32_t> istart(tkeys + 1, 0);
+            for (int64_t k = 0; k < tkeys; k++)
+                istart[k + 1] = istart[k] + (int32_t)ceil_div(ts[k + 1] - ts[k], kTgSegment);
+            DMR_CHECK(istart[tkeys] == (int64_t)titems.size(), DMR_ERR_UNSUPPORTED, "gridding item count mismatch");
+            DMR_TRY(plan_alloc(dev, &p->tg_item_start, istart.size(), st));
+            DMR_CUDA(cudaMemcpyAsync(p->tg_item_start, istart.data(), istart.size() * sizeof(int32_t),
+                                     cudaMemcpyHostToDevice, st));
+            DMR_CUDA(cudaStreamSynchronize(st));
+            p->tg_nwork = (int)titems.size();
+            p->tg_nbins = tbins;
+            for (int a = 0; a < 3; a++) {
+                p->tg_T[a] = tT[a];
+                p->tg_nb[a] = tnb[a];
+            }
+        }
+    }
+    return DMR_OK;
+}
+
+}  // namespace dmr
+
+extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os_shape,
+                               const int32_t *width, const float *beta, const float *oversamp,
+                               const float *coord, const int64_t *frame_offsets, int64_t nframes,
+                               const int32_t *tile, void *stream, dmr_plan **out)
+{
+    DMR_CHECK(out, DMR_ERR_INVALID, "out is NULL");
+    *out = nullptr;
+    DMR_CHECK(ndim >= 1 && ndim <= 3, DMR_ERR_INVALID, "ndim must be 1, 2 or 3 (got %d)", ndim);
+    DMR_CHECK(shape && os_shape && width && beta && oversamp && frame_offsets, DMR_ERR_INVALID,
+              "NULL parameter array");
+    DMR_CHECK(nframes >= 1 && nframes < (1 << 20), DMR_ERR_INVALID, "bad nframes %lld",
+              (long long)nframes);
+    const int64_t total = frame_offsets[nframes];
+    DMR_CHECK(frame_offsets[0] == 0 && total >= 0 && total < INT32_MAX, DMR_ERR_INVALID,
+              "frame offsets must start at 0 and total samples must fit in int32");
+    for (int64_t f = 0; f < nframes; f++)
+        DMR_CHECK(frame_offsets[f + 1] >= frame_offsets[f], DMR_ERR_INVALID,
+                  "frame offsets must be non-decreasing");
+    DMR_CHECK(coord || total == 0, DMR_ERR_INVALID, "coord is NULL");
+
+    cudaStream_t st = (cudaStream_t)stream;
+    std::unique_ptr<dmr_plan> p(new dmr_plan());
+    DMR_CUDA(cudaGetDevice(&p->device));
+    Geom &g = p->g;
+    memset(&g, 0, sizeof(g));
+    g.ndim = ndim;
+    g.nframes = (int)nframes;
+    g.total = total;
+    int T[3];
+    default_tile(ndim, T);
+    for (int a = 0; a < 3; a++) {
+        g.G[a] = g.N[a] = g.W[a] = g.T[a] = g.nb[a] = 1;
+        g.half[a] = 0;
+        g.beta[a] = 0.0f;
+        g.inv_hw[a] = 1.0;
+        p->os[a] = 1.0f;
+    }
+    for (int i = 0; i < ndim; i++) {
+        const int a = ndim - 1 - i;  // (z, y, x) input -> x = 0
+        g.N[a] = shape[i];
+        g.G[a] = os_shape[i];
+        g.W[a] = width[i];
+        g.beta[a] = beta[i];
+        p->os[a] = oversamp[i];
+        DMR_CHECK(g.N[a] >= 1 && g.G[a] >= 1 && g.W[a] >= 1 && g.W[a] <= 16, DMR_ERR_INVALID,
+                  "bad axis %d: shape %d os_shape %d width %d (widths up to 16)", i, g.N[a],
+                  g.G[a], g.W[a]);
+        DMR_CHECK(g.W[a] == 1 || g.G[a] >= g.W[a], DMR_ERR_UNSUPPORTED,
+                  "oversampled grid %d smaller than kernel width %d on axis %d", g.G[a], g.W[a], i);
+        g.half[a] = g.G[a] / 2;
+        g.inv_hw[a] = 1.0 / (g.W[a] / 2.0);
+        const int t = tile ? tile[i] : T[a];
+        DMR_CHECK(t >= 1, DMR_ERR_INVALID, "bad tile");
+        g.T[a] = std::min(t, g.G[a]);
+        g.nb[a] = (int)ceil_div(g.G[a], g.T[a]);
+    }
+    g.nbins = g.nb[0] * g.nb[1] * g.nb[2];
+    g.gsize = (int64_t)g.G[0] * g.G[1] * g.G[2];
+    g.isize = (int64_t)g.N[0] * g.N[1] * g.N[2];
+    DMR_CHECK((int64_t)g.nbins * nframes * g.T[0] * g.T[1] * g.T[2] < INT32_MAX, DMR_ERR_UNSUPPORTED,
+              "too many bins x cells for 32-bit sort keys");
+    p->scale = kernel_scale(g);
+    p->frame_offsets.assign(frame_offsets, frame_offsets + nframes + 1);
+
+    // one upload: apodisation tables (image index) of the three axes, frame offsets
+    const int dev = p->device;
+    std::vector<float> ap[3];
+    size_t words = 0;
+    for (int a = 0; a < 3; a++) {
+        ap[a] = apod_table(g.N[a], a < ndim ? g.W[a] : 1, p->os[a], g.beta[a]);
+        words += (ap[a].size() + 3) / 4 * 4;
+    }
+    std::vector<char> host(words * sizeof(float) + (nframes + 1) * sizeof(int64_t));
+    DMR_TRY(plan_alloc(dev, &p->tables, host.size(), st));
+    size_t off = 0;
+    for (int a = 0; a < 3; a++) {
+        memcpy(host.data() + off, ap[a].data(), ap[a].size() * sizeof(float));
+        p->apod[a] = (float *)(p->tables + off);
+        off += (ap[a].size() + 3) / 4 * 4 * sizeof(float);
+    }
+    memcpy(host.data() + off, frame_offsets, (nframes + 1) * sizeof(int64_t));
+    p->foff_dev = (int64_t *)(p->tables + off);
+    DMR_CUDA(cudaMemcpyAsync(p->tables, host.data(), host.size(), cudaMemcpyHostToDevice, st));
+
+    // rescale constants (nufft.py:415-418), float32 like numpy
+    float sc[3] = {1, 1, 1}, sh[3] = {0, 0, 0};
+    for (int a = 0; a < ndim; a++) {
+        const float gos = std::ceil(p->os[a] * (float)g.N[a]);
+        sc[a] = gos / (float)g.N[a];
+        sh[a] = std::floor(gos / 2.0f);
+    }
+    // status word, then the coordinate error flag
+    DMR_TRY(plan_alloc(dev, &p->status, 2, st));
+    DMR_CUDA(cudaMemsetAsync(p->status, 0, 2 * sizeof(int32_t), st));
+    int *d_err = p->status + 1;
+    for (int a = 0; a < ndim; a++) DMR_TRY(plan_alloc(dev, &p->rk[a], total, st));
+    PlanTemp tmp(dev, st);
+    int32_t *keys = nullptr, *keys_s = nullptr, *vals = nullptr;
+    MarchTotals totals;
+    if (total > 0) {
+        DMR_TRY(tmp.alloc(&keys, total));
+        DMR_TRY(tmp.alloc(&keys_s, total));
+        DMR_TRY(tmp.alloc(&vals, total));
+        rescale_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, coord, sc[0], sc[1], sc[2], sh[0], sh[1], sh[2],
+                                                                p->rk[0], p->rk[1], p->rk[2], vals, d_err);
+        DMR_LAUNCHED("rescale_kernel");
+        DMR_TRY(d2_build(p.get(), p->rk, st));
+        DMR_TRY(march_build(p.get(), p->rk, keys, keys_s, vals, totals, st));
+    }
+    int h_err = 0;
+    DMR_CUDA(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    DMR_CUDA(cudaStreamSynchronize(st));
+    DMR_CHECK(h_err == 0, DMR_ERR_COORD, "non-finite (or |k| >= 1e8) k-space coordinate");
+    march_lists(p.get(), totals);
+    DMR_TRY(tg_build(p.get(), keys, keys_s, vals, st));
+    // plans of the interleaved kernels build the bin structures when a call
+    // needs them (plan_bins)
+    if (!p->il_forward()) DMR_TRY(plan_bins(p.get(), st));
     *out = p.release();
     return DMR_OK;
 }

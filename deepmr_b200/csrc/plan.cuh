@@ -67,6 +67,36 @@ struct FftPlan {
 // Process-wide cache of cuFFT plans keyed by (device, rank, dims, batch).
 std::shared_ptr<FftPlan> get_fft_plan(int ndim, const int *dims_zyx, int64_t batch, int *err);
 
+// stream-ordered plan memory: n elements of T from the plans' pool on `dev`
+int plan_alloc_bytes(int dev, void **p, size_t bytes, cudaStream_t st);
+
+template <typename T>
+int plan_alloc(int dev, T **p, size_t n, cudaStream_t st)
+{
+    return plan_alloc_bytes(dev, (void **)p, n * sizeof(T), st);
+}
+
+// temporaries of plan building, freed (stream-ordered) at the end of the scope
+struct PlanTemp {
+    int dev;
+    cudaStream_t st;
+    std::vector<void *> ptrs;
+    PlanTemp(int d, cudaStream_t s) : dev(d), st(s) {}
+    ~PlanTemp()
+    {
+        for (void *q : ptrs) cudaFreeAsync(q, st);
+    }
+    template <typename T>
+    int alloc(T **p, size_t n)
+    {
+        const int rc = plan_alloc(dev, p, n, st);
+        if (rc == DMR_OK) ptrs.push_back(*p);
+        return rc;
+    }
+};
+
+// the bin kernels' structures, built on first use (plan.cu)
+int plan_bins(const ::dmr_plan *p, cudaStream_t st);
 // Register-tile gridding: whether the geometry admits it (3D, grid at least
 // a block region plus the kernel support on every axis); plan the block items after the bin sort (host
 // bin offsets h_start, nframes * nbins + 1 entries); scratch bytes a call of
@@ -137,7 +167,13 @@ struct dmr_plan {
     double scale;                       // kernel-sum normalisation
     std::vector<int64_t> frame_offsets;  // host CSR
     float os[3];
-    // device buffers
+    // device buffers: apodisation tables and frame offsets, rescaled coordinates
+    // in acquisition order
+    char *tables = nullptr;
+    float *rk[3] = {nullptr, nullptr, nullptr};
+    // bin structures (plan_bins)
+    std::mutex bins_mu;
+    bool bins_ready = false;
     float *scoord[3] = {nullptr, nullptr, nullptr};  // sorted rescaled coordinates
     int32_t *sidx = nullptr;            // sorted position -> global sample index
     // 3D tensor-core gridding: bins of its own (tile tg_T, x y z) whose region
@@ -212,38 +248,42 @@ struct dmr_plan {
     // (dmr_plan_status; 0 while every result is valid)
     int32_t *status = nullptr;
 
+// (the owner has synchronised the device: nothing uses the buffers any more)
     ~dmr_plan()
     {
+        auto drop = [](void *q) {
+            if (q) cudaFreeAsync(q, cudaStreamPerThread);
+        };
+        drop(tables);
         for (int a = 0; a < 3; a++) {
-            cudaFree(scoord[a]);
-            cudaFree(apod[a]);
+            drop(scoord[a]);
+            drop(rk[a]);
         }
-        cudaFree(sidx);
-        for (int a = 0; a < 3; a++) cudaFree(tg_scoord[a]);
-        cudaFree(tg_sidx);
-        cudaFree(tg_w);
-        cudaFree(tg_l);
-        cudaFree(tg_work);
-        cudaFree(tg_order);
-        cudaFree(tg_item_start);
-        cudaFree(bin_start);
-        cudaFree(work);
-        cudaFree(work_order);
-        cudaFree(tiles);
-        cudaFree(det_work);
-        cudaFree(foff_dev);
+        drop(sidx);
+        for (int a = 0; a < 3; a++) drop(tg_scoord[a]);
+        drop(tg_sidx);
+        drop(tg_w);
+        drop(tg_l);
+        drop(tg_work);
+        drop(tg_order);
+        drop(tg_item_start);
+        drop(bin_start);
+        drop(work);
+        drop(work_order);
+        drop(tiles);
+        drop(det_work);
         cudaFree(rt_items);
         cudaFree(rt_reduce);
-        cudaFree(status);
-        cudaFree(mp_cstart);
-        cudaFree(mp_sidx);
-        cudaFree(mp_inv);
-        cudaFree(mp_zc);
-        cudaFree(mp_rec);
-        for (void *u : mp_units) cudaFree(u);
-        cudaFree(mp_ustart);
-        cudaFree(mp_items);
-        cudaFree(d2_rec);
-        cudaFree(d2_base);
+        drop(status);
+        drop(mp_cstart);
+        drop(mp_sidx);
+        drop(mp_inv);
+        drop(mp_zc);
+        drop(mp_rec);
+        for (void *u : mp_units) drop(u);
+        drop(mp_ustart);
+        drop(mp_items);
+        drop(d2_rec);
+        drop(d2_base);
     }
 };

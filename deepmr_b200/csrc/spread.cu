@@ -1365,11 +1365,12 @@ static int cube_width(const Geom &g)
 int interp_dispatch(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_t batch,
                     const float *weight, int wpb, cudaStream_t st)
 {
-    if (p->nwork == 0) return DMR_OK;
+    if (p->g.total == 0) return DMR_OK;
     if (p->il_forward()) {
         const int rc = march_interp_pool(p, grid, ksp, batch, weight, wpb, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }
+    DMR_TRY(plan_bins(p, st));
     const int cw = cube_width(p->g);
     if (cw > 0) {
         switch (p->g.ndim * 100 + cw) {
@@ -1434,6 +1435,7 @@ int grid_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, i
         const int rc = grid_tc_dispatch(p, ksp, kreal, grid, batch, weight, wpb, det, scratch, scratch_bytes, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }
+    DMR_TRY(plan_bins(p, st));
     // deterministic 3D gridding of 8+ coils otherwise: register tiles (one owner
     // per grid point, no colour passes) when the plan has them
     if (det) {
