@@ -43,9 +43,14 @@ __host__ __device__ constexpr int march_tile(int W) { return W <= 4 ? 4 : 3; }
 __host__ __device__ constexpr int march_rec(int W, int ndim = 3) { return (ndim * W + 3) / 4 * 4; }
 
 // visits of a gridding unit / samples of an interpolation item, at most: heavier
-// ones (the centre of k-space) are split so that no warp runs far behind
-constexpr int kUnitVisits = 512;
-constexpr int kUnitVisits2 = 128;  // 2D: few tiles, and no z axis to spread a dense one over
+// ones (the centre of k-space) are split so that no warp runs far behind. A
+// unit's sums are chains in float32, so its length also sets the rounding error
+// where k-space is dense (radial 100^3, 4,000 views of 180, 12 coils: 10.4e-7 of
+// the result at 512 visits, 9.3 at 128, 9.0 at 64, 8.8 with no chain to speak
+// of), and several planes to a warp cost no more in short units (512 and 64: 772
+// and 790 us; 64^3, 8 coils: 265 and 240). With a plane per warp a unit's flush
+// weighs more (192^3, 32 coils: 12.2 and 13.7 ms)
+constexpr int unit_visits(int ndim, int np) { return ndim == 3 && np == 1 ? 512 : 64; }
 constexpr int kItemSamples = 144;
 constexpr int kItemZ = 8;  // z cells of an interpolation item
 // rows of cell columns of an interpolation item (a tile has T / march_rows items per z block)
@@ -1021,7 +1026,7 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     if (g.ndim == 2 && g.total < 4 * nft) return DMR_OK;
     const bool d3 = g.ndim == 3;
     // lists: gridding units of 1, 2, 4, 8 planes (2D: 1), interpolation items (3D)
-    const int most = d3 ? kUnitVisits : kUnitVisits2, nl = d3 ? 5 : 1;
+    const int nl = d3 ? 5 : 1;
     const int np[4] = {1, 2, 4, 8};
     const int nzb = (int)ceil_div(g.G[2], kItemZ), cols = T * march_rows(W), nzbh = nzb * (TT / cols);
     int per[5];           // entries per frame tile before splitting
@@ -1064,6 +1069,7 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     // before its length is known
     for (int l = 0; l < nl; l++) {
         const int64_t n = off[l + 1] - off[l];
+        const int most = l < 4 ? unit_visits(g.ndim, np[l]) : kItemSamples;
         int4 *list = nullptr;
         if (l < 4) {
             const int64_t visits = g.total * (d3 ? ceil_div(np[l] + W - 1, np[l]) + 1 : 1);
@@ -1071,7 +1077,7 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
             march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], d3 ? W : 1, np[l],
                                                                     per[l], most, counts);
         } else {
-            DMR_TRY(plan_alloc(dev, &list, std::min(n, g.total) + g.total / kItemSamples + 1, st));
+            DMR_TRY(plan_alloc(dev, &list, std::min(n, g.total) + g.total / most + 1, st));
             march_item_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, cols, g.G[2], nzb, counts);
         }
         (l < 4 ? p->mp_units[l] : p->mp_items) = list;
