@@ -12,6 +12,7 @@
 // memory so that the k-space side runs along the samples. Weights and the
 // first tap's grid position come from the plan (d2_rec, d2_base).
 #include <algorithm>
+#include <cmath>
 
 #include "kb.cuh"
 #include "march.cuh"
@@ -166,6 +167,101 @@ __global__ void __launch_bounds__(256) grid2_kernel(D2Geom g, const float *__res
     }
 }
 
+// Trajectory gradient (gradient.cu): out[i, a] = post * sum_b Re(conj(v_b[i])
+// dy_b[i] / dcoord[i, a]) over coils b0 .. of `nch` interleaved chunks.
+// The block evaluates its samples' tap weights and their derivatives once; lane
+// = (sample, coil) sums its coil's taps, coils are added with shuffles.
+struct D2Grad {
+    float beta[2], inv_hw[2], rs[2];
+};
+
+template <int W, int CC>
+__global__ void __launch_bounds__(256) grad2_kernel(D2Geom g, D2Grad gr, const float *__restrict__ rk0,
+                                                    const float *__restrict__ rk1, const float *__restrict__ rec,
+                                                    const int2 *__restrict__ base, const float2 *__restrict__ grid,
+                                                    const float2 *__restrict__ v, int64_t batch, int64_t nch,
+                                                    const float *__restrict__ weight, int wpb, float scale, float post,
+                                                    int64_t b00, float *__restrict__ out)
+{
+    constexpr int NS = d2_tile(CC), GS = CC;  // samples per block, lanes per sample
+    __shared__ float2 s[NS][CC + 1];
+    __shared__ float dw[NS][2 * W + 1];
+    const int64_t i0 = blockIdx.x * (int64_t)NS;
+    const int n = (int)min((int64_t)NS, g.total - i0);
+    for (int e = threadIdx.x; e < 2 * W * NS; e += 256) {
+        const int t = e / (2 * W), q = e - t * (2 * W), a = q / W, k = q - a * W;
+        if (t >= n) continue;
+        const float c = a ? rk1[i0 + t] : rk0[i0 + t];
+        const int x0 = first_tap_dev(c, W);
+        const float u = (float)(((double)(x0 + k) - (double)c) * (2.0 / W));
+        float d;
+        kb_and_derivative(u, gr.beta[a], &d);
+        dw[t][q] = d * -gr.inv_hw[a] * gr.rs[a];
+    }
+    const int c = threadIdx.x % CC;
+    constexpr int K = (NS * CC + 255) / 256;  // samples of this lane
+    float acc[K][2];
+#pragma unroll
+    for (int k = 0; k < K; k++) acc[k][0] = acc[k][1] = 0.0f;
+    for (int64_t ch = 0; ch < nch; ch++) {
+        const int64_t b0 = b00 + ch * g.CS;
+        const int cact = (int)min((int64_t)g.CS, batch - b0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < NS * CC; e += 256) {
+            const int cc = e / NS, t = e % NS;
+            if (cc >= cact || t >= n) continue;
+            const int64_t o = (b0 + cc) * g.total + i0 + t;
+            const float2 x = v[o];
+            float w = scale;
+            if (weight) w *= weight[wpb ? o : i0 + t];
+            s[t][cc] = make_float2(x.x * w, x.y * w);
+        }
+        __syncthreads();
+        const float2 *gc = grid + ch * g.npts * g.CS + c;
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const int r = threadIdx.x / CC + k * (256 / CC);
+            if (r >= n || c >= cact) continue;
+            const Taps<W> t(g, rec + (i0 + r) * d2_rec(W), __ldg(base + i0 + r));
+            float2 dx = make_float2(0.0f, 0.0f), dy = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int jy = 0; jy < W; jy++) {
+                float2 q = make_float2(0.0f, 0.0f), qd = make_float2(0.0f, 0.0f);
+#pragma unroll
+                for (int jx = 0; jx < W; jx++) {
+                    const float2 x = __ldg(gc + t.yo[jy] + t.xo[jx]);
+                    q.x = fmaf(t.w[jx], x.x, q.x);
+                    q.y = fmaf(t.w[jx], x.y, q.y);
+                    qd.x = fmaf(dw[r][jx], x.x, qd.x);
+                    qd.y = fmaf(dw[r][jx], x.y, qd.y);
+                }
+                dx.x = fmaf(t.w[W + jy], qd.x, dx.x);
+                dx.y = fmaf(t.w[W + jy], qd.y, dx.y);
+                dy.x = fmaf(dw[r][W + jy], q.x, dy.x);
+                dy.y = fmaf(dw[r][W + jy], q.y, dy.y);
+            }
+            const float2 vb = s[r][c];
+            acc[k][0] += vb.x * dx.x + vb.y * dx.y;  // Re(conj(v) D)
+            acc[k][1] += vb.x * dy.x + vb.y * dy.y;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+        const int r = threadIdx.x / CC + k * (256 / CC);
+#pragma unroll
+        for (int d = 1; d < GS; d <<= 1) {
+            acc[k][0] += __shfl_xor_sync(0xffffffffu, acc[k][0], d);
+            acc[k][1] += __shfl_xor_sync(0xffffffffu, acc[k][1], d);
+        }
+        if (r < n && c == 0) {
+            // (chunks given one call at a time add to the first one's)
+            float *o = out + (i0 + r) * 2;
+            o[0] = (b00 ? o[0] : 0.0f) + acc[k][0] * post;
+            o[1] = (b00 ? o[1] : 0.0f) + acc[k][1] * post;
+        }
+    }
+}
+
 D2Geom d2_geom(const dmr_plan *p, int CS)
 {
     D2Geom g;
@@ -195,6 +291,24 @@ int launch_grid2(const dmr_plan *p, const D2Geom &g, const void *ksp, int kreal,
     grid2_kernel<W, CC><<<dim3((unsigned)ceil_div(g.total, d2_tile(CC)), (unsigned)nch), 256, 0, st>>>(
         g, p->d2_rec, (const int2 *)p->d2_base, ksp, kreal, grid, b0, batch, weight, wpb, (float)(1.0 / p->scale));
     DMR_LAUNCHED("grid2_kernel");
+    return DMR_OK;
+}
+
+template <int W, int CC>
+int launch_grad2(const dmr_plan *p, const D2Geom &g, const float2 *grid, const float2 *v, int64_t b0, int64_t nch,
+                 int64_t batch,
+                 const float *weight, int wpb, float post, float *out, cudaStream_t st)
+{
+    D2Grad gr;
+    for (int a = 0; a < 2; a++) {
+        gr.beta[a] = p->g.beta[a];
+        gr.inv_hw[a] = (float)p->g.inv_hw[a];
+        gr.rs[a] = std::ceil(p->os[a] * (float)p->g.N[a]) / (float)p->g.N[a];
+    }
+    grad2_kernel<W, CC><<<(unsigned)ceil_div(g.total, d2_tile(CC)), 256, 0, st>>>(
+        g, gr, p->rk[0], p->rk[1], p->d2_rec, (const int2 *)p->d2_base, grid, v, batch, nch, weight, wpb,
+        (float)(1.0 / p->scale), post, b0, out);
+    DMR_LAUNCHED("grad2_kernel");
     return DMR_OK;
 }
 
@@ -244,6 +358,13 @@ int d2_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t
 {
     const D2Geom g = d2_geom(p, CS);
     DMR_D2(launch_grid2, CS, p, g, ksp, kreal, grid, b0, nch, batch, weight, wpb, st)
+}
+
+int d2_grad(const dmr_plan *p, const float2 *grid, const float2 *v, int64_t b0, int64_t nch, int CS, int64_t batch,
+            const float *weight, int wpb, float post, float *out, cudaStream_t st)
+{
+    const D2Geom g = d2_geom(p, CS);
+    DMR_D2(launch_grad2, CS, p, g, grid, v, b0, nch, batch, weight, wpb, post, out, st)
 }
 
 }  // namespace dmr

@@ -857,7 +857,7 @@ int launch_rows(int L, bool crop, const FftGeom &g, const float2 *tw, const void
     }
 }
 
-FftGeom make_geom(const dmr_plan *p, int64_t batch, float scale)
+FftGeom make_geom(const dmr_plan *p, int64_t batch, int64_t nframes, float scale)
 {
     const Geom &gg = p->g;
     FftGeom g;
@@ -867,7 +867,7 @@ FftGeom make_geom(const dmr_plan *p, int64_t batch, float scale)
         g.apod[a] = gg.W[a] != 1 ? p->apod[a] : nullptr;
         g.off[a] = -(gg.N[a] / 2);  // FFT order: centred index N/2 at 0
     }
-    g.nbf = batch * gg.nframes;
+    g.nbf = batch * nframes;
     g.gsize = gg.gsize;
     g.isize = gg.isize;
     g.scale = scale;
@@ -924,10 +924,10 @@ bool fft3_applies(const dmr_plan *p)
 }
 
 // apodise + zero-pad + forward 3D FFT of `image` into `grid` (FFT order)
-int fft3_forward(const dmr_plan *p, const void *image, int image_real, int64_t batch, float2 *grid,
+int fft3_forward(const dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nframes, float2 *grid,
                  cudaStream_t st)
 {
-    const FftGeom g = make_geom(p, batch, 1.0f);
+    const FftGeom g = make_geom(p, batch, nframes, 1.0f);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
     for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
     if (g.nbf == 0) return DMR_OK;
@@ -938,9 +938,9 @@ int fft3_forward(const dmr_plan *p, const void *image, int image_real, int64_t b
 }
 
 // inverse 3D FFT of `grid` (FFT order, overwritten) + crop + 1/G + apodisation into `image`
-int fft3_adjoint(const dmr_plan *p, float2 *grid, int64_t batch, float2 *image, cudaStream_t st)
+int fft3_adjoint(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nframes, float2 *image, cudaStream_t st)
 {
-    const FftGeom g = make_geom(p, batch, (float)(1.0 / (double)p->g.gsize));
+    const FftGeom g = make_geom(p, batch, nframes, (float)(1.0 / (double)p->g.gsize));
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
     for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
     if (g.nbf == 0) return DMR_OK;
@@ -961,22 +961,22 @@ FftGeom il_cols(const FftGeom &g)
     return c;
 }
 
-FftGeom il_geom(const dmr_plan *p, int64_t batch, int64_t nchunks, int CS, float scale)
+FftGeom il_geom(const dmr_plan *p, int64_t batch, int64_t nframes, int64_t nchunks, int CS, float scale)
 {
-    FftGeom g = make_geom(p, nchunks, scale);  // nbf: (chunk, frame) sets
+    FftGeom g = make_geom(p, nchunks, nframes, scale);  // nbf: (chunk, frame) sets
     g.CS = CS;
-    g.nframes = p->g.nframes;
+    g.nframes = (int)nframes;
     g.batch = batch;
     return g;
 }
 
 }  // namespace
 
-int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nchunks, int CS,
-                    float2 *grid, cudaStream_t st)
+int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nframes,
+                    int64_t nchunks, int CS, float2 *grid, cudaStream_t st)
 {
-    if (CS == 1) return fft3_forward(p, image, image_real, batch, grid, st);  // the same layout
-    const FftGeom g = il_geom(p, batch, nchunks, CS, 1.0f), c = il_cols(g);
+    if (CS == 1) return fft3_forward(p, image, image_real, batch, nframes, grid, st);  // the same layout
+    const FftGeom g = il_geom(p, batch, nframes, nchunks, CS, 1.0f), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
     for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
     DMR_TRY(launch_rows<true>(g.G[0], false, g, tw[0], image, image_real, grid, st));
@@ -985,11 +985,11 @@ int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_
     return launch_cols(g.G[2], c, z_pass(c, false), tw[2], grid, st);
 }
 
-int fft3_adjoint_il(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nchunks, int CS, float2 *image,
-                    cudaStream_t st)
+int fft3_adjoint_il(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nframes, int64_t nchunks, int CS,
+                    float2 *image, cudaStream_t st)
 {
-    if (CS == 1) return fft3_adjoint(p, grid, batch, image, st);
-    const FftGeom g = il_geom(p, batch, nchunks, CS, (float)(1.0 / (double)p->g.gsize)), c = il_cols(g);
+    if (CS == 1) return fft3_adjoint(p, grid, batch, nframes, image, st);
+    const FftGeom g = il_geom(p, batch, nframes, nchunks, CS, (float)(1.0 / (double)p->g.gsize)), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
     for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
     if (g.G[2] > 1) DMR_TRY(launch_cols(g.G[2], c, z_pass(c, true), tw[2], grid, st));

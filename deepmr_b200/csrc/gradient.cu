@@ -15,47 +15,10 @@
 #include <cmath>
 
 #include "kb.cuh"
+#include "march.cuh"
 #include "plan.cuh"
 
 namespace dmr {
-
-// KB(u) and dKB/du of the A&S approximation used by the reference
-// (src/deepmr/fft/_interp/plan.py:216-248), differentiated term by term.
-__device__ __forceinline__ float kb_and_derivative(float u, float beta, float *dkb)
-{
-    if (fabsf(u) > 1.0f) {
-        *dkb = 0.0f;
-        return 0.0f;
-    }
-    const float s = fmaxf(1.0f - u * u, 0.0f);
-    const float a = beta * sqrtf(s);
-    float i0, di0_over_a;
-    if (a < 3.75f) {
-        const float t = a / 3.75f;
-        const float t2 = t * t;
-        i0 = 1.0f + t2 * (3.5156229f + t2 * (3.0899424f + t2 * (1.2067492f
-             + t2 * (0.2659732f + t2 * (0.0360768f + t2 * 0.0045813f)))));
-        // d/da sum c_k t^(2k) = sum 2k c_k t^(2k-1) / 3.75; divided by a = 3.75 t
-        const float p = 2.0f * 3.5156229f + t2 * (4.0f * 3.0899424f + t2 * (6.0f * 1.2067492f
-                        + t2 * (8.0f * 0.2659732f + t2 * (10.0f * 0.0360768f + t2 * 12.0f * 0.0045813f))));
-        di0_over_a = p / (3.75f * 3.75f);
-    } else {
-        const float v = 3.75f / a;
-        const float P = 0.39894228f + v * (0.01328592f + v * (0.00225319f + v * (-0.00157565f
-                        + v * (0.00916281f + v * (-0.02057706f + v * (0.02635537f
-                        + v * (-0.01647633f + v * 0.00392377f)))))));
-        const float dP = 0.01328592f + v * (2.0f * 0.00225319f + v * (3.0f * -0.00157565f
-                         + v * (4.0f * 0.00916281f + v * (5.0f * -0.02057706f + v * (6.0f * 0.02635537f
-                         + v * (7.0f * -0.01647633f + v * 8.0f * 0.00392377f))))));
-        const float e = expf(a) * rsqrtf(a);
-        i0 = P * e;
-        const float di0 = e * (P * (1.0f - 0.5f / a) - dP * 3.75f / (a * a));
-        di0_over_a = di0 / a;
-    }
-    // da/du = -beta^2 u / a
-    *dkb = -beta * beta * u * di0_over_a;
-    return i0;
-}
 
 // One warp per sample; lanes loop over coils. Grid in FFT order.
 template <int NDIM, int WMAX>
@@ -151,6 +114,8 @@ __global__ void traj_grad_kernel(Geom g, const float *__restrict__ sc0, const fl
 
 int forward_grid(dmr_plan *p, const void *image, int image_real, int64_t batch, void *workspace,
                  size_t workspace_bytes, cudaStream_t st, float2 **grid_out);
+int forward_grid_il(dmr_plan *p, const void *image, int image_real, int64_t batch, void *workspace,
+                    size_t workspace_bytes, cudaStream_t st, float2 **grid_out, float2 **il_out);
 
 }  // namespace dmr
 
@@ -168,6 +133,27 @@ extern "C" int dmr_nufft_traj_grad(dmr_plan *p, const void *image, int image_rea
     for (int a = 0; a < g.ndim; a++) wm = std::max(wm, g.W[a]);
     DMR_CHECK(wm <= 8, DMR_ERR_UNSUPPORTED, "trajectory gradient supports widths up to 8");
     float2 *grid = nullptr;
+    // 2D: the kernel of direct2d.cu on the interleaved grid (256^2, 12 coils,
+    // 205,824 samples: 69 us; the warp per sample on planar grids below took 406
+    // and needed the plan's bins, which a step with new coordinates builds anew).
+    // cuFFT lengths go a planar chunk at a time for the same reason (98..223
+    // points, 2 to 14 coils: 0.85 to 1.2 times the old step's speed before, 1.0
+    // to 2.1 now)
+    if (p->d2_W) {
+        const MarchChunks ch = march_chunks(p, batch);
+        float2 *il = nullptr;
+        DMR_TRY(forward_grid_il(p, image, image_real, batch, workspace, workspace_bytes, st, &grid, &il));
+        if (!il)
+            return d2_grad(p, grid, (const float2 *)v, 0, ch.n, ch.CS, batch, weight, weight_per_batch,
+                           (float)post_scale, grad, st);
+        for (int64_t b0 = 0; b0 < batch; b0 += ch.CS) {
+            DMR_TRY(march_interleave(p, grid + b0 * g.nframes * g.gsize, il, (int)std::min<int64_t>(ch.CS, batch - b0),
+                                     ch.CS, st));
+            DMR_TRY(d2_grad(p, il, (const float2 *)v, b0, 1, ch.CS, batch, weight, weight_per_batch, (float)post_scale,
+                            grad, st));
+        }
+        return DMR_OK;
+    }
     DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));
     if (g.total == 0) return DMR_OK;
     DMR_TRY(plan_bins(p, st));

@@ -45,6 +45,44 @@ __device__ __forceinline__ float kb_f32_select(float u, float beta)
     return fabsf(u) > 1.0f ? 0.0f : r;
 }
 
+// KB(u) and dKB/du of the A&S approximation used by the reference
+// (src/deepmr/fft/_interp/plan.py:216-248), differentiated term by term.
+__device__ __forceinline__ float kb_and_derivative(float u, float beta, float *dkb)
+{
+    if (fabsf(u) > 1.0f) {
+        *dkb = 0.0f;
+        return 0.0f;
+    }
+    const float s = fmaxf(1.0f - u * u, 0.0f);
+    const float a = beta * sqrtf(s);
+    float i0, di0_over_a;
+    if (a < 3.75f) {
+        const float t = a / 3.75f;
+        const float t2 = t * t;
+        i0 = 1.0f + t2 * (3.5156229f + t2 * (3.0899424f + t2 * (1.2067492f
+             + t2 * (0.2659732f + t2 * (0.0360768f + t2 * 0.0045813f)))));
+        // d/da sum c_k t^(2k) = sum 2k c_k t^(2k-1) / 3.75; divided by a = 3.75 t
+        const float p = 2.0f * 3.5156229f + t2 * (4.0f * 3.0899424f + t2 * (6.0f * 1.2067492f
+                        + t2 * (8.0f * 0.2659732f + t2 * (10.0f * 0.0360768f + t2 * 12.0f * 0.0045813f))));
+        di0_over_a = p / (3.75f * 3.75f);
+    } else {
+        const float v = 3.75f / a;
+        const float P = 0.39894228f + v * (0.01328592f + v * (0.00225319f + v * (-0.00157565f
+                        + v * (0.00916281f + v * (-0.02057706f + v * (0.02635537f
+                        + v * (-0.01647633f + v * 0.00392377f)))))));
+        const float dP = 0.01328592f + v * (2.0f * 0.00225319f + v * (3.0f * -0.00157565f
+                         + v * (4.0f * 0.00916281f + v * (5.0f * -0.02057706f + v * (6.0f * 0.02635537f
+                         + v * (7.0f * -0.01647633f + v * 8.0f * 0.00392377f))))));
+        const float e = expf(a) * rsqrtf(a);
+        i0 = P * e;
+        const float di0 = e * (P * (1.0f - 0.5f / a) - dP * 3.75f / (a * a));
+        di0_over_a = di0 / a;
+    }
+    // da/du = -beta^2 u / a
+    *dkb = -beta * beta * u * di0_over_a;
+    return i0;
+}
+
 inline double kb_f64(double u, double beta)
 {
     if (fabs(u) > 1.0) return 0.0;

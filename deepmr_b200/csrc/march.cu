@@ -1192,6 +1192,11 @@ static int transpose(const float2 *src, float2 *dst, int64_t npts, int cact, int
     return DMR_OK;
 }
 
+int march_interleave(const dmr_plan *p, const float2 *src, float2 *dst, int cact, int CS, cudaStream_t st)
+{
+    return transpose<false>(src, dst, (int64_t)p->g.nframes * p->g.gsize, cact, CS, st);
+}
+
 int march_interp(const dmr_plan *p, const float2 *grid, bool planar, float2 *ksp, int64_t batch, const float *weight,
                  int wpb, float2 *rows, float2 *il, cudaStream_t st)
 {

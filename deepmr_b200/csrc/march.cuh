@@ -41,6 +41,11 @@ int d2_interp(const ::dmr_plan *p, const float2 *grid, float2 *ksp, int64_t b0, 
 int d2_grid(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t b0, int64_t nch, int CS,
             int64_t batch, const float *weight, int wpb, cudaStream_t st);
 
+// trajectory gradient from `nch` chunks of the interleaved forward grid, the
+// first coil b0; calls with b0 > 0 add to the gradient of the coils before
+int d2_grad(const ::dmr_plan *p, const float2 *grid, const float2 *v, int64_t b0, int64_t nch, int CS, int64_t batch,
+            const float *weight, int wpb, float post, float *out, cudaStream_t st);
+
 MarchChunks march_chunks(const ::dmr_plan *p, int64_t batch);
 size_t march_rows_bytes(const ::dmr_plan *p, int CS);
 size_t march_il_bytes(const ::dmr_plan *p, int CS);
@@ -55,6 +60,8 @@ int march_interp(const ::dmr_plan *p, const float2 *grid, bool planar, float2 *k
                  int wpb, float2 *rows, float2 *il, cudaStream_t st);
 int march_grid(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool planar, int64_t batch,
                const float *weight, int wpb, int det, int64_t det_limit, float2 *rows, float2 *il, cudaStream_t st);
+// one chunk of a planar grid to interleaved
+int march_interleave(const ::dmr_plan *p, const float2 *src, float2 *dst, int cact, int CS, cudaStream_t st);
 // the same on planar grids with rows and il from the library pool
 int march_interp_pool(const ::dmr_plan *p, const float2 *grid, float2 *ksp, int64_t batch, const float *weight,
                       int wpb, cudaStream_t st);

@@ -352,7 +352,7 @@ int forward_grid(dmr_plan *p, const void *image, int image_real, int64_t batch, 
     NufftWs w;
     DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
     if (!w.fft) {
-        DMR_TRY(fft3_forward(p, image, image_real, batch, w.grid, st));
+        DMR_TRY(fft3_forward(p, image, image_real, batch, g.nframes, w.grid, st));
         *grid_out = w.grid;
         return DMR_OK;
     }
@@ -378,6 +378,20 @@ int forward_grid(dmr_plan *p, const void *image, int image_real, int64_t batch, 
     return DMR_OK;
 }
 
+// the grid of plans whose transforms run on interleaved grids: interleaved
+// (*il_out NULL), or planar where cuFFT computes it (*il_out: room for one
+// interleaved chunk)
+int forward_grid_il(dmr_plan *p, const void *image, int image_real, int64_t batch, void *workspace,
+                    size_t workspace_bytes, cudaStream_t st, float2 **grid_out, float2 **il_out)
+{
+    NufftWs w;
+    DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
+    *grid_out = w.grid;
+    *il_out = w.fft ? w.il : nullptr;
+    if (w.fft) return forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, grid_out);
+    return fft3_forward_il(p, image, image_real, batch, p->g.nframes, w.march.n, w.march.CS, w.grid, st);
+}
+
 }  // namespace dmr
 
 extern "C" int dmr_nufft_forward(dmr_plan *p, const void *image, int image_real, void *kspace,
@@ -391,7 +405,7 @@ extern "C" int dmr_nufft_forward(dmr_plan *p, const void *image, int image_real,
         NufftWs w;
         DMR_TRY(nufft_ws(p, batch, workspace, workspace_bytes, w, nullptr));
         if (w.fft) DMR_TRY(forward_grid(p, image, image_real, batch, workspace, workspace_bytes, st, &grid));
-        else DMR_TRY(fft3_forward_il(p, image, image_real, batch, w.march.n, w.march.CS, w.grid, st));
+        else DMR_TRY(fft3_forward_il(p, image, image_real, batch, p->g.nframes, w.march.n, w.march.CS, w.grid, st));
         return march_interp(p, w.grid, w.fft != nullptr, (float2 *)kspace, batch, weight, weight_per_batch, w.rows,
                             w.il, st);
     }
@@ -414,13 +428,13 @@ extern "C" int dmr_nufft_adjoint(dmr_plan *p, const void *kspace, int kspace_rea
         rc = march_grid(p, kspace, kspace_real, w.grid, w.fft != nullptr, batch, weight, weight_per_batch,
                         deterministic, det_scratch_limit(), w.rows, w.il, st);
         if (rc == DMR_OK && !w.fft)
-            return fft3_adjoint_il(p, w.grid, batch, w.march.n, w.march.CS, (float2 *)image, st);
+            return fft3_adjoint_il(p, w.grid, batch, g.nframes, w.march.n, w.march.CS, (float2 *)image, st);
     }
     if (rc == DMR_ERR_UNSUPPORTED)
         rc = grid_dispatch(p, kspace, kspace_real, w.grid, batch, weight, weight_per_batch, deterministic,
                            w.rt_scratch, w.rt_bytes, st);
     DMR_TRY(rc);
-    if (!w.fft) return fft3_adjoint(p, w.grid, batch, (float2 *)image, st);
+    if (!w.fft) return fft3_adjoint(p, w.grid, batch, g.nframes, (float2 *)image, st);
     DMR_TRY(fft_exec(*w.fft, w.grid, CUFFT_INVERSE, w.fft_work, st));
     ResizeArgs r;
     memset(&r, 0, sizeof(r));
@@ -466,63 +480,112 @@ namespace dmr {
 
 constexpr int kMaxCoeff = 32;
 
-// out[b, i, p] = sum_j M[i, j] in[b, j, p] with few inputs (nin <= kMaxCoeff):
-// a thread holds the nin input values of one grid point
-__global__ void __launch_bounds__(256) combine_few_in_kernel(const float2 *__restrict__ in, float2 *__restrict__ out,
-                                                            const float2 *__restrict__ M, int nin, int nout,
-                                                            int64_t npts, int64_t nbatch)
+// out[b, i, p] = sum_j M[i, j] in[b, j, p] with at most NC of the two counts
+// small: FEW_IN holds the nin input values of a point and writes nout sums,
+// otherwise a thread streams the inputs and keeps the nout sums. M sits in
+// shared memory; inputs are loaded eight at a time. NC is the small count
+// rounded up, so that no instruction is issued for coefficients that are not
+// there (a fixed bound of 32 made the sum of 120 frames instruction-bound:
+// 1.08 ms for 442 MB, 8 coils of 240^2).
+template <int NC, bool FEW_IN>
+__global__ void __launch_bounds__(256) combine_kernel(const float2 *__restrict__ in, float2 *__restrict__ out,
+                                                     const float2 *__restrict__ M, int nin, int nout, int64_t npts)
 {
-    for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
-        for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npts;
-             p += (int64_t)gridDim.x * blockDim.x) {
-            float2 v[kMaxCoeff];
+    extern __shared__ float2 sm[];  // M as [j][i < NC] (few outputs) or [i][j < NC] (few inputs), zero-padded
+    const int many = FEW_IN ? nout : nin;
+    for (int e = threadIdx.x; e < many * NC; e += 256) {
+        const int a = e / NC, k = e - a * NC;
+        float2 m = make_float2(0.0f, 0.0f);
+        if (FEW_IN ? k < nin : k < nout) m = FEW_IN ? M[(int64_t)a * nin + k] : M[(int64_t)k * nin + a];
+        sm[e] = m;
+    }
+    __syncthreads();
+    in += (int64_t)blockIdx.y * nin * npts;
+    out += (int64_t)blockIdx.y * nout * npts;
+    for (int64_t p = blockIdx.x * (int64_t)256 + threadIdx.x; p < npts; p += (int64_t)gridDim.x * 256) {
+        float2 r[NC];
+        if (FEW_IN) {
 #pragma unroll
-            for (int j = 0; j < kMaxCoeff; j++)
-                v[j] = j < nin ? in[(b * nin + j) * npts + p] : make_float2(0.0f, 0.0f);
-            for (int i = 0; i < nout; i++) {
+            for (int k = 0; k < NC; k++) r[k] = k < nin ? in[k * npts + p] : make_float2(0.0f, 0.0f);
+            for (int a = 0; a < nout; a++) {
                 float2 acc = make_float2(0.0f, 0.0f);
 #pragma unroll
-                for (int j = 0; j < kMaxCoeff; j++) {
-                    if (j < nin) {
-                        const float2 m = __ldg(M + (int64_t)i * nin + j);
-                        acc.x += m.x * v[j].x - m.y * v[j].y;
-                        acc.y += m.x * v[j].y + m.y * v[j].x;
+                for (int k = 0; k < NC; k++) {
+                    if (k >= nin) break;
+                    const float2 m = sm[a * NC + k];
+                    acc.x += m.x * r[k].x - m.y * r[k].y;
+                    acc.y += m.x * r[k].y + m.y * r[k].x;
+                }
+                out[a * npts + p] = acc;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < NC; k++) r[k] = make_float2(0.0f, 0.0f);
+            constexpr int U = 8;
+            for (int a = 0; a < nin; a += U) {
+                float2 v[U];
+#pragma unroll
+                for (int u = 0; u < U; u++)
+                    if (a + u < nin) v[u] = __ldcs(in + (a + u) * npts + p);
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (a + u >= nin) break;
+#pragma unroll
+                    for (int k = 0; k < NC; k++) {
+                        const float2 m = sm[(a + u) * NC + k];
+                        r[k].x += m.x * v[u].x - m.y * v[u].y;
+                        r[k].y += m.x * v[u].y + m.y * v[u].x;
                     }
                 }
-                out[(b * nout + i) * npts + p] = acc;
             }
+#pragma unroll
+            for (int k = 0; k < NC; k++)
+                if (k < nout) out[k * npts + p] = r[k];
         }
     }
 }
 
-// the same with few outputs (nout <= kMaxCoeff): a thread streams the inputs
-// of one grid point and keeps the nout sums
-__global__ void __launch_bounds__(256) combine_few_out_kernel(const float2 *__restrict__ in, float2 *__restrict__ out,
-                                                             const float2 *__restrict__ M, int nin, int nout,
-                                                             int64_t npts, int64_t nbatch)
+template <bool FEW_IN>
+static int launch_combine_t(const float2 *in, float2 *out, const float2 *M, int nin, int nout, int64_t npts,
+                            int64_t nbatch, cudaStream_t st)
 {
-    for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y) {
-        for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npts;
-             p += (int64_t)gridDim.x * blockDim.x) {
-            float2 acc[kMaxCoeff];
-#pragma unroll
-            for (int i = 0; i < kMaxCoeff; i++) acc[i] = make_float2(0.0f, 0.0f);
-            for (int j = 0; j < nin; j++) {
-                const float2 v = in[(b * nin + j) * npts + p];
-#pragma unroll
-                for (int i = 0; i < kMaxCoeff; i++) {
-                    if (i < nout) {
-                        const float2 m = __ldg(M + (int64_t)i * nin + j);
-                        acc[i].x += m.x * v.x - m.y * v.y;
-                        acc[i].y += m.x * v.y + m.y * v.x;
-                    }
-                }
-            }
-#pragma unroll
-            for (int i = 0; i < kMaxCoeff; i++)
-                if (i < nout) out[(b * nout + i) * npts + p] = acc[i];
-        }
+    const int few = FEW_IN ? nin : nout, many = FEW_IN ? nout : nin;
+    const int NC = few <= 4 ? 4 : (few <= 8 ? 8 : (few <= 16 ? 16 : 32));
+    const size_t smem = (size_t)many * NC * sizeof(float2);
+    int dev = 0, limit = 0;
+    DMR_CUDA(cudaGetDevice(&dev));
+    DMR_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    if (smem > (size_t)limit) return DMR_ERR_UNSUPPORTED;
+    const auto kern = NC == 4 ? combine_kernel<4, FEW_IN>
+                              : (NC == 8 ? combine_kernel<8, FEW_IN>
+                                         : (NC == 16 ? combine_kernel<16, FEW_IN> : combine_kernel<32, FEW_IN>));
+    DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (int64_t b = 0; b < nbatch; b += 65535) {
+        const unsigned gy = (unsigned)std::min<int64_t>(nbatch - b, 65535);
+        const unsigned gx = (unsigned)std::max<int64_t>(1, std::min<int64_t>(ceil_div(npts, 256), 65535 * 16));
+        kern<<<dim3(gx, gy), 256, smem, st>>>(in + b * nin * npts, out + b * nout * npts, M, nin, nout, npts);
+        DMR_LAUNCHED("combine_kernel");
     }
+    return DMR_OK;
+}
+
+// frames that do not fit in shared memory (more than 900 for 32 coefficients)
+__global__ void __launch_bounds__(256) combine_long_kernel(const float2 *__restrict__ in, float2 *__restrict__ out,
+                                                          const float2 *__restrict__ M, int nin, int nout, int64_t npts,
+                                                          int64_t nbatch)
+{
+    for (int64_t b = blockIdx.y; b < nbatch; b += gridDim.y)
+        for (int64_t e = blockIdx.x * (int64_t)256 + threadIdx.x; e < npts * nout; e += (int64_t)gridDim.x * 256) {
+            const int i = (int)(e / npts);
+            const int64_t p = e - i * npts;
+            float2 acc = make_float2(0.0f, 0.0f);
+            for (int j = 0; j < nin; j++) {
+                const float2 m = __ldg(M + (int64_t)i * nin + j), v = in[(b * nin + j) * npts + p];
+                acc.x += m.x * v.x - m.y * v.y;
+                acc.y += m.x * v.y + m.y * v.x;
+            }
+            out[(b * nout + i) * npts + p] = acc;
+        }
 }
 
 static int launch_combine(const float2 *in, float2 *out, const float2 *M, int nin, int nout, int64_t npts,
@@ -530,17 +593,14 @@ static int launch_combine(const float2 *in, float2 *out, const float2 *M, int ni
 {
     DMR_CHECK(nin <= kMaxCoeff || nout <= kMaxCoeff, DMR_ERR_UNSUPPORTED,
               "subspace projection with more than %d coefficients", kMaxCoeff);
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int rc = nin <= kMaxCoeff && (nin <= nout || nout > kMaxCoeff)
+                       ? launch_combine_t<true>(in, out, M, nin, nout, npts, nbatch, st)
+                       : launch_combine_t<false>(in, out, M, nin, nout, npts, nbatch, st);
+    if (rc != DMR_ERR_UNSUPPORTED) return rc;
     const unsigned gy = (unsigned)std::min<int64_t>(nbatch, 65535);
-    const unsigned gx = (unsigned)std::max<int64_t>(
-        1, std::min<int64_t>(ceil_div(npts, 256), ceil_div((int64_t)sms * 8, gy)));
-    if (nin <= kMaxCoeff && (nin <= nout || nout > kMaxCoeff))
-        combine_few_in_kernel<<<dim3(gx, gy), 256, 0, st>>>(in, out, M, nin, nout, npts, nbatch);
-    else
-        combine_few_out_kernel<<<dim3(gx, gy), 256, 0, st>>>(in, out, M, nin, nout, npts, nbatch);
-    DMR_LAUNCHED("combine_kernel");
+    combine_long_kernel<<<dim3((unsigned)std::min<int64_t>(ceil_div(npts * nout, 256), 148 * 16), gy), 256, 0, st>>>(
+        in, out, M, nin, nout, npts, nbatch);
+    DMR_LAUNCHED("combine_long_kernel");
     return DMR_OK;
 }
 
@@ -551,6 +611,11 @@ struct LowrankWs {
     void *rt_scratch;
     size_t rt_bytes;
     std::shared_ptr<FftPlan> fft;
+    // interleaved buffers, in the same workspace (used instead of the planar
+    // ones, never with them): coefficient and frame grids, rows of one chunk
+    bool il = false;
+    MarchChunks march;
+    float2 *il_coef, *il_frame, *rows;
 };
 
 static int lowrank_ws(dmr_plan *p, int64_t batch, int64_t ncoeff, void *ws, size_t ws_bytes, LowrankWs &out,
@@ -568,7 +633,16 @@ static int lowrank_ws(dmr_plan *p, int64_t batch, int64_t ncoeff, void *ws, size
     const size_t frame_bytes = align_up((size_t)batch * g.nframes * g.gsize * sizeof(float2), 256);
     const size_t fft_bytes = align_up(fp->work_bytes, 256);
     const size_t rt_bytes = align_up(grid_scratch_bytes(p, batch), 256);
-    const size_t total = coef_bytes + frame_bytes + fft_bytes + rt_bytes;
+    size_t total = coef_bytes + frame_bytes + fft_bytes + rt_bytes;
+    size_t ic = 0, ifr = 0;
+    out.il = p->il_forward() && fft3_applies(p);
+    if (out.il) {
+        out.march = march_chunks(p, batch);
+        const size_t slot = (size_t)out.march.n * out.march.CS * g.gsize * sizeof(float2);
+        ic = align_up(slot * ncoeff, 256);
+        ifr = align_up(slot * g.nframes, 256);
+        total = std::max(total, ic + ifr + march_rows_bytes(p, out.march.CS));
+    }
     if (need) *need = total;
     if (!ws) return DMR_OK;
     DMR_CHECK(ws_bytes >= total, DMR_ERR_WORKSPACE, "workspace too small: %zu < %zu", ws_bytes, total);
@@ -580,6 +654,9 @@ static int lowrank_ws(dmr_plan *p, int64_t batch, int64_t ncoeff, void *ws, size
     out.rt_scratch = rt_bytes ? c + coef_bytes + frame_bytes + fft_bytes : nullptr;
     out.rt_bytes = rt_bytes;
     out.fft = fp;
+    out.il_coef = (float2 *)c;
+    out.il_frame = (float2 *)(c + ic);
+    out.rows = (float2 *)(c + ic + ifr);
     return DMR_OK;
 }
 
@@ -602,6 +679,14 @@ extern "C" int dmr_nufft_forward_lowrank(dmr_plan *p, const void *image, int ima
     const Geom &g = p->g;
     LowrankWs w;
     DMR_TRY(lowrank_ws(p, batch, ncoeff, workspace, workspace_bytes, w, nullptr));
+    if (w.il) {
+        // on interleaved grids, points and coils of a frame are one axis
+        const int64_t n = g.gsize * w.march.CS;
+        DMR_TRY(fft3_forward_il(p, image, image_real, batch, ncoeff, w.march.n, w.march.CS, w.il_coef, st));
+        DMR_TRY(launch_combine(w.il_coef, w.il_frame, (const float2 *)basis_adjoint, (int)ncoeff, g.nframes, n,
+                               w.march.n, st));
+        return march_interp(p, w.il_frame, false, (float2 *)kspace, batch, weight, weight_per_batch, w.rows, nullptr, st);
+    }
     ResizeArgs r;
     memset(&r, 0, sizeof(r));
     for (int a = 0; a < 3; a++) {
@@ -635,6 +720,16 @@ extern "C" int dmr_nufft_adjoint_lowrank(dmr_plan *p, const void *kspace, int ks
     const Geom &g = p->g;
     LowrankWs w;
     DMR_TRY(lowrank_ws(p, batch, ncoeff, workspace, workspace_bytes, w, nullptr));
+    if (w.il && grid_march_applies(p, batch, deterministic)) {
+        const int rc = march_grid(p, kspace, kspace_real, w.il_frame, false, batch, weight, weight_per_batch,
+                                  deterministic, det_scratch_limit(), w.rows, nullptr, st);
+        if (rc == DMR_OK) {
+            DMR_TRY(launch_combine(w.il_frame, w.il_coef, (const float2 *)basis, g.nframes, (int)ncoeff,
+                                   g.gsize * w.march.CS, w.march.n, st));
+            return fft3_adjoint_il(p, w.il_coef, batch, ncoeff, w.march.n, w.march.CS, (float2 *)image, st);
+        }
+        if (rc != DMR_ERR_UNSUPPORTED) return rc;
+    }
     DMR_TRY(grid_dispatch(p, kspace, kspace_real, w.frame, batch, weight, weight_per_batch, deterministic,
                           w.rt_scratch, w.rt_bytes, st));
     DMR_TRY(launch_combine(w.frame, w.coef, (const float2 *)basis, g.nframes, (int)ncoeff, g.gsize, batch, st));

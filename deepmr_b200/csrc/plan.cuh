@@ -117,15 +117,17 @@ cudaMemPool_t scratch_pool(int dev);
 // (apodise + pad + FFT into the grid) and the adjoint (inverse FFT of the grid,
 // which it overwrites, + crop + 1/G + apodisation into the image)
 bool fft3_applies(const ::dmr_plan *p);
-int fft3_forward(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, float2 *grid,
+// nframes: grids per batch element (the plan's frames, or the coefficients of a
+// subspace transform)
+int fft3_forward(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nframes, float2 *grid,
                  cudaStream_t st);
-int fft3_adjoint(const ::dmr_plan *p, float2 *grid, int64_t batch, float2 *image, cudaStream_t st);
+int fft3_adjoint(const ::dmr_plan *p, float2 *grid, int64_t batch, int64_t nframes, float2 *image, cudaStream_t st);
 // the same with the coil-interleaved grid of march.cuh: nchunks chunks of CS
 // coils, (chunk, frame, z, y, x, coil)
-int fft3_forward_il(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nchunks, int CS,
-                    float2 *grid, cudaStream_t st);
-int fft3_adjoint_il(const ::dmr_plan *p, float2 *grid, int64_t batch, int64_t nchunks, int CS, float2 *image,
-                    cudaStream_t st);
+int fft3_forward_il(const ::dmr_plan *p, const void *image, int image_real, int64_t batch, int64_t nframes,
+                    int64_t nchunks, int CS, float2 *grid, cudaStream_t st);
+int fft3_adjoint_il(const ::dmr_plan *p, float2 *grid, int64_t batch, int64_t nframes, int64_t nchunks, int CS,
+                    float2 *image, cudaStream_t st);
 // the same passes for the 3D Toeplitz self-adjoint: whether they apply
 // (kernel extents at least the image's and with a compiled transform), and
 // pad + FFT + kernel multiply + inverse FFT + crop (data: batch kernel grids)

@@ -164,3 +164,66 @@ def test_2d_vs_oracle(shape, width, os, nsamples):
                 F.set_deterministic_gridding(old)
             assert rel(x, x_ref[:k]) < TOL, (k, det)
             assert not det or torch.equal(x, x2), k
+
+
+@pytest.mark.parametrize("width,os,shape,coils", [(4, 1.25, (24, 32), (1, 5, 12, 35)), (3, 2.0, (16, 20), (2, 17)),
+                                                  (6, 2.0, (11, 13), (1, 34)), (2, 1.5, (18, 9), (3, 33))])
+def test_2d_trajectory_gradient_frames_weights(width, os, shape, coils):
+    """The 2D gradient kernel around its lane groups and coil chunks, on fused
+    FFT lengths (interleaved grids) and cuFFT ones (a planar chunk at a time),
+    against central differences of the float64 operator.
+
+    Tolerance 2e-5 of the gradient's norm: the rescaled coordinate is a float32
+    up to 48 (rounding 2e-6, times the second derivative, about the first's
+    size) and the differences add 1e-8 (step squared) + 1e-9 (1e-13 / step)."""
+    import deepmr_b200.fft as F
+    from oracle import nufft_ref as R
+
+    nf, npts, most, eps = 2, 30, max(coils), 1e-4
+    rng = np.random.default_rng(7)
+    n = np.asarray(shape[::-1], dtype=np.float64)
+    grid = np.ceil(os * n)
+    # samples off the points where the tap set changes
+    t = rng.integers(1, grid - 2, (nf, npts, 2)) + (0.5 if width % 2 else 0.0) + rng.uniform(0.05, 0.95, (nf, npts, 2))
+    c = ((t - grid // 2) * n / grid).astype(np.float32)
+    plan = F.plan_nufft(torch.as_tensor(c[:, None]), shape, width, os, device="cuda")
+    gen = torch.Generator().manual_seed(8)
+    cplx = lambda *s: torch.complex(torch.randn(s, generator=gen), torch.randn(s, generator=gen))  # noqa: E731
+    img, v, w = cplx(most, nf, *shape), cplx(most, nf, 1, npts), torch.rand(nf, 1, npts, generator=gen)
+    per_coil = np.zeros((most, nf, npts, 2))  # Re(conj(v) w dy/dc)
+    for f in range(nf):
+        f64 = R.Forward64(img[:, f].numpy(), c[f][None], shape, width, os)
+        for p in range(npts):
+            for a in range(2):
+                d = np.zeros(2)
+                d[a] = eps
+                x = c[f, p].astype(np.float64)
+                dy = (f64.sample(x + d) - f64.sample(x - d)) / (2 * eps)
+                per_coil[:, f, p, a] = np.real(np.conj(v[:, f, 0, p].numpy()) * dy) * float(w[f, 0, p])
+    for k in coils:
+        got = F.traj_grad(plan, img[:k].cuda(), v[:k].cuda(), weight=w.cuda(), post_scale=0.5)
+        assert rel(got.reshape(nf, npts, 2), 0.5 * per_coil[:k].sum(0)) < 2e-5, k
+
+
+@pytest.mark.parametrize("ndim,shape,nf,ncoeff,coils", [(2, (24, 32), 40, 9, 5), (2, (24, 32), 3, 7, 33),
+                                                        (3, (16, 12, 20), 5, 17, 2), (2, (16, 16), 950, 20, 1)])
+def test_lowrank_coefficient_counts(ndim, shape, nf, ncoeff, coils):
+    """The projection's rounded coefficient counts (4, 8, 16, 32), more
+    coefficients than frames, two coil chunks, and a basis that is larger than
+    shared memory (950 frames of 20 coefficients), on interleaved grids."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+    from oracle import nufft_ref as R
+
+    rng = np.random.default_rng(9)
+    c = torch.as_tensor((rng.uniform(-0.49, 0.49, (nf, 1, 60, ndim)) * np.asarray(shape[::-1])).astype(np.float32))
+    gen = torch.Generator().manual_seed(10)
+    basis = torch.complex(torch.randn(ncoeff, nf, generator=gen), torch.randn(ncoeff, nf, generator=gen))
+    img = synth.complex_gaussian((coils, ncoeff) + shape, seed=1)
+    ksp = synth.complex_gaussian((coils, nf, 1, 60), seed=2)
+    plan = F.plan_nufft(c, shape, 4, 1.25, device="cuda")
+    oplan = R.plan_nufft(c, shape, 4, 1.25)
+    y = F.apply_nufft(img.cuda(), plan, basis_adjoint=basis.conj().t())
+    assert rel(y, R.apply_nufft_lowrank(img, oplan, basis.conj().t())) < TOL
+    x = F.apply_nufft_adj(ksp.cuda(), plan, basis=basis)
+    assert rel(x, R.apply_nufft_adj_lowrank(ksp, oplan, basis)) < TOL
