@@ -19,16 +19,30 @@
 // With G = 1.25 N that is 15.5 GB of DRAM traffic per 240^3 x 32 transform
 // against 26.6 GB for a full-grid pad kernel plus three full passes.
 //
-// Each block transforms 16 lines at once in one shared-memory buffer
-// ([position][line], line pitch 17 so that 8-byte accesses of a half-warp hit
-// distinct banks): a Stockham autosort FFT (Govindaraju et al., "High performance discrete
-// Fourier transforms on graphics processors", SC 2008) with radix-4, 2, 3 and
-// 5 stages, twiddles from a per-length table computed in double precision on
-// the host.
+// Each block transforms 16 lines in two steps (the four-step form of the
+// Cooley-Tukey algorithm, L = L1 L2): a thread takes L1 points of a line
+// straight from global memory into registers, transforms and twiddles them,
+// one exchange through shared memory, and L2 points per thread go from
+// registers to global memory. Nothing is staged in shared memory before or
+// after: with 16 lines of 8 bytes next to each other (columns, interleaved
+// rows) a half-warp reads and writes 128 contiguous bytes, along image rows
+// neighbouring threads take neighbouring points.
+// What bounds these passes is DRAM, once there are few instructions and enough
+// warps: 500 x 16 images of 224^2 to 280^2 and back take 1.53 + 1.60 ms and
+// 1.55 + 1.40 ms, 4.7 to 5.6 TB/s; 192^3 x 32 coils 0.80 + 2.25 and 2.22 + 0.76.
+// Tiles staged by asynchronous copies, roots of unity read from shared memory and
+// a run-time direction took 93 instructions per point (now about 55) at 18 warps
+// per SM: 2.44 + 2.08, 2.11 + 2.12, and 1.23 + 2.56, 2.52 + 1.07. So constants are
+// immediates, co-prime factors of a register transform need no twiddles (Good, "The interaction
+// algorithm and practical Fourier analysis", 1958), the direction is a template
+// argument, and the twiddles between the steps are stored in the order in which
+// they are used, in double precision rounded once.
 #include <algorithm>
 #include <cmath>
 #include <map>
 #include <mutex>
+#include <tuple>
+#include <utility>
 #include <vector>
 
 #include "plan.cuh"
@@ -37,24 +51,9 @@ namespace dmr {
 
 namespace {
 
-#ifndef DMR_FFT_LINES
-#define DMR_FFT_LINES 16
-#endif
-// resident blocks per SM the compiler plans registers for: the row and column
-// passes of blocks of at most 256 threads at 3 (about 80 registers; 39.5 vs
-// 39.9 ms per 240^3 x 32 forward + adjoint pair at 2), larger blocks (a factor
-// above 16: 320 or 384 threads) at 2, where 3 would cap them at 56-64
-// registers and spill; the fused Toeplitz z pass at 2 (its forward transform,
-// kernel multiply and inverse transform need the registers)
-#ifndef DMR_FFT_MINB
-#define DMR_FFT_MINB 3
-#endif
-#ifndef DMR_FFT_TOEP_MINB
-#define DMR_FFT_TOEP_MINB 2
-#endif
-constexpr int kFftLines = DMR_FFT_LINES;  // lines per block (16 or 32)
-constexpr int kFftLP = kFftLines + 2;     // shared-memory pitch of a position (16-byte rows)
-constexpr int kFftShift = kFftLines == 32 ? 5 : 4;
+// lines per block: 8 are as fast on small grids, but their 64-byte pieces cost a
+// quarter on large ones (192^3, 32 coils, columns: 2.27 ms with 16, 2.96 with 8)
+constexpr int kFftLines = 16;
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b)
 {
@@ -64,218 +63,224 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b)
 // complex add / subtract as packed FP32 (one instruction each)
 __device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
-
-// R-point DFT of v in place, V[m] = sum_q v[q] w^(q m), w = exp(-+2 pi i / R),
-// for R = 2, 4 (no multiplications), 3 and 5 (roots of unity from the table
-// of the transform length L)
-template <int R, int L>
-__device__ __forceinline__ void small_dft(float2 *v, const float2 *tw, bool inv)
+// a + s b and s b for a real constant s
+__device__ __forceinline__ float2 axpy(float s, float2 b, float2 a)
 {
-    if constexpr (R == 2) {
+    return make_float2(fmaf(s, b.x, a.x), fmaf(s, b.y, a.y));
+}
+__device__ __forceinline__ float2 scl(float s, float2 b) { return make_float2(s * b.x, s * b.y); }
+
+// cos and sin of 2 pi t / n at compile time: the angle is brought to [0, pi/4]
+// exactly (in eighths of a turn), then the power series in double precision
+constexpr double series(double x, bool odd)
+{
+    double term = odd ? x : 1.0, sum = term;
+    for (int k = odd ? 3 : 2; k < 26; k += 2) {
+        term *= -x * x / ((double)k * (k - 1));
+        sum += term;
+    }
+    return sum;
+}
+constexpr double cos_turn(int t, int n)  // 0 <= t < n
+{
+    if (2 * t > n) t = n - t;                              // cos(2 pi - a)
+    if (4 * t > n) return -cos_turn(n - 2 * t, 2 * n);     // -cos(pi - a)
+    const double x = 6.283185307179586476925286766559 / n;
+    // above an eighth of a turn: sin(pi/2 - a), the complement as an exact fraction
+    return 8 * t > n ? series((n - 4 * t) * (x / 4), true) : series(t * x, false);
+}
+constexpr double sin_turn(int t, int n)
+{
+    // sin a = cos(a - quarter turn), in quarters of 1/n
+    int q = (4 * t - n) % (4 * n);
+    if (q < 0) q += 4 * n;
+    return cos_turn(q, 4 * n);
+}
+// exp(-+2 pi i t / n): forward (INV false) and inverse
+template <int T, int N, bool INV>
+struct Root {
+    static constexpr float re = (float)cos_turn(T % N, N);
+    static constexpr float im = (float)(INV ? sin_turn(T % N, N) : -sin_turn(T % N, N));
+};
+// v times exp(-+2 pi i T / N), without arithmetic for quarter turns
+template <int T, int N, bool INV>
+__device__ __forceinline__ float2 rot(float2 v)
+{
+    if constexpr (T % N == 0) {
+        return v;
+    } else if constexpr (4 * (T % N) == N) {
+        return INV ? make_float2(-v.y, v.x) : make_float2(v.y, -v.x);
+    } else if constexpr (2 * (T % N) == N) {
+        return make_float2(-v.x, -v.y);
+    } else if constexpr (4 * (T % N) == 3 * N) {
+        return INV ? make_float2(v.y, -v.x) : make_float2(-v.y, v.x);
+    } else {
+        constexpr float c = Root<T, N, INV>::re, s = Root<T, N, INV>::im;
+        return make_float2(v.x * c - v.y * s, v.x * s + v.y * c);
+    }
+}
+
+template <int... I, class Fn>
+__device__ __forceinline__ void unroll_seq(std::integer_sequence<int, I...>, Fn &&fn)
+{
+    (fn(std::integral_constant<int, I>{}), ...);
+}
+template <int N, class Fn>
+__device__ __forceinline__ void unroll(Fn &&fn)
+{
+    unroll_seq(std::make_integer_sequence<int, N>{}, fn);
+}
+
+// factors of a register transform: co-prime where there are any
+template <int M>
+struct Split {
+    static constexpr int pow2 = M % 32 == 0 ? 32 : (M % 16 == 0 ? 16 : (M % 8 == 0 ? 8 : (M % 4 == 0 ? 4 : (M % 2 == 0 ? 2 : 1))));
+    static constexpr int odd = M / pow2;
+    static constexpr int A = odd > 1 && pow2 > 1 ? pow2 : (odd == 1 ? (M == 8 ? 2 : 4) : (M % 3 == 0 ? 3 : 5));
+    static constexpr int B = M / A;
+    static constexpr bool coprime = A % 2 != B % 2 && !(A % 3 == 0 && B % 3 == 0) && !(A % 5 == 0 && B % 5 == 0) ||
+                                    (A == 3 && B % 3 != 0) || (A == 5 && B % 5 != 0);
+};
+
+// M-point DFT of registers v, natural order in and out. Odd prime lengths R:
+// with a_k = v_k + v_(R-k), b_k = v_k - v_(R-k),
+//   V_m, V_(R-m) = v0 + sum_k cos(k m) a_k -+ i sum_k sin(k m) b_k.
+// M = A B co-prime: n = B n1 + A n2 and k = (k mod A, k mod B) separate the two
+// (no twiddles); otherwise n = B n1 + n2, k = k1 + A k2 with twiddles w_M^(n2 k1).
+// Every index is a compile-time constant once unrolled.
+template <int M, bool INV>
+__device__ __forceinline__ void reg_dft(float2 *v)
+{
+    if constexpr (M == 2) {
         const float2 a = v[0], b = v[1];
         v[0] = cadd(a, b);
         v[1] = csub(a, b);
-    } else if constexpr (R == 4) {
+    } else if constexpr (M == 4) {
         const float2 s02 = cadd(v[0], v[2]), d02 = csub(v[0], v[2]);
-        const float2 s13 = cadd(v[1], v[3]), d13 = csub(v[1], v[3]);
-        // w d13 with w = -i (forward) or +i (inverse)
-        const float2 jd = inv ? make_float2(-d13.y, d13.x) : make_float2(d13.y, -d13.x);
+        const float2 s13 = cadd(v[1], v[3]), jd = rot<1, 4, INV>(csub(v[1], v[3]));
         v[0] = cadd(s02, s13);
         v[1] = cadd(d02, jd);
         v[2] = csub(s02, s13);
         v[3] = csub(d02, jd);
-    } else if constexpr (R == 3) {
-        // w^2 = conj(w): V1,2 = v0 + Re(w) (v1 + v2) +- i Im(w) (v1 - v2)
-        float2 w = tw[L / 3];
-        if (inv) w.y = -w.y;
-        const float2 a = make_float2(v[1].x + v[2].x, v[1].y + v[2].y);
-        const float2 b = make_float2(v[1].x - v[2].x, v[1].y - v[2].y);
-        const float2 m = make_float2(v[0].x + w.x * a.x, v[0].y + w.x * a.y);
-        const float2 ib = make_float2(-w.y * b.y, w.y * b.x);
-        v[0] = make_float2(v[0].x + a.x, v[0].y + a.y);
-        v[1] = make_float2(m.x + ib.x, m.y + ib.y);
-        v[2] = make_float2(m.x - ib.x, m.y - ib.y);
-    } else if constexpr (R == 7) {
-        // odd R: w^(R-j) = conj(w^j); a_k = v_k + v_(R-k), b_k = v_k - v_(R-k):
-        // V_m, V_(R-m) = v0 + sum_k Re(w^(k m)) a_k +- i sum_k Im(w^(k m)) b_k
-        constexpr int H = R / 2;
-        float2 w[H + 1];
-#pragma unroll
-        for (int j = 1; j <= H; j++) {
-            w[j] = tw[j * (L / R)];
-            if (inv) w[j].y = -w[j].y;
-        }
+    } else if constexpr (M == 3 || M == 5 || M == 7) {
+        constexpr int H = M / 2;
         float2 a[H + 1], b[H + 1];
+        const float2 v0 = v[0];
 #pragma unroll
         for (int k = 1; k <= H; k++) {
-            a[k] = cadd(v[k], v[R - k]);
-            b[k] = csub(v[k], v[R - k]);
+            a[k] = cadd(v[k], v[M - k]);
+            b[k] = csub(v[k], v[M - k]);
+            v[0] = cadd(v[0], a[k]);
         }
-        float2 o[R];
-        o[0] = v[0];
-#pragma unroll
-        for (int k = 1; k <= H; k++) o[0] = cadd(o[0], a[k]);
-#pragma unroll
-        for (int m = 1; m <= H; m++) {
-            float2 re = v[0], im = make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int k = 1; k <= H; k++) {
-                const int j = (k * m) % R;
-                const float c = j <= H ? w[j].x : w[R - j].x;
-                const float sn = j <= H ? w[j].y : -w[R - j].y;
-                re = make_float2(re.x + c * a[k].x, re.y + c * a[k].y);
-                im = make_float2(im.x + sn * b[k].x, im.y + sn * b[k].y);
-            }
-            // i * im = (-im.y, im.x)
-            o[m] = make_float2(re.x - im.y, re.y + im.x);
-            o[R - m] = make_float2(re.x + im.y, re.y - im.x);
-        }
-#pragma unroll
-        for (int m = 0; m < R; m++) v[m] = o[m];
-    } else {
-        static_assert(R == 5, "radix");
-        // w^4 = conj(w), w^3 = conj(w^2); a1 = v1 + v4, b1 = v1 - v4,
-        // a2 = v2 + v3, b2 = v2 - v3:
-        // V1,4 = v0 + Re(w) a1 + Re(w2) a2 +- i (Im(w) b1 + Im(w2) b2)
-        // V2,3 = v0 + Re(w2) a1 + Re(w) a2 +- i (Im(w2) b1 - Im(w) b2)
-        float2 w1 = tw[L / 5], w2 = tw[2 * (L / 5)];
-        if (inv) {
-            w1.y = -w1.y;
-            w2.y = -w2.y;
-        }
-        const float2 a1 = make_float2(v[1].x + v[4].x, v[1].y + v[4].y);
-        const float2 b1 = make_float2(v[1].x - v[4].x, v[1].y - v[4].y);
-        const float2 a2 = make_float2(v[2].x + v[3].x, v[2].y + v[3].y);
-        const float2 b2 = make_float2(v[2].x - v[3].x, v[2].y - v[3].y);
-        const float2 m1 = make_float2(v[0].x + w1.x * a1.x + w2.x * a2.x, v[0].y + w1.x * a1.y + w2.x * a2.y);
-        const float2 m2 = make_float2(v[0].x + w2.x * a1.x + w1.x * a2.x, v[0].y + w2.x * a1.y + w1.x * a2.y);
-        const float2 s1 = make_float2(w1.y * b1.x + w2.y * b2.x, w1.y * b1.y + w2.y * b2.y);
-        const float2 s2 = make_float2(w2.y * b1.x - w1.y * b2.x, w2.y * b1.y - w1.y * b2.y);
-        v[0] = make_float2(v[0].x + a1.x + a2.x, v[0].y + a1.y + a2.y);
-        v[1] = make_float2(m1.x - s1.y, m1.y + s1.x);
-        v[4] = make_float2(m1.x + s1.y, m1.y - s1.x);
-        v[2] = make_float2(m2.x - s2.y, m2.y + s2.x);
-        v[3] = make_float2(m2.x + s2.y, m2.y - s2.x);
-    }
-}
-
-template <int M>
-struct Split {
-    static constexpr int A = M % 4 == 0 ? 4 : (M % 2 == 0 ? 2 : (M % 3 == 0 ? 3 : (M % 5 == 0 ? 5 : 7)));
-    static constexpr int B = M / A;
-};
-
-// M-point DFT of registers v (M divides L), natural order in and out: radix
-// 2 / 3 / 4 / 5 directly, else M = A B in registers (index n = B n1 + n2):
-// A-point DFTs over n1, twiddles w_M^(n2 k1), B-point DFTs over n2, output
-// k1 + A k2. Every index is a compile-time constant once unrolled.
-template <int M, int L>
-__device__ __forceinline__ void reg_dft(float2 *v, const float2 *tw, bool inv)
-{
-    if constexpr (M == 2 || M == 3 || M == 4 || M == 5 || M == 7) {
-        small_dft<M, L>(v, tw, inv);
+        unroll<H>([&](auto mi) {
+            constexpr int m = decltype(mi)::value + 1;
+            float2 re = axpy(Root<m, M, INV>::re, a[1], v0), im = scl(Root<m, M, INV>::im, b[1]);
+            unroll<H - 1>([&](auto ki) {
+                constexpr int k = decltype(ki)::value + 2;
+                re = axpy(Root<k * m, M, INV>::re, a[k], re);
+                im = axpy(Root<k * m, M, INV>::im, b[k], im);
+            });
+            v[m] = make_float2(re.x - im.y, re.y + im.x);  // + i im
+            v[M - m] = make_float2(re.x + im.y, re.y - im.x);
+        });
     } else {
         constexpr int A = Split<M>::A, B = Split<M>::B;
+        static_assert(A > 1 && B > 1 && A * B == M, "factors");
         float2 y[M];
-#pragma unroll
-        for (int n2 = 0; n2 < B; n2++) {
+        unroll<B>([&](auto bi) {
+            constexpr int n2 = decltype(bi)::value;
             float2 a[A];
 #pragma unroll
-            for (int n1 = 0; n1 < A; n1++) a[n1] = v[B * n1 + n2];
-            reg_dft<A, L>(a, tw, inv);
-#pragma unroll
-            for (int k1 = 0; k1 < A; k1++) {
-                if ((n2 * k1) % M != 0) {
-                    float2 w = tw[((n2 * k1) % M) * (L / M)];
-                    if (inv) w.y = -w.y;
-                    a[k1] = cmulf(a[k1], w);
-                }
-                y[n2 * A + k1] = a[k1];
-            }
-        }
-#pragma unroll
-        for (int k1 = 0; k1 < A; k1++) {
+            for (int n1 = 0; n1 < A; n1++) a[n1] = v[Split<M>::coprime ? (B * n1 + A * n2) % M : B * n1 + n2];
+            reg_dft<A, INV>(a);
+            unroll<A>([&](auto ai) {
+                constexpr int k1 = decltype(ai)::value;
+                y[n2 * A + k1] = Split<M>::coprime ? a[k1] : rot<n2 * k1, M, INV>(a[k1]);
+            });
+        });
+        unroll<A>([&](auto ai) {
+            constexpr int k1 = decltype(ai)::value;
             float2 b[B];
 #pragma unroll
             for (int n2 = 0; n2 < B; n2++) b[n2] = y[n2 * A + k1];
-            reg_dft<B, L>(b, tw, inv);
+            reg_dft<B, INV>(b);
+            if constexpr (!Split<M>::coprime) {
 #pragma unroll
-            for (int k2 = 0; k2 < B; k2++) v[k1 + A * k2] = b[k2];
-        }
+                for (int k2 = 0; k2 < B; k2++) v[k1 + A * k2] = b[k2];
+            } else {
+#pragma unroll
+                for (int k = 0; k < M; k++)
+                    if (k % A == k1) v[k] = b[k % B];
+            }
+        });
     }
 }
 
 // A transform length L = L1 L2 (both at most 32, products of 2, 3, 4, 5, 7).
+// Step A, one thread per (line, n2): the L1 points L2 n1 + n2, times w_L^(n2 k1)
+// after the transform. Step B, one thread per (line, k1): the L2 values n2,
+// which become the transform at k1 + L1 k2.
 template <int L_, int L1_, int L2_>
 struct Len {
     static constexpr int L = L_, L1 = L1_, L2 = L2_;
-    // one thread per (line, column) of step A and per (line, row) of step B
-    static constexpr int T = kFftLines * (L1 > L2 ? L1 : L2);
-    static constexpr int MINB = T <= 256 ? DMR_FFT_MINB : (T <= 384 ? 2 : 1);
-    static constexpr int TOEP_MINB = T <= 384 ? DMR_FFT_TOEP_MINB : 1;
+    static constexpr int MX = L1 > L2 ? L1 : L2;
+    static constexpr int T = kFftLines * MX;
+    // resident blocks that the registers are planned for, from registers a thread
+    // would like; more warps beat a few spilled words (280 points, 500 x 16 images
+    // forward: 3.13 ms at 64 registers, 3 blocks; 3.95 at 96, 2 blocks) up to 24
+    // points a thread. The Toeplitz pass holds two transforms' values (288 points:
+    // 0.73 ms at 3 blocks, 0.91 at 4)
+    static constexpr int blocks(int regs) { return 65536 / (T * regs) > 0 ? 65536 / (T * regs) : 1; }
+    static constexpr int MINB = blocks(MX > 24 ? 128 : 56), TOEP_MINB = blocks(MX > 24 ? 128 : 64);
     static_assert(L1 * L2 == L, "factors");
 };
 
-// Step A of the four-step transform of the block's 16 lines in buf
-// ([position][line]): line c, column n2 takes positions L2 n1 + n2, an
-// L1-point DFT, twiddles w_L^(n2 k1), back to positions L2 k1 + n2 (the
-// positions it read: no barrier needed between its reads and writes).
-// With `scale` the inputs are first multiplied by scale_line[c] * scale[position].
-template <class F>
-__device__ __forceinline__ void step_a(float2 *buf, const float2 *tw, bool inv, const float *scale = nullptr,
-                                       const float *scale_line = nullptr)
+// v times the twiddle between the steps, conjugated for the inverse
+template <bool INV>
+__device__ __forceinline__ float2 twiddle(float2 v, float2 w)
 {
-    constexpr int L = F::L, L1 = F::L1, L2 = F::L2;
-    const int w = threadIdx.x;
-    if (w < kFftLines * L2) {
-        const int c = w & (kFftLines - 1), n2 = w >> kFftShift;
-        float2 a[L1];
-#pragma unroll
-        for (int n1 = 0; n1 < L1; n1++) a[n1] = buf[(L2 * n1 + n2) * kFftLP + c];
-        if (scale) {
-            const float sl = scale_line[c];
-#pragma unroll
-            for (int n1 = 0; n1 < L1; n1++) {
-                const float sc = sl * scale[L2 * n1 + n2];
-                a[n1].x *= sc;
-                a[n1].y *= sc;
-            }
-        }
-        reg_dft<L1, L>(a, tw, inv);
-        // twiddles w_L^(n2 k1), index n2 k1 mod L kept incrementally
-        int ti = 0;
-#pragma unroll
-        for (int k1 = 1; k1 < L1; k1++) {
-            ti += n2;
-            if (ti >= L) ti -= L;
-            float2 t = tw[ti];
-            if (inv) t.y = -t.y;
-            a[k1] = cmulf(a[k1], t);
-        }
-#pragma unroll
-        for (int k1 = 0; k1 < L1; k1++) buf[(L2 * k1 + n2) * kFftLP + c] = a[k1];
-    }
+    return INV ? make_float2(v.x * w.x + v.y * w.y, v.y * w.x - v.x * w.y)
+               : make_float2(v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
 }
 
-// Step B for line c, row k1: positions L2 k1 + n2 (n2 < L2), an L2-point DFT;
-// b[k2] is the transform at position k1 + L1 k2.
-template <class F>
-__device__ __forceinline__ void step_b(const float2 *buf, const float2 *tw, bool inv, int c, int k1, float2 *b)
+// step A from registers (a[n1]) into the exchange buffer, rows k1 of pitch S1,
+// positions n2 of pitch S2; `sm` points at (n2, line), tw at table entry n2
+template <class F, bool INV, int S1>
+__device__ __forceinline__ void step_a(float2 *a, float2 *sm, const float2 *__restrict__ tw)
 {
-    constexpr int L = F::L, L2 = F::L2;
+    reg_dft<F::L1, INV>(a);
+    sm[0] = a[0];
 #pragma unroll
-    for (int n2 = 0; n2 < L2; n2++) b[n2] = buf[(L2 * k1 + n2) * kFftLP + c];
-    reg_dft<L2, L>(b, tw, inv);
+    for (int k1 = 1; k1 < F::L1; k1++) sm[k1 * S1] = twiddle<INV>(a[k1], __ldg(tw + k1 * F::L2));
 }
+
+// step B from the exchange buffer (`sm` at row k1, line) into registers
+template <class F, bool INV, int S2>
+__device__ __forceinline__ void step_b(const float2 *sm, float2 *b)
+{
+#pragma unroll
+    for (int n2 = 0; n2 < F::L2; n2++) b[n2] = sm[n2 * S2];
+    reg_dft<F::L2, INV>(b);
+}
+
+// positions of a line that hold data: l < e1 or s2 <= l < e2 (a cyclic range)
+struct Range {
+    int e1, s2, e2;
+    __device__ __forceinline__ bool has(int l) const { return l < e1 || (l >= s2 && l < e2); }
+};
 
 // the lengths with a compiled transform (grid extents of common matrix sizes
-// at oversampling 1.25 and 2), as (L, L1, L2); other lengths use cuFFT
+// at oversampling 1.25 and 2), as (L, L1, L2); other lengths use cuFFT. The
+// smaller factor first: more threads wait for fewer loads each in step A, and no
+// warp is idle there (rows forward, 280 = 14 x 20, 500 x 16 images of 224^2:
+// 1.98 ms with 20 first, 1.53 with 14; columns 1.73 and 1.60). The cropping row
+// pass is the other way round (1.40 ms, 1.56; its stores are the scattered side)
 #define DMR_FFT_LENGTHS(X)                                                                            \
-    X(32, 8, 4) X(40, 8, 5) X(48, 16, 3) X(56, 8, 7) X(64, 8, 8) X(80, 16, 5) X(96, 16, 6)              \
-    X(112, 16, 7) X(120, 12, 10) X(128, 16, 8) X(140, 20, 7) X(144, 12, 12) X(160, 16, 10)               \
-    X(168, 12, 14) X(192, 16, 12) X(200, 20, 10) X(224, 16, 14) X(240, 16, 15) X(256, 16, 16)            \
-    X(280, 20, 14) X(288, 18, 16) X(320, 20, 16) X(336, 24, 14) X(384, 24, 16) X(400, 20, 20)            \
-    X(480, 24, 20) X(512, 32, 16) X(640, 32, 20)
+    X(32, 4, 8) X(40, 5, 8) X(48, 3, 16) X(56, 7, 8) X(64, 8, 8) X(80, 5, 16) X(96, 6, 16)              \
+    X(112, 7, 16) X(120, 10, 12) X(128, 8, 16) X(140, 7, 20) X(144, 12, 12) X(160, 10, 16)               \
+    X(168, 12, 14) X(192, 12, 16) X(200, 10, 20) X(224, 14, 16) X(240, 15, 16) X(256, 16, 16)            \
+    X(280, 14, 20) X(288, 16, 18) X(320, 16, 20) X(336, 14, 24) X(384, 16, 24) X(400, 20, 20)            \
+    X(480, 20, 24) X(512, 16, 32) X(640, 20, 32)
 
 bool has_len(int L)
 {
@@ -307,82 +312,68 @@ __host__ __device__ __forceinline__ int wrapi(int v, int n)
     return v < 0 ? v + n : v;
 }
 
-// whether position l of a length-L line lies in the cyclic range [q0, q0 + n)
-__device__ __forceinline__ bool in_range(int l, int q0, int n, int L)
+// the cyclic range [q0, q0 + n) of a length-L line
+Range range(int q0, int n, int L)
 {
-    int d = l - q0;
-    if (d < 0) d += L;
-    return d < n;
+    return q0 + n > L ? Range{q0 + n - L, q0, L} : Range{0, q0, q0 + n};
 }
 
-// asynchronous copy of `bytes` (4 or 8) into shared memory; when !valid the
-// destination is zero-filled and nothing is read (src must still be mapped)
-__device__ __forceinline__ void cp_async_fill(void *sdst, const void *src, int bytes, bool valid)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(sdst);
-    const int n = valid ? bytes : 0;
-    if (bytes == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
-}
+// division of 0 <= v < 2^31 by a run-time constant
+struct FastDiv {
+    unsigned d, m, s;
+    explicit FastDiv(unsigned d_ = 1) : d(d_), s(31)
+    {
+        while ((1ull << (s - 31)) < d) s++;
+        m = (unsigned)(((1ull << s) + d - 1) / d);
+    }
+    __device__ __forceinline__ unsigned div(unsigned v) const { return (unsigned)(((unsigned long long)v * m) >> s); }
+};
 
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Lines of a row pass: line `row` of set bf (a (batch, frame) grid; with IL a
+// (chunk, frame) and line row % CS of image row row / CS).
+struct RowArgs {
+    FftGeom g;
+    FastDiv cs, n1, nf;
+    int nrows;   // lines of a set
+    int64_t bf0; // first set of the launch
+};
 
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// Per-line data of a row tile, computed once by the first 16 threads: the
-// image row offset, the grid row offset and the apodisation of the row's
-// (y, z) times the scale; rows past the end get offset -1.
+// image offset (-1: a coil past the batch), grid offset and, times the scale,
+// the apodisation of a line
 struct RowLine {
     int64_t img, grid;
     float s;
 };
 
-// With IL line `row` is coil row % CS of image row row / CS of a (chunk, frame);
-// coils past the batch have no image row (offset -1) but a grid row.
 template <bool IL>
-__device__ __forceinline__ void row_lines(const FftGeom &g, int64_t row0, int64_t nrows, RowLine *lines)
+__device__ __forceinline__ RowLine row_line(const RowArgs &ra, int row)
 {
-    const int c = threadIdx.x;
-    if (c >= kFftLines) return;
-    int64_t row = row0 + c;
-    RowLine ln;
-    ln.img = -1;
-    ln.grid = -1;
-    ln.s = 0.0f;
-    if (row < nrows) {
-        const int N1 = g.N[1], N2 = g.N[2];
-        const int64_t plane = (int64_t)N2 * N1;
-        int coil = 0;
-        if (IL) {
-            const int64_t r = row / g.CS;
-            coil = (int)(row - r * g.CS);
-            row = r;
-        }
-        const int64_t bf = row / plane;
-        const int rr = (int)(row - bf * plane);
-        const int y = rr % N1, z = rr / N1;
-        const int qy = wrapi(y + g.off[1], g.G[1]), qz = wrapi(z + g.off[2], g.G[2]);
-        ln.img = bf * g.isize + (int64_t)rr * g.N[0];
-        ln.grid = bf * g.gsize + ((int64_t)qz * g.G[1] + qy) * g.G[0];
-        if (IL) {
-            const int64_t chunk = bf / g.nframes, f = bf - chunk * g.nframes, b = chunk * g.CS + coil;
-            ln.img = b < g.batch ? (b * g.nframes + f) * g.isize + (int64_t)rr * g.N[0] : -1;
-            ln.grid = ln.grid * g.CS + coil;
-        }
-        float s = g.scale;
-        if (g.apod[1]) s *= g.apod[1][y];
-        if (g.apod[2]) s *= g.apod[2][z];
-        ln.s = s;
+    const FftGeom &g = ra.g;
+    const int64_t bf = ra.bf0 + blockIdx.y;
+    int coil = 0, rr = row;
+    if (IL) {
+        rr = ra.cs.div(row);
+        coil = row - rr * g.CS;
     }
-    lines[c] = ln;
+    const int z = ra.n1.div(rr), y = rr - z * g.N[1];
+    int qy = y + g.off[1], qz = z + g.off[2];
+    if (qy < 0) qy += g.G[1];
+    if (qz < 0) qz += g.G[2];
+    RowLine ln;
+    ln.img = bf * g.isize + (int64_t)rr * g.N[0];
+    ln.grid = bf * g.gsize + ((int64_t)qz * g.G[1] + qy) * g.G[0];
+    if (IL) {
+        const int64_t chunk = ra.nf.div((unsigned)bf), f = bf - chunk * g.nframes, b = chunk * g.CS + coil;
+        ln.img = b < g.batch ? (b * g.nframes + f) * g.isize + (int64_t)rr * g.N[0] : -1;
+        ln.grid = ln.grid * g.CS + coil;
+    }
+    ln.s = g.scale;
+    if (g.apod[1]) ln.s *= g.apod[1][y];
+    if (g.apod[2]) ln.s *= g.apod[2][z];
+    return ln;
 }
 
-// Row passes (x): tiles of 16 rows, double-buffered (the next tile's loads
-// are in flight while the current one is transformed); shared memory holds
-// two [L][17] tiles, the twiddle table and the x apodisation.
+// Row passes (x), a block per 16 rows.
 //   forward (CROP false): image rows (real or complex) are placed at their
 //   FFT-order positions (zero elsewhere), apodised, transformed and written
 //   as full grid rows;
@@ -391,340 +382,214 @@ __device__ __forceinline__ void row_lines(const FftGeom &g, int64_t row0, int64_
 // With IL the lines are 16 neighbouring (row, coil) pairs and the grid is
 // interleaved, so its accesses run along the lines; the image's along x.
 template <class F, bool CROP, bool IL>
-__global__ void __launch_bounds__(F::T, F::MINB) fft_rows_kernel(FftGeom g, const float2 *__restrict__ tw,
+struct RowShape {
+    // lanes of step A / B along the points of a line (else across the lines)
+    static constexpr bool XA = !(IL && CROP), XB = !(IL && !CROP);
+    // pitches of the exchange buffer (row k1, position n2, line): the lanes of a
+    // half-warp are neighbours when they write and an odd pitch apart when they
+    // read across, so that they hit distinct banks
+    static constexpr int S2 = XA ? 1 : kFftLines, SC = XA ? F::L2 | 1 : 1;
+    static constexpr int R = XA ? kFftLines * SC : F::L2 * S2, S1 = XB ? R | 1 : R;
+    static constexpr size_t SMEM = (size_t)F::L1 * S1 * sizeof(float2);
+};
+
+template <class F, bool CROP, bool IL>
+__global__ void __launch_bounds__(F::T, F::MINB) fft_rows_kernel(RowArgs ra, const float2 *__restrict__ tw,
                                                         const void *__restrict__ src, int src_real,
                                                         float2 *__restrict__ dst)
 {
-    constexpr int L = F::L, L1 = F::L1, L2 = F::L2, T = F::T;
+    using S = RowShape<F, CROP, IL>;
+    constexpr int L = F::L, L1 = F::L1, L2 = F::L2, S1 = S::S1, S2 = S::S2, SC = S::SC;
     extern __shared__ __align__(16) float2 fsm[];
-    float2 *bufs = fsm;                               // 2 x L * 17
-    float2 *tws = fsm + 2 * L * kFftLP;               // L
-    // L floats: the forward pass's x apodisation by grid position q (zero
-    // outside the image), the adjoint's by image index i
-    float *apx = reinterpret_cast<float *>(tws + L);
-    __shared__ RowLine lines[2][kFftLines];
-    __shared__ float line_s[2][kFftLines];
-    // h0: grid position q holds image index (q + h0) mod L (when below N0)
-    const int N0 = g.N[0], h0 = wrapi(-g.off[0], L);
-    for (int i = threadIdx.x; i < L; i += T) {
-        tws[i] = tw[i];
-        if (CROP) {
-            apx[i] = (g.apod[0] && i < N0) ? g.apod[0][i] : 1.0f;
-        } else {
-            int ii = i + h0;
-            if (ii >= L) ii -= L;
-            apx[i] = ii < N0 ? (g.apod[0] ? g.apod[0][ii] : 1.0f) : 0.0f;
-        }
-    }
-    const int64_t nrows = g.nbf * g.N[2] * g.N[1] * (IL ? g.CS : 1);
-    const int64_t ntiles = (nrows + kFftLines - 1) / kFftLines;
-    // loads of tile t into buffer `slot` (line data first, so a barrier)
-    auto prefetch = [&](int64_t t, int slot) {
-        row_lines<IL>(g, t * kFftLines, nrows, lines[slot]);
-        __syncthreads();
-        if (threadIdx.x < kFftLines) line_s[slot][threadIdx.x] = lines[slot][threadIdx.x].s;
-        float2 *buf = bufs + slot * L * kFftLP;
-        if (IL && CROP) {
-            if ((g.CS & 1) == 0) {
-                // pairs of coils (16 bytes): a pair never straddles two rows
-                constexpr int P = kFftLines / 2;
-                const int c = 2 * (threadIdx.x % P);
-                const int64_t go = lines[slot][c].grid;
-                const float2 *sp = reinterpret_cast<const float2 *>(src) + (go >= 0 ? go : 0);
-                const int64_t st = go >= 0 ? g.CS : 0;
-                for (int q = threadIdx.x / P; q < L; q += T / P) {
-                    const unsigned d = (unsigned)__cvta_generic_to_shared(buf + q * kFftLP + c);
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(sp + q * st),
-                                 "r"(go >= 0 ? 16 : 0)
-                                 : "memory");
-                }
-            } else {
-                const int c = threadIdx.x & (kFftLines - 1);
-                const int64_t go = lines[slot][c].grid;
-                for (int q = threadIdx.x >> kFftShift; q < L; q += T / kFftLines)
-                    cp_async_fill(buf + q * kFftLP + c,
-                                  reinterpret_cast<const float2 *>(src) + (go >= 0 ? go + (int64_t)q * g.CS : 0), 8,
-                                  go >= 0);
-            }
-            cp_async_commit();
-            return;
-        }
-        for (int e = threadIdx.x; e < kFftLines * L; e += T) {
-            const int c = e / L, q = e - c * L;
-            const RowLine ln = lines[slot][c];
-            float2 *d = buf + q * kFftLP + c;
-            if (!CROP) {
-                int i = q + h0;
-                if (i >= L) i -= L;
-                const bool ok = ln.img >= 0 && i < N0;
+    const FftGeom &g = ra.g;
+    const int w = threadIdx.x, row0 = blockIdx.x * kFftLines;
+    // grid position q holds image index (q + h0) mod L (when below N0)
+    const int N0 = g.N[0], h0 = g.off[0] > 0 ? L - g.off[0] : -g.off[0];
+    if (w < kFftLines * L2) {
+        const int c = S::XA ? w / L2 : w & (kFftLines - 1), n2 = S::XA ? w % L2 : w / kFftLines;
+        float2 a[L1];
+#pragma unroll
+        for (int n1 = 0; n1 < L1; n1++) a[n1] = make_float2(0.0f, 0.0f);
+        if (row0 + c < ra.nrows) {
+            const RowLine ln = row_line<IL>(ra, row0 + c);
+            if (CROP) {
+                const float2 *sp = reinterpret_cast<const float2 *>(src) + ln.grid + (int64_t)n2 * (IL ? g.CS : 1);
+                const int step = IL ? L2 * g.CS : L2;
+#pragma unroll
+                for (int n1 = 0; n1 < L1; n1++) a[n1] = IL ? __ldcg(sp + (int64_t)step * n1) : sp[step * n1];
+            } else if (ln.img >= 0) {
+                const float *ap = g.apod[0];
+                // image index of position L2 n1 + n2: i0 + L2 n1, less L after the wrap
+                const int i0 = n2 + h0;
                 if (src_real) {
-                    const float *sp = reinterpret_cast<const float *>(src) + (ok ? ln.img + i : 0);
-                    cp_async_fill(d, sp, 4, ok);
-                    cp_async_fill(reinterpret_cast<float *>(d) + 1, sp, 4, false);
+                    const float *sp = reinterpret_cast<const float *>(src) + ln.img;
+#pragma unroll
+                    for (int n1 = 0; n1 < L1; n1++) {
+                        const int i = i0 + L2 * n1 - (i0 + L2 * n1 >= L ? L : 0);
+                        if (i < N0) a[n1].x = sp[i] * (ap ? ln.s * __ldg(ap + i) : ln.s);
+                    }
                 } else {
-                    cp_async_fill(d, reinterpret_cast<const float2 *>(src) + (ok ? ln.img + i : 0), 8, ok);
+                    const float2 *sp = reinterpret_cast<const float2 *>(src) + ln.img;
+#pragma unroll
+                    for (int n1 = 0; n1 < L1; n1++) {
+                        const int i = i0 + L2 * n1 - (i0 + L2 * n1 >= L ? L : 0);
+                        if (i < N0) a[n1] = sp[i];
+                    }
+#pragma unroll
+                    for (int n1 = 0; n1 < L1; n1++) {
+                        const int i = i0 + L2 * n1 - (i0 + L2 * n1 >= L ? L : 0);
+                        if (i < N0) a[n1] = scl(ap ? ln.s * __ldg(ap + i) : ln.s, a[n1]);
+                    }
                 }
-            } else {
-                const bool ok = ln.grid >= 0;
-                cp_async_fill(d, reinterpret_cast<const float2 *>(src) + (ok ? ln.grid + q : 0), 8, ok);
             }
         }
-        cp_async_commit();
-    };
-    int64_t t = blockIdx.x;
-    if (t < ntiles) prefetch(t, 0);
-    for (int it = 0; t < ntiles; t += gridDim.x, it++) {
-        const int cur = it & 1;
-        float2 *buf = bufs + cur * L * kFftLP;
-        if (t + gridDim.x < ntiles) prefetch(t + gridDim.x, cur ^ 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        // forward: apodisation (position q of line c holds image index
-        // (q + N0/2) mod L, or zero) applied as step A reads its inputs
-        if (CROP) step_a<F>(buf, tws, true);
-        else step_a<F>(buf, tws, false, apx, line_s[cur]);
-        __syncthreads();
-        // step B into registers, then (after every thread has read its
-        // inputs) back into the tile in transform order
-        const int w = threadIdx.x;
-        const int c = w & (kFftLines - 1), k1 = w >> kFftShift;
-        float2 b[L2];
-        if (k1 < L1) step_b<F>(buf, tws, CROP, c, k1, b);
-        if (IL && !CROP) {
-            // straight to the grid: the 16 lines are neighbours there
-            const int64_t go = lines[cur][c].grid;
-            if (k1 < L1 && go >= 0) {
-#pragma unroll
-                for (int k2 = 0; k2 < L2; k2++) dst[go + (int64_t)(k1 + L1 * k2) * g.CS] = b[k2];
-            }
-            __syncthreads();
-            continue;
-        }
-        __syncthreads();
-        if (k1 < L1) {
-#pragma unroll
-            for (int k2 = 0; k2 < L2; k2++) buf[(k1 + L1 * k2) * kFftLP + c] = b[k2];
-        }
-        __syncthreads();
-        if (!CROP) {
-            for (int e = threadIdx.x; e < kFftLines * L; e += T) {
-                const int cc = e / L, l = e - cc * L;
-                const int64_t go = lines[cur][cc].grid;
-                if (go >= 0) dst[go + l] = buf[l * kFftLP + cc];
-            }
-        } else {
-            for (int e = threadIdx.x; e < kFftLines * N0; e += T) {
-                const int cc = e / N0, i = e - cc * N0;
-                const RowLine ln = lines[cur][cc];
-                if (ln.img < 0) continue;
-                int q = i - h0;
-                if (q < 0) q += L;
-                float2 v = buf[q * kFftLP + cc];
-                const float sc = ln.s * apx[i];
-                v.x *= sc;
-                v.y *= sc;
-                dst[ln.img + i] = v;
-            }
-        }
-        // the tile's buffer is loaded again two iterations on
-        __syncthreads();
+        step_a<F, CROP, S1>(a, fsm + n2 * S2 + c * SC, tw + n2);
     }
-    cp_async_wait<0>();
+    __syncthreads();
+    if (w < kFftLines * L1) {
+        const int c = S::XB ? w / L1 : w & (kFftLines - 1), k1 = S::XB ? w % L1 : w / kFftLines;
+        float2 b[L2];
+        step_b<F, CROP, S2>(fsm + k1 * S1 + c * SC, b);
+        if (row0 + c >= ra.nrows) return;
+        const RowLine ln = row_line<IL>(ra, row0 + c);
+        if (!CROP) {
+            float2 *d = dst + ln.grid + (int64_t)k1 * (IL ? g.CS : 1);
+            const int step = IL ? L1 * g.CS : L1;
+#pragma unroll
+            for (int k2 = 0; k2 < L2; k2++) d[(int64_t)step * k2] = b[k2];
+        } else if (ln.img >= 0) {
+            const float *ap = g.apod[0];
+            const int i0 = k1 + h0;
+            float2 *d = dst + ln.img;
+#pragma unroll
+            for (int k2 = 0; k2 < L2; k2++) {
+                const int i = i0 + L1 * k2 - (i0 + L1 * k2 >= L ? L : 0);
+                if (i < N0) d[i] = scl(ap ? ln.s * __ldg(ap + i) : ln.s, b[k2]);
+            }
+        }
+    }
 }
 
-// Column pass along y or z, in place on the grid: tiles of 16 consecutive x
-// of one line set (batch*frame, outer index), the line running along the axis
-// with element stride S. Input positions outside [in_q0, in_q0 + in_n)
-// (cyclic) are zero and not read; outputs outside [out_q0, out_q0 + out_n)
-// are not written. Outer index k in [0, nouter) selects plane / row
-// (outer_q0 + k) mod outer_G with stride outer_stride. Double-buffered like
-// the row passes; step B writes straight to the grid (16 consecutive x per
-// half-warp).
+// Column pass along y or z, in place on the grid: a block per 16 consecutive x
+// (x, coil) of one line set (set, outer index), the line running along the axis
+// with element stride S. Input positions outside `in` are zero and not read;
+// outputs outside `out` are not written. Outer index k selects plane / row
+// (outer_q0 + k) mod outer_G with stride outer_stride.
 struct ColArgs {
     int64_t S, outer_stride;
     int nouter, outer_q0, outer_G;
     int in_q0, in_n, out_q0, out_n;
     int inv;
+    Range in, out;
 };
 
-template <class F, bool IN_ALL, bool OUT_ALL>
-__global__ void __launch_bounds__(F::T, F::MINB) fft_cols_kernel(FftGeom g, ColArgs a, const float2 *__restrict__ tw,
-                                                        float2 *grid)
+template <class F, bool IN_ALL, bool OUT_ALL, bool INV>
+__global__ void __launch_bounds__(F::T, F::MINB) fft_cols_kernel(int G0, int64_t gsize, ColArgs a,
+                                                        const float2 *__restrict__ tw, float2 *grid)
 {
-    constexpr int L = F::L, L1 = F::L1, L2 = F::L2, T = F::T;
+    constexpr int L1 = F::L1, L2 = F::L2, S2 = kFftLines, S1 = L2 * S2;
     extern __shared__ __align__(16) float2 fsm[];
-    float2 *bufs = fsm, *tws = fsm + 2 * L * kFftLP;
-    for (int i = threadIdx.x; i < L; i += T) tws[i] = tw[i];
-    const int G0 = g.G[0];
-    const int ntx = (G0 + kFftLines - 1) / kFftLines;
-    const int64_t ntiles = g.nbf * a.nouter * ntx;
-    const bool inv = a.inv != 0;
-    // first x and base pointer of tile t
-    auto tile = [&](int64_t t, int &x0) -> float2 * {
-        const int tx = (int)(t % ntx);
-        const int64_t rest = t / ntx;
-        const int k = (int)(rest % a.nouter);
-        const int64_t bf = rest / a.nouter;
-        int qo = a.outer_q0 + k;
-        if (qo >= a.outer_G) qo -= a.outer_G;
-        x0 = tx * kFftLines;
-        return grid + bf * g.gsize + (int64_t)qo * a.outer_stride + x0;
-    };
-    auto prefetch = [&](int64_t t, int slot) {
-        int x0;
-        const float2 *base = tile(t, x0);
-        float2 *buf = bufs + slot * L * kFftLP;
-        // pairs of x (16 bytes; grid extents are even, so a pair never
-        // straddles the end of a row)
-        constexpr int P = kFftLines / 2;
-        for (int e = threadIdx.x; e < P * L; e += T) {
-            const int l = e / P, c = 2 * (e - l * P);
-            const bool ok = x0 + c < G0 && (IN_ALL || in_range(l, a.in_q0, a.in_n, L));
-            const unsigned d = (unsigned)__cvta_generic_to_shared(buf + l * kFftLP + c);
-            const float2 *sp = ok ? base + (int64_t)l * a.S + c : base;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(sp), "r"(ok ? 16 : 0)
-                         : "memory");
-        }
-        cp_async_commit();
-    };
-    int64_t t = blockIdx.x;
-    if (t < ntiles) prefetch(t, 0);
-    for (int it = 0; t < ntiles; t += gridDim.x, it++) {
-        const int cur = it & 1;
-        float2 *buf = bufs + cur * L * kFftLP;
-        if (t + gridDim.x < ntiles) prefetch(t + gridDim.x, cur ^ 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        step_a<F>(buf, tws, inv);
-        __syncthreads();
-        const int w = threadIdx.x;
-        const int c = w & (kFftLines - 1), k1 = w >> kFftShift;
-        int x0;
-        float2 *base = tile(t, x0);
-        if (k1 < L1 && x0 + c < G0) {
-            float2 b[L2];
-            step_b<F>(buf, tws, inv, c, k1, b);
+    int qo = a.outer_q0 + blockIdx.y;
+    if (qo >= a.outer_G) qo -= a.outer_G;
+    const int w = threadIdx.x, c = w % kFftLines, r = w / kFftLines, x = blockIdx.x * kFftLines + c;
+    float2 *base = grid + blockIdx.z * gsize + (int64_t)qo * a.outer_stride + x + r * a.S;
+    if (r < L2) {
+        float2 v[L1];
+        const int step = (int)(L2 * a.S);
 #pragma unroll
-            for (int k2 = 0; k2 < L2; k2++) {
-                const int l = k1 + L1 * k2;
-                if (OUT_ALL || in_range(l, a.out_q0, a.out_n, L)) base[(int64_t)l * a.S + c] = b[k2];
-            }
+        for (int n1 = 0; n1 < L1; n1++) {
+            v[n1] = make_float2(0.0f, 0.0f);
+            if (x < G0 && (IN_ALL || a.in.has(r + L2 * n1))) v[n1] = __ldcg(base + (int64_t)step * n1);
         }
-        // the tile's buffer is loaded again two iterations on
-        __syncthreads();
+        step_a<F, INV, S1>(v, fsm + w, tw + r);
     }
-    cp_async_wait<0>();
+    __syncthreads();
+    if (r < L1 && x < G0) {
+        float2 b[L2];
+        step_b<F, INV, S2>(fsm + r * S1 + c, b);
+        const int step = (int)(L1 * a.S);
+#pragma unroll
+        for (int k2 = 0; k2 < L2; k2++)
+            if (OUT_ALL || a.out.has(r + L1 * k2)) base[(int64_t)step * k2] = b[k2];
+    }
 }
 
-// Toeplitz z pass: per tile of 16 x of one (batch, y), the z columns (reading
-// the N2 z with data only), forward FFT, times kernel[b mod nk][z][y][x] *
-// kscale, inverse FFT, and the N2 kept z written back; nothing leaves shared
-// memory between the two transforms. Tiles run batch-fastest, so the blocks
-// that read one kernel tile run together and share it in L2.
+// Toeplitz z pass: per 16 x of one (batch, y), the z columns (reading the N2 z
+// with data only), forward FFT, times kernel[b mod nk][z][y][x] * kscale,
+// inverse FFT, and the N2 kept z written back. After step B a thread holds the
+// transform at k1 + L1 k2, all k2: the inverse runs the two steps backwards from
+// there (L2 points over k2, twiddles, the same row of the exchange buffer, L1
+// points over k1), so two barriers serve both transforms. Blocks run
+// batch-fastest: those that read one kernel tile run together and share it in L2.
 template <class F>
-__global__ void __launch_bounds__(F::T, F::TOEP_MINB) fft_toep_z_kernel(FftGeom g, ColArgs a, int64_t nk,
+__global__ void __launch_bounds__(F::T, F::TOEP_MINB) fft_toep_z_kernel(int G0, int64_t gsize, ColArgs a, int64_t nk,
                                                           const float2 *__restrict__ kern, float kscale,
                                                           const float2 *__restrict__ tw, float2 *grid)
 {
-    constexpr int L = F::L, L1 = F::L1, L2 = F::L2, T = F::T;
+    constexpr int L1 = F::L1, L2 = F::L2, S2 = kFftLines, S1 = L2 * S2;
     extern __shared__ __align__(16) float2 fsm[];
-    float2 *bufs = fsm, *tws = fsm + 2 * L * kFftLP;
-    for (int i = threadIdx.x; i < L; i += T) tws[i] = tw[i];
-    const int G0 = g.G[0];
-    const int ntx = (G0 + kFftLines - 1) / kFftLines;
-    const int64_t ntiles = g.nbf * a.nouter * ntx;
-    // batch index, first x, and the tile's offset in a grid (y row a.outer)
-    auto tile = [&](int64_t t, int64_t &bf, int &x0) -> int64_t {
-        bf = t % g.nbf;
-        const int64_t rest = t / g.nbf;
-        const int tx = (int)(rest % ntx);
-        const int k = (int)(rest / ntx);
-        x0 = tx * kFftLines;
-        return (int64_t)k * a.outer_stride + x0;
-    };
-    auto prefetch = [&](int64_t t, int slot) {
-        int64_t bf;
-        int x0;
-        const float2 *base = grid + tile(t, bf, x0) + bf * g.gsize;
-        float2 *buf = bufs + slot * L * kFftLP;
-        constexpr int P = kFftLines / 2;
-        for (int e = threadIdx.x; e < P * L; e += T) {
-            const int l = e / P, c = 2 * (e - l * P);
-            const bool ok = x0 + c < G0 && in_range(l, a.in_q0, a.in_n, L);
-            const unsigned d = (unsigned)__cvta_generic_to_shared(buf + l * kFftLP + c);
-            const float2 *sp = ok ? base + (int64_t)l * a.S + c : base;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(sp), "r"(ok ? 16 : 0)
-                         : "memory");
-        }
-        cp_async_commit();
-    };
-    int64_t t = blockIdx.x;
-    if (t < ntiles) prefetch(t, 0);
-    for (int it = 0; t < ntiles; t += gridDim.x, it++) {
-        const int cur = it & 1;
-        float2 *buf = bufs + cur * L * kFftLP;
-        if (t + gridDim.x < ntiles) prefetch(t + gridDim.x, cur ^ 1);
-        else cp_async_commit();
-        cp_async_wait<1>();
-        __syncthreads();
-        int64_t bf;
-        int x0;
-        const int64_t to = tile(t, bf, x0);
-        const int w = threadIdx.x;
-        const int c = w & (kFftLines - 1), k1 = w >> kFftShift;
-        // forward transform back into the tile (transform order)
-        step_a<F>(buf, tws, false);
-        __syncthreads();
-        float2 b[L2];
-        if (k1 < L1) step_b<F>(buf, tws, false, c, k1, b);
-        __syncthreads();
-        if (k1 < L1) {
+    const int w = threadIdx.x, c = w % kFftLines, r = w / kFftLines, x = blockIdx.y * kFftLines + c;
+    const int64_t bf = blockIdx.x, to = (int64_t)blockIdx.z * a.outer_stride + x + r * a.S;
+    float2 *base = grid + bf * gsize + to;
+    const int step_in = (int)(L2 * a.S), step_k = (int)(L1 * a.S);
+    if (r < L2) {
+        float2 v[L1];
 #pragma unroll
-            for (int k2 = 0; k2 < L2; k2++) buf[(k1 + L1 * k2) * kFftLP + c] = b[k2];
+        for (int n1 = 0; n1 < L1; n1++) {
+            v[n1] = make_float2(0.0f, 0.0f);
+            if (x < G0 && a.in.has(r + L2 * n1)) v[n1] = __ldcg(base + (int64_t)step_in * n1);
         }
-        __syncthreads();
-        // kernel multiply
-        const float2 *kb = kern + (bf % nk) * g.gsize + to;
-        for (int e = threadIdx.x; e < kFftLines * L; e += T) {
-            const int l = e >> kFftShift, cc = e & (kFftLines - 1);
-            if (x0 + cc < G0) {
-                const float2 kv = kb[(int64_t)l * a.S + cc];
-                float2 &v = buf[l * kFftLP + cc];
-                const float2 m = cmulf(kv, v);
-                v = make_float2(m.x * kscale, m.y * kscale);
-            }
-        }
-        __syncthreads();
-        // inverse transform, kept z to the grid
-        step_a<F>(buf, tws, true);
-        __syncthreads();
-        if (k1 < L1 && x0 + c < G0) {
-            step_b<F>(buf, tws, true, c, k1, b);
-            float2 *base = grid + bf * g.gsize + to;
-#pragma unroll
-            for (int k2 = 0; k2 < L2; k2++) {
-                const int l = k1 + L1 * k2;
-                if (in_range(l, a.out_q0, a.out_n, L)) base[(int64_t)l * a.S + c] = b[k2];
-            }
-        }
-        // the tile's buffer is loaded again two iterations on
-        __syncthreads();
+        step_a<F, false, S1>(v, fsm + w, tw + r);
     }
-    cp_async_wait<0>();
+    __syncthreads();
+    if (r < L1) {
+        float2 b[L2];
+        float2 *row = fsm + r * S1 + c;
+        step_b<F, false, S2>(row, b);
+        const float2 *kb = kern + (bf % nk) * gsize + to;
+#pragma unroll
+        for (int k2 = 0; k2 < L2; k2++) {
+            const float2 m = x < G0 ? cmulf(__ldg(kb + (int64_t)step_k * k2), b[k2]) : make_float2(0.0f, 0.0f);
+            b[k2] = make_float2(m.x * kscale, m.y * kscale);
+        }
+        reg_dft<L2, true>(b);
+#pragma unroll
+        for (int n2 = 0; n2 < L2; n2++) row[n2 * S2] = twiddle<true>(b[n2], __ldg(tw + r * L2 + n2));
+    }
+    __syncthreads();
+    if (r < L2 && x < G0) {
+        float2 v[L1];
+#pragma unroll
+        for (int k1 = 0; k1 < L1; k1++) v[k1] = fsm[k1 * S1 + w];
+        reg_dft<L1, true>(v);
+#pragma unroll
+        for (int n1 = 0; n1 < L1; n1++)
+            if (a.out.has(r + L2 * n1)) base[(int64_t)step_in * n1] = v[n1];
+    }
 }
 
-// per-device twiddle tables exp(-2 pi i t / L), t in [0, L), from double precision
+// per-device twiddle tables of the compiled lengths: entry k1 L2 + n2 is
+// exp(-2 pi i n2 k1 / L), from double precision; `crop`: with the factors
+// exchanged, for the cropping row pass
 std::mutex g_tw_mu;
-std::map<std::pair<int, int>, float2 *> g_tw;
+std::map<std::tuple<int, int, bool>, float2 *> g_tw;
 
-int twiddles(int L, const float2 **out)
+int second_factor(int L, bool crop)
+{
+    switch (L) {
+#define DMR_FFT_CASE(L, L1, L2) case L: return crop ? L1 : L2;
+        DMR_FFT_LENGTHS(DMR_FFT_CASE)
+#undef DMR_FFT_CASE
+    default: return 0;
+    }
+}
+
+int twiddles(int L, bool crop, const float2 **out)
 {
     int dev = 0;
     DMR_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_tw_mu);
-    auto key = std::make_pair(dev, L);
+    const auto key = std::make_tuple(dev, L, crop);
     auto it = g_tw.find(key);
     if (it != g_tw.end()) {
         *out = it->second;
@@ -732,8 +597,9 @@ int twiddles(int L, const float2 **out)
     }
     std::vector<float2> h(L);
     const double two_pi = 6.283185307179586476925286766559;
+    const int L2 = second_factor(L, crop);
     for (int t = 0; t < L; t++) {
-        const double ang = two_pi * (double)t / (double)L;
+        const double ang = two_pi * (double)((t / L2) * (t % L2)) / (double)L;
         h[t] = make_float2((float)std::cos(ang), (float)-std::sin(ang));
     }
     float2 *d = nullptr;
@@ -753,33 +619,28 @@ int fft_disabled()
     return v;
 }
 
-// two tiles, the twiddle table and the x apodisation (row passes)
-size_t smem_bytes(int L) { return (size_t)(2 * L * kFftLP + L) * sizeof(float2) + L * sizeof(float); }
+// sets (batch, frame) per launch: the grid's y and z extents are 16 bits
+constexpr int64_t kMaxSets = 65535;
 
-// grid size for a kernel looping over `ntiles` tiles: a few waves of resident blocks
-int blocks_for(const void *kern, int threads, size_t smem, int64_t ntiles, int *blocks)
+template <class K>
+int opt_in(K kern, size_t smem)
 {
-    int dev = 0, sms = 0, per_sm = 0;
-    DMR_CUDA(cudaGetDevice(&dev));
-    DMR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    DMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, smem));
-    DMR_CHECK(per_sm >= 1, DMR_ERR_UNSUPPORTED, "FFT pass does not fit on an SM");
-    const int64_t cap = (int64_t)sms * per_sm;
-    *blocks = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, cap));
+    if (smem > 48 * 1024) DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return DMR_OK;
 }
 
-template <class F, bool IN_ALL, bool OUT_ALL>
+template <class F, bool IN_ALL, bool OUT_ALL, bool INV>
 int launch_cols_tt(const FftGeom &g, const ColArgs &a, const float2 *tw, float2 *grid, cudaStream_t st)
 {
-    const size_t smem = smem_bytes(F::L);
-    const int64_t ntiles = g.nbf * a.nouter * ((g.G[0] + kFftLines - 1) / kFftLines);
-    if (ntiles == 0) return DMR_OK;
-    int blocks = 0;
-    DMR_TRY(blocks_for((const void *)fft_cols_kernel<F, IN_ALL, OUT_ALL>, F::T, smem, ntiles, &blocks));
-    fft_cols_kernel<F, IN_ALL, OUT_ALL><<<blocks, F::T, smem, st>>>(g, a, tw, grid);
-    DMR_LAUNCHED("fft_cols_kernel");
+    const size_t smem = (size_t)F::L * kFftLines * sizeof(float2);
+    const auto kern = fft_cols_kernel<F, IN_ALL, OUT_ALL, INV>;
+    DMR_TRY(opt_in(kern, smem));
+    for (int64_t b = 0; b < g.nbf; b += kMaxSets) {
+        const dim3 blocks((unsigned)ceil_div(g.G[0], kFftLines), (unsigned)a.nouter,
+                          (unsigned)std::min<int64_t>(g.nbf - b, kMaxSets));
+        kern<<<blocks, F::T, smem, st>>>(g.G[0], g.gsize, a, tw, grid + b * g.gsize);
+        DMR_LAUNCHED("fft_cols_kernel");
+    }
     return DMR_OK;
 }
 
@@ -788,22 +649,24 @@ int launch_cols_tt(const FftGeom &g, const ColArgs &a, const float2 *tw, float2 
 template <class F>
 int launch_cols_t(const FftGeom &g, const ColArgs &a, const float2 *tw, float2 *grid, cudaStream_t st)
 {
-    const int L = F::L;
-    if (a.out_n == L) return launch_cols_tt<F, false, true>(g, a, tw, grid, st);
-    if (a.in_n == L) return launch_cols_tt<F, true, false>(g, a, tw, grid, st);
-    return launch_cols_tt<F, false, false>(g, a, tw, grid, st);
+    return a.inv ? launch_cols_tt<F, true, false, true>(g, a, tw, grid, st)
+                 : launch_cols_tt<F, false, true, false>(g, a, tw, grid, st);
 }
 
 template <class F, bool CROP, bool IL>
 int launch_rows_t(const FftGeom &g, const float2 *tw, const void *src, int src_real, float2 *dst, cudaStream_t st)
 {
-    const size_t smem = smem_bytes(F::L);
-    const int64_t ntiles = (g.nbf * g.N[2] * g.N[1] * (IL ? g.CS : 1) + kFftLines - 1) / kFftLines;
-    if (ntiles == 0) return DMR_OK;
-    int blocks = 0;
-    DMR_TRY(blocks_for((const void *)fft_rows_kernel<F, CROP, IL>, F::T, smem, ntiles, &blocks));
-    fft_rows_kernel<F, CROP, IL><<<blocks, F::T, smem, st>>>(g, tw, src, src_real, dst);
-    DMR_LAUNCHED(CROP ? "fft_crop_rows_kernel" : "fft_pad_rows_kernel");
+    const size_t smem = RowShape<F, CROP, IL>::SMEM;
+    const auto kern = fft_rows_kernel<F, CROP, IL>;
+    DMR_TRY(opt_in(kern, smem));
+    const int64_t nrows = (int64_t)g.N[2] * g.N[1] * (IL ? g.CS : 1);
+    DMR_CHECK(nrows < INT32_MAX - kFftLines && g.nbf <= INT32_MAX, DMR_ERR_UNSUPPORTED, "too many image rows");
+    RowArgs ra{g, FastDiv(IL ? g.CS : 1), FastDiv(g.N[1]), FastDiv(g.nframes), (int)nrows, 0};
+    for (; ra.bf0 < g.nbf; ra.bf0 += kMaxSets) {
+        const dim3 blocks((unsigned)ceil_div(nrows, kFftLines), (unsigned)std::min<int64_t>(g.nbf - ra.bf0, kMaxSets));
+        kern<<<blocks, F::T, smem, st>>>(ra, tw, src, src_real, dst);
+        DMR_LAUNCHED(CROP ? "fft_crop_rows_kernel" : "fft_pad_rows_kernel");
+    }
     return DMR_OK;
 }
 
@@ -811,12 +674,10 @@ template <class F>
 int launch_toep_z_t(const FftGeom &g, const ColArgs &a, int64_t nk, const float2 *kern, float kscale,
                     const float2 *tw, float2 *grid, cudaStream_t st)
 {
-    const size_t smem = smem_bytes(F::L);
-    const int64_t ntiles = g.nbf * a.nouter * ((g.G[0] + kFftLines - 1) / kFftLines);
-    if (ntiles == 0) return DMR_OK;
-    int blocks = 0;
-    DMR_TRY(blocks_for((const void *)fft_toep_z_kernel<F>, F::T, smem, ntiles, &blocks));
-    fft_toep_z_kernel<F><<<blocks, F::T, smem, st>>>(g, a, nk, kern, kscale, tw, grid);
+    const size_t smem = (size_t)F::L * kFftLines * sizeof(float2);
+    DMR_TRY(opt_in(fft_toep_z_kernel<F>, smem));
+    const dim3 blocks((unsigned)g.nbf, (unsigned)ceil_div(g.G[0], kFftLines), (unsigned)a.nouter);
+    fft_toep_z_kernel<F><<<blocks, F::T, smem, st>>>(g.G[0], g.gsize, a, nk, kern, kscale, tw, grid);
     DMR_LAUNCHED("fft_toep_z_kernel");
     return DMR_OK;
 }
@@ -849,7 +710,7 @@ int launch_rows(int L, bool crop, const FftGeom &g, const float2 *tw, const void
     switch (L) {
 #define DMR_FFT_CASE(L, L1, L2)                                                                     \
     case L:                                                                                         \
-        return crop ? launch_rows_t<Len<L, L1, L2>, true, IL>(g, tw, src, src_real, dst, st)        \
+        return crop ? launch_rows_t<Len<L, L2, L1>, true, IL>(g, tw, src, src_real, dst, st)        \
                     : launch_rows_t<Len<L, L1, L2>, false, IL>(g, tw, src, src_real, dst, st);
         DMR_FFT_LENGTHS(DMR_FFT_CASE)
 #undef DMR_FFT_CASE
@@ -874,6 +735,12 @@ FftGeom make_geom(const dmr_plan *p, int64_t batch, int64_t nframes, float scale
     return g;
 }
 
+void set_ranges(ColArgs &a, int L)
+{
+    a.in = range(a.in_q0, a.in_n, L);
+    a.out = range(a.out_q0, a.out_n, L);
+}
+
 ColArgs y_pass(const FftGeom &g, bool inv)
 {
     // y columns of the N2 planes that hold data; the forward reads the N1
@@ -890,6 +757,7 @@ ColArgs y_pass(const FftGeom &g, bool inv)
     a.out_q0 = inv ? q0 : 0;
     a.out_n = inv ? g.N[1] : g.G[1];
     a.inv = inv;
+    set_ranges(a, g.G[1]);
     return a;
 }
 
@@ -909,6 +777,7 @@ ColArgs z_pass(const FftGeom &g, bool inv)
     a.out_q0 = inv ? q0 : 0;
     a.out_n = inv ? g.N[2] : g.G[2];
     a.inv = inv;
+    set_ranges(a, g.G[2]);
     return a;
 }
 
@@ -929,7 +798,7 @@ int fft3_forward(const dmr_plan *p, const void *image, int image_real, int64_t b
 {
     const FftGeom g = make_geom(p, batch, nframes, 1.0f);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], false, &tw[a]));
     if (g.nbf == 0) return DMR_OK;
     DMR_TRY(launch_rows(g.G[0], false, g, tw[0], image, image_real, grid, st));
     DMR_TRY(launch_cols(g.G[1], g, y_pass(g, false), tw[1], grid, st));
@@ -942,7 +811,7 @@ int fft3_adjoint(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nframes
 {
     const FftGeom g = make_geom(p, batch, nframes, (float)(1.0 / (double)p->g.gsize));
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], a == 0, &tw[a]));
     if (g.nbf == 0) return DMR_OK;
     if (g.G[2] > 1) DMR_TRY(launch_cols(g.G[2], g, z_pass(g, true), tw[2], grid, st));
     DMR_TRY(launch_cols(g.G[1], g, y_pass(g, true), tw[1], grid, st));
@@ -978,7 +847,7 @@ int fft3_forward_il(const dmr_plan *p, const void *image, int image_real, int64_
     if (CS == 1) return fft3_forward(p, image, image_real, batch, nframes, grid, st);  // the same layout
     const FftGeom g = il_geom(p, batch, nframes, nchunks, CS, 1.0f), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], false, &tw[a]));
     DMR_TRY(launch_rows<true>(g.G[0], false, g, tw[0], image, image_real, grid, st));
     DMR_TRY(launch_cols(g.G[1], c, y_pass(c, false), tw[1], grid, st));
     if (g.G[2] == 1) return DMR_OK;  // 2D
@@ -991,7 +860,7 @@ int fft3_adjoint_il(const dmr_plan *p, float2 *grid, int64_t batch, int64_t nfra
     if (CS == 1) return fft3_adjoint(p, grid, batch, nframes, image, st);
     const FftGeom g = il_geom(p, batch, nframes, nchunks, CS, (float)(1.0 / (double)p->g.gsize)), c = il_cols(g);
     const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    for (int a = 0; a < p->g.ndim; a++) DMR_TRY(twiddles(g.G[a], a == 0, &tw[a]));
     if (g.G[2] > 1) DMR_TRY(launch_cols(g.G[2], c, z_pass(c, true), tw[2], grid, st));
     DMR_TRY(launch_cols(g.G[1], c, y_pass(c, true), tw[1], grid, st));
     return launch_rows<true>(g.G[0], true, g, tw[0], grid, 0, image, st);
@@ -1031,8 +900,9 @@ int fft3_toeplitz(int ndim, const int32_t *kshape_zyx, const int32_t *ishape_zyx
     }
     g.nbf = batch;
     g.scale = 1.0f;
-    const float2 *tw[3] = {nullptr, nullptr, nullptr};
-    for (int a = 0; a < ndim; a++) DMR_TRY(twiddles(g.G[a], &tw[a]));
+    const float2 *tw[3] = {nullptr, nullptr, nullptr}, *twc = nullptr;
+    for (int a = 0; a < ndim; a++) DMR_TRY(twiddles(g.G[a], false, &tw[a]));
+    DMR_TRY(twiddles(g.G[0], true, &twc));
     if (batch == 0) return DMR_OK;
     const float kscale = (float)(1.0 / (double)g.gsize);
     DMR_TRY(launch_rows(g.G[0], false, g, tw[0], image, image_real, data, st));
@@ -1041,16 +911,18 @@ int fft3_toeplitz(int ndim, const int32_t *kshape_zyx, const int32_t *ishape_zyx
         ColArgs y = y_pass(g, false);
         y.out_q0 = y.in_q0;
         y.out_n = y.in_n;
+        set_ranges(y, g.G[1]);
         DMR_TRY(launch_toep_z(g.G[1], g, y, nk, kernel, kscale, tw[1], data, st));
     } else {
         DMR_TRY(launch_cols(g.G[1], g, y_pass(g, false), tw[1], data, st));
         ColArgs z = z_pass(g, false);
         z.out_q0 = z.in_q0;
         z.out_n = z.in_n;  // only the kept z leave the fused transform
+        set_ranges(z, g.G[2]);
         DMR_TRY(launch_toep_z(g.G[2], g, z, nk, kernel, kscale, tw[2], data, st));
         DMR_TRY(launch_cols(g.G[1], g, y_pass(g, true), tw[1], data, st));
     }
-    return launch_rows(g.G[0], true, g, tw[0], data, 0, out, st);
+    return launch_rows(g.G[0], true, g, twc, data, 0, out, st);
 }
 
 }  // namespace dmr
