@@ -175,16 +175,28 @@ __device__ __forceinline__ void reg_dft(float2 *v)
         }
         unroll<H>([&](auto mi) {
             constexpr int m = decltype(mi)::value + 1;
-            // (long sums take v0 last: fewer roundings at its size)
-            constexpr bool LONG = M > 7;
-            float2 re = LONG ? scl(Root<m, M, INV>::re, a[1]) : axpy(Root<m, M, INV>::re, a[1], v0);
-            float2 im = scl(Root<m, M, INV>::im, b[1]);
+            float2 re = axpy(Root<m, M, INV>::re, a[1], v0), im = scl(Root<m, M, INV>::im, b[1]);
+            // sums of five and more: two chains, added last (rounding)
+            constexpr int SPLIT = M > 7 ? H / 2 : H;
+            float2 re2 = make_float2(0.0f, 0.0f), im2 = re2;
             unroll<H - 1>([&](auto ki) {
                 constexpr int k = decltype(ki)::value + 2;
-                re = axpy(Root<k * m, M, INV>::re, a[k], re);
-                im = axpy(Root<k * m, M, INV>::im, b[k], im);
+                constexpr float c = Root<k * m, M, INV>::re, s = Root<k * m, M, INV>::im;
+                if constexpr (k <= SPLIT) {
+                    re = axpy(c, a[k], re);
+                    im = axpy(s, b[k], im);
+                } else if constexpr (k == SPLIT + 1) {
+                    re2 = scl(c, a[k]);
+                    im2 = scl(s, b[k]);
+                } else {
+                    re2 = axpy(c, a[k], re2);
+                    im2 = axpy(s, b[k], im2);
+                }
             });
-            if (LONG) re = cadd(v0, re);
+            if constexpr (SPLIT < H) {
+                re = cadd(re, re2);
+                im = cadd(im, im2);
+            }
             v[m] = make_float2(re.x - im.y, re.y + im.x);  // + i im
             v[M - m] = make_float2(re.x + im.y, re.y - im.x);
         });
@@ -552,11 +564,21 @@ __device__ __forceinline__ void toep_b(const ColArgs &a, int G0, int x, float2 *
     float2 b[L2];
     float2 *row = fsm + r * L2 * kFftLines + w % kFftLines;
     step_b<L2, false>(row, kFftLines, b);
+    // kernel values six loads at a time (left to itself the compiler takes one load,
+    // one use: 288 points, 8 coils of 144^3, 1.31 ms against 0.75, and 512 points 48
+    // us a call against 24; all at once spills: 28 us)
+    constexpr int GRP = 6;
+    const bool on = x < G0;
     kb += r * a.S;
 #pragma unroll
-    for (int k2 = 0; k2 < L2; k2++) {
-        const float2 m = x < G0 ? cmulf(__ldg(kb + (int64_t)step * k2), b[k2]) : make_float2(0.0f, 0.0f);
-        b[k2] = make_float2(m.x * kscale, m.y * kscale);
+    for (int k0 = 0; k0 < L2; k0 += GRP) {
+        float2 kv[GRP];
+#pragma unroll
+        for (int j = 0; j < GRP; j++)
+            kv[j] = on && k0 + j < L2 ? __ldg(kb + (int64_t)step * (k0 + j)) : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < GRP; j++)
+            if (k0 + j < L2) b[k0 + j] = scl(kscale, cmulf(kv[j], b[k0 + j]));
     }
     reg_dft<L2, true>(b);
 #pragma unroll
