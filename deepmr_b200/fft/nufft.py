@@ -5,12 +5,12 @@ reference module (src/deepmr/fft/nufft.py); the work runs in the sm_100a CUDA
 library through its C ABI:
 
 * ``plan_nufft``  -> Cartesian-axis test on the device, then a device-resident
-  plan (rescaled coordinates sorted by spatial bin), nufft.py:27-132.
-* ``apply_nufft`` -> one fused apodise/zero-pad/ifftshift kernel, cuFFT, and
-  the bin-tiled interpolation kernel, nufft.py:212-245, 450-528.
-* ``apply_nufft_adj`` -> bin-tiled gridding, cuFFT, one fused
-  fftshift/crop/apodise kernel, nufft.py:289-322, 531-606.
-* ``apply_nufft_selfadj`` -> Toeplitz pad/FFT/multiply/iFFT/crop,
+  plan (sorted samples, tap weights, work lists), nufft.py:27-132.
+* ``apply_nufft`` -> fused apodise/zero-pad/FFT passes onto a coil-interleaved
+  grid and the interpolation kernel, nufft.py:212-245, 450-528.
+* ``apply_nufft_adj`` -> gridding, fused inverse FFT/crop/apodise passes,
+  nufft.py:289-322, 531-606.
+* ``apply_nufft_selfadj`` -> Toeplitz passes with the kernel multiply inside,
   nufft.py:351-375, 609-669.
 
 Computation always happens on a CUDA device. ``device="cpu"`` (the reference
@@ -28,6 +28,7 @@ __all__ = [
     "NUFFTPlan",
 ]
 
+import contextlib
 import ctypes
 import math
 import weakref
@@ -54,6 +55,14 @@ def compute_device(device):
     if d.type == "cuda":
         return torch.device("cuda", d.index if d.index is not None else torch.cuda.current_device())
     return torch.device("cuda", torch.cuda.current_device())
+
+
+_HERE = contextlib.nullcontext()
+
+
+def _on_device(dev):
+    """Context that makes ``dev`` the current device: nothing to enter where it is."""
+    return _HERE if torch.cuda.current_device() == dev.index else torch.cuda.device(dev)
 
 
 def _destroy(handle):
@@ -134,13 +143,13 @@ class DevicePlan:
 
     def workspace(self, batch):
         n = ctypes.c_size_t()
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             _lib.check(_lib.lib().dmr_nufft_workspace_bytes(self.handle, int(batch), ctypes.byref(n)))
         return torch.empty(int(n.value), dtype=torch.uint8, device=self.device)
 
     def workspace_lowrank(self, batch, ncoeff):
         n = ctypes.c_size_t()
-        with torch.cuda.device(self.device):
+        with _on_device(self.device):
             _lib.check(_lib.lib().dmr_nufft_lowrank_workspace_bytes(self.handle, int(batch), int(ncoeff),
                                                                     ctypes.byref(n)))
         return torch.empty(int(n.value), dtype=torch.uint8, device=self.device)
@@ -340,13 +349,26 @@ class ApplyNUFFTSelfAdjoint(autograd.Function):
                 None, None, None)
 
 
+def _call(function, x, *args):
+    """``function.apply(x, *args)`` without the lookup of the forward's signature
+    that ``apply`` does first to fill in defaults (18 of the 72 us of a one-coil
+    64^2 call): here every argument is given. The autograd function is entered
+    all the same, so saved-tensor hooks, forward mode and tracing see it; inside
+    function transforms, for their tensors and while compiling, ``apply`` itself
+    runs."""
+    if (torch._C._are_functorch_transforms_active() or torch.compiler.is_compiling()
+            or (isinstance(x, torch.Tensor) and torch._C._functorch.is_functorch_wrapped_tensor(x))):
+        return function.apply(x, *args)
+    return super(autograd.Function, function).apply(x, *args)
+
+
 def apply_nufft(image, nufft_plan, basis_adjoint=None, weight=None, device=None, threadsperblock=128):
     """Apply the NUFFT (reference: nufft.py:212-245).
 
     image ``(..., [ncontrasts,] *shape)`` -> kspace ``(..., [ncontrasts,] nviews, nsamples)``.
     ``threadsperblock`` is accepted for compatibility and ignored.
     """
-    return ApplyNUFFT.apply(image, nufft_plan, basis_adjoint, weight, device, threadsperblock)
+    return _call(ApplyNUFFT, image, nufft_plan, basis_adjoint, weight, device, threadsperblock)
 
 
 def apply_nufft_adj(kspace, nufft_plan, basis=None, weight=None, device=None, threadsperblock=128):
@@ -354,12 +376,12 @@ def apply_nufft_adj(kspace, nufft_plan, basis=None, weight=None, device=None, th
 
     kspace ``(..., [ncontrasts,] nviews, nsamples)`` -> image ``(..., [ncontrasts,] *shape)``.
     """
-    return ApplyNUFFTAdjoint.apply(kspace, nufft_plan, basis, weight, device, threadsperblock)
+    return _call(ApplyNUFFTAdjoint, kspace, nufft_plan, basis, weight, device, threadsperblock)
 
 
 def apply_nufft_selfadj(image, toeplitz_kern, device=None, threadsperblock=128):
     """Self-adjoint NUFFT through Toeplitz convolution (reference: nufft.py:351-375)."""
-    return ApplyNUFFTSelfAdjoint.apply(image, toeplitz_kern, device, threadsperblock)
+    return _call(ApplyNUFFTSelfAdjoint, image, toeplitz_kern, device, threadsperblock)
 
 
 # ---------------------------------------------------------------------------
@@ -558,7 +580,7 @@ def _apply_nufft(image, nufft_plan, basis_adjoint, weight, device, threadsperblo
             raise ValueError(f"expected {nframes} frames before the spatial axes, got {tuple(image.shape)}")
     if tuple(image.shape[-ndim:]) != tuple(int(s) for s in nufft_plan.shape):
         raise ValueError(f"image spatial shape {tuple(image.shape[-ndim:])} != plan shape {nufft_plan.shape}")
-    batch = int(np.prod(batch_shape))
+    batch = int(math.prod(batch_shape))
     kshape = _kspace_shape(interp, batch_shape)
     real = int(not image.is_complex())
 
@@ -580,7 +602,7 @@ def _apply_nufft(image, nufft_plan, basis_adjoint, weight, device, threadsperblo
     out = torch.empty(kshape, dtype=torch.complex64, device=dev)
     if batch > 0 and interp.total > 0:
         w, wpb = _weight_arg(weight, batch_shape, interp, frames_shape, dev)
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             run(x, out, 0, batch, interp.workspace(batch), _lib.stream_ptr(dev))
     out = _to_origin(out, image)
     return out.numpy(force=True) if isnumpy else out
@@ -604,7 +626,7 @@ def _apply_nufft_adj(kspace, nufft_plan, basis, weight, device, threadsperblock,
         batch_shape = kspace.shape[: -nsd - 1]
     if list(kspace.shape) != _kspace_shape(interp, batch_shape):
         raise ValueError(f"kspace shape {tuple(kspace.shape)} does not match the plan samples {_sample_shape(interp)}")
-    batch = int(np.prod(batch_shape))
+    batch = int(math.prod(batch_shape))
     item = list(frames_shape) + [int(s) for s in nufft_plan.shape]
     real = int(not kspace.is_complex())
     det = int(DETERMINISTIC_GRIDDING if deterministic is None else deterministic)
@@ -618,7 +640,7 @@ def _apply_nufft_adj(kspace, nufft_plan, basis, weight, device, threadsperblock,
         )
 
     min_chunk = (ADJOINT_MIN_CHUNK_3D_DET if det else ADJOINT_MIN_CHUNK_3D) if nufft_plan.ndim == 3 else 1
-    if batch >= 2 * min_chunk and _pipelinable(kspace, dev, batch, 8 * int(np.prod(item))):
+    if batch >= 2 * min_chunk and _pipelinable(kspace, dev, batch, 8 * int(math.prod(item))):
         w, wpb = _weight_arg(weight, batch_shape, interp, frames_shape, dev)
         out = torch.empty([batch] + item, dtype=torch.complex64, pin_memory=True)
         _pipelined(kspace.reshape((batch,) + tuple(kspace.shape[len(batch_shape):])), out, batch, dev, run,
@@ -629,7 +651,7 @@ def _apply_nufft_adj(kspace, nufft_plan, basis, weight, device, threadsperblock,
     out = torch.empty(list(batch_shape) + item, dtype=torch.complex64, device=dev)
     if batch > 0:
         w, wpb = _weight_arg(weight, batch_shape, interp, frames_shape, dev)
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             run(y, out, 0, batch, interp.workspace(batch), _lib.stream_ptr(dev))
     out = _to_origin(out, kspace)
     if batch > 0 and (CHECK_STATUS or out.device.type == "cpu"):
@@ -655,13 +677,13 @@ def _apply_nufft_lowrank(image, nufft_plan, basis_adjoint, weight, device):
     ba = _basis_arg(basis_adjoint, nframes, ncoeff, dev, "basis_adjoint")
     batch_shape = x.shape[: -ndim - 1]
     frames_shape = (nframes,) if nframes > 1 else ()
-    batch = int(np.prod(batch_shape))
+    batch = int(math.prod(batch_shape))
     x = x.contiguous()
     out = torch.empty(_kspace_shape(interp, batch_shape), dtype=torch.complex64, device=dev)
     if batch > 0 and interp.total > 0:
         w, wpb = _weight_arg(weight, batch_shape, interp, frames_shape, dev)
         ws = interp.workspace_lowrank(batch, ncoeff)
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             _lib.check(_lib.lib().dmr_nufft_forward_lowrank(
                 interp.handle, _lib.ptr(x), int(not x.is_complex()), ncoeff, _lib.ptr(ba), _lib.ptr(out),
                 batch, _lib.ptr(w), wpb, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
@@ -693,7 +715,7 @@ def _apply_nufft_adj_lowrank(kspace, nufft_plan, basis, weight, device, determin
     ncoeff = int(b.shape[0])
     bb = _basis_arg(b, ncoeff, nframes, dev, "basis")
     frames_shape = (nframes,) if nframes > 1 else ()
-    batch = int(np.prod(batch_shape))
+    batch = int(math.prod(batch_shape))
     y = y.contiguous()
     out = torch.empty(list(batch_shape) + [ncoeff] + [int(s) for s in nufft_plan.shape],
                       dtype=torch.complex64, device=dev)
@@ -701,7 +723,7 @@ def _apply_nufft_adj_lowrank(kspace, nufft_plan, basis, weight, device, determin
         w, wpb = _weight_arg(weight, batch_shape, interp, frames_shape, dev)
         ws = interp.workspace_lowrank(batch, ncoeff)
         det = int(DETERMINISTIC_GRIDDING if deterministic is None else deterministic)
-        with torch.cuda.device(dev):
+        with _on_device(dev):
             _lib.check(_lib.lib().dmr_nufft_adjoint_lowrank(
                 interp.handle, _lib.ptr(y), int(not y.is_complex()), ncoeff, _lib.ptr(bb), _lib.ptr(out), batch,
                 _lib.ptr(w), wpb, det, _lib.ptr(ws), ws.numel(), _lib.stream_ptr(dev)))
