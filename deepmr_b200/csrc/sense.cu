@@ -5,9 +5,10 @@
 // src/deepmr/linops/nufft.py:189-241, src/deepmr/linops/coil.py:11-205) and
 // cg_solve / CGStep (src/deepmr/optim/cg.py:16-221). The reference chains
 // torch operations (coil multiply, Toeplitz self-adjoint per coil, coil sum)
-// and computes CG inner products in complex64; here coil expansion is fused
-// into the zero-pad kernel, coil combination (+ lambda x) into the crop
-// kernel, and inner products accumulate in float64 with a fixed two-stage
+// and computes CG inner products in complex64; here coil expansion and coil
+// combination (+ lambda x) are one kernel each around the fused Toeplitz passes
+// (fftpass.cu; for other lengths fused into the pad and crop kernels around
+// cuFFT), and inner products accumulate in float64 with a fixed two-stage
 // reduction (bitwise reproducible, independent of what else runs on the GPU).
 #include <algorithm>
 #include <cmath>

@@ -88,10 +88,11 @@ int dmr_tc_test_stall(int enable);
 
 /*
  * Query, no reference counterpart: 1 if the plan's forward / adjoint NUFFT
- * run their 3D FFT as the library's fused passes (apodise + zero-pad + FFT,
- * inverse FFT + crop + 1/G + apodisation, pruned to the lines with data),
- * 0 if they use cuFFT with separate pad / crop kernels (grid extents without
- * a compiled transform, 1D / 2D plans, or DMR_CUFFT=1 in the environment).
+ * run their 2D or 3D FFT as the library's fused passes (apodise + zero-pad +
+ * FFT, inverse FFT + crop + 1/G + apodisation, pruned to the lines with data),
+ * 0 if they use cuFFT with separate pad / crop kernels (a grid extent below 32
+ * or that is no product of two factors up to 26 (512 and 640 are taken), 1D
+ * plans, or DMR_CUFFT=1 in the environment).
  * Replaces the FFT step of src/deepmr/fft/nufft.py:502-505 and 583-590.
  */
 int dmr_fft3_fused(dmr_plan *plan);
@@ -214,8 +215,9 @@ int dmr_grid(const dmr_plan *plan, const void *kspace, int kspace_real,
 int dmr_nufft_workspace_bytes(dmr_plan *plan, int64_t batch, size_t *bytes);
 
 /*
- * Forward NUFFT: apodise + zero-pad + ifftshift (one kernel), cuFFT forward,
- * interpolation (fftshift folded into its indexing) with 1/scale and weight.
+ * Forward NUFFT: apodise + zero-pad + ifftshift + FFT (fused passes; for other
+ * extents a pad kernel and cuFFT), interpolation (fftshift folded into its
+ * indexing) with 1/scale and weight.
  * Replaces _apply_nufft (src/deepmr/fft/nufft.py:450-528).
  *  image: (batch, nframes, *shape) complex64, or float32 if image_real == 1.
  *  kspace: (batch, total) complex64.
@@ -226,8 +228,8 @@ int dmr_nufft_forward(dmr_plan *plan, const void *image, int image_real,
                       size_t workspace_bytes, void *stream);
 
 /*
- * Adjoint NUFFT: gridding (weight, 1/scale, ifftshift folded), cuFFT inverse,
- * fftshift + crop + 1/G + apodisation (one kernel).
+ * Adjoint NUFFT: gridding (weight, 1/scale, ifftshift folded), inverse FFT +
+ * fftshift + crop + 1/G + apodisation (fused passes, or cuFFT and a crop kernel).
  * Replaces _apply_nufft_adj (src/deepmr/fft/nufft.py:531-606).
  *  kspace: (batch, total) complex64, or float32 if kspace_real == 1.
  *  image: (batch, nframes, *shape) complex64.
