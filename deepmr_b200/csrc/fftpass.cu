@@ -15,7 +15,8 @@ using namespace fftp;
 namespace {
 
 // the lengths with a compiled transform (grid extents of common matrix sizes
-// at oversampling 1.25 and 2), as (L, L1, L2); other lengths use cuFFT. The
+// at oversampling 1.25 and 2), as (L, L1, L2); other lengths run with
+// their factors at run time (any_factors) or through cuFFT. The
 // smaller factor first: more threads wait for fewer loads each in step A, and no
 // warp is idle there (rows forward, 280 = 14 x 20, 500 x 16 images of 224^2:
 // 1.98 ms with 20 first, 1.53 with 14; columns 1.73 and 1.60). The cropping row
