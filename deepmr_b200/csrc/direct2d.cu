@@ -335,6 +335,9 @@ int d2_build(dmr_plan *p, float *const rk[3], cudaStream_t st)
     const Geom &g = p->g;
     const int W = g.W[0];
     if (g.ndim != 2 || g.total == 0 || W < 2 || W > 6 || g.W[1] != W) return DMR_OK;
+    // a record holds its first tap as x | y << 16, y in the upper half of a
+    // signed int: longer grids keep the bin kernels
+    if (g.G[0] > 65536 || g.G[1] > 32768) return DMR_OK;
     DMR_TRY(plan_alloc(p->device, &p->d2_rec, (size_t)g.total * d2_rec(W), st));
     int2 *base = nullptr;
     DMR_TRY(plan_alloc(p->device, &base, g.total, st));

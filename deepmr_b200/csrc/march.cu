@@ -1022,8 +1022,9 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     // their samples (their plans keep the bin kernels)
     if (ncells >= INT32_MAX || ncells > 16 * g.total + (1 << 24)) return DMR_OK;
     // 2D tiles pay from a few samples per tile on (below, a tile's flush costs
-    // more than its samples' own additions: direct2d.cu)
-    if (g.ndim == 2 && g.total < 4 * nft) return DMR_OK;
+    // more than its samples' own additions: direct2d.cu), and go with the
+    // interleaved grids of direct2d.cu, which has built its records before
+    if (g.ndim == 2 && (p->d2_W == 0 || g.total < 4 * nft)) return DMR_OK;
     const bool d3 = g.ndim == 3;
     // lists: gridding units of 1, 2, 4, 8 planes (2D: 1), interpolation items (3D)
     const int nl = d3 ? 5 : 1;

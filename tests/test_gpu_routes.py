@@ -1,0 +1,108 @@
+"""Calls at the limits of the interleaved kernels: what they do not take runs on
+the other kernels with the same results, and what a plan asks of its caller does
+not depend on which calls it has seen.
+
+Tolerance: relative L2 error <= 1e-5 in float32 against float64 sums or the
+oracle, as in the other parity tests.
+"""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+TOL = 1e-5
+
+
+def rel(a, b):
+    a = np.asarray(torch.as_tensor(a).detach().cpu(), dtype=np.complex128).ravel()
+    b = np.asarray(torch.as_tensor(b).detach().cpu(), dtype=np.complex128).ravel()
+    return float(np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+class CPlan:
+    """A plan through the C ABI with grid extents of its own (the public call keeps
+    extents in 16 bits), no oversampling: sample k sits at grid position k + G // 2."""
+
+    def __init__(self, grid, width, coord):
+        from deepmr_b200 import _lib
+
+        self.L, self.lib = _lib.lib(), _lib
+        self.grid, self.width, self.n, nd = grid, width, len(coord), len(grid)
+        self.beta = 2.34 * width
+        self.coord = torch.as_tensor(coord).cuda()
+        self.handle = ctypes.c_void_p()
+        shape, ones = _lib.i32_array(grid), _lib.f32_array([1.0] * nd)
+        _lib.check(self.L.dmr_plan_create(
+            nd, shape, shape, _lib.i32_array([width] * nd), _lib.f32_array([self.beta] * nd), ones, _lib.ptr(self.coord),
+            (ctypes.c_int64 * 2)(0, self.n), 1, None, self.stream(), ctypes.byref(self.handle)))
+        # taps of every sample: FFT-order positions and weights, float64 from the float32 coordinate
+        idx, w = np.zeros(self.n, dtype=np.int64)[:, None], np.ones((self.n, 1))
+        for a in reversed(range(nd)):  # z first: row-major
+            G = grid[nd - 1 - a]
+            k = (coord[:, a] + np.float32(G // 2)).astype(np.float64)
+            x = np.ceil(k - width / 2)[:, None] + np.arange(width)
+            u = (x - k[:, None]) / (width / 2)
+            wa = np.where(np.abs(u) <= 1, np.i0(self.beta * np.sqrt(np.maximum(1 - u * u, 0))), 0)
+            idx = (idx[:, :, None] * G + ((x.astype(np.int64) - G // 2) % G)[:, None, :]).reshape(self.n, -1)
+            w = (w[:, :, None] * wa[:, None, :]).reshape(self.n, -1)
+        scale = ctypes.c_double()
+        _lib.check(self.L.dmr_plan_scale(self.handle, ctypes.byref(scale)))
+        self.idx, self.w = idx, w / scale.value
+
+    def stream(self):
+        return self.lib.stream_ptr(torch.device("cuda", torch.cuda.current_device()))
+
+    def interp(self, g):
+        y = torch.full((g.shape[0], self.n), float("nan"), dtype=torch.complex64, device="cuda")
+        self.lib.check(self.L.dmr_interp(self.handle, self.lib.ptr(g), self.lib.ptr(y), len(g), None, 0, self.stream()))
+        return y
+
+    def gridding(self, y, det):
+        g = torch.full((y.shape[0],) + tuple(self.grid), float("nan"), dtype=torch.complex64, device="cuda")
+        self.lib.check(self.L.dmr_grid(self.handle, self.lib.ptr(y), 0, self.lib.ptr(g), len(y), None, 0, int(det),
+                                       self.stream()))
+        return g
+
+    def exact_interp(self, g):
+        g = g.cpu().numpy().astype(np.complex128).reshape(g.shape[0], -1)
+        return np.stack([(c[self.idx] * self.w).sum(1) for c in g])
+
+    def exact_gridding(self, y):
+        n = int(np.prod(self.grid))
+        out = []
+        for c in y.cpu().numpy().astype(np.complex128):
+            v, i = (c[:, None] * self.w).ravel(), self.idx.ravel()
+            out.append(np.bincount(i, v.real, n) + 1j * np.bincount(i, v.imag, n))
+        return np.stack(out)
+
+    def close(self):
+        self.lib.check(self.L.dmr_plan_destroy(self.handle))
+
+
+def _samples(grid, n, seed):
+    """All over the grid and its last cells on each side."""
+    rng = np.random.default_rng(seed)
+    ext = np.asarray(grid[::-1], dtype=np.float64)
+    c = rng.uniform(-0.5, 0.5, (n, len(grid))) * (ext - 1)
+    c[-16:] = np.sign(c[-16:]) * (ext / 2 - rng.uniform(0.5, 3.0, (16, len(grid))))
+    return c.astype(np.float32)
+
+
+@pytest.mark.parametrize("grid", [(8, 65536), (8, 65537), (32768, 8), (32769, 8)], ids=lambda g: f"{g[0]}x{g[1]}")
+@pytest.mark.parametrize("nsamples", [300, 140000], ids=["sparse", "dense"])
+def test_long_2d_grids(grid, nsamples):
+    """The longest grids whose positions fit a 2D record (65,536 x, 32,768 y) and
+    the next ones, below and above the density that tiles are used from."""
+    from deepmr_b200 import synth
+
+    p = CPlan(grid, 4, _samples(grid, nsamples, 1))
+    for k in (1, 3):
+        g = synth.complex_gaussian((k,) + grid, seed=1).cuda()
+        y = synth.complex_gaussian((k, nsamples), seed=2).cuda()
+        assert rel(p.interp(g), p.exact_interp(g)) < TOL, k
+        assert rel(p.gridding(y, False), p.exact_gridding(y)) < TOL, k
+    p.close()
