@@ -34,6 +34,7 @@ SYMBOLS = (
     "dmr_tc_timeouts",
     "dmr_plan_status",
     "dmr_tc_test_stall",
+    "dmr_plan_test_alloc",
     "dmr_fft3_fused",
     "dmr_tc_min_coils",
     "dmr_scratch_release",
@@ -90,6 +91,7 @@ _SIGS = {
     "dmr_tc_timeouts": (ctypes.c_int, [i64p, ctypes.c_int]),
     "dmr_plan_status": (ctypes.c_int, [vp, i32p, ctypes.c_int, vp]),
     "dmr_tc_test_stall": (ctypes.c_int, [ctypes.c_int]),
+    "dmr_plan_test_alloc": (ctypes.c_int, [ctypes.c_int]),
     "dmr_fft3_fused": (ctypes.c_int, [vp]),
     "dmr_tc_min_coils": (ctypes.c_int, [ctypes.c_int]),
     "dmr_scratch_release": (ctypes.c_int, [ctypes.c_int]),

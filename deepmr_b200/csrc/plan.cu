@@ -278,8 +278,13 @@ cudaMemPool_t plan_pool(int dev)
     return pool;
 }
 
+// test hook (dmr_plan_test_alloc): plan allocations of this thread until one
+// fails, 0: none does
+static thread_local int t_fail_alloc = 0;
+
 int plan_alloc_bytes(int dev, void **p, size_t bytes, cudaStream_t st)
 {
+    DMR_CHECK(t_fail_alloc == 0 || --t_fail_alloc > 0, DMR_ERR_OOM, "plan allocation of %zu bytes failed (test)", bytes);
     cudaMemPool_t pool = plan_pool(dev);
     DMR_CHECK(pool, DMR_ERR_CUDA, "no memory pool on device %d", dev);
     DMR_CUDA(cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st));
@@ -328,6 +333,12 @@ extern "C" int dmr_detect_cartesian(const float *coord, int64_t npts, int ndim,
     if (rc == DMR_OK)
         for (int a = 0; a < ndim; a++) is_cart_xyz[a] = h[a];
     return rc;
+}
+
+extern "C" int dmr_plan_test_alloc(int n)
+{
+    t_fail_alloc = std::max(n, 0);
+    return DMR_OK;
 }
 
 extern "C" int dmr_plan_destroy(dmr_plan *p)
@@ -632,6 +643,21 @@ static int tg_build(dmr_plan *p, int32_t *keys, int32_t *keys_s, int32_t *vals, 
 
 }  // namespace dmr
 
+namespace {
+
+// a plan under construction: work on its buffers may be in flight on `st` when
+// an error returns early, and the destructor frees them on another stream
+struct Unfinished {
+    cudaStream_t st;
+    void operator()(dmr_plan *p) const
+    {
+        cudaStreamSynchronize(st);
+        delete p;
+    }
+};
+
+}  // namespace
+
 extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os_shape,
                                const int32_t *width, const float *beta, const float *oversamp,
                                const float *coord, const int64_t *frame_offsets, int64_t nframes,
@@ -653,7 +679,7 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     DMR_CHECK(coord || total == 0, DMR_ERR_INVALID, "coord is NULL");
 
     cudaStream_t st = (cudaStream_t)stream;
-    std::unique_ptr<dmr_plan> p(new dmr_plan());
+    std::unique_ptr<dmr_plan, Unfinished> p(new dmr_plan(), Unfinished{st});
     DMR_CUDA(cudaGetDevice(&p->device));
     Geom &g = p->g;
     memset(&g, 0, sizeof(g));

@@ -250,7 +250,8 @@ struct dmr_plan {
     // (dmr_plan_status; 0 while every result is valid)
     int32_t *status = nullptr;
 
-// (the owner has synchronised the device: nothing uses the buffers any more)
+    // (the owner has synchronised the device, or the stream that a plan was being
+    // built on: nothing uses the buffers any more)
     ~dmr_plan()
     {
         auto drop = [](void *q) {

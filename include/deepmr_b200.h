@@ -87,6 +87,13 @@ int dmr_plan_status(dmr_plan *plan, int32_t *failed, int reset, void *stream);
 int dmr_tc_test_stall(int enable);
 
 /*
+ * Test hook, no reference counterpart: the n-th allocation of plan memory that
+ * the calling thread makes from now on fails with DMR_ERR_OOM (once; n <= 0:
+ * none does). Returns 0.
+ */
+int dmr_plan_test_alloc(int n);
+
+/*
  * Query, no reference counterpart: 1 if the plan's forward / adjoint NUFFT
  * run their 2D or 3D FFT as the library's fused passes (apodise + zero-pad +
  * FFT, inverse FFT + crop + 1/G + apodisation, pruned to the lines with data),

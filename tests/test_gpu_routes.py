@@ -106,3 +106,59 @@ def test_long_2d_grids(grid, nsamples):
         assert rel(p.interp(g), p.exact_interp(g)) < TOL, k
         assert rel(p.gridding(y, False), p.exact_gridding(y)) < TOL, k
     p.close()
+
+
+def test_failed_plan_creation_leaves_nothing_in_flight():
+    """Whatever allocation fails while a plan is being made, the call returns only
+    when the work on the plan's buffers is done (they are freed on another
+    stream), and the next plan is made as ever."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import _lib, synth
+    from oracle import nufft_ref as R
+
+    c3 = torch.as_tensor(synth.kooshball_3d(60, 32, 16).astype(np.float32))
+    c2 = torch.as_tensor(synth.radial_2d(24, 32, 16).astype(np.float32))
+    s = torch.cuda.Stream()
+    failed = 0
+    with torch.cuda.stream(s):
+        for c, shape in ((c3, (16, 16, 16)), (c2, (16, 16))):
+            args = _plan_args(c, shape)
+            for n in range(1, 200):
+                torch.cuda._sleep(10_000_000)  # some milliseconds of other work first
+                _lib.lib().dmr_plan_test_alloc(n)
+                try:
+                    h = args()
+                except _lib.DmrError as e:
+                    assert e.code == -3 and s.query(), n
+                    failed += 1
+                    continue
+                finally:
+                    _lib.lib().dmr_plan_test_alloc(0)
+                _lib.check(_lib.lib().dmr_plan_destroy(h))
+                break
+            else:
+                pytest.fail("no plan was made")
+    assert failed > 20
+    img = synth.complex_gaussian((3, 16, 16, 16), seed=1)
+    plan = F.plan_nufft(c3, 16, 4, 1.25, device="cuda")
+    assert rel(F.apply_nufft(img.cuda(), plan), R.apply_nufft(img, R.plan_nufft(c3, 16, 4, 1.25))) < TOL
+
+
+def _plan_args(coord, shape):
+    """A call that makes a plan of width 4 and oversampling 1.25 on the current
+    stream and returns its handle (no other allocations in between)."""
+    from deepmr_b200 import _lib
+
+    nd = len(shape)
+    flat = coord.reshape(-1, nd).cuda().contiguous()
+    torch.cuda.synchronize()
+
+    def make():
+        h = ctypes.c_void_p()
+        _lib.check(_lib.lib().dmr_plan_create(
+            nd, _lib.i32_array(shape), _lib.i32_array([-(-5 * s // 4) for s in shape]), _lib.i32_array([4] * nd),
+            _lib.f32_array([7.2] * nd), _lib.f32_array([1.25] * nd), _lib.ptr(flat), (ctypes.c_int64 * 2)(0, len(flat)), 1,
+            None, _lib.stream_ptr(flat.device), ctypes.byref(h)))
+        return h
+
+    return make
