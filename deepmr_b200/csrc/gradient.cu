@@ -168,7 +168,7 @@ extern "C" int dmr_nufft_traj_grad(dmr_plan *p, const void *image, int image_rea
     const float inv = (float)(1.0 / p->scale);
     const float post = (float)post_scale;
 #define TG(N, W)                                                                                              \
-    traj_grad_kernel<N, W><<<blocks, threads, 0, st>>>(g, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx, \
+    traj_grad_kernel<N, W><<<blocks, threads, 0, st>>>(g, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, \
                                                        d_foff, grid, (const float2 *)v, batch, weight,        \
                                                        weight_per_batch, inv, rs[0], rs[1], rs[2], post, grad)
     const int w4 = wm <= 4 ? 4 : 8;

@@ -14,6 +14,7 @@
 #include <map>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <numeric>
 #include <string>
 
@@ -359,16 +360,9 @@ namespace dmr {
 // whose calls run on the interleaved kernels build them on the first call that
 // needs them (trajectory gradients in 3D, deterministic gridding over its
 // scratch limit, no pool memory): a host loop over all bins, milliseconds.
-int plan_bins(const dmr_plan *cp, cudaStream_t st)
+static int bins_build(const dmr_plan *p, PlanBins &out, cudaStream_t st)
 {
-    dmr_plan *p = const_cast<dmr_plan *>(cp);
-    std::lock_guard<std::mutex> lock(p->bins_mu);
-    if (p->bins_ready) return DMR_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    DMR_CUDA(cudaStreamIsCapturing(st, &cap));
-    DMR_CHECK(cap == cudaStreamCaptureStatusNone, DMR_ERR_UNSUPPORTED,
-              "this call builds bin structures on its first use: run it once before capturing it");
-    Geom &g = p->g;
+    const Geom &g = p->g;
     const int ndim = g.ndim, dev = p->device;
     const int64_t total = g.total, nframes = g.nframes;
     float *const *rk = p->rk;
@@ -379,8 +373,8 @@ int plan_bins(const dmr_plan *cp, cudaStream_t st)
     DMR_TRY(tmp.alloc(&keys_s, total));
     DMR_TRY(tmp.alloc(&vals, total));
     DMR_TRY(tmp.alloc(&counts, nkeys));
-    for (int a = 0; a < ndim; a++) DMR_TRY(plan_alloc(dev, &p->scoord[a], total, st));
-    DMR_TRY(plan_alloc(dev, &p->sidx, total, st));
+    for (int a = 0; a < ndim; a++) DMR_TRY(plan_alloc(dev, &out.scoord[a], total, st));
+    DMR_TRY(plan_alloc(dev, &out.sidx, total, st));
     DMR_CUDA(cudaMemsetAsync(counts, 0, nkeys * sizeof(int32_t), st));
 
     // Within a bin, samples are sorted by the cell of their first tap (register
@@ -396,15 +390,15 @@ int plan_bins(const dmr_plan *cp, cudaStream_t st)
         int end_bit = 1;
         while ((1ll << end_bit) < nsort) end_bit++;
         size_t temp_bytes = 0;
-        DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_s, vals, p->sidx,
+        DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, temp_bytes, keys, keys_s, vals, out.sidx,
                                                  (int)total, 0, end_bit, st));
         char *temp = nullptr;
         DMR_TRY(tmp.alloc(&temp, temp_bytes));
-        DMR_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_s, vals, p->sidx,
+        DMR_CUDA(cub::DeviceRadixSort::SortPairs(temp, temp_bytes, keys, keys_s, vals, out.sidx,
                                                  (int)total, 0, end_bit, st));
         g_launches.fetch_add(1);
         gather_sorted_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(
-            total, ndim, p->sidx, rk[0], rk[1], rk[2], p->scoord[0], p->scoord[1], p->scoord[2]);
+            total, ndim, out.sidx, rk[0], rk[1], rk[2], out.scoord[0], out.scoord[1], out.scoord[2]);
         DMR_LAUNCHED("gather_sorted_kernel");
     }
     std::vector<int32_t> h_counts(nkeys);
@@ -492,18 +486,18 @@ int plan_bins(const dmr_plan *cp, cudaStream_t st)
         by_color[col].push_back({(int)key, h_start[key], h_start[key + 1]});
     }
     std::vector<WorkItem> det;
-    p->det_color_start.assign(1, 0);
+    out.det_color_start.assign(1, 0);
     for (int c = 0; c < ncolors; c++) {
         // heaviest bins first inside a pass (shorter tail)
         std::stable_sort(by_color[c].begin(), by_color[c].end(), [](const WorkItem &x, const WorkItem &y) {
             return (x.end - x.begin) > (y.end - y.begin);
         });
         det.insert(det.end(), by_color[c].begin(), by_color[c].end());
-        p->det_color_start.push_back((int)det.size());
+        out.det_color_start.push_back((int)det.size());
     }
-    DMR_TRY(plan_alloc(dev, &p->det_work, det.size(), st));
+    DMR_TRY(plan_alloc(dev, &out.det_work, det.size(), st));
     if (!det.empty())
-        DMR_CUDA(cudaMemcpyAsync(p->det_work, det.data(), det.size() * sizeof(WorkItem),
+        DMR_CUDA(cudaMemcpyAsync(out.det_work, det.data(), det.size() * sizeof(WorkItem),
                                  cudaMemcpyHostToDevice, st));
 
     // the same items visited in 4x4x4-bin tiles (frame, tile z, y, x, bin z, y, x):
@@ -527,26 +521,51 @@ int plan_bins(const dmr_plan *cp, cudaStream_t st)
         std::stable_sort(worder.begin(), worder.end(),
                          [&](int32_t a, int32_t b) { return tkey(items[a]) < tkey(items[b]); });
     }
-    p->nwork = (int)items.size();
-    p->ntiles = (int)order.size();
-    DMR_TRY(plan_alloc(dev, &p->bin_start, nkeys + 1, st));
-    DMR_TRY(plan_alloc(dev, &p->work, items.size(), st));
-    DMR_TRY(plan_alloc(dev, &p->tiles, order.size(), st));
-    DMR_CUDA(cudaMemcpyAsync(p->bin_start, h_start.data(), (nkeys + 1) * sizeof(int32_t),
+    out.nwork = (int)items.size();
+    out.ntiles = (int)order.size();
+    DMR_TRY(plan_alloc(dev, &out.bin_start, nkeys + 1, st));
+    DMR_TRY(plan_alloc(dev, &out.work, items.size(), st));
+    DMR_TRY(plan_alloc(dev, &out.tiles, order.size(), st));
+    DMR_CUDA(cudaMemcpyAsync(out.bin_start, h_start.data(), (nkeys + 1) * sizeof(int32_t),
                              cudaMemcpyHostToDevice, st));
-    DMR_TRY(plan_alloc(dev, &p->work_order, items.size(), st));
+    DMR_TRY(plan_alloc(dev, &out.work_order, items.size(), st));
     if (!items.empty()) {
-        DMR_CUDA(cudaMemcpyAsync(p->work, items.data(), items.size() * sizeof(WorkItem),
+        DMR_CUDA(cudaMemcpyAsync(out.work, items.data(), items.size() * sizeof(WorkItem),
                                  cudaMemcpyHostToDevice, st));
-        DMR_CUDA(cudaMemcpyAsync(p->work_order, worder.data(), worder.size() * sizeof(int32_t),
+        DMR_CUDA(cudaMemcpyAsync(out.work_order, worder.data(), worder.size() * sizeof(int32_t),
                                  cudaMemcpyHostToDevice, st));
     }
-    DMR_CUDA(cudaMemcpyAsync(p->tiles, order.data(), order.size() * sizeof(int32_t),
+    DMR_CUDA(cudaMemcpyAsync(out.tiles, order.data(), order.size() * sizeof(int32_t),
                              cudaMemcpyHostToDevice, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    DMR_TRY(rt_build(p, h_start, st));
+    DMR_TRY(rt_build(p, out, h_start, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    p->bins_ready = true;
+    return DMR_OK;
+}
+
+int plan_bins(const dmr_plan *p, cudaStream_t st)
+{
+    if (p->bins_ptr.load(std::memory_order_acquire)) return DMR_OK;
+    std::lock_guard<std::mutex> lock(p->bins_mu);
+    if (p->bins_ptr.load(std::memory_order_relaxed)) return DMR_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    DMR_CUDA(cudaStreamIsCapturing(st, &cap));
+    DMR_CHECK(cap == cudaStreamCaptureStatusNone, DMR_ERR_UNSUPPORTED,
+              "this call builds bin structures on its first use: run it once before capturing it");
+    int rc = DMR_OK;
+    std::unique_ptr<PlanBins> b;
+    try {
+        b.reset(new PlanBins());
+        rc = bins_build(p, *b, st);
+    } catch (const std::bad_alloc &) {  // (the host lists)
+        set_error("no host memory for the plan's bins");
+        rc = DMR_ERR_OOM;
+    }
+    if (rc != DMR_OK) {
+        cudaStreamSynchronize(st);  // the buffers that go now may be in use
+        return rc;
+    }
+    p->bins_ptr.store(b.release(), std::memory_order_release);
     return DMR_OK;
 }
 

@@ -3,6 +3,7 @@
 
 #include <cufft.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -29,8 +30,10 @@ struct Geom {
     int64_t gsize;  // grid points per (batch, frame)
     int64_t isize;  // image points per (batch, frame)
     int64_t total;  // samples over all frames
-    int nr[3];      // register-tile gridding: block regions per axis (0: not planned)
-    int nregions;   // block regions per frame
+    // register-tile gridding, set for its launches (PlanBins): block regions per
+    // axis, and per frame
+    int nr[3];
+    int nregions;
 };
 
 // One block-level unit of interpolation / atomic-gridding work: a chunk of
@@ -95,14 +98,49 @@ struct PlanTemp {
     }
 };
 
-// the bin kernels' structures, built on first use (plan.cu)
+// The bin kernels' structures of a plan: built aside by plan_bins and then
+// published whole (dmr_plan::bins), so that a call sees all of them or none and
+// nothing a call reads without them ever changes.
+struct PlanBins {
+    float *scoord[3] = {nullptr, nullptr, nullptr};  // sorted rescaled coordinates
+    int32_t *sidx = nullptr;            // sorted position -> global sample index
+    int32_t *bin_start = nullptr;       // (nframes * nbins + 1)
+    WorkItem *work = nullptr;           // interpolation / atomic gridding items
+    int nwork = 0;
+    int32_t *work_order = nullptr;      // item order in 4x4x4-bin tiles (L2 reuse of halos and spokes)
+    int32_t *tiles = nullptr;           // owner-gridding tile order (heavy first)
+    int ntiles = 0;
+    // deterministic gridding: whole non-empty bins grouped by colour; bins of
+    // one colour have disjoint tile + halo regions
+    WorkItem *det_work = nullptr;
+    std::vector<int> det_color_start;   // host, ncolors + 1
+    // register-tile gridding (3D): block regions per axis (0: not planned) and
+    // frame, block items, reduction items for regions split over several blocks,
+    // and the number of partial-sum slots
+    int nr[3] = {0, 0, 0};
+    int nregions = 0;
+    RtItem *rt_items = nullptr;
+    int nrt = 0;
+    RtItem *rt_reduce = nullptr;
+    int nrt_reduce = 0;
+    int rt_slots = 0;
+    // (the owner has synchronised, as ~dmr_plan's)
+    ~PlanBins()
+    {
+        for (void *q : {(void *)scoord[0], (void *)scoord[1], (void *)scoord[2], (void *)sidx, (void *)bin_start,
+                        (void *)work, (void *)work_order, (void *)tiles, (void *)det_work, (void *)rt_items,
+                        (void *)rt_reduce})
+            if (q) cudaFreeAsync(q, cudaStreamPerThread);
+    }
+};
+// builds them on first use (plan.cu)
 int plan_bins(const ::dmr_plan *p, cudaStream_t st);
 // Register-tile gridding: whether the geometry admits it (3D, grid at least
 // a block region plus the kernel support on every axis); plan the block items after the bin sort (host
 // bin offsets h_start, nframes * nbins + 1 entries); scratch bytes a call of
 // `batch` coils needs (0 when the kernel does not apply).
 bool rt_geometry_ok(const Geom &g);
-int rt_build(::dmr_plan *p, const std::vector<int32_t> &h_start, cudaStream_t st);
+int rt_build(const ::dmr_plan *p, PlanBins &b, const std::vector<int32_t> &h_start, cudaStream_t st);
 size_t rt_scratch_bytes(const ::dmr_plan *p, int64_t batch);
 // scratch bytes of deterministic tensor-core gridding (every work item's
 // region partial sums, 2 KB per item and coil)
@@ -173,11 +211,10 @@ struct dmr_plan {
     // in acquisition order
     char *tables = nullptr;
     float *rk[3] = {nullptr, nullptr, nullptr};
-    // bin structures (plan_bins)
-    std::mutex bins_mu;
-    bool bins_ready = false;
-    float *scoord[3] = {nullptr, nullptr, nullptr};  // sorted rescaled coordinates
-    int32_t *sidx = nullptr;            // sorted position -> global sample index
+    // bin structures: null until plan_bins has published them
+    mutable std::mutex bins_mu;
+    mutable std::atomic<const dmr::PlanBins *> bins_ptr{nullptr};
+    const dmr::PlanBins &bins() const { return *bins_ptr.load(std::memory_order_acquire); }
     // 3D tensor-core gridding: bins of its own (tile tg_T, x y z) whose region
     // (tile + W - 1 per axis) is at most 7 x 6 x 6 = 252 points, one N = 256
     // MMA; the samples of a bin in acquisition order (consecutive samples of a
@@ -202,25 +239,8 @@ struct dmr_plan {
     // tg_item_start[k + 1]) of tg_work for bin key k (frame * tg_nbins + bin;
     // items are numbered in key order, a bin's segments in sample order)
     int32_t *tg_item_start = nullptr;
-    int32_t *bin_start = nullptr;       // (nframes * nbins + 1)
-    dmr::WorkItem *work = nullptr;      // interpolation / atomic gridding items
-    int nwork = 0;
-    int32_t *work_order = nullptr;      // item order in 4x4x4-bin tiles (L2 reuse of halos and spokes)
-    int32_t *tiles = nullptr;           // owner-gridding tile order (heavy first)
-    int ntiles = 0;
-    // deterministic gridding: whole non-empty bins grouped by colour; bins of
-    // one colour have disjoint tile + halo regions
-    dmr::WorkItem *det_work = nullptr;
-    std::vector<int> det_color_start;   // host, ncolors + 1
     float *apod[3] = {nullptr, nullptr, nullptr};  // per-axis apodisation (image index)
     int64_t *foff_dev = nullptr;        // frame offsets on the device (nframes + 1)
-    // register-tile gridding (3D): block items, reduction items for regions
-    // split over several blocks, and the number of partial-sum slots
-    dmr::RtItem *rt_items = nullptr;
-    int nrt = 0;
-    dmr::RtItem *rt_reduce = nullptr;
-    int nrt_reduce = 0;
-    int rt_slots = 0;
     // march order (march.cu; mp_W == 0: not planned; 3D, and 2D plans dense enough
     // for tiles, which have gridding units only): tiles along x and y,
     // CSR offsets per cell, sorted position -> sample and back, per sorted
@@ -258,11 +278,8 @@ struct dmr_plan {
             if (q) cudaFreeAsync(q, cudaStreamPerThread);
         };
         drop(tables);
-        for (int a = 0; a < 3; a++) {
-            drop(scoord[a]);
-            drop(rk[a]);
-        }
-        drop(sidx);
+        delete bins_ptr.load();
+        for (int a = 0; a < 3; a++) drop(rk[a]);
         for (int a = 0; a < 3; a++) drop(tg_scoord[a]);
         drop(tg_sidx);
         drop(tg_w);
@@ -270,13 +287,6 @@ struct dmr_plan {
         drop(tg_work);
         drop(tg_order);
         drop(tg_item_start);
-        drop(bin_start);
-        drop(work);
-        drop(work_order);
-        drop(tiles);
-        drop(det_work);
-        cudaFree(rt_items);
-        cudaFree(rt_reduce);
         drop(status);
         drop(mp_cstart);
         drop(mp_sidx);

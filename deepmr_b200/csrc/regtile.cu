@@ -492,11 +492,9 @@ bool rt_geometry_ok(const Geom &g)
     return true;
 }
 
-int rt_build(dmr_plan *p, const std::vector<int32_t> &h_start, cudaStream_t st)
+int rt_build(const dmr_plan *p, PlanBins &b, const std::vector<int32_t> &h_start, cudaStream_t st)
 {
-    Geom &g = p->g;
-    g.nr[0] = g.nr[1] = g.nr[2] = 0;
-    g.nregions = 0;
+    const Geom &g = p->g;
     if (!rt_geometry_ok(g)) return DMR_OK;
     int nr[3];
     for (int a = 0; a < 3; a++) nr[a] = (int)ceil_div(g.G[a], rt_extent(a));
@@ -565,36 +563,31 @@ int rt_build(dmr_plan *p, const std::vector<int32_t> &h_start, cudaStream_t st)
                      [&](const Reg &x, const Reg &y) { return tile_key(x.region) < tile_key(y.region); });
     for (const Reg &r : light) items.push_back({r.region, 0, 1, -1});
 
-    cudaFree(p->rt_items);
-    cudaFree(p->rt_reduce);
-    p->rt_items = nullptr;
-    p->rt_reduce = nullptr;
-    DMR_CUDA(cudaMalloc(&p->rt_items, std::max<size_t>(1, items.size()) * sizeof(RtItem)));
-    DMR_CUDA(cudaMalloc(&p->rt_reduce, std::max<size_t>(1, red.size()) * sizeof(RtItem)));
-    DMR_CUDA(cudaMemcpyAsync(p->rt_items, items.data(), items.size() * sizeof(RtItem),
-                             cudaMemcpyHostToDevice, st));
+    DMR_TRY(plan_alloc(p->device, &b.rt_items, items.size(), st));
+    DMR_TRY(plan_alloc(p->device, &b.rt_reduce, red.size(), st));
+    DMR_CUDA(cudaMemcpyAsync(b.rt_items, items.data(), items.size() * sizeof(RtItem), cudaMemcpyHostToDevice, st));
     if (!red.empty())
-        DMR_CUDA(cudaMemcpyAsync(p->rt_reduce, red.data(), red.size() * sizeof(RtItem),
-                                 cudaMemcpyHostToDevice, st));
+        DMR_CUDA(cudaMemcpyAsync(b.rt_reduce, red.data(), red.size() * sizeof(RtItem), cudaMemcpyHostToDevice, st));
     DMR_CUDA(cudaStreamSynchronize(st));
-    p->nrt = (int)items.size();
-    p->nrt_reduce = (int)red.size();
-    p->rt_slots = slots;
-    for (int a = 0; a < 3; a++) g.nr[a] = nr[a];
-    g.nregions = nregions;
+    b.nrt = (int)items.size();
+    b.nrt_reduce = (int)red.size();
+    b.rt_slots = slots;
+    for (int a = 0; a < 3; a++) b.nr[a] = nr[a];
+    b.nregions = nregions;
     return DMR_OK;
 }
 
 static bool rt_applies(const dmr_plan *p, int64_t batch)
 {
-    return p->g.nregions > 0 && p->nrt > 0 && batch >= kRtMinBatch && getenv("DMR_NO_RT") == nullptr;
+    const PlanBins *b = p->bins_ptr.load(std::memory_order_acquire);
+    return b && b->nregions > 0 && b->nrt > 0 && batch >= kRtMinBatch && getenv("DMR_NO_RT") == nullptr;
 }
 
 size_t rt_scratch_bytes(const dmr_plan *p, int64_t batch)
 {
-    if (!rt_applies(p, batch) || p->rt_slots == 0) return 0;
+    if (!rt_applies(p, batch) || p->bins().rt_slots == 0) return 0;
     const int64_t ncc = ceil_div(batch, kRtCoils);
-    return (size_t)p->rt_slots * ncc * kRtPts * kRtCoils * sizeof(float2);
+    return (size_t)p->bins().rt_slots * ncc * kRtPts * kRtCoils * sizeof(float2);
 }
 
 // Library-owned stream-ordered pool for the scratch of calls without a
@@ -625,6 +618,14 @@ static cudaMemPool_t find_pool(int dev, bool create)
 
 cudaMemPool_t scratch_pool(int dev) { return find_pool(dev, true); }
 
+static Geom rt_geom(const dmr_plan *p)
+{
+    Geom g = p->g;
+    for (int a = 0; a < 3; a++) g.nr[a] = p->bins().nr[a];
+    g.nregions = p->bins().nregions;
+    return g;
+}
+
 template <int W>
 static int rt_launch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
                      const float *weight, int wpb, float2 *scratch, int ncc, float inv_scale, cudaStream_t st)
@@ -632,8 +633,8 @@ static int rt_launch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     auto kern = grid_rt_kernel<W>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RtShared));
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute", __FILE__, __LINE__);
-    kern<<<dim3(p->nrt, ncc), kRtThreads, sizeof(RtShared), st>>>(
-        p->g, p->rt_items, p->bin_start, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx, ksp, kreal,
+    kern<<<dim3(p->bins().nrt, ncc), kRtThreads, sizeof(RtShared), st>>>(
+        rt_geom(p), p->bins().rt_items, p->bins().bin_start, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, ksp, kreal,
         grid, scratch, batch, weight, wpb, inv_scale);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     e = cudaGetLastError();
@@ -670,8 +671,8 @@ int grid_rt_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     case 7: rc = rt_launch<7>(p, ksp, kreal, grid, batch, weight, wpb, sp, ncc, inv_scale, st); break;
     default: rc = rt_launch<8>(p, ksp, kreal, grid, batch, weight, wpb, sp, ncc, inv_scale, st); break;
     }
-    if (rc == DMR_OK && p->nrt_reduce > 0) {
-        grid_rt_reduce_kernel<<<dim3(p->nrt_reduce, ncc), 256, 0, st>>>(p->g, p->rt_reduce,
+    if (rc == DMR_OK && p->bins().nrt_reduce > 0) {
+        grid_rt_reduce_kernel<<<dim3(p->bins().nrt_reduce, ncc), 256, 0, st>>>(rt_geom(p), p->bins().rt_reduce,
                                                                         (const float2 *)scratch, grid,
                                                                         batch, inv_scale);
         g_launches.fetch_add(1, std::memory_order_relaxed);

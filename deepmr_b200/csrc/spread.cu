@@ -1087,8 +1087,8 @@ static int launch_interp(const dmr_plan *p, const float2 *grid, float2 *ksp, int
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t chunks = ceil_div(batch, 1ll << l);
     DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
-    dim3 grd(p->nwork, (unsigned)chunks);
-    kern<<<grd, 256, smem, st>>>(g, p->work, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx,
+    dim3 grd(p->bins().nwork, (unsigned)chunks);
+    kern<<<grd, 256, smem, st>>>(g, p->bins().work, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx,
                                  grid, ksp, batch, weight, wpb, (float)p->scale, l);
     DMR_LAUNCHED("interp_kernel");
     return DMR_OK;
@@ -1111,9 +1111,9 @@ static int launch_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *gr
         DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         const int64_t chunks = ceil_div(batch, 1ll << l);
         DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
-        if (p->nwork == 0) return DMR_OK;
-        dim3 grd(p->nwork, (unsigned)chunks);
-        kern<<<grd, 256, smem, st>>>(g, p->work, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx,
+        if (p->bins().nwork == 0) return DMR_OK;
+        dim3 grd(p->bins().nwork, (unsigned)chunks);
+        kern<<<grd, 256, smem, st>>>(g, p->bins().work, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx,
                                      ksp, kreal, grid, batch, weight, wpb, (float)p->scale, l);
         DMR_LAUNCHED("grid_atomic_kernel");
         return DMR_OK;
@@ -1129,9 +1129,9 @@ static int launch_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *gr
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t chunks = ceil_div(batch, 1ll << l);
     DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
-    dim3 grd((unsigned)ceil_div(p->ntiles, kOwnerWarps), (unsigned)chunks);
-    kern<<<grd, 32 * kOwnerWarps, smem, st>>>(g, p->tiles, p->ntiles, p->bin_start, p->scoord[0],
-                                              p->scoord[1], p->scoord[2], p->sidx, ksp, kreal, grid,
+    dim3 grd((unsigned)ceil_div(p->bins().ntiles, kOwnerWarps), (unsigned)chunks);
+    kern<<<grd, 32 * kOwnerWarps, smem, st>>>(g, p->bins().tiles, p->bins().ntiles, p->bins().bin_start, p->bins().scoord[0],
+                                              p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, ksp, kreal, grid,
                                               batch, weight, wpb, (float)p->scale, l);
     DMR_LAUNCHED("grid_owner_kernel");
     return DMR_OK;
@@ -1216,8 +1216,8 @@ static int launch_interp_cube(const dmr_plan *p, const float2 *grid, float2 *ksp
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t chunks = ceil_div(batch, 1ll << l);
     DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
-    kern<<<dim3(p->nwork, (unsigned)chunks), kCubeThreads, smem, st>>>(
-        p->g, rg, p->work, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx, grid, ksp, batch, weight,
+    kern<<<dim3(p->bins().nwork, (unsigned)chunks), kCubeThreads, smem, st>>>(
+        p->g, rg, p->bins().work, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, grid, ksp, batch, weight,
         wpb, (float)(1.0 / p->scale), l);
     DMR_LAUNCHED("interp_cube_kernel");
     return DMR_OK;
@@ -1236,13 +1236,13 @@ static int launch_grid_cube(const dmr_plan *p, const void *ksp, int kreal, float
     const int l = cube_config<NDIM, W, CR>(p->g, batch, rg, smem, 32);
     DMR_CHECK(l >= 0, DMR_ERR_UNSUPPORTED, "gridding tile does not fit in shared memory");
     DMR_CUDA(cudaMemsetAsync(grid, 0, (size_t)batch * p->g.nframes * p->g.gsize * sizeof(float2), st));
-    if (p->nwork == 0) return DMR_OK;
+    if (p->bins().nwork == 0) return DMR_OK;
     auto kern = grid_cube_kernel<NDIM, W, CR>;
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t chunks = ceil_div(batch, 1ll << l);
     DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
-    kern<<<dim3(p->nwork, (unsigned)chunks), kCubeThreads, smem, st>>>(
-        p->g, rg, p->work, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx, ksp, kreal, grid, batch,
+    kern<<<dim3(p->bins().nwork, (unsigned)chunks), kCubeThreads, smem, st>>>(
+        p->g, rg, p->bins().work, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, ksp, kreal, grid, batch,
         weight, wpb, (float)(1.0 / p->scale), l);
     DMR_LAUNCHED("grid_cube_kernel");
     return DMR_OK;
@@ -1263,17 +1263,17 @@ static int launch_grid_slab_nr(const dmr_plan *p, const void *ksp, int kreal, fl
     DMR_CHECK(chunks < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
     const float inv = (float)(1.0 / p->scale);
     if (ATOMIC) {
-        kern<<<dim3(p->nwork, (unsigned)chunks), 32 * W, smem, st>>>(
-            p->g, rg, p->work, p->scoord[0], p->scoord[1], p->scoord[2], p->sidx, ksp, kreal, grid, batch,
+        kern<<<dim3(p->bins().nwork, (unsigned)chunks), 32 * W, smem, st>>>(
+            p->g, rg, p->bins().work, p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx, ksp, kreal, grid, batch,
             weight, wpb, inv, l);
         DMR_LAUNCHED("grid_slab_kernel");
         return DMR_OK;
     }
-    for (size_t c = 0; c + 1 < p->det_color_start.size(); c++) {
-        const int n = p->det_color_start[c + 1] - p->det_color_start[c];
+    for (size_t c = 0; c + 1 < p->bins().det_color_start.size(); c++) {
+        const int n = p->bins().det_color_start[c + 1] - p->bins().det_color_start[c];
         if (n == 0) continue;
         kern<<<dim3(n, (unsigned)chunks), 32 * W, smem, st>>>(
-            p->g, rg, p->det_work + p->det_color_start[c], p->scoord[0], p->scoord[1], p->scoord[2], p->sidx,
+            p->g, rg, p->bins().det_work + p->bins().det_color_start[c], p->bins().scoord[0], p->bins().scoord[1], p->bins().scoord[2], p->bins().sidx,
             ksp, kreal, grid, batch, weight, wpb, inv, l);
         DMR_LAUNCHED("grid_slab_kernel");
     }
@@ -1299,7 +1299,7 @@ static int launch_grid_slab(const dmr_plan *p, const void *ksp, int kreal, float
     }
     DMR_CHECK(l >= 0, DMR_ERR_UNSUPPORTED, "gridding tile does not fit in shared memory");
     DMR_CUDA(cudaMemsetAsync(grid, 0, (size_t)batch * p->g.nframes * p->g.gsize * sizeof(float2), st));
-    if (p->nwork == 0) return DMR_OK;
+    if (p->bins().nwork == 0) return DMR_OK;
     switch (l) {
     case 5: return launch_grid_slab_nr<NDIM, W, 1, ATOMIC>(p, ksp, kreal, grid, batch, weight, wpb, l, rg, smem, st);
     case 4: return launch_grid_slab_nr<NDIM, W, 2, ATOMIC>(p, ksp, kreal, grid, batch, weight, wpb, l, rg, smem, st);

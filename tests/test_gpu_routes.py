@@ -162,3 +162,80 @@ def _plan_args(coord, shape):
         return h
 
     return make
+
+
+def _problem3(n=24, views=160, samples=64, coils=9):
+    """A 3D plan of width 4 whose bin structures are not built, images, k-space."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+
+    c = torch.as_tensor(synth.kooshball_3d(views, samples, n).astype(np.float32))
+    plan = F.plan_nufft(c, n, 4, 1.25, device="cuda")
+    img = synth.complex_gaussian((coils, n, n, n), seed=1).cuda()
+    ksp = synth.complex_gaussian((coils,) + tuple(c.shape[:-1]), seed=2).cuda()
+    return plan, img, ksp
+
+
+def test_bins_build_that_fails_leaves_the_plan_as_it_was():
+    """Bin structures that could not be allocated are given back, and the next
+    call builds them: any number of failures costs no memory (4 x 80 MB each
+    here, were they kept)."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import _lib
+
+    rng = np.random.default_rng(3)
+    c = torch.as_tensor((rng.uniform(-0.5, 0.5, (1, 20_000_000, 3)) * 64).astype(np.float32))
+    plan = F.plan_nufft(c, 64, 4, 1.25, device="cuda")
+    img = torch.ones((1, 64, 64, 64), dtype=torch.complex64, device="cuda")
+    v = torch.ones((1,) + tuple(c.shape[:-1]), dtype=torch.complex64, device="cuda")
+    free = []
+    for n in (10,) * 12:  # after the sorted coordinates and indices
+        _lib.lib().dmr_plan_test_alloc(n)
+        try:
+            with pytest.raises(_lib.DmrError) as e:
+                F.traj_grad(plan, img, v)
+        finally:
+            _lib.lib().dmr_plan_test_alloc(0)
+        assert e.value.code == -3
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert free[1] - free[-1] < 400 << 20, [f >> 20 for f in free]
+    g = F.traj_grad(plan, img, v)
+    assert torch.isfinite(g).all() and float(g.abs().max()) > 0
+
+
+def test_threads_on_a_plan_without_bins():
+    """Several threads' calls on one plan while one of them builds its bin
+    structures: every result is that of a thread alone."""
+    import threading
+
+    import deepmr_b200.fft as F
+
+    plan, img, ksp = _problem3()
+    adj = F.apply_nufft_adj(ksp, plan)
+    fwd = F.apply_nufft(img, plan)
+    ref = F.traj_grad(_problem3()[0], img, ksp)
+    errors, out = [], {}
+    start = threading.Barrier(6)
+
+    def work(i):
+        try:
+            torch.cuda.set_device(0)
+            with torch.cuda.stream(torch.cuda.Stream()):
+                start.wait()
+                for _ in range(5):
+                    out[i] = (F.traj_grad(plan, img, ksp) if i < 2 else
+                              F.apply_nufft_adj(ksp, plan) if i < 4 else F.apply_nufft(img, plan))
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    torch.cuda.synchronize()
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    for i in range(6):
+        assert rel(out[i], (ref, ref, adj, adj, fwd, fwd)[i]) < 1e-6, i
