@@ -206,9 +206,12 @@ static int nufft_ws(dmr_plan *p, int64_t batch, void *ws, size_t ws_bytes, Nufft
     }
     const size_t grid_bytes = align_up((size_t)slots * g.nframes * g.gsize * sizeof(float2), 256);
     const size_t fft_bytes = fp ? align_up(fp->work_bytes, 256) : 0;
-    const size_t rt_bytes = align_up(grid_scratch_bytes(p, batch), 256);
-    // the register-tile scratch and the march buffers are never in use together
-    const size_t total = grid_bytes + fft_bytes + std::max(rt_bytes, rows_bytes + il_bytes);
+    // (plans of the interleaved kernels build the register tiles' lists with the
+    // bins, when a call needs them: their scratch, whose size is not known before,
+    // comes from the library pool, so that a plan asks for the same workspace all
+    // its life)
+    const size_t rt_bytes = p->il_forward() ? 0 : align_up(grid_scratch_bytes(p, batch), 256);
+    const size_t total = grid_bytes + fft_bytes + rt_bytes + rows_bytes + il_bytes;
     if (need) *need = total;
     if (!ws) return DMR_OK;
     DMR_CHECK(ws_bytes >= total, DMR_ERR_WORKSPACE, "workspace too small: %zu < %zu", ws_bytes, total);
@@ -632,7 +635,7 @@ static int lowrank_ws(dmr_plan *p, int64_t batch, int64_t ncoeff, void *ws, size
     const size_t coef_bytes = align_up((size_t)batch * ncoeff * g.gsize * sizeof(float2), 256);
     const size_t frame_bytes = align_up((size_t)batch * g.nframes * g.gsize * sizeof(float2), 256);
     const size_t fft_bytes = align_up(fp->work_bytes, 256);
-    const size_t rt_bytes = align_up(grid_scratch_bytes(p, batch), 256);
+    const size_t rt_bytes = p->il_forward() ? 0 : align_up(grid_scratch_bytes(p, batch), 256);  // as in nufft_ws
     size_t total = coef_bytes + frame_bytes + fft_bytes + rt_bytes;
     size_t ic = 0, ifr = 0;
     out.il = p->il_forward() && fft3_applies(p);

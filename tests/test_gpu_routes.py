@@ -239,3 +239,45 @@ def test_threads_on_a_plan_without_bins():
     assert not errors, errors
     for i in range(6):
         assert rel(out[i], (ref, ref, adj, adj, fwd, fwd)[i]) < 1e-6, i
+
+
+@pytest.mark.parametrize("width,os", [(4, 1.25), (6, 1.25)])
+def test_workspace_does_not_grow(width, os):
+    """A workspace sized before the plan's bin structures were built serves the
+    calls after it, all that a plan can make: dense samples (register tiles split
+    over blocks), 8 coils and more."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import _lib
+
+    L, n, total, k = _lib.lib(), 32, 1_000_000, 8
+    rng = np.random.default_rng(4)
+    c = torch.as_tensor((rng.uniform(-0.5, 0.5, (1, total, 3)) * n).astype(np.float32))
+    plan = F.plan_nufft(c, n, width, os, device="cuda")
+    ip = plan.interpolator
+    ws, wl = ip.workspace(k), ip.workspace_lowrank(k, 1)
+    ksp = torch.ones((k,) + tuple(c.shape[:-1]), dtype=torch.complex64, device="cuda")
+    img = torch.ones((k, n, n, n), dtype=torch.complex64, device="cuda")
+    one = torch.ones((1, 1), dtype=torch.complex64, device="cuda")
+    st = _lib.stream_ptr(ip.device)
+
+    def adjoint(w, det):
+        out = torch.empty_like(img)
+        _lib.check(L.dmr_nufft_adjoint(ip.handle, _lib.ptr(ksp), 0, _lib.ptr(out), k, None, 0, det, _lib.ptr(w), w.numel(), st))
+        return out
+
+    def lowrank(w, det):
+        out = torch.empty_like(img)
+        _lib.check(L.dmr_nufft_adjoint_lowrank(ip.handle, _lib.ptr(ksp), 0, 1, _lib.ptr(one), _lib.ptr(out), k, None, 0, det,
+                                               _lib.ptr(w), w.numel(), st))
+        return out
+
+    before = [adjoint(ws, d) for d in (0, 1)] + [lowrank(wl, d) for d in (0, 1)]
+    F.traj_grad(plan, img, ksp)  # builds the bins
+    assert (ip.workspace(k).numel(), ip.workspace_lowrank(k, 1).numel()) == (ws.numel(), wl.numel())
+    after = [adjoint(ws, d) for d in (0, 1)] + [lowrank(wl, d) for d in (0, 1)]
+    assert torch.equal(before[1], after[1]) and torch.equal(before[3], after[3])
+    old = F.set_deterministic_scratch_limit(1)  # register tiles
+    try:
+        assert all(torch.isfinite(t).all() for t in after + [adjoint(ws, 1), lowrank(wl, 1)])
+    finally:
+        F.set_deterministic_scratch_limit(old)
