@@ -957,13 +957,17 @@ int launch_planes(const dmr_plan *p, const MarchGeom &m, const float2 *rows, flo
     return launch_planes_np<W, 8, 3>(p, m, rows, grid, scratch, st);
 }
 
+// dynamic shared memory of a gather block: cover lists of the x positions, unit
+// ranges of up to 8 rows of tiles
+size_t gather_smem(const MarchGeom &m) { return (size_t)m.G[0] * sizeof(uint4) + (size_t)8 * m.nt0 * sizeof(int2); }
+
 template <int W>
 int launch_gather(const dmr_plan *p, const MarchGeom &m, const float2 *scratch, float2 *grid, cudaStream_t st)
 {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = (size_t)m.G[0] * sizeof(uint4) + (size_t)8 * m.nt0 * sizeof(int2);
+    const size_t smem = gather_smem(m);
     auto kern = grid_planes_gather_kernel<W>;
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const int64_t nrows = (int64_t)p->g.nframes * m.G[2] * m.G[1];
@@ -1224,6 +1228,22 @@ int march_interp(const dmr_plan *p, const float2 *grid, bool planar, float2 *ksp
     return DMR_OK;
 }
 
+// scratch of deterministic gridding: every unit's plane of one chunk of coils.
+// DMR_ERR_UNSUPPORTED (another deterministic kernel takes the call) where that
+// is over the caller's limit, and on grids too wide for the gather: its lists
+// must fit in shared memory (7,264 x positions at widths 2..4, 6,225 at 5 and 6)
+// and its entries hold a tile in 13 bits
+static int det_scratch(const dmr_plan *p, const MarchGeom &m, int64_t det_limit, size_t *need)
+{
+    const int R = m.T + p->mp_W - 1;
+    *need = std::max<size_t>((size_t)p->mp_nunits[0] * R * R * m.CS * sizeof(float2), 256);
+    if (det_limit > 0 && *need > (size_t)det_limit) return DMR_ERR_UNSUPPORTED;
+    int dev = 0, limit = 0;
+    DMR_CUDA(cudaGetDevice(&dev));
+    DMR_CUDA(cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    return gather_smem(m) > (size_t)limit || std::max(m.nt0, m.nt1) > 8191 ? DMR_ERR_UNSUPPORTED : DMR_OK;
+}
+
 int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool planar, int64_t batch,
                const float *weight, int wpb, int det, int64_t det_limit, float2 *rows, float2 *il, cudaStream_t st)
 {
@@ -1249,11 +1269,8 @@ int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool
         return DMR_OK;
     }
     if (det) {
-        // every unit's plane of one chunk of coils; over the caller's limit, or
-        // no memory for it: another deterministic kernel takes the call
-        const int R = march_tile(p->mp_W) + p->mp_W - 1;
-        const size_t need = std::max<size_t>((size_t)p->mp_nunits[0] * R * R * ch.CS * sizeof(float2), 256);
-        if (det_limit > 0 && need > (size_t)det_limit) return DMR_ERR_UNSUPPORTED;
+        size_t need = 0;
+        DMR_TRY(det_scratch(p, m, det_limit, &need));
         cudaMemPool_t pool = scratch_pool(p->device);
         if (pool == nullptr) return DMR_ERR_UNSUPPORTED;
         void *owned = nullptr;
@@ -1318,6 +1335,10 @@ int march_interp_pool(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_
 int march_grid_pool(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch, const float *weight,
                     int wpb, int det, int64_t det_limit, cudaStream_t st)
 {
+    if (det && p->mp_W) {  // (before the buffers are allocated)
+        size_t need = 0;
+        DMR_TRY(det_scratch(p, march_geom(p, march_chunks(p, batch).CS), det_limit, &need));
+    }
     MarchPool b(p, batch, st);
     if (!b.owned) return DMR_ERR_UNSUPPORTED;
     return march_grid(p, ksp, kreal, grid, true, batch, weight, wpb, det, det_limit, b.rows, b.il, st);

@@ -54,8 +54,8 @@ size_t march_il_bytes(const ::dmr_plan *p, int CS);
 // chunks, or planar (coil, frame, z, y, x) with `il` the interleaved grid of one
 // chunk; `rows`: the rows of one chunk. Deterministic gridding takes its
 // scratch (every unit's plane of a chunk) from the library pool;
-// DMR_ERR_UNSUPPORTED, before any launch, when that exceeds det_limit (> 0) or
-// the pool has no memory.
+// DMR_ERR_UNSUPPORTED, before any launch, when that exceeds det_limit (> 0), the
+// grid is too wide for its gather, or the pool has no memory.
 int march_interp(const ::dmr_plan *p, const float2 *grid, bool planar, float2 *ksp, int64_t batch, const float *weight,
                  int wpb, float2 *rows, float2 *il, cudaStream_t st);
 int march_grid(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool planar, int64_t batch,

@@ -281,3 +281,20 @@ def test_workspace_does_not_grow(width, os):
         assert all(torch.isfinite(t).all() for t in after + [adjoint(ws, 1), lowrank(wl, 1)])
     finally:
         F.set_deterministic_scratch_limit(old)
+
+
+@pytest.mark.parametrize("grid,width,nsamples", [((8, 7264), 4, 20000), ((8, 7265), 4, 20000), ((8, 6400), 6, 24000),
+                                                 ((32768, 8), 4, 140000), ((8, 8, 7300), 4, 5000)],
+                         ids=lambda v: "x".join(map(str, v)) if isinstance(v, tuple) else str(v))
+def test_deterministic_on_wide_grids(grid, width, nsamples):
+    """Deterministic gridding on the widest grid that the planes' gather holds in
+    shared memory and on wider ones, which the other deterministic kernels take."""
+    from deepmr_b200 import synth
+
+    p = CPlan(grid, width, _samples(grid, nsamples, 5))
+    for k in (1, 3):
+        y = synth.complex_gaussian((k, nsamples), seed=2).cuda()
+        g = p.gridding(y, True)
+        assert rel(g, p.exact_gridding(y)) < TOL, k
+        assert torch.equal(g, p.gridding(y, True)), k
+    p.close()
