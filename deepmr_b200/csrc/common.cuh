@@ -22,6 +22,7 @@ extern std::atomic<int64_t> g_launches;
 inline int cuda_fail(cudaError_t e, const char *what, const char *file, int line)
 {
     set_error("%s:%d %s: %s", file, line, what, cudaGetErrorString(e));
+    cudaGetLastError();  // reported: the next launch's check is not to find it again
     return e == cudaErrorMemoryAllocation ? DMR_ERR_OOM : DMR_ERR_CUDA;
 }
 

@@ -298,3 +298,19 @@ def test_deterministic_on_wide_grids(grid, width, nsamples):
         assert rel(g, p.exact_gridding(y)) < TOL, k
         assert torch.equal(g, p.gridding(y, True)), k
     p.close()
+
+
+def test_a_reported_error_is_not_reported_again():
+    """After an allocation has failed, the next call works (its launches do not
+    find the earlier error)."""
+    from deepmr_b200 import _lib, synth
+
+    make = _plan_args(torch.as_tensor(synth.kooshball_3d(60, 32, 16).astype(np.float32)), (16, 16, 16))
+    _lib.lib().dmr_plan_test_alloc(8)
+    try:
+        with pytest.raises(_lib.DmrError) as e:
+            make()
+    finally:
+        _lib.lib().dmr_plan_test_alloc(0)
+    assert e.value.code == -3
+    _lib.check(_lib.lib().dmr_plan_destroy(make()))
