@@ -543,6 +543,18 @@ static int bins_build(const dmr_plan *p, PlanBins &out, cudaStream_t st)
     return DMR_OK;
 }
 
+namespace {
+
+// For its scope the thread's calls that a stream capture forbids elsewhere
+// (allocation, synchronisation of other streams) are allowed
+struct Uncaptured {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+}  // namespace
+
 int plan_bins(const dmr_plan *p, cudaStream_t st)
 {
     if (p->bins_ptr.load(std::memory_order_acquire)) return DMR_OK;
@@ -550,8 +562,14 @@ int plan_bins(const dmr_plan *p, cudaStream_t st)
     if (p->bins_ptr.load(std::memory_order_relaxed)) return DMR_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     DMR_CUDA(cudaStreamIsCapturing(st, &cap));
-    DMR_CHECK(cap == cudaStreamCaptureStatusNone, DMR_ERR_UNSUPPORTED,
-              "this call builds bin structures on its first use: run it once before capturing it");
+    // while the caller captures, the structures are built on a stream of their
+    // own: what they are built from was complete when the plan was made
+    const Uncaptured mode;
+    cudaStream_t own = nullptr;
+    if (cap != cudaStreamCaptureStatusNone) {
+        DMR_CUDA(cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking));
+        st = own;
+    }
     int rc = DMR_OK;
     std::unique_ptr<PlanBins> b;
     try {
@@ -561,10 +579,13 @@ int plan_bins(const dmr_plan *p, cudaStream_t st)
         set_error("no host memory for the plan's bins");
         rc = DMR_ERR_OOM;
     }
-    if (rc != DMR_OK) {
-        cudaStreamSynchronize(st);  // the buffers that go now may be in use
-        return rc;
+    // (on an error the buffers that go now may be in use)
+    if (rc != DMR_OK) cudaStreamSynchronize(st);
+    if (own) {
+        cudaStreamSynchronize(own);
+        cudaStreamDestroy(own);
     }
+    if (rc != DMR_OK) return rc;
     p->bins_ptr.store(b.release(), std::memory_order_release);
     return DMR_OK;
 }

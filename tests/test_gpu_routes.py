@@ -314,3 +314,41 @@ def test_a_reported_error_is_not_reported_again():
         _lib.lib().dmr_plan_test_alloc(0)
     assert e.value.code == -3
     _lib.check(_lib.lib().dmr_plan_destroy(make()))
+
+
+@pytest.mark.parametrize("call", ["gradient 3D", "deterministic sparse 2D", "over the scratch limit", "over the limit, 3 coils"])
+def test_first_call_that_needs_bins_is_captured(call):
+    """A plan's first call that needs its bin structures builds them while it is
+    being captured, and the replays give what the call gives by itself."""
+    import gc
+
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+
+    if call == "deterministic sparse 2D":
+        c = torch.as_tensor(synth.radial_2d(6, 64, 32).astype(np.float32))
+        make = lambda: F.plan_nufft(c, 32, 4, 1.25, device="cuda")  # noqa: E731
+        ksp = synth.complex_gaussian((3,) + tuple(c.shape[:-1]), seed=2).cuda()
+    else:
+        make = lambda: _problem3()[0]  # noqa: E731
+        _, img, ksp = _problem3()
+        if call.endswith("3 coils"):
+            ksp = ksp[:3].contiguous()
+    run = (lambda p: F.traj_grad(p, img, ksp)) if call == "gradient 3D" else (lambda p: F.apply_nufft_adj(ksp, p))
+    old = F.set_deterministic_gridding(True), F.set_deterministic_scratch_limit(1 if "limit" in call else 0)
+    try:
+        ref = run(make())  # (another plan: kernels and tables are loaded)
+        plan = make()
+        gc.collect()  # (a plan that is destroyed synchronises the device, which a capture forbids)
+        torch.cuda.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = run(plan)
+        for _ in range(2):
+            out.zero_()
+            graph.replay()
+            assert torch.equal(out, ref)
+        assert torch.equal(run(plan), ref)
+    finally:
+        F.set_deterministic_gridding(old[0])
+        F.set_deterministic_scratch_limit(old[1])
