@@ -67,6 +67,14 @@ __host__ __device__ __forceinline__ int pmod(int v, int n)
 
 __host__ __device__ __forceinline__ int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+// For its scope the thread's calls that a stream capture forbids elsewhere
+// (allocation, synchronisation of other streams) are allowed
+struct Uncaptured {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace dmr

@@ -3,7 +3,6 @@
 #include <cmath>
 #include <map>
 #include <mutex>
-#include <tuple>
 #include <vector>
 
 #include "fftpass.cuh"
@@ -50,11 +49,12 @@ bool has_len(int L)
     }
 }
 
-// per-device twiddle tables: entry k1 L2 + n2 is
-// exp(-2 pi i n2 k1 / L), from double precision; `crop`: with the factors
-// exchanged, for the cropping row pass
+// per-device twiddle tables of a length: entry k1 L2 + n2 is
+// exp(-2 pi i n2 k1 / L), from double precision; then the same with the factors
+// exchanged, for the cropping row pass (`crop`). Both are uploaded at once, on a
+// stream of their own, so that a call can be captured whatever ran before it
 std::mutex g_tw_mu;
-std::map<std::tuple<int, int, bool>, float2 *> g_tw;
+std::map<std::pair<int, int>, float2 *> g_tw;
 
 int second_factor(int L, bool crop)
 {
@@ -71,24 +71,30 @@ int twiddles(int L, bool crop, const float2 **out)
     int dev = 0;
     DMR_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lk(g_tw_mu);
-    const auto key = std::make_tuple(dev, L, crop);
-    auto it = g_tw.find(key);
-    if (it != g_tw.end()) {
-        *out = it->second;
-        return DMR_OK;
+    float2 *&d = g_tw[{dev, L}];
+    if (!d) {
+        std::vector<float2> h(2 * L);
+        const double two_pi = 6.283185307179586476925286766559;
+        for (int t = 0; t < 2 * L; t++) {
+            const int L2 = second_factor(L, t >= L), e = t % L;
+            const double ang = two_pi * (double)((e / L2) * (e % L2)) / (double)L;
+            h[t] = make_float2((float)std::cos(ang), (float)-std::sin(ang));
+        }
+        const Uncaptured mode;
+        cudaStream_t st = nullptr;
+        float2 *p = nullptr;
+        DMR_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        cudaError_t e = cudaMalloc(&p, h.size() * sizeof(float2));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p, h.data(), h.size() * sizeof(float2), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        cudaStreamDestroy(st);
+        if (e != cudaSuccess) {
+            if (p) cudaFree(p);
+            return cuda_fail(e, "twiddle table", __FILE__, __LINE__);
+        }
+        d = p;
     }
-    std::vector<float2> h(L);
-    const double two_pi = 6.283185307179586476925286766559;
-    const int L2 = second_factor(L, crop);
-    for (int t = 0; t < L; t++) {
-        const double ang = two_pi * (double)((t / L2) * (t % L2)) / (double)L;
-        h[t] = make_float2((float)std::cos(ang), (float)-std::sin(ang));
-    }
-    float2 *d = nullptr;
-    DMR_CUDA(cudaMalloc(&d, L * sizeof(float2)));
-    DMR_CUDA(cudaMemcpy(d, h.data(), L * sizeof(float2), cudaMemcpyHostToDevice));
-    g_tw[key] = d;
-    *out = d;
+    *out = d + (crop ? L : 0);
     return DMR_OK;
 }
 

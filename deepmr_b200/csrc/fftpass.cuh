@@ -42,7 +42,6 @@
 #include <cmath>
 #include <map>
 #include <mutex>
-#include <tuple>
 #include <utility>
 #include <vector>
 

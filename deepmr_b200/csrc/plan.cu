@@ -543,18 +543,6 @@ static int bins_build(const dmr_plan *p, PlanBins &out, cudaStream_t st)
     return DMR_OK;
 }
 
-namespace {
-
-// For its scope the thread's calls that a stream capture forbids elsewhere
-// (allocation, synchronisation of other streams) are allowed
-struct Uncaptured {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~Uncaptured() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
-}  // namespace
-
 int plan_bins(const dmr_plan *p, cudaStream_t st)
 {
     if (p->bins_ptr.load(std::memory_order_acquire)) return DMR_OK;

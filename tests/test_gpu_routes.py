@@ -352,3 +352,36 @@ def test_first_call_that_needs_bins_is_captured(call):
     finally:
         F.set_deterministic_gridding(old[0])
         F.set_deterministic_scratch_limit(old[1])
+
+
+@pytest.mark.parametrize("warm,shape", [(None, (187, 209)), ("forward", (221, 143)), ("adjoint", (165, 253))],
+                         ids=["cold", "forward warmed", "adjoint warmed"])
+def test_captures_of_calls_that_have_not_run(warm, shape):
+    """Both directions captured when neither or only the other has run, at
+    transform lengths that nothing else here uses (twiddle tables)."""
+    import gc
+
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+    from oracle import nufft_ref as R
+
+    c = torch.as_tensor(synth.radial_2d(30, 64, 64).astype(np.float32))
+    plan = F.plan_nufft(c, shape, 4, 2.0, device="cuda")
+    img = synth.complex_gaussian((3,) + shape, seed=1)
+    ksp = synth.complex_gaussian((3,) + tuple(c.shape[:-1]), seed=2)
+    x, y = img.cuda(), ksp.cuda()
+    calls = {"forward": lambda: F.apply_nufft(x, plan), "adjoint": lambda: F.apply_nufft_adj(y, plan)}
+    if warm:
+        calls[warm]()
+    gc.collect()
+    torch.cuda.synchronize()
+    out = {}
+    for name, call in calls.items():
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            out[name] = call()
+        g.replay()
+    torch.cuda.synchronize()
+    oplan = R.plan_nufft(c, shape, 4, 2.0)
+    assert rel(out["forward"], R.apply_nufft(img, oplan)) < TOL
+    assert rel(out["adjoint"], R.apply_nufft_adj(ksp, oplan)) < TOL
