@@ -44,13 +44,21 @@ __host__ __device__ constexpr int march_rec(int W, int ndim = 3) { return (ndim 
 
 // visits of a gridding unit / samples of an interpolation item, at most: heavier
 // ones (the centre of k-space) are split so that no warp runs far behind. A
-// unit's sums are chains in float32, so its length also sets the rounding error
-// where k-space is dense (radial 100^3, 4,000 views of 180, 12 coils: 10.4e-7 of
-// the result at 512 visits, 9.3 at 128, 9.0 at 64, 8.8 with no chain to speak
-// of), and several planes to a warp cost no more in short units (512 and 64: 772
-// and 790 us; 64^3, 8 coils: 265 and 240). With a plane per warp a unit's flush
-// weighs more (192^3, 32 coils: 12.2 and 13.7 ms)
-constexpr int unit_visits(int ndim, int np) { return ndim == 3 && np == 1 ? 512 : 64; }
+// unit's sums are a chain in float32 and the units of a plane are another (a
+// quarter as long where a block's warps add theirs first), so that errors grow
+// with a unit's length and with its inverse: 64 visits is where they are least
+// (adjoint of 48^3, 12 coils, W 6, os 1.25, against 64 bits: 7.4e-6 of the result
+// at 8 visits, 4.4 at 64, 3.7 with blocks adding first, 5.9 at 512; 64^3, 8 coils,
+// W 4: 8.1e-7 at 64, 10.2 at 512), and several planes to a warp cost no more in
+// short units (512 and 64: 772 and 790 us; 64^3, 8 coils: 265 and 240). With a
+// plane per warp a unit's flush weighs more (192^3, 32 coils: 12.2 ms at 512, 13.7
+// at 64), so these have lists of both: see launch_planes. At width 6 all are short
+// (144^3, 32 coils: 5.1 and 5.4 ms)
+constexpr int kShortUnit = 64, kLongUnit = 512;
+// unit lists: planes per warp, the last one of short units
+constexpr int kUnitLists = 5;
+constexpr int kUnitPlanes[kUnitLists] = {1, 2, 4, 8, 1};
+constexpr int unit_visits(int ndim, int W, int list) { return ndim == 3 && W <= 5 && list == 0 ? kLongUnit : kShortUnit; }
 constexpr int kItemSamples = 144;
 constexpr int kItemZ = 8;  // z cells of an interpolation item
 // rows of cell columns of an interpolation item (a tile has T / march_rows items per z block)
@@ -353,8 +361,9 @@ __global__ void __launch_bounds__(256) transpose_kernel(const float2 *__restrict
 // side by side in the warp), and visits every sample that touches the plane:
 // per column of cells (compile-time tap positions, one case of a switch) the
 // samples of its W z-cells. The plane is then added to the grid once, 8 B per
-// lane and point, coils contiguous. No shared-memory sums, no barriers; the
-// only atomics are the R^2 additions per unit, 10.8 GB for the 192^3, 32-coil
+// lane and point, coils contiguous (pieces of a heavy plane that a block's warps
+// hold are added first). The only atomics are the R^2 additions per unit, 10.8 GB
+// for the 192^3, 32-coil
 // kooshball against 24.8 GB of per-bin regions. Rows and weight records of 16
 // visits at a time come through a double-buffered shared-memory ring of the
 // warp (cp.async).
@@ -372,7 +381,9 @@ struct PlaneShape {
     static constexpr int ROWB = CC * 8;    // bytes of a staged row
     static constexpr int RECS = kVisitBatch * ROWB, ZCS = RECS + kVisitBatch * REC * 4;
     static constexpr int BUF = ZCS + kVisitBatch * 4;  // one buffer of the ring: rows, records, z cells
-    static constexpr int SMEM = kGridWarps * 2 * BUF;
+    // shared memory of a pair of warps: their rings, then one of their planes
+    static constexpr int PLANE = R * R * 32 * 8, PAIR = 4 * BUF > PLANE ? 4 * BUF : PLANE;
+    static constexpr int SMEM = kGridWarps / 2 * PAIR;
 };
 
 template <int W, int NP, int ND>
@@ -386,8 +397,8 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
     extern __shared__ __align__(16) unsigned char msm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int u = blockIdx.x * kGridWarps + warp;
-    if (u >= nunits) return;  // warp-uniform; the kernel has no block barriers
-    const int ring = warp * 2 * S::BUF;
+    if (u >= nunits) return;  // warp-uniform; barriers join warps of one tile and plane only
+    const int ring = (warp >> 1) * S::PAIR + (warp & 1) * 2 * S::BUF;
     const int4 un = units[u];
     const int ft = un.x, z0 = un.y * NP, z1 = min(z0 + NP, g.G[2]) - 1;
     const int c = lane % CC, z = z0 + lane / CC;
@@ -536,6 +547,51 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
         }
         return;
     }
+    // pieces of one tile's plane that neighbouring warps hold are added before they
+    // go to the grid: warps 1 and 3 to 0 and 2, then 2 to 0 (through the pair's
+    // shared memory, `give` to `take`, whose barriers both sides reach). A heavy
+    // plane's sum is then a tree over units of a block and a chain over blocks, a
+    // quarter as long: it is the chain in the grid that rounds most (64^3, 8 coils:
+    // 8.4e-7 of the result without, see unit_visits)
+    static_assert(kGridWarps == 4, "pairs of warps");
+    auto same = [&](int v) {  // unit v is a piece of the same plane
+        if (v < 0 || v >= nunits) return false;
+        const int4 o = units[v];
+        return o.x == un.x && o.y == un.y;
+    };
+    auto join = [](int id) {
+        __syncwarp();
+        asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory");
+    };
+    auto give = [&](int at) {
+        float2 *d = reinterpret_cast<float2 *>(msm + at) + lane;
+#pragma unroll
+        for (int i = 0; i < R; i++)
+#pragma unroll
+            for (int k = 0; k < R; k++) d[(i * R + k) * 32] = acc[i][k];
+    };
+    auto take = [&](int at) {
+        const float2 *d = reinterpret_cast<const float2 *>(msm + at) + lane;
+#pragma unroll
+        for (int i = 0; i < R; i++)
+#pragma unroll
+            for (int k = 0; k < R; k++) acc[i][k] = __fadd2_rn(acc[i][k], d[(i * R + k) * 32]);
+    };
+    const int pair = (warp >> 1) * S::PAIR;
+    if (same(warp & 1 ? u - 1 : u + 1)) {
+        join(1 + (warp >> 1));  // both are done with their rings
+        if (warp & 1) give(pair);
+        join(1 + (warp >> 1));
+        if (warp & 1) return;
+        take(pair);
+    }
+    if (!(warp & 1) && same(warp ? u - 2 : u + 2)) {  // (the unit between is one of the plane's, too)
+        join(3);  // warp 0 has taken what lay in its pair's memory
+        if (warp) give(0);
+        join(3);
+        if (warp) return;
+        take(0);
+    }
     if (c >= g.CS || z > z1) return;
     const int ntile = g.nt0 * g.nt1;
     const int f = ft / ntile, t2 = ft - f * ntile, ty = t2 / g.nt0, tx = t2 - ty * g.nt0;
@@ -631,8 +687,12 @@ __global__ void __launch_bounds__(256) grid_planes_gather_kernel(MarchGeom g, in
                 const int dy = cover_at(ycov, ky) & 7;
                 return scratch + ((int64_t)s * (R * R) + dy * R + (vx & 7)) * g.CS + c;
             };
-            auto rest = [&](int2 u, int ky, int vx) {  // a split unit's further pieces
-                for (int s = 1; s < u.y; s++) acc = __fadd2_rn(acc, __ldcs(slot(u.x + s, ky, vx)));
+            auto rest = [&](int2 u, int ky, int vx) {  // a split unit's further pieces, added eight at a time (rounding)
+                for (int s = 1; s < u.y;) {
+                    float2 sum = __ldcs(slot(u.x + s, ky, vx));
+                    for (const int e = min(s + 8, u.y); ++s < e;) sum = __fadd2_rn(sum, __ldcs(slot(u.x + s, ky, vx)));
+                    acc = __fadd2_rn(acc, sum);
+                }
             };
             if (ny <= 2 && cover_at(xc, 2) < 0) {
                 int2 u[4];
@@ -925,11 +985,10 @@ MarchGeom march_geom(const dmr_plan *p, int CS)
 }
 
 template <int W, int NP, int ND>
-int launch_planes_np(const dmr_plan *p, const MarchGeom &m, const float2 *rows, float2 *grid, float2 *scratch,
+int launch_planes_np(const dmr_plan *p, const MarchGeom &m, int L, const float2 *rows, float2 *grid, float2 *scratch,
                      cudaStream_t st)
 {
     using S = PlaneShape<W, NP, ND>;
-    constexpr int L = NP == 1 ? 0 : (NP == 2 ? 1 : (NP == 4 ? 2 : 3));
     const int n = p->mp_nunits[L];
     if (n == 0) return DMR_OK;
     auto kern = grid_planes_kernel<W, NP, ND>;
@@ -948,13 +1007,17 @@ template <int W>
 int launch_planes(const dmr_plan *p, const MarchGeom &m, const float2 *rows, float2 *grid, float2 *scratch,
                   cudaStream_t st)
 {
-    // deterministic units are always single planes, so that a coil's sums do
-    // not depend on how many coils it is gridded with
-    if (p->g.ndim == 2) return launch_planes_np<W, 1, 2>(p, m, rows, grid, scratch, st);
-    if (scratch || m.CS > 16) return launch_planes_np<W, 1, 3>(p, m, rows, grid, scratch, st);
-    if (m.CS > 8) return launch_planes_np<W, 2, 3>(p, m, rows, grid, scratch, st);
-    if (m.CS > 4) return launch_planes_np<W, 4, 3>(p, m, rows, grid, scratch, st);
-    return launch_planes_np<W, 8, 3>(p, m, rows, grid, scratch, st);
+    if (p->g.ndim == 2) return launch_planes_np<W, 1, 2>(p, m, 0, rows, grid, scratch, st);
+    // deterministic units are always single planes of one list, so that a coil's
+    // sums do not depend on how many coils it is gridded with
+    if (scratch) return launch_planes_np<W, 1, 3>(p, m, 0, rows, grid, scratch, st);
+    // single planes in long units from 20 coils on, where these took the place of
+    // tensor-core sums (64^3, W 4: 3.7e-6 of the result, now 1.1e-6); fewer coils
+    // had the sums of the cell-cube kernel (8.0e-7; 8.1e-7 in short units)
+    if (m.CS > 16) return launch_planes_np<W, 1, 3>(p, m, m.CS < 20 && W <= 5 ? 4 : 0, rows, grid, scratch, st);
+    if (m.CS > 8) return launch_planes_np<W, 2, 3>(p, m, 1, rows, grid, scratch, st);
+    if (m.CS > 4) return launch_planes_np<W, 4, 3>(p, m, 2, rows, grid, scratch, st);
+    return launch_planes_np<W, 8, 3>(p, m, 3, rows, grid, scratch, st);
 }
 
 // dynamic shared memory of a gather block: cover lists of the x positions, unit
@@ -1030,14 +1093,14 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     // interleaved grids of direct2d.cu, which has built its records before
     if (g.ndim == 2 && (p->d2_W == 0 || g.total < 4 * nft)) return DMR_OK;
     const bool d3 = g.ndim == 3;
-    // lists: gridding units of 1, 2, 4, 8 planes (2D: 1), interpolation items (3D)
-    const int nl = d3 ? 5 : 1;
-    const int np[4] = {1, 2, 4, 8};
+    // lists: gridding units (2D: the first), interpolation items (3D)
+    const int nl = d3 ? kUnitLists + 1 : 1;
+    const auto np = kUnitPlanes;
     const int nzb = (int)ceil_div(g.G[2], kItemZ), cols = T * march_rows(W), nzbh = nzb * (TT / cols);
-    int per[5];           // entries per frame tile before splitting
-    int64_t off[6] = {0};
+    int per[kUnitLists + 1];  // entries per frame tile before splitting
+    int64_t off[kUnitLists + 2] = {0};
     for (int l = 0; l < nl; l++) {
-        per[l] = l < 4 ? (int)ceil_div(g.G[2], np[l]) : nzbh;
+        per[l] = l < kUnitLists ? (int)ceil_div(g.G[2], np[l]) : nzbh;
         off[l + 1] = off[l] + nft * per[l] + 1;
     }
     PlanTemp tmp(dev, st);
@@ -1074,9 +1137,9 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     // before its length is known
     for (int l = 0; l < nl; l++) {
         const int64_t n = off[l + 1] - off[l];
-        const int most = l < 4 ? unit_visits(g.ndim, np[l]) : kItemSamples;
+        const int most = l < kUnitLists ? unit_visits(g.ndim, W, l) : kItemSamples;
         int4 *list = nullptr;
-        if (l < 4) {
+        if (l < kUnitLists) {
             const int64_t visits = g.total * (d3 ? ceil_div(np[l] + W - 1, np[l]) + 1 : 1);
             DMR_TRY(plan_alloc(dev, &list, std::min(n, visits) + visits / most + 1, st));
             march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], d3 ? W : 1, np[l],
@@ -1085,11 +1148,11 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
             DMR_TRY(plan_alloc(dev, &list, std::min(n, g.total) + g.total / most + 1, st));
             march_item_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, cols, g.G[2], nzb, counts);
         }
-        (l < 4 ? p->mp_units[l] : p->mp_items) = list;
+        (l < kUnitLists ? p->mp_units[l] : p->mp_items) = list;
         DMR_LAUNCHED("march_count_kernel");
         DMR_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb, counts, starts + off[l], (int)n, st));
         g_launches.fetch_add(1);
-        if (l < 4)
+        if (l < kUnitLists)
             march_unit_fill_kernel<<<march_blocks(n), 256, 0, st>>>(starts + off[l], nft, per[l], most, list);
         else
             march_item_fill_kernel<<<march_blocks(n), 256, 0, st>>>(starts + off[l], nft, per[l], list);
@@ -1107,7 +1170,7 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
 
 void march_lists(dmr_plan *p, const MarchTotals &totals)
 {
-    for (int l = 0; l < totals.n; l++) (l < 4 ? p->mp_nunits[l] : p->mp_nitems) = totals.v[l];
+    for (int l = 0; l < totals.n; l++) (l < kUnitLists ? p->mp_nunits[l] : p->mp_nitems) = totals.v[l];
 }
 
 MarchChunks march_chunks(const dmr_plan *p, int64_t batch)

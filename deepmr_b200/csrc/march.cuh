@@ -26,7 +26,7 @@ struct MarchChunks {
 // takes them once the stream has been synchronised
 struct MarchTotals {
     int n = 0;
-    int32_t v[5] = {0};
+    int32_t v[6] = {0};
 };
 int march_build(::dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
                 MarchTotals &totals, cudaStream_t st);

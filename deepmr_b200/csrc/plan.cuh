@@ -245,7 +245,7 @@ struct dmr_plan {
     // for tiles, which have gridding units only): tiles along x and y,
     // CSR offsets per cell, sorted position -> sample and back, per sorted
     // sample the tap weights and z cell, gridding units for 1, 2, 4 and 8
-    // planes per warp (int4), the first unit of each (frame tile, plane), and
+    // planes per warp and short ones for 1 (int4), the first unit of each (frame tile, plane), and
     // interpolation items (int4)
     int mp_W = 0;
     int mp_nt[2] = {0, 0};
@@ -254,8 +254,8 @@ struct dmr_plan {
     int32_t *mp_inv = nullptr;
     int32_t *mp_zc = nullptr;
     float *mp_rec = nullptr;
-    void *mp_units[4] = {nullptr, nullptr, nullptr, nullptr};
-    int mp_nunits[4] = {0, 0, 0, 0};
+    void *mp_units[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+    int mp_nunits[5] = {0, 0, 0, 0, 0};
     int32_t *mp_ustart = nullptr;
     void *mp_items = nullptr;
     int mp_nitems = 0;

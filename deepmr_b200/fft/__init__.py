@@ -67,7 +67,7 @@ def set_deterministic_gridding(flag=True):
     """Select the gridding kernel used by the adjoint NUFFT.
 
     True: bitwise reproducible — 3D plans store the plane of every gridding
-    unit (a tile's plane, or 512 samples of a heavier one), and a gather then
+    unit (a tile's plane, or 512 samples of a heavier one, 64 at width 6), and a gather then
     adds the planes per grid point in a fixed order (they take 392 bytes per
     unit and coil at width 4 in the library's scratch pool: see
     release_scratch); other plans with one owner per grid point or per tile.
