@@ -753,7 +753,7 @@ struct InterpShape {
     static constexpr int RX = T + W - 1, RYE = H + W - 1, RZ = kItemZ + W - 1, PTS = RX * RYE * RZ;
     static constexpr int TILE = (PTS * CC * 8 + 15) / 16 * 16;
     static constexpr int SMEM = TILE + kItemCap * (REC * 4 + 4);
-    static constexpr int MINB = NZ == 1 ? 2 : 4;
+    static constexpr int MINB = NZ == 1 || SPL * RY * W > 64 ? 2 : 4;
 };
 
 template <int W, int NZ, int NY>
@@ -958,6 +958,99 @@ __global__ void __launch_bounds__(32 * InterpShape<W, NZ, NY>::NW, InterpShape<W
     }
 }
 
+// Few coils: the same items and regions, a thread per sample. Lanes as (plane
+// group, coil) leave most of a warp idle then, and a region staged for more coils
+// than there are keeps blocks off the SM.
+constexpr int kFewThreads = 128;
+
+template <int W, int CC>
+__global__ void __launch_bounds__(kFewThreads)
+    interp_few_kernel(MarchGeom g, const int4 *__restrict__ items, const int32_t *__restrict__ cstart,
+                      const float *__restrict__ rec, const int32_t *__restrict__ zc, const float2 *__restrict__ grid,
+                      float2 *__restrict__ rows)
+{
+    using S = InterpShape<W, W, 1>;
+    constexpr int T = S::T, TT = T * T, REC = S::REC, RX = S::RX, RYE = S::RYE, COLS = S::COLS, NH = TT / COLS;
+    __shared__ __align__(16) float2 tile[S::PTS * CC];
+    __shared__ int s_beg[COLS], s_pre[COLS + 1];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int4 it = items[blockIdx.x];
+    const int ft = it.x, h = it.y % NH, z0 = it.y / NH * kItemZ, z1 = min(z0 + kItemZ, g.G[2]);
+    const int ntile = g.nt0 * g.nt1;
+    const int f = ft / ntile, t2 = ft - f * ntile, ty = t2 / g.nt0, tx = t2 - ty * g.nt0;
+    // region points, CC coils each
+    const float2 *gf = grid + f * g.gsize * g.CS;
+    for (int e = tid; e < S::PTS * CC; e += kFewThreads) {
+        const int pt = e / CC, c = e - pt * CC;
+        const int x = pt % RX, r = pt / RX, y = r % RYE, z = r / RYE;
+        const int gx = (tx * T + x + g.G[0] - g.half[0]) % g.G[0], gy = (ty * T + h * S::H + y + g.G[1] - g.half[1]) % g.G[1],
+                  gz = (z0 + z + g.G[2] - g.half[2]) % g.G[2];
+        if (c < g.CS) cp8(smem_addr(tile + e), gf + (gz * g.plane + (int64_t)gy * g.G[0] + gx) * g.CS + c);
+    }
+    cp_commit();
+    if (tid < 32) {
+        // the columns' sample ranges (this part of them) and their offsets in the item
+        int beg = 0, cnt = 0;
+        if (lane < COLS) {
+            const int32_t *cs = cstart + ((int64_t)ft * TT + h * COLS + lane) * g.G[2];
+            const int b = cs[z0], n = cs[z1] - b;
+            const int lo = (int)((int64_t)n * it.z / it.w), hi = (int)((int64_t)n * (it.z + 1) / it.w);
+            beg = b + lo;
+            cnt = hi - lo;
+        }
+        int incl = cnt;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int o = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += o;
+        }
+        if (lane < COLS) {
+            s_beg[lane] = beg;
+            s_pre[lane + 1] = incl;
+        }
+        if (lane == 0) s_pre[0] = 0;
+    }
+    cp_wait<0>();
+    __syncthreads();
+    const int n = s_pre[COLS];
+    for (int q = tid; q < n; q += kFewThreads) {
+        int s = 0;
+        while (s_pre[s + 1] <= q) s++;
+        const int64_t j = s_beg[s] + q - s_pre[s];
+        float w[REC];
+#pragma unroll
+        for (int e = 0; e < REC / 4; e++)
+            *reinterpret_cast<float4 *>(w + 4 * e) = __ldg(reinterpret_cast<const float4 *>(rec + j * REC) + e);
+        const float2 *tp = tile + ((((zc[j] - z0) * RYE + s / T) * RX) + s % T) * CC;
+        float2 acc[CC];
+#pragma unroll
+        for (int c = 0; c < CC; c++) acc[c] = make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            float2 t[CC];
+#pragma unroll
+            for (int i = 0; i < W; i++) {
+                float2 r[CC];
+#pragma unroll
+                for (int x = 0; x < W; x++)
+#pragma unroll
+                    for (int c = 0; c < CC; c++) {
+                        const float2 v = tp[((k * RYE + i) * RX + x) * CC + c];
+                        r[c] = x == 0 ? __fmul2_rn(dup(w[x]), v) : __ffma2_rn(dup(w[x]), v, r[c]);
+                    }
+#pragma unroll
+                for (int c = 0; c < CC; c++)
+                    t[c] = i == 0 ? __fmul2_rn(dup(w[W + i]), r[c]) : __ffma2_rn(dup(w[W + i]), r[c], t[c]);
+            }
+#pragma unroll
+            for (int c = 0; c < CC; c++) acc[c] = __ffma2_rn(dup(w[2 * W + k]), t[c], acc[c]);
+        }
+#pragma unroll
+        for (int c = 0; c < CC; c++)
+            if (c < g.CS) rows[j * g.RS + c] = acc[c];
+    }
+}
+
 int march_blocks(int64_t n)
 {
     int dev = 0, sms = 148;
@@ -1052,9 +1145,29 @@ int launch_interp_n(const dmr_plan *p, const MarchGeom &m, const float2 *grid, f
     return DMR_OK;
 }
 
+template <int W, int CC>
+int launch_interp_few(const dmr_plan *p, const MarchGeom &m, const float2 *grid, float2 *rows, cudaStream_t st)
+{
+    interp_few_kernel<W, CC><<<p->mp_nitems, kFewThreads, 0, st>>>(m, (const int4 *)p->mp_items, p->mp_cstart, p->mp_rec,
+                                                                  p->mp_zc, grid, rows);
+    DMR_LAUNCHED("interp_few_kernel");
+    return DMR_OK;
+}
+
 template <int W>
 int launch_interp(const dmr_plan *p, const MarchGeom &m, const float2 *grid, float2 *rows, cudaStream_t st)
 {
+    // a thread per sample for 1 coil (96^3, 1.8 M samples: W 3, os 1.25, 247 us with
+    // lane groups and 105 with this; W 6, os 2, 1,477 and 535), and for 2 at the
+    // widths whose groups take 3 coils or more at a time (W 2 and 3: 0.95 to 1.8
+    // times the groups' speed, W 6 1.1 to 2.1, W 4 and 5 0.86 to 1.5; 4 coils at W 4
+    // 0.6 to 1.0)
+    if (m.CS == 1) return launch_interp_few<W, 1>(p, m, grid, rows, st);
+    if constexpr (W <= 3 || W == 6)
+        if (m.CS == 2) return launch_interp_few<W, 2>(p, m, grid, rows, st);
+    // width 6: 10 coils at a time take 1.7 times as long as 5
+    if constexpr (W == 6)
+        if (5 * ceil_div(m.CS, 10) < 3 * ceil_div(m.CS, 5)) return launch_interp_n<6, 3, 1>(p, m, grid, rows, st);
     // lane groups by the coils of the chunk: as few as leave the lanes filled
     // (each group adds a share of a plane's work and a round of shuffles); a
     // lane holds at most 64 taps

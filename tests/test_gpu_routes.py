@@ -404,3 +404,26 @@ def test_rounding_by_coils_and_mode(width, n, calls):
     ref = err("adj", 12)
     for call in calls:
         assert err(*call) < 1.15 * ref, call
+
+
+@pytest.mark.parametrize("width,coils", [(2, (1, 2, 3)), (3, (1, 2, 3)), (4, (1, 2)), (5, (1, 2)),
+                                         (6, (1, 2, 3, 10, 11, 20, 21, 31))])
+def test_forward_lane_layouts(width, coils):
+    """Interpolation around the coil counts where its lanes change, items with
+    hundreds of samples (parts, more samples than threads), with few and with
+    none, and regions that wrap."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import synth
+    from oracle import nufft_ref as R
+
+    shape = (13, 9, 21)
+    rng = np.random.default_rng(width)
+    c = rng.uniform(-0.5, 0.5, (1, 3000, 3)) * np.asarray(shape[::-1])
+    c[:, :2000] *= 0.02
+    c[:, -8:] = np.sign(c[:, -8:]) * np.asarray(shape[::-1]) * 0.4999
+    c = torch.as_tensor(c.astype(np.float32))
+    plan, oplan = F.plan_nufft(c, shape, width, 2.0, device="cuda"), R.plan_nufft(c, shape, width, 2.0)
+    img = synth.complex_gaussian((max(coils),) + shape, seed=1)
+    ref = R.apply_nufft(img, oplan)
+    for k in coils:
+        assert rel(F.apply_nufft(img[:k].cuda(), plan), ref[:k]) < TOL, k
