@@ -427,3 +427,43 @@ def test_forward_lane_layouts(width, coils):
     ref = R.apply_nufft(img, oplan)
     for k in coils:
         assert rel(F.apply_nufft(img[:k].cuda(), plan), ref[:k]) < TOL, k
+
+
+def test_arguments_that_outlive_their_transform():
+    """A weight that leaked from a function transform is taken, and what function
+    transforms and tracing compute are the values that ``apply`` computes."""
+    import deepmr_b200.fft as F
+
+    c = torch.as_tensor(np.random.default_rng(0).uniform(-8, 8, (1, 40, 2)).astype(np.float32))
+    plan = F.plan_nufft(c, (16, 16), 4, 1.25, device="cuda")
+    g = torch.Generator().manual_seed(1)
+    y = torch.complex(torch.randn(2, 1, 40, generator=g), torch.randn(2, 1, 40, generator=g)).cuda()
+    w = torch.rand(1, 40, generator=g).cuda()
+    leaked = []
+
+    def leak(t):
+        leaked.append(t)
+        return (t * t).sum()
+
+    torch.func.grad(leak)(w)
+    ref = F.apply_nufft_adj(y, plan, weight=w)
+    assert rel(F.apply_nufft_adj(y, plan, weight=leaked[0]), ref) < 1e-6
+
+    x = ref.clone()
+    N = __import__("importlib").import_module("deepmr_b200.fft.nufft")
+    runs = {
+        "vmap": lambda f: torch.func.vmap(f)(x),
+        "grad": lambda f: torch.func.grad(lambda t: (f(t).abs() ** 2).sum())(x),
+        "trace": lambda f: torch.jit.trace(f, (x,), check_trace=False)(x),
+    }
+    for name, run in runs.items():
+        res = []
+        for f in ((lambda t: N.apply_nufft(t, plan)), (lambda t: N.ApplyNUFFT.apply(t, plan, None, None, None, 128))):
+            try:
+                res.append(run(f))
+            except Exception as e:  # noqa: BLE001
+                res.append(type(e))
+        if isinstance(res[1], torch.Tensor):
+            assert rel(res[0].detach(), res[1].detach()) < 1e-6, name
+        else:
+            assert res[0] is res[1], name
