@@ -616,8 +616,8 @@ __global__ void __launch_bounds__(F::T, F::TOEP_MINB) fft_toep_z_kernel(int G0, 
 }
 
 // Other lengths L = L1 L2, both at most MX: the same steps with the factors at
-// run time, a switch over the register transforms. Two sizes of kernel, so that
-// small factors do not pay for the registers of large ones.
+// run time, a switch over the register transforms. Three sizes of kernel (13, 20
+// and 26), so that small factors do not pay for the registers of large ones.
 struct Fac {
     int L = 0, L1 = 0, L2 = 0;
 };
@@ -626,7 +626,7 @@ template <int MX>
 struct Gen {
     static constexpr int T = kFftLines * MX, MINB = 65536 / (T * (MX > 20 ? 72 : 64));
 };
-// the run-time lengths' passes (fft_any_rows.cu, fft_any_cols.cu, fft_any_toep.cu)
+// the run-time lengths' passes (fft_any_rows.cuh, fft_any_cols.cu, fft_any_toep.cu)
 template <bool CROP, bool IL>
 int launch_rows_any(Fac f, const FftGeom &g, const float2 *tw, const void *src, int src_real, float2 *dst, cudaStream_t st);
 int launch_cols_any(const Fac &f, const FftGeom &g, const ColArgs &a, const float2 *tw, float2 *grid, cudaStream_t st);

@@ -648,15 +648,6 @@ static int tg_build(dmr_plan *p, int32_t *keys, int32_t *keys_s, int32_t *vals, 
                 DMR_CUDA(cudaMemcpyAsync(p->tg_order, torder.data(), torder.size() * sizeof(int32_t),
                                          cudaMemcpyHostToDevice, st));
             }
-            // deterministic mode: the items of each bin (make_items numbers
-            // them in key order, kTgSegment samples each)
-            std::vector<int32_t> istart(tkeys + 1, 0);
-            for (int64_t k = 0; k < tkeys; k++)
-                istart[k + 1] = istart[k] + (int32_t)ceil_div(ts[k + 1] - ts[k], kTgSegment);
-            DMR_CHECK(istart[tkeys] == (int64_t)titems.size(), DMR_ERR_UNSUPPORTED, "gridding item count mismatch");
-            DMR_TRY(plan_alloc(dev, &p->tg_item_start, istart.size(), st));
-            DMR_CUDA(cudaMemcpyAsync(p->tg_item_start, istart.data(), istart.size() * sizeof(int32_t),
-                                     cudaMemcpyHostToDevice, st));
             DMR_CUDA(cudaStreamSynchronize(st));
             p->tg_nwork = (int)titems.size();
             p->tg_nbins = tbins;

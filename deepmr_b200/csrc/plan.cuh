@@ -142,9 +142,6 @@ int plan_bins(const ::dmr_plan *p, cudaStream_t st);
 bool rt_geometry_ok(const Geom &g);
 int rt_build(const ::dmr_plan *p, PlanBins &b, const std::vector<int32_t> &h_start, cudaStream_t st);
 size_t rt_scratch_bytes(const ::dmr_plan *p, int64_t batch);
-// scratch bytes of deterministic tensor-core gridding (every work item's
-// region partial sums, 2 KB per item and coil)
-size_t tm_scratch_bytes(const ::dmr_plan *p, int64_t batch);
 // scratch bytes a gridding call of `batch` coils may need (either kernel)
 size_t grid_scratch_bytes(const ::dmr_plan *p, int64_t batch);
 // library-owned stream-ordered pool for the scratch of calls without a workspace
@@ -179,8 +176,7 @@ int fft3_toeplitz(int ndim, const int32_t *kshape_zyx, const int32_t *ishape_zyx
 // tensor-core gridding of 3D plans (tcgrid.cu: dispatch and health state,
 // tmgrid.cu: the kernel); DMR_ERR_UNSUPPORTED when the plan has no gridding bins
 int grid_tc_dispatch(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
-                     const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes,
-                     cudaStream_t st);
+                     const float *weight, int wpb, cudaStream_t st);
 // smallest batch of atomic tensor-core gridding (dmr_tc_min_coils), DMR_NO_TC,
 // and the deterministic scratch limit (dmr_det_scratch_limit)
 int tc_min_coils();
@@ -188,16 +184,11 @@ bool tc_disabled();
 int64_t det_scratch_limit();
 // whether gridding of `batch` coils runs on the plane kernel (march.cuh)
 bool grid_march_applies(const ::dmr_plan *p, int64_t batch, int det);
-// tensor-core gridding with the plan's gridding bins (tmgrid.cu), atomic or
-// deterministic (partial sums per work item, then a gather per grid point;
-// scratch from the caller when it holds tm_scratch_bytes, else from the
-// library pool; DMR_ERR_UNSUPPORTED, before any launch, when it needs more
-// than `det_limit` bytes (> 0) or the pool has no memory for it, so that the
-// caller takes another deterministic kernel); `timeouts` is the device
-// address of the process-wide counter of blocks that stopped on a bounded wait
+// atomic tensor-core gridding with the plan's gridding bins (tmgrid.cu);
+// `timeouts` is the device address of the process-wide counter of blocks that
+// stopped on a bounded wait
 int grid_tm_dispatch(const ::dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
-                     const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes, int *timeouts,
-                     int stall, int64_t det_limit, cudaStream_t st);
+                     const float *weight, int wpb, int *timeouts, int stall, cudaStream_t st);
 
 }  // namespace dmr
 
@@ -235,10 +226,6 @@ struct dmr_plan {
     dmr::WorkItem *tg_work = nullptr;
     int tg_nwork = 0;
     int32_t *tg_order = nullptr;
-    // deterministic mode: the items of each bin, [tg_item_start[k],
-    // tg_item_start[k + 1]) of tg_work for bin key k (frame * tg_nbins + bin;
-    // items are numbered in key order, a bin's segments in sample order)
-    int32_t *tg_item_start = nullptr;
     float *apod[3] = {nullptr, nullptr, nullptr};  // per-axis apodisation (image index)
     int64_t *foff_dev = nullptr;        // frame offsets on the device (nframes + 1)
     // march order (march.cu; mp_W == 0: not planned; 3D, and 2D plans dense enough
@@ -286,7 +273,6 @@ struct dmr_plan {
         drop(tg_l);
         drop(tg_work);
         drop(tg_order);
-        drop(tg_item_start);
         drop(status);
         drop(mp_cstart);
         drop(mp_sidx);

@@ -1401,8 +1401,8 @@ int interp_dispatch(const dmr_plan *p, const float2 *grid, float2 *ksp, int64_t 
 int grid_rt_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
                      const float *weight, int wpb, void *scratch, size_t scratch_bytes, cudaStream_t st);
 
-// (the deterministic tensor-core gridding takes its larger scratch from the
-// library pool, so that callers' workspaces do not hold it in atomic mode)
+// (deterministic plane gridding takes its larger scratch from the library pool,
+// so that callers' workspaces do not hold it in atomic mode)
 size_t grid_scratch_bytes(const dmr_plan *p, int64_t batch)
 {
     return rt_scratch_bytes(p, batch);
@@ -1432,7 +1432,7 @@ int grid_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, i
     // atomic 3D gridding on the tensor cores where dmr_tc_min_coils asks for it
     // (plans made under that setting have its gridding bins)
     if (p->g.ndim == 3 && grid_variant() == 0 && !det && batch >= tc_min_coils()) {
-        const int rc = grid_tc_dispatch(p, ksp, kreal, grid, batch, weight, wpb, det, scratch, scratch_bytes, st);
+        const int rc = grid_tc_dispatch(p, ksp, kreal, grid, batch, weight, wpb, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }
     DMR_TRY(plan_bins(p, st));

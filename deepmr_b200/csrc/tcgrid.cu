@@ -33,8 +33,8 @@ bool tc_disabled()
 }
 
 static std::atomic<int> g_tc_stall{0};  // test hook (dmr_tc_test_stall)
-// largest scratch (bytes) deterministic tensor-core gridding may take, 0: no
-// limit (dmr_det_scratch_limit)
+// largest scratch (bytes) deterministic plane gridding may take, 0: no limit
+// (dmr_det_scratch_limit)
 static std::atomic<int64_t> g_det_scratch_max{0};
 
 int64_t det_scratch_limit() { return g_det_scratch_max.load(); }
@@ -51,20 +51,18 @@ static int timeouts_ptr(int dev, int **out)
     return DMR_OK;
 }
 
-// Tensor-core gridding of a 3D plan with the kernel of tmgrid.cu (atomic, or
-// deterministic through per-item partial sums); DMR_ERR_UNSUPPORTED when it does not
-// apply or DMR_NO_TC=1 (then the caller uses the CUDA-core kernels).
+// Atomic tensor-core gridding of a 3D plan with the kernel of tmgrid.cu;
+// DMR_ERR_UNSUPPORTED when it does not apply or DMR_NO_TC=1 (then the caller uses
+// the CUDA-core kernels).
 int grid_tc_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
-                     const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes,
-                     cudaStream_t st)
+                     const float *weight, int wpb, cudaStream_t st)
 {
     if (tc_disabled()) return DMR_ERR_UNSUPPORTED;
     int dev = 0;
     DMR_CUDA(cudaGetDevice(&dev));
     int *timeouts = nullptr;
     DMR_TRY(timeouts_ptr(dev, &timeouts));
-    return grid_tm_dispatch(p, ksp, kreal, grid, batch, weight, wpb, det, scratch, scratch_bytes, timeouts,
-                            g_tc_stall.load(), g_det_scratch_max.load(), st);
+    return grid_tm_dispatch(p, ksp, kreal, grid, batch, weight, wpb, timeouts, g_tc_stall.load(), st);
 }
 
 }  // namespace dmr

@@ -110,7 +110,6 @@ struct TmShape {
     int R[3];        // region extents (tile + W - 1)
     int P;           // region points (<= 256)
     int CC;          // coils per block (<= 32)
-    int ccp;         // deterministic scratch: coil stride of a region point (CC rounded up to the gather's group)
     int vrows;       // R[0] + R[1] + R[2]
     int table_off;   // per builder group two chunk weight tables (offset in dynamic shared memory)
     int goff_off;    // read-back: grid offsets of the current item's region points
@@ -267,8 +266,8 @@ __device__ __forceinline__ void bin_origin(const Geom &g, int bin, int &f, int o
 __global__ void __launch_bounds__(kTmThreads, 1) grid_tmem_kernel(
     Geom g, TmShape sh, const WorkItem *__restrict__ work, const int32_t *__restrict__ order, int nwork,
     int nchunks, const float *__restrict__ tw, const int32_t *__restrict__ tl, const int32_t *__restrict__ sidx, const void *__restrict__ ksp, int kreal, float2 *__restrict__ grid,
-    int64_t batch, const float *__restrict__ weight, int wpb, float inv_scale, float2 *__restrict__ scratch,
-    int *__restrict__ status, int *__restrict__ timeouts, int stall)
+    int64_t batch, const float *__restrict__ weight, int wpb, float inv_scale, int *__restrict__ status,
+    int *__restrict__ timeouts, int stall)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t bars[kBarCount];
@@ -500,11 +499,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) grid_tmem_kernel(
                 goff[et] = (gz * g.G[1] + gy) * g.G[0] + gx;
             }
             const float2 *gitem = grid + (b0 * g.nframes + f) * g.gsize;
-            // deterministic mode: the item stores its partial sums into its
-            // scratch slot (the item's index), [region point][coil]
-            float2 *part = scratch ? scratch + ((int64_t)order[ps.task / nchunks] * nchunks + ps.task % nchunks) *
-                                                   kTmN * sh.ccp
-                                   : nullptr;
             const int64_t cstride = (int64_t)g.nframes * g.gsize;
             uint32_t r[16], rn[16];
             tc_ld16(tbase + lanebase + (uint32_t)(acc * kTmN + 16 * hcol), r);
@@ -533,23 +527,11 @@ __global__ void __launch_bounds__(kTmThreads, 1) grid_tmem_kernel(
                                             (xb[(2 * c + 1) * kTmXS + lane] + xb[(65 + 2 * c) * kTmXS + lane]) *
                                                 inv_scale);
                     }
-                    if (part) {
-                        // coils 4e .. 4e + 3 of the point: one 32-byte sector in
-                        // one 256-bit store (coils past the batch hold the zero
-                        // rows of V)
-                        if (e * 4 < cact)
-                            asm volatile("st.global.cs.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(
-                                             part + pp * sh.ccp + e * 4),
-                                         "f"(v[0].x), "f"(v[0].y), "f"(v[1].x), "f"(v[1].y), "f"(v[2].x), "f"(v[2].y),
-                                         "f"(v[3].x), "f"(v[3].y)
-                                         : "memory");
-                    } else {
 #pragma unroll
-                        for (int cc = 0; cc < 4; cc++) {
-                            const int c = e * 4 + cc;
-                            if (c < cact && (v[cc].x != 0.0f || v[cc].y != 0.0f))
-                                atomicAdd(const_cast<float2 *>(gp) + c * cstride, v[cc]);
-                        }
+                    for (int cc = 0; cc < 4; cc++) {
+                        const int c = e * 4 + cc;
+                        if (c < cact && (v[cc].x != 0.0f || v[cc].y != 0.0f))
+                            atomicAdd(const_cast<float2 *>(gp) + c * cstride, v[cc]);
                     }
                 }
                 if (more) {
@@ -707,173 +689,6 @@ __global__ void __launch_bounds__(kTmThreads, 1) grid_tmem_kernel(
     }
 }
 
-// The regions that cover grid position `pos` along one axis: bins b with
-// offsets u in their region, (b T + u - half) = pos (mod G), 0 <= u < R <= 8,
-// as 16-bit entries (b << 3 | u) + 1 in increasing u, 0 after the last. With
-// R <= G a bin covers a position at most once; b T = (pos + half - u) mod G
-// < G implies b < nb. Increasing u puts neighbouring positions of one bin at
-// the same index.
-__device__ __forceinline__ uint4 tm_cover(int pos, int G, int T, int R, int half)
-{
-    uint32_t e[4] = {0, 0, 0, 0};
-    int n = 0;
-    const int t = (pos + half) % G;
-    for (int u = 0; u < R; u++) {
-        int o = t - u;
-        if (o < 0) o += G;
-        if (o % T == 0) {
-            e[n >> 1] |= (uint32_t)((o / T) << 3 | u) + 1u << (16 * (n & 1));
-            n++;
-        }
-    }
-    return make_uint4(e[0], e[1], e[2], e[3]);
-}
-
-__device__ __forceinline__ int tm_cover_count(const uint4 &c)
-{
-    const uint32_t w[4] = {c.x, c.y, c.z, c.w};
-    int n = 0;
-#pragma unroll
-    for (int q = 0; q < 4; q++) n += ((w[q] & 0xffffu) != 0) + ((w[q] >> 16) != 0);
-    return n;
-}
-
-// G coils of one region point of a deterministic scratch slot (8 G
-// contiguous bytes, 256-bit loads), and their addition to the accumulators
-template <int G>
-__device__ __forceinline__ void tm_ldg(const float2 *src, float (&v)[2 * G])
-{
-#pragma unroll
-    for (int j = 0; j < G / 4; j++)
-        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-            : "=f"(v[8 * j]), "=f"(v[8 * j + 1]), "=f"(v[8 * j + 2]), "=f"(v[8 * j + 3]), "=f"(v[8 * j + 4]),
-              "=f"(v[8 * j + 5]), "=f"(v[8 * j + 6]), "=f"(v[8 * j + 7])
-            : "l"(src + 4 * j));
-}
-
-template <int G>
-__device__ __forceinline__ void tm_addg(float2 (&acc)[G], const float (&v)[2 * G])
-{
-#pragma unroll
-    for (int c = 0; c < G; c++) {
-        acc[c].x += v[2 * c];
-        acc[c].y += v[2 * c + 1];
-    }
-}
-
-__device__ __forceinline__ int tm_cover_at(const uint4 &c, int k)
-{
-    const int q = k >> 1;  // entries 2q and 2q + 1 share a word
-    const uint32_t w = q < 2 ? (q < 1 ? c.x : c.y) : (q < 3 ? c.z : c.w);
-    return (int)((w >> (16 * (k & 1))) & 0xffff) - 1;
-}
-
-// Deterministic mode: every grid point adds, for kTmGatherCoils coils of one
-// coil chunk, in a fixed order (covering bins by z, y, x offset, then each
-// bin's items in sample order) the partial sums that the covering items
-// stored in their scratch slots ([region point][coil]), and writes the grid
-// once (0 where no item covers it). A thread reads its coils of a region
-// point as 8 kTmGatherCoils contiguous bytes; lanes run along x, so a warp writes 32
-// neighbouring grid points per coil. The coil groups of the same points are
-// neighbouring blocks (blockIdx.x = point block * groups + group, blockIdx.y
-// = chunk), so each point's coils (256 bytes of a slot) come from DRAM once.
-// The cover lists of all positions (two entries per 32-bit word, up to 8 per
-// position) are built per block in shared memory (G[0] + G[1] + G[2] uint4).
-constexpr int kTmGatherCoils = 8;
-
-__global__ void __launch_bounds__(256, 2) grid_tm_gather_kernel(Geom g, TmShape sh, const int32_t *__restrict__ istart,
-                                                            const float2 *__restrict__ scratch,
-                                                            float2 *__restrict__ grid, int64_t batch, int nchunks)
-{
-    extern __shared__ uint4 s_cover[];
-    uint4 *cov[3] = {s_cover, s_cover + g.G[0], s_cover + g.G[0] + g.G[1]};
-    for (int a = 0; a < 3; a++)
-        for (int pos = threadIdx.x; pos < g.G[a]; pos += blockDim.x)
-            cov[a][pos] = tm_cover(pos, g.G[a], g.T[a], sh.R[a], g.half[a]);
-    __syncthreads();
-    const int ngrp = (sh.CC + kTmGatherCoils - 1) / kTmGatherCoils;
-    const int cch = blockIdx.y, c0 = (blockIdx.x % ngrp) * kTmGatherCoils;
-    const int pblock = blockIdx.x / ngrp, pblocks = gridDim.x / ngrp;
-    const int64_t b0 = (int64_t)cch * sh.CC + c0;
-    // coils of this chunk (the last chunk may hold fewer than CC), of this group
-    const int ccoils = (int)min((int64_t)sh.CC, batch - (int64_t)cch * sh.CC);
-    const int cact = min(kTmGatherCoils, ccoils - c0);
-    const int64_t npts = (int64_t)g.nframes * g.gsize;
-    const int gxy = g.G[0] * g.G[1];
-    for (int64_t i = (int64_t)pblock * blockDim.x + threadIdx.x; i < npts; i += (int64_t)pblocks * blockDim.x) {
-        const int f = (int)(i / g.gsize), r = (int)(i - (int64_t)f * g.gsize);
-        const int z = r / gxy, y = (r - z * gxy) / g.G[0], x = r - z * gxy - y * g.G[0];
-        const uint4 cz = cov[2][z], cy = cov[1][y], cx = cov[0][x];
-        float2 acc[kTmGatherCoils];
-#pragma unroll
-        for (int c = 0; c < kTmGatherCoils; c++) acc[c] = make_float2(0.0f, 0.0f);
-        const int ncz = tm_cover_count(cz), ncy = tm_cover_count(cy), ncx = tm_cover_count(cx);
-        auto slot = [&](int s, int pt) {
-            return scratch + (((int64_t)s * nchunks + cch) * kTmN + pt) * sh.ccp + c0;
-        };
-        if (ncz <= 2 && ncy <= 2 && ncx <= 2) {
-            // at most two covering bins per axis (every position of the usual
-            // geometries): the item ranges of all 8 candidates first, then the
-            // first items of 4 candidates at a time, so that their loads are
-            // in flight together; the additions keep the general order
-            int beg[8], cnt[8], pts[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-                const int kz = q >> 2, ky = (q >> 1) & 1, kx = q & 1;
-                beg[q] = cnt[q] = pts[q] = 0;
-                if (kz < ncz && ky < ncy && kx < ncx) {
-                    const int vz = tm_cover_at(cz, kz), vy = tm_cover_at(cy, ky), vx = tm_cover_at(cx, kx);
-                    const int key = f * g.nbins + ((vz >> 3) * g.nb[1] + (vy >> 3)) * g.nb[0] + (vx >> 3);
-                    beg[q] = __ldg(istart + key);
-                    cnt[q] = __ldg(istart + key + 1) - beg[q];
-                    pts[q] = ((vz & 7) * sh.R[1] + (vy & 7)) * sh.R[0] + (vx & 7);
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                float v[2][2 * kTmGatherCoils];
-#pragma unroll
-                for (int j = 0; j < 2; j++)
-                    if (cnt[2 * h + j] > 0) tm_ldg<kTmGatherCoils>(slot(beg[2 * h + j], pts[2 * h + j]), v[j]);
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const int q = 2 * h + j;
-                    if (cnt[q] > 0) {
-                        tm_addg<kTmGatherCoils>(acc, v[j]);
-                        for (int s = beg[q] + 1; s < beg[q] + cnt[q]; s++) {
-                            float w[2 * kTmGatherCoils];
-                            tm_ldg<kTmGatherCoils>(slot(s, pts[q]), w);
-                            tm_addg<kTmGatherCoils>(acc, w);
-                        }
-                    }
-                }
-            }
-        } else {
-            for (int kz = 0; kz < ncz; kz++) {
-                const int vz = tm_cover_at(cz, kz);
-                for (int ky = 0; ky < ncy; ky++) {
-                    const int vy = tm_cover_at(cy, ky);
-                    const int kyz = f * g.nbins + ((vz >> 3) * g.nb[1] + (vy >> 3)) * g.nb[0];
-                    const int pyz = ((vz & 7) * sh.R[1] + (vy & 7)) * sh.R[0];
-                    for (int kx = 0; kx < ncx; kx++) {
-                        const int vx = tm_cover_at(cx, kx);
-                        const int key = kyz + (vx >> 3);
-                        const int s1 = istart[key + 1];
-                        for (int s = istart[key]; s < s1; s++) {
-                            float w[2 * kTmGatherCoils];
-                            tm_ldg<kTmGatherCoils>(slot(s, pyz + (vx & 7)), w);
-                            tm_addg<kTmGatherCoils>(acc, w);
-                        }
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < kTmGatherCoils; c++)
-            if (c < cact) grid[(b0 + c) * npts + i] = acc[c];
-    }
-}
-
 bool tm_shape(const dmr_plan *p, int64_t batch, int wpb, int smem_limit, TmShape &s)
 {
     const Geom &g = p->g;
@@ -885,7 +700,6 @@ bool tm_shape(const dmr_plan *p, int64_t batch, int wpb, int smem_limit, TmShape
     s.vrows = s.R[0] + s.R[1] + s.R[2];
     if (s.vrows > kTmMaxRows) return false;
     s.CC = (int)std::min<int64_t>(batch, kTmCC);
-    s.ccp = (s.CC + kTmGatherCoils - 1) / kTmGatherCoils * kTmGatherCoils;
     s.wp = p->tg_wp;
     int off = kTmSB * 3 * s.wp * 4;  // tap weights of the pass, [sample][axis][wp]
     s.l_off = off;
@@ -924,20 +738,8 @@ bool tm_shape(const dmr_plan *p, int64_t batch, int wpb, int smem_limit, TmShape
 // Tensor-core gridding of a 3D plan with its gridding bins; DMR_ERR_UNSUPPORTED
 // when the plan has none or the geometry does not fit (the caller then uses
 // the other kernels).
-// scratch of deterministic tensor-core gridding: one slot of kTmN region
-// points per (work item, coil chunk), each point the chunk's coils rounded up
-// to the gather's coil group
-size_t tm_scratch_bytes(const dmr_plan *p, int64_t batch)
-{
-    if (p->g.ndim != 3 || p->tg_T[0] == 0 || p->tg_nwork == 0 || batch < 1) return 0;
-    const int64_t cc = std::min<int64_t>(batch, kTmCC);
-    return (size_t)p->tg_nwork * ceil_div(batch, cc) * kTmN * ((cc + kTmGatherCoils - 1) / kTmGatherCoils * kTmGatherCoils) *
-           sizeof(float2);
-}
-
 int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
-                     const float *weight, int wpb, int det, void *scratch, size_t scratch_bytes, int *timeouts,
-                     int stall, int64_t det_limit, cudaStream_t st)
+                     const float *weight, int wpb, int *timeouts, int stall, cudaStream_t st)
 {
     int dev = 0, sms = 0, smem_blk = 0;
     DMR_CUDA(cudaGetDevice(&dev));
@@ -953,14 +755,7 @@ int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     int per_sm = 0;
     DMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_tmem_kernel, kTmThreads, smem));
     if (per_sm != 1) return DMR_ERR_UNSUPPORTED;
-    // deterministic mode needs the points of one region on distinct grid
-    // points and at most 8 region points per axis (the gather's cover lists)
-    if (det)
-        for (int a = 0; a < 3; a++)
-            if (sh.R[a] > p->g.G[a] || sh.R[a] > 8) return DMR_ERR_UNSUPPORTED;
-    // the deterministic gather writes every grid point
-    if (!det || p->tg_nwork == 0)
-        DMR_CUDA(cudaMemsetAsync(grid, 0, (size_t)batch * p->g.nframes * p->g.gsize * sizeof(float2), st));
+    DMR_CUDA(cudaMemsetAsync(grid, 0, (size_t)batch * p->g.nframes * p->g.gsize * sizeof(float2), st));
     if (p->tg_nwork == 0) return DMR_OK;
     const int64_t nchunks = ceil_div(batch, sh.CC);
     DMR_CHECK((int64_t)p->tg_nwork * nchunks < (1ll << 31), DMR_ERR_UNSUPPORTED, "too many gridding tasks");
@@ -972,60 +767,12 @@ int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     }
     g.nbins = p->tg_nbins;
     const float inv_scale = (float)(1.0 / p->scale);
-    if (!det) {
-        const int blocks = (int)std::min<int64_t>((int64_t)p->tg_nwork * nchunks, (int64_t)sms);
-        grid_tmem_kernel<<<blocks, kTmThreads, smem, st>>>(
-            g, sh, p->tg_work, p->tg_order, p->tg_nwork, (int)nchunks, p->tg_w, p->tg_l, p->tg_sidx, ksp, kreal,
-            grid, batch, weight, wpb, inv_scale, nullptr, p->status, timeouts, stall);
-        DMR_LAUNCHED("grid_tmem_kernel");
-        return DMR_OK;
-    }
-    // deterministic: the items store their partial sums into scratch slots
-    // (no grid writes), then the gather sums them per grid point in a fixed
-    // order: every run adds the same values in the same order
-    const int ngrp = (sh.CC + kTmGatherCoils - 1) / kTmGatherCoils;
-    DMR_CHECK(nchunks <= 65535, DMR_ERR_UNSUPPORTED, "batch too large");
-    // the gather's cover lists: one uint4 per grid position of each axis
-    const size_t gsmem = (size_t)(p->g.G[0] + p->g.G[1] + p->g.G[2]) * sizeof(uint4);
-    if (gsmem > 48 * 1024) {
-        DMR_CHECK(gsmem <= (size_t)smem_blk, DMR_ERR_UNSUPPORTED, "grid too large for the gather");
-        DMR_CUDA(cudaFuncSetAttribute(grid_tm_gather_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gsmem));
-    }
-    const size_t need = tm_scratch_bytes(p, batch);
-    // over the caller's limit, or no memory for it: another deterministic
-    // kernel takes the call (nothing has been launched yet)
-    if (det_limit > 0 && need > (size_t)det_limit) return DMR_ERR_UNSUPPORTED;
-    void *owned = nullptr;
-    if (scratch == nullptr || scratch_bytes < need) {
-        cudaMemPool_t pool = scratch_pool(p->device);
-        if (pool == nullptr) return DMR_ERR_UNSUPPORTED;
-        const cudaError_t e = cudaMallocFromPoolAsync(&owned, need, pool, st);
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            return DMR_ERR_UNSUPPORTED;
-        }
-        if (e != cudaSuccess) return cuda_fail(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);
-        scratch = owned;
-    }
-    int rc = DMR_OK;
     const int blocks = (int)std::min<int64_t>((int64_t)p->tg_nwork * nchunks, (int64_t)sms);
     grid_tmem_kernel<<<blocks, kTmThreads, smem, st>>>(
         g, sh, p->tg_work, p->tg_order, p->tg_nwork, (int)nchunks, p->tg_w, p->tg_l, p->tg_sidx, ksp, kreal, grid,
-        batch, weight, wpb, inv_scale, (float2 *)scratch, p->status, timeouts, stall);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) rc = cuda_fail(e, "grid_tmem_kernel", __FILE__, __LINE__);
-    if (rc == DMR_OK) {
-        const int64_t npts = (int64_t)g.nframes * g.gsize;
-        const int gblocks = (int)std::min<int64_t>(ceil_div(npts, 256), (int64_t)sms * 16);
-        grid_tm_gather_kernel<<<dim3(gblocks * ngrp, (unsigned)nchunks), 256, gsmem, st>>>(
-            g, sh, p->tg_item_start, (const float2 *)scratch, grid, batch, (int)nchunks);
-        g_launches.fetch_add(1, std::memory_order_relaxed);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) rc = cuda_fail(e, "grid_tm_gather_kernel", __FILE__, __LINE__);
-    }
-    if (owned) cudaFreeAsync(owned, st);
-    return rc;
+        batch, weight, wpb, inv_scale, p->status, timeouts, stall);
+    DMR_LAUNCHED("grid_tmem_kernel");
+    return DMR_OK;
 }
 
 }  // namespace dmr
