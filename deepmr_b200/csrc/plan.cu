@@ -132,10 +132,10 @@ __global__ void gather_sorted_kernel(int64_t total, int ndim, const int32_t *__r
 }
 
 // sort key of the tensor-core gridding bins: (frame, bin) with tile tg_T
-__global__ void tg_key_kernel(Geom g, int t0, int t1, int t2, int n0, int n1, int n2, int nbins,
+__global__ void tg_key_kernel(Geom g, int t0, int t1, int t2, int n0, int n1, int nbins,
                               const int64_t *__restrict__ foff, const float *__restrict__ rk0,
                               const float *__restrict__ rk1, const float *__restrict__ rk2,
-                              int32_t *__restrict__ keys, int32_t *__restrict__ counts)
+                              int32_t *__restrict__ keys, int32_t *__restrict__ vals, int32_t *__restrict__ counts)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.total;
          i += (int64_t)gridDim.x * blockDim.x) {
@@ -149,6 +149,7 @@ __global__ void tg_key_kernel(Geom g, int t0, int t1, int t2, int n0, int n1, in
         const int bz = pmod(first_tap(rk2[i], g.W[2]), g.G[2]) / t2;
         const int key = lo * nbins + (bz * n1 + by) * n0 + bx;
         keys[i] = key;
+        vals[i] = (int32_t)i;
         atomicAdd(&counts[key], 1);
     }
 }
@@ -543,11 +544,13 @@ static int bins_build(const dmr_plan *p, PlanBins &out, cudaStream_t st)
     return DMR_OK;
 }
 
-int plan_bins(const dmr_plan *p, cudaStream_t st)
+// builds structures aside with `build` and publishes them in `slot`, once
+template <class B, class Fn>
+static int publish(const dmr_plan *p, std::atomic<const B *> &slot, cudaStream_t st, Fn build)
 {
-    if (p->bins_ptr.load(std::memory_order_acquire)) return DMR_OK;
+    if (slot.load(std::memory_order_acquire)) return DMR_OK;
     std::lock_guard<std::mutex> lock(p->bins_mu);
-    if (p->bins_ptr.load(std::memory_order_relaxed)) return DMR_OK;
+    if (slot.load(std::memory_order_relaxed)) return DMR_OK;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     DMR_CUDA(cudaStreamIsCapturing(st, &cap));
     // while the caller captures, the structures are built on a stream of their
@@ -559,10 +562,10 @@ int plan_bins(const dmr_plan *p, cudaStream_t st)
         st = own;
     }
     int rc = DMR_OK;
-    std::unique_ptr<PlanBins> b;
+    std::unique_ptr<B> b;
     try {
-        b.reset(new PlanBins());
-        rc = bins_build(p, *b, st);
+        b.reset(new B());
+        rc = build(p, *b, st);
     } catch (const std::bad_alloc &) {  // (the host lists)
         set_error("no host memory for the plan's bins");
         rc = DMR_ERR_OOM;
@@ -574,91 +577,92 @@ int plan_bins(const dmr_plan *p, cudaStream_t st)
         cudaStreamDestroy(own);
     }
     if (rc != DMR_OK) return rc;
-    p->bins_ptr.store(b.release(), std::memory_order_release);
+    slot.store(b.release(), std::memory_order_release);
     return DMR_OK;
 }
 
-// Tensor-core gridding order of 3D plans made while dmr_tc_min_coils is set
-static int tg_build(dmr_plan *p, int32_t *keys, int32_t *keys_s, int32_t *vals, cudaStream_t st)
+int plan_bins(const dmr_plan *p, cudaStream_t st) { return publish(p, p->bins_ptr, st, bins_build); }
+
+// grid extents in tensor-core bins: region (T + W - 1) of 7 x 6 x 6 points (x, y,
+// z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..4 (at width 5 with 32 coils the
+// kernel's bounded waits ran out)
+static int64_t tg_tiles(const Geom &g, int T[3], int nb[3])
+{
+    const int W = g.W[0];
+    int64_t n = g.nframes;
+    for (int a = 0; a < 3; a++) {
+        T[a] = std::min(a == 0 ? 8 - W : 7 - W, g.G[a]);
+        nb[a] = (int)ceil_div(g.G[a], T[a]);
+        n *= nb[a];
+    }
+    return n;
+}
+
+bool tg_geometry_ok(const dmr_plan *p)
 {
     const Geom &g = p->g;
-    const int64_t total = g.total, nframes = g.nframes;
+    if (g.ndim != 3 || g.total == 0 || g.W[0] != g.W[1] || g.W[1] != g.W[2] || g.W[0] < 2 || g.W[0] > 4) return false;
+    int T[3], nb[3];
+    return tg_tiles(g, T, nb) < INT32_MAX;
+}
+
+static int tg_build(const dmr_plan *p, TgBins &out, cudaStream_t st)
+{
+    const Geom &g = p->g;
+    const int64_t total = g.total;
     float *const *rk = p->rk;
     const int dev = p->device;
+    const int64_t tkeys = tg_tiles(g, out.T, out.nb);
+    out.nbins = out.nb[0] * out.nb[1] * out.nb[2];
     PlanTemp tmp(dev, st);
-    // bins of the 3D tensor-core gridding: region (T + W - 1) of 7 x 6 x 6
-    // points (x, y, z), i.e. T = (8 - W, 7 - W, 7 - W), for widths 2..4 (at width
-    // 5 with 32 coils the kernel's bounded waits ran out)
-    // (only where dmr_tc_min_coils was set: 1.3 GB and a second sort for the
-    // 192^3 kooshball)
-    if (tc_min_coils() == INT_MAX || g.ndim != 3 || total == 0 || g.W[0] != g.W[1] || g.W[1] != g.W[2] || g.W[0] < 2 ||
-        g.W[0] > 4)
-        return DMR_OK;
-    {
-        const int W = g.W[0];
-        int tT[3] = {8 - W, 7 - W, 7 - W}, tnb[3];
-        for (int a = 0; a < 3; a++) {
-            tT[a] = std::min(tT[a], g.G[a]);
-            tnb[a] = (int)ceil_div(g.G[a], tT[a]);
-        }
-        const int tbins = tnb[0] * tnb[1] * tnb[2];
-        const int64_t tkeys = (int64_t)nframes * tbins;
-        if (tkeys < INT32_MAX) {
-            int32_t *tcounts = nullptr;
-            DMR_TRY(tmp.alloc(&tcounts, tkeys));
-            DMR_CUDA(cudaMemsetAsync(tcounts, 0, tkeys * sizeof(int32_t), st));
-            tg_key_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], tnb[0], tnb[1], tnb[2],
-                                                                   tbins, p->foff_dev, rk[0], rk[1], rk[2], keys, tcounts);
-            DMR_LAUNCHED("tg_key_kernel");
-            int tbit = 1;
-            while ((1ll << tbit) < tkeys) tbit++;
-            for (int a = 0; a < 3; a++) DMR_TRY(plan_alloc(dev, &p->tg_scoord[a], total, st));
-            DMR_TRY(plan_alloc(dev, &p->tg_sidx, total, st));
-            size_t tb = 0;
-            DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
-                                                     tbit, st));
-            char *ttemp = nullptr;
-            DMR_TRY(tmp.alloc(&ttemp, tb));
-            DMR_CUDA(cub::DeviceRadixSort::SortPairs(ttemp, tb, keys, keys_s, vals, p->tg_sidx, (int)total, 0,
-                                                     tbit, st));
-            g_launches.fetch_add(1);
-            gather_sorted_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(
-                total, 3, p->tg_sidx, rk[0], rk[1], rk[2], p->tg_scoord[0], p->tg_scoord[1], p->tg_scoord[2]);
-            DMR_LAUNCHED("gather_sorted_kernel");
-            p->tg_wp = W <= 4 ? 4 : 8;
-            DMR_TRY(plan_alloc(dev, &p->tg_w, (size_t)total * 3 * p->tg_wp, st));
-            DMR_TRY(plan_alloc(dev, &p->tg_l, total, st));
-            tg_weights_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, tT[0], tT[1], tT[2], p->tg_wp,
-                                                                       p->tg_scoord[0], p->tg_scoord[1],
-                                                                       p->tg_scoord[2], p->tg_w, p->tg_l);
-            DMR_LAUNCHED("tg_weights_kernel");
-            std::vector<int32_t> hc(tkeys);
-            DMR_CUDA(cudaMemcpyAsync(hc.data(), tcounts, tkeys * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-            DMR_CUDA(cudaStreamSynchronize(st));
-            std::vector<int32_t> ts(tkeys + 1, 0);
-            for (int64_t i = 0; i < tkeys; i++) ts[i + 1] = ts[i] + hc[i];
-            std::vector<WorkItem> titems;
-            std::vector<int32_t> torder;
-            make_items(ts, tbins, tnb, kTgSegment, titems, torder);
-            DMR_TRY(plan_alloc(dev, &p->tg_work, titems.size(), st));
-            DMR_TRY(plan_alloc(dev, &p->tg_order, torder.size(), st));
-            if (!titems.empty()) {
-                DMR_CUDA(cudaMemcpyAsync(p->tg_work, titems.data(), titems.size() * sizeof(WorkItem),
-                                         cudaMemcpyHostToDevice, st));
-                DMR_CUDA(cudaMemcpyAsync(p->tg_order, torder.data(), torder.size() * sizeof(int32_t),
-                                         cudaMemcpyHostToDevice, st));
-            }
-            DMR_CUDA(cudaStreamSynchronize(st));
-            p->tg_nwork = (int)titems.size();
-            p->tg_nbins = tbins;
-            for (int a = 0; a < 3; a++) {
-                p->tg_T[a] = tT[a];
-                p->tg_nb[a] = tnb[a];
-            }
-        }
-    }
+    int32_t *keys = nullptr, *keys_s = nullptr, *vals = nullptr, *counts = nullptr;
+    float *sc[3] = {nullptr, nullptr, nullptr};
+    DMR_TRY(tmp.alloc(&keys, total));
+    DMR_TRY(tmp.alloc(&keys_s, total));
+    DMR_TRY(tmp.alloc(&vals, total));
+    DMR_TRY(tmp.alloc(&counts, tkeys));
+    for (int a = 0; a < 3; a++) DMR_TRY(tmp.alloc(&sc[a], total));
+    DMR_TRY(plan_alloc(dev, &out.sidx, total, st));
+    out.wp = 4;
+    DMR_TRY(plan_alloc(dev, &out.w, (size_t)total * 3 * out.wp, st));
+    DMR_TRY(plan_alloc(dev, &out.l, total, st));
+    DMR_CUDA(cudaMemsetAsync(counts, 0, tkeys * sizeof(int32_t), st));
+    tg_key_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, out.T[0], out.T[1], out.T[2], out.nb[0], out.nb[1],
+                                                           out.nbins, p->foff_dev, rk[0], rk[1], rk[2], keys, vals,
+                                                           counts);
+    DMR_LAUNCHED("tg_key_kernel");
+    int bits = 1;
+    while ((1ll << bits) < tkeys) bits++;
+    size_t tb = 0;
+    DMR_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_s, vals, out.sidx, (int)total, 0, bits, st));
+    char *temp = nullptr;
+    DMR_TRY(tmp.alloc(&temp, tb));
+    DMR_CUDA(cub::DeviceRadixSort::SortPairs(temp, tb, keys, keys_s, vals, out.sidx, (int)total, 0, bits, st));
+    g_launches.fetch_add(1);
+    gather_sorted_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(total, 3, out.sidx, rk[0], rk[1], rk[2], sc[0], sc[1],
+                                                                  sc[2]);
+    DMR_LAUNCHED("gather_sorted_kernel");
+    tg_weights_kernel<<<grid_blocks(total, 256), 256, 0, st>>>(g, out.T[0], out.T[1], out.T[2], out.wp, sc[0], sc[1],
+                                                               sc[2], out.w, out.l);
+    DMR_LAUNCHED("tg_weights_kernel");
+    std::vector<int32_t> hc(tkeys);
+    DMR_CUDA(cudaMemcpyAsync(hc.data(), counts, tkeys * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    DMR_CUDA(cudaStreamSynchronize(st));
+    std::vector<int32_t> ts(tkeys + 1, 0);
+    for (int64_t i = 0; i < tkeys; i++) ts[i + 1] = ts[i] + hc[i];
+    std::vector<WorkItem> items;
+    std::vector<int32_t> order;
+    make_items(ts, out.nbins, out.nb, kTgSegment, items, order);
+    DMR_TRY(plan_alloc(dev, &out.work, items.size(), st));
+    DMR_TRY(plan_alloc(dev, &out.order, order.size(), st));
+    DMR_CUDA(cudaMemcpyAsync(out.work, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, st));
+    DMR_CUDA(cudaMemcpyAsync(out.order, order.data(), order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+    DMR_CUDA(cudaStreamSynchronize(st));
+    out.nwork = (int)items.size();
     return DMR_OK;
 }
+
+int plan_tg(const dmr_plan *p, cudaStream_t st) { return publish(p, p->tg_ptr, st, tg_build); }
 
 }  // namespace dmr
 
@@ -791,7 +795,6 @@ extern "C" int dmr_plan_create(int ndim, const int32_t *shape, const int32_t *os
     DMR_CUDA(cudaStreamSynchronize(st));
     DMR_CHECK(h_err == 0, DMR_ERR_COORD, "non-finite (or |k| >= 1e8) k-space coordinate");
     march_lists(p.get(), totals);
-    DMR_TRY(tg_build(p.get(), keys, keys_s, vals, st));
     // plans of the interleaved kernels build the bin structures when a call
     // needs them (plan_bins)
     if (!p->il_forward()) DMR_TRY(plan_bins(p.get(), st));

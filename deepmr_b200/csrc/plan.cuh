@@ -135,6 +135,36 @@ struct PlanBins {
 };
 // builds them on first use (plan.cu)
 int plan_bins(const ::dmr_plan *p, cudaStream_t st);
+
+// The bins of 3D tensor-core gridding (dmr_tc_min_coils), built and published the
+// same way: bins of its own (tile T, x y z) whose region (tile + W - 1 per axis)
+// is at most 7 x 6 x 6 = 252 points, one N = 256 MMA; the samples of a bin in
+// acquisition order (consecutive samples of a spoke, which share 32-byte sectors
+// of k-space, are read together); work items of at most kTgSegment samples,
+// visited in 4 x 4 x 4-bin tiles.
+struct TgBins {
+    int T[3] = {0, 0, 0};
+    int nb[3] = {1, 1, 1};
+    int nbins = 0;
+    int32_t *sidx = nullptr;
+    // per sample (gridding order): the Kaiser-Bessel weights of its W taps on
+    // each axis, [sample][axis][wp] (wp = 4), and the offsets of its first taps
+    // inside its bin, x | y << 8 | z << 16
+    float *w = nullptr;
+    int32_t *l = nullptr;
+    int wp = 0;
+    WorkItem *work = nullptr;
+    int nwork = 0;
+    int32_t *order = nullptr;
+    ~TgBins()
+    {
+        for (void *q : {(void *)sidx, (void *)w, (void *)l, (void *)work, (void *)order})
+            if (q) cudaFreeAsync(q, cudaStreamPerThread);
+    }
+};
+// whether a plan can have them (3D, one width of 2..4 on all axes), and the same for them
+bool tg_geometry_ok(const ::dmr_plan *p);
+int plan_tg(const ::dmr_plan *p, cudaStream_t st);
 // Register-tile gridding: whether the geometry admits it (3D, grid at least
 // a block region plus the kernel support on every axis); plan the block items after the bin sort (host
 // bin offsets h_start, nframes * nbins + 1 entries); scratch bytes a call of
@@ -206,26 +236,7 @@ struct dmr_plan {
     mutable std::mutex bins_mu;
     mutable std::atomic<const dmr::PlanBins *> bins_ptr{nullptr};
     const dmr::PlanBins &bins() const { return *bins_ptr.load(std::memory_order_acquire); }
-    // 3D tensor-core gridding: bins of its own (tile tg_T, x y z) whose region
-    // (tile + W - 1 per axis) is at most 7 x 6 x 6 = 252 points, one N = 256
-    // MMA; the samples of a bin in acquisition order (consecutive samples of a
-    // spoke, which share 32-byte sectors of k-space, are read together);
-    // work items of at most 2048 samples, visited in 4 x 4 x 4-bin tiles.
-    // tg_T[0] == 0: not planned.
-    int tg_T[3] = {0, 0, 0};
-    int tg_nb[3] = {1, 1, 1};
-    int tg_nbins = 0;
-    float *tg_scoord[3] = {nullptr, nullptr, nullptr};
-    int32_t *tg_sidx = nullptr;
-    // per sample (gridding order): the Kaiser-Bessel weights of its W taps on
-    // each axis, [sample][axis][tg_wp] (tg_wp = 4 for W <= 4, else 8), and the
-    // offsets of its first taps inside its bin, x | y << 8 | z << 16
-    float *tg_w = nullptr;
-    int32_t *tg_l = nullptr;
-    int tg_wp = 0;
-    dmr::WorkItem *tg_work = nullptr;
-    int tg_nwork = 0;
-    int32_t *tg_order = nullptr;
+    mutable std::atomic<const dmr::TgBins *> tg_ptr{nullptr};
     float *apod[3] = {nullptr, nullptr, nullptr};  // per-axis apodisation (image index)
     int64_t *foff_dev = nullptr;        // frame offsets on the device (nframes + 1)
     // march order (march.cu; mp_W == 0: not planned; 3D, and 2D plans dense enough
@@ -266,13 +277,8 @@ struct dmr_plan {
         };
         drop(tables);
         delete bins_ptr.load();
+        delete tg_ptr.load();
         for (int a = 0; a < 3; a++) drop(rk[a]);
-        for (int a = 0; a < 3; a++) drop(tg_scoord[a]);
-        drop(tg_sidx);
-        drop(tg_w);
-        drop(tg_l);
-        drop(tg_work);
-        drop(tg_order);
         drop(status);
         drop(mp_cstart);
         drop(mp_sidx);

@@ -1418,7 +1418,7 @@ bool grid_march_applies(const dmr_plan *p, int64_t batch, int det)
 {
     if ((p->mp_W == 0 && p->d2_W == 0) || grid_variant() != 0) return false;
     if (det) return p->mp_W && !(p->g.ndim == 3 && tc_disabled());
-    return p->tg_T[0] == 0 || batch < tc_min_coils();
+    return batch < tc_min_coils() || tc_disabled() || !tg_geometry_ok(p);
 }
 
 int grid_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
@@ -1430,8 +1430,9 @@ int grid_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, i
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }
     // atomic 3D gridding on the tensor cores where dmr_tc_min_coils asks for it
-    // (plans made under that setting have its gridding bins)
-    if (p->g.ndim == 3 && grid_variant() == 0 && !det && batch >= tc_min_coils()) {
+    // (its bins, 1.3 GB for the 192^3 kooshball, are built by the first such call)
+    if (grid_variant() == 0 && !det && batch >= tc_min_coils() && !tc_disabled() && tg_geometry_ok(p)) {
+        DMR_TRY(plan_tg(p, st));
         const int rc = grid_tc_dispatch(p, ksp, kreal, grid, batch, weight, wpb, st);
         if (rc != DMR_ERR_UNSUPPORTED) return rc;
     }

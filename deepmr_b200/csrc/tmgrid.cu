@@ -689,18 +689,18 @@ __global__ void __launch_bounds__(kTmThreads, 1) grid_tmem_kernel(
     }
 }
 
-bool tm_shape(const dmr_plan *p, int64_t batch, int wpb, int smem_limit, TmShape &s)
+bool tm_shape(const dmr_plan *p, const TgBins &b, int64_t batch, int wpb, int smem_limit, TmShape &s)
 {
     const Geom &g = p->g;
-    if (g.ndim != 3 || batch < 1 || p->tg_T[0] == 0) return false;
+    if (g.ndim != 3 || batch < 1) return false;
     const int W = g.W[0];
-    for (int a = 0; a < 3; a++) s.R[a] = p->tg_T[a] + W - 1;
+    for (int a = 0; a < 3; a++) s.R[a] = b.T[a] + W - 1;
     s.P = s.R[0] * s.R[1] * s.R[2];
     if (s.P > kTmN) return false;
     s.vrows = s.R[0] + s.R[1] + s.R[2];
     if (s.vrows > kTmMaxRows) return false;
     s.CC = (int)std::min<int64_t>(batch, kTmCC);
-    s.wp = p->tg_wp;
+    s.wp = b.wp;
     int off = kTmSB * 3 * s.wp * 4;  // tap weights of the pass, [sample][axis][wp]
     s.l_off = off;
     off += kTmSB * 4;
@@ -741,6 +741,7 @@ bool tm_shape(const dmr_plan *p, int64_t batch, int wpb, int smem_limit, TmShape
 int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, int64_t batch,
                      const float *weight, int wpb, int *timeouts, int stall, cudaStream_t st)
 {
+    const TgBins &b = *p->tg_ptr.load(std::memory_order_acquire);
     int dev = 0, sms = 0, smem_blk = 0;
     DMR_CUDA(cudaGetDevice(&dev));
     DMR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -748,7 +749,7 @@ int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     cudaFuncAttributes fa;
     DMR_CUDA(cudaFuncGetAttributes(&fa, grid_tmem_kernel));
     TmShape sh;
-    if (!tm_shape(p, batch, wpb, smem_blk - (int)fa.sharedSizeBytes, sh)) return DMR_ERR_UNSUPPORTED;
+    if (!tm_shape(p, b, batch, wpb, smem_blk - (int)fa.sharedSizeBytes, sh)) return DMR_ERR_UNSUPPORTED;
     const size_t smem = (size_t)sh.goff_off + kTmN * 4;
     // one block per SM: it allocates all 512 tensor-memory columns
     DMR_CUDA(cudaFuncSetAttribute(grid_tmem_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -756,20 +757,20 @@ int grid_tm_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
     DMR_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, grid_tmem_kernel, kTmThreads, smem));
     if (per_sm != 1) return DMR_ERR_UNSUPPORTED;
     DMR_CUDA(cudaMemsetAsync(grid, 0, (size_t)batch * p->g.nframes * p->g.gsize * sizeof(float2), st));
-    if (p->tg_nwork == 0) return DMR_OK;
+    if (b.nwork == 0) return DMR_OK;
     const int64_t nchunks = ceil_div(batch, sh.CC);
-    DMR_CHECK((int64_t)p->tg_nwork * nchunks < (1ll << 31), DMR_ERR_UNSUPPORTED, "too many gridding tasks");
+    DMR_CHECK((int64_t)b.nwork * nchunks < (1ll << 31), DMR_ERR_UNSUPPORTED, "too many gridding tasks");
     DMR_CHECK(nchunks * sh.CC < (1ll << 31), DMR_ERR_UNSUPPORTED, "batch too large");
     Geom g = p->g;
     for (int a = 0; a < 3; a++) {
-        g.T[a] = p->tg_T[a];
-        g.nb[a] = p->tg_nb[a];
+        g.T[a] = b.T[a];
+        g.nb[a] = b.nb[a];
     }
-    g.nbins = p->tg_nbins;
+    g.nbins = b.nbins;
     const float inv_scale = (float)(1.0 / p->scale);
-    const int blocks = (int)std::min<int64_t>((int64_t)p->tg_nwork * nchunks, (int64_t)sms);
+    const int blocks = (int)std::min<int64_t>((int64_t)b.nwork * nchunks, (int64_t)sms);
     grid_tmem_kernel<<<blocks, kTmThreads, smem, st>>>(
-        g, sh, p->tg_work, p->tg_order, p->tg_nwork, (int)nchunks, p->tg_w, p->tg_l, p->tg_sidx, ksp, kreal, grid,
+        g, sh, b.work, b.order, b.nwork, (int)nchunks, b.w, b.l, b.sidx, ksp, kreal, grid,
         batch, weight, wpb, inv_scale, p->status, timeouts, stall);
     DMR_LAUNCHED("grid_tmem_kernel");
     return DMR_OK;

@@ -106,12 +106,13 @@ int dmr_fft3_fused(dmr_plan *plan);
 
 /*
  * Tuning knob, no reference counterpart: atomic gridding of 3D plans of widths
- * 2..4 that are made while it is set runs on the tensor cores for batches of
- * at least `coils` coils and on the CUDA cores otherwise. By default
- * (INT32_MAX) none does: the CUDA-core plane kernel is faster at every batch
- * (192^3 kooshball, 32 coils: 8.1 ms with its row transposition, tensor cores
- * 16.2 ms) and closer to the exact sums. coils <= 0 only queries. Returns the
- * previous value. Process-wide; deterministic gridding is not affected.
+ * 2..4 runs on the tensor cores for batches of at least `coils` coils and on the
+ * CUDA cores otherwise (a plan's first such call builds the bins of that kernel,
+ * 1.3 GB for the 192^3 kooshball). By default (INT32_MAX) none does: the CUDA-core
+ * plane kernel is faster at every batch (192^3 kooshball, 32 coils: 8.1 ms with its
+ * row transposition, tensor cores 16.2 ms) and closer to the exact sums. coils <= 0
+ * only queries. Returns the previous value. Process-wide; deterministic gridding is
+ * not affected.
  */
 int dmr_tc_min_coils(int coils);
 

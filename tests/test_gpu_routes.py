@@ -467,3 +467,52 @@ def test_arguments_that_outlive_their_transform():
             assert rel(res[0].detach(), res[1].detach()) < 1e-6, name
         else:
             assert res[0] is res[1], name
+
+
+def test_tensor_core_gridding_of_a_plan_that_exists():
+    """dmr_tc_min_coils moves the calls of a plan made before it was set (the
+    kernel's test stall, which only it obeys, shows that it ran), captured as well,
+    and back."""
+    import gc
+
+    import deepmr_b200.fft as F
+    from deepmr_b200 import _lib
+    from oracle import nufft_ref as R
+    from deepmr_b200 import synth
+
+    L = _lib.lib()
+    plan, _, ksp = _problem3()
+    c = torch.as_tensor(synth.kooshball_3d(160, 64, 24).astype(np.float32))
+    ref = R.apply_nufft_adj(ksp.cpu(), R.plan_nufft(c, 24, 4, 1.25))
+
+    def ran_on_tensor_cores():
+        L.dmr_tc_test_stall(1)
+        try:
+            F.apply_nufft_adj(ksp, plan)
+            plan.interpolator.check_status()
+        except _lib.DmrError as e:
+            assert e.code == -8
+            return True
+        finally:
+            L.dmr_tc_test_stall(0)
+        return False
+
+    assert not ran_on_tensor_cores()
+    old = L.dmr_tc_min_coils(9)
+    try:
+        gc.collect()
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            x = F.apply_nufft_adj(ksp, plan)
+        g.replay()
+        assert rel(x, ref) < TOL and rel(F.apply_nufft_adj(ksp, plan), ref) < TOL
+        assert ran_on_tensor_cores()
+        L.dmr_tc_min_coils(10)
+        assert not ran_on_tensor_cores()
+    finally:
+        L.dmr_tc_min_coils(old)
+    assert rel(F.apply_nufft_adj(ksp, plan), ref) < TOL
+    g = None
+    n = ctypes.c_int64()
+    _lib.check(L.dmr_tc_timeouts(ctypes.byref(n), 1))
