@@ -258,13 +258,14 @@ static void default_tile(int ndim, int T[3])
 // Plan memory comes from a pool of its own (stream-ordered, so that a plan
 // costs no device-wide allocator calls: 20 cudaMalloc / cudaFree pairs took
 // over 2 ms); the pool keeps at most 256 MB for the next plan.
-cudaMemPool_t plan_pool(int dev)
+cudaMemPool_t plan_pool(int dev, bool create)
 {
     static std::mutex mu;
     static std::map<int, cudaMemPool_t> pools;
     std::lock_guard<std::mutex> lk(mu);
     auto it = pools.find(dev);
     if (it != pools.end()) return it->second;
+    if (!create) return nullptr;
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -287,7 +288,7 @@ static thread_local int t_fail_alloc = 0;
 int plan_alloc_bytes(int dev, void **p, size_t bytes, cudaStream_t st)
 {
     if (t_fail_alloc > 0 && --t_fail_alloc == 0) bytes = (size_t)1 << 60;  // more than any device has
-    cudaMemPool_t pool = plan_pool(dev);
+    cudaMemPool_t pool = plan_pool(dev, true);
     DMR_CHECK(pool, DMR_ERR_CUDA, "no memory pool on device %d", dev);
     DMR_CUDA(cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 16), pool, st));
     return DMR_OK;

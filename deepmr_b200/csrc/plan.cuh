@@ -174,6 +174,8 @@ int rt_build(const ::dmr_plan *p, PlanBins &b, const std::vector<int32_t> &h_sta
 size_t rt_scratch_bytes(const ::dmr_plan *p, int64_t batch);
 // scratch bytes a gridding call of `batch` coils may need (either kernel)
 size_t grid_scratch_bytes(const ::dmr_plan *p, int64_t batch);
+// the plans' pool (nullptr where none exists and `create` is false)
+cudaMemPool_t plan_pool(int dev, bool create);
 // library-owned stream-ordered pool for the scratch of calls without a workspace
 cudaMemPool_t scratch_pool(int dev);
 // fused, pruned FFT passes of the NUFFT pipelines (fftpass.cu): whether they

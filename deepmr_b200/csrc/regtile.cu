@@ -685,16 +685,17 @@ int grid_rt_dispatch(const dmr_plan *p, const void *ksp, int kreal, float2 *grid
 
 }  // namespace dmr
 
-// Return the scratch pool's free memory on `device` to the device.
+// Return the free memory of the library's pools on `device` to the device.
 extern "C" int dmr_scratch_release(int device)
 {
-    cudaMemPool_t pool = dmr::find_pool(device, false);
-    if (!pool) return DMR_OK;
+    cudaMemPool_t pools[2] = {dmr::find_pool(device, false), dmr::plan_pool(device, false)};
+    if (!pools[0] && !pools[1]) return DMR_OK;
     int old = 0;
     DMR_CUDA(cudaGetDevice(&old));
     DMR_CUDA(cudaSetDevice(device));
     cudaError_t e = cudaDeviceSynchronize();
-    if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
+    for (cudaMemPool_t pool : pools)
+        if (e == cudaSuccess && pool) e = cudaMemPoolTrimTo(pool, 0);
     cudaSetDevice(old);
     if (e != cudaSuccess) return dmr::cuda_fail(e, "dmr_scratch_release", __FILE__, __LINE__);
     return DMR_OK;

@@ -118,12 +118,14 @@ int dmr_tc_min_coils(int coils);
 
 /*
  * Housekeeping, no reference counterpart: gives back to `device` the memory
- * that the library's scratch pool holds beyond what is in use. Calls without
+ * that the library's pools hold beyond what is in use: that of destroyed plans
+ * (at most 256 MB are kept) and gridding scratch. Calls without
  * a large enough workspace take their gridding scratch from this pool, which
  * keeps it for the next call; deterministic 3D gridding keeps every gridding
  * unit's plane there (392 bytes per unit and coil at width 4: 10.9 GB for 32
  * coils of the 192^3, 19.2 M-sample kooshball), and dmr_interp / dmr_grid of
- * 3D plans a chunk's rows and interleaved grid. Synchronises the device first. Returns 0 or a DMR_ERR_* code.
+ * 3D plans a chunk's rows and interleaved grid. Synchronises the device first.
+ * Returns 0 or a DMR_ERR_* code.
  */
 int dmr_scratch_release(int device);
 

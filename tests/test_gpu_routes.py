@@ -516,3 +516,26 @@ def test_tensor_core_gridding_of_a_plan_that_exists():
     g = None
     n = ctypes.c_int64()
     _lib.check(L.dmr_tc_timeouts(ctypes.byref(n), 1))
+
+
+def test_release_gives_back_the_memory_of_destroyed_plans():
+    """After a plan of several hundred MB is gone, releasing the library's pools
+    leaves the device with the memory it had before."""
+    import gc
+
+    import deepmr_b200.fft as F
+
+    gc.collect()
+    torch.cuda.synchronize()
+    F.release_scratch()
+    torch.cuda.empty_cache()
+    before = torch.cuda.mem_get_info()[0]
+    c = torch.rand((1, 4_000_000, 3)) * 60 - 30
+    plan = F.plan_nufft(c, 64, 4, 1.25, device="cuda")
+    during = torch.cuda.mem_get_info()[0]
+    del plan
+    gc.collect()
+    F.release_scratch()
+    torch.cuda.empty_cache()
+    assert before - during > 300 << 20  # (the plan is larger than what the pool keeps)
+    assert before - torch.cuda.mem_get_info()[0] < 32 << 20
