@@ -539,3 +539,37 @@ def test_release_gives_back_the_memory_of_destroyed_plans():
     torch.cuda.empty_cache()
     assert before - during > 300 << 20  # (the plan is larger than what the pool keeps)
     assert before - torch.cuda.mem_get_info()[0] < 32 << 20
+
+
+@pytest.mark.parametrize("shape,os,grid", [((17, 30, 19), (2.0, 1.5, 2.0), (34, 45, 38)),
+                                           ((22, 17, 26), (1.5, 2.0, 1.5), (33, 34, 39))])
+@pytest.mark.parametrize("width", [3, 4])
+def test_run_time_lengths_3d(shape, os, grid, width):
+    """Run-time FFT lengths on all axes of a 3D grid, planar (1 coil) and interleaved
+    (3 and 9), both directions and modes, real images, and the 3D Toeplitz pass."""
+    import deepmr_b200.fft as F
+    from deepmr_b200 import _lib, synth
+    from oracle import nufft_ref as R
+
+    rng = np.random.default_rng(width)
+    c = torch.as_tensor((rng.uniform(-0.5, 0.5, (3, 60, 3)) * np.asarray(shape[::-1])).astype(np.float32))
+    plan, oplan = F.plan_nufft(c, shape, width, os, device="cuda"), R.plan_nufft(c, shape, width, os)
+    assert _lib.lib().dmr_fft3_fused(plan.interpolator.handle) == 1
+    assert tuple(int(g) for g in oplan.os_shape) == grid
+    img = synth.complex_gaussian((9,) + shape, seed=1)
+    ksp = synth.complex_gaussian((9, 3, 60), seed=2)
+    y, x = R.apply_nufft(img, oplan), R.apply_nufft_adj(ksp, oplan)
+    for k in (1, 3, 9):
+        assert rel(F.apply_nufft(img[:k].cuda(), plan), y[:k]) < TOL, k
+        for det in (False, True):
+            old = F.set_deterministic_gridding(det)
+            try:
+                assert rel(F.apply_nufft_adj(ksp[:k].cuda(), plan), x[:k]) < TOL, (k, det)
+            finally:
+                F.set_deterministic_gridding(old)
+    assert rel(F.apply_nufft(img.real.contiguous().cuda(), plan), R.apply_nufft(img.real, oplan)) < TOL
+    dcf = torch.as_tensor(rng.uniform(0.5, 1.5, (3, 60)).astype(np.float32))
+    T = F.plan_toeplitz_nufft(c, shape, dcf=dcf, device="cuda")
+    ref = R.apply_selfadj(img, R.plan_toeplitz(c, shape, dcf=dcf))
+    for k in (1, 9):
+        assert rel(F.apply_nufft_selfadj(img[:k].cuda(), T), ref[:k]) < TOL, k
