@@ -34,6 +34,7 @@ import numpy as np
 import torch
 
 from . import fft as _fft
+from .fft import _nufft
 
 
 # ---------------------------------------------------------------------------
@@ -164,6 +165,17 @@ def _cartesian_acs(kspace):
     return _fft.fft(sub, axes=(1,))
 
 
+def _adjoint(ksp, coord, shape):
+    """Adjoint NUFFT at oversampling 2, gridded in a fixed order: the phase that an
+    SVD gives a voxel's maps can turn on the last bit of the calibration data, and
+    calibrating twice should give the same maps."""
+    grads = [t for t in (ksp, coord) if isinstance(t, torch.Tensor) and t.requires_grad]
+    if grads and torch.is_grad_enabled():
+        return _fft.nufft_adj(ksp, coord, shape, oversamp=2.0)
+    plan = _nufft.plan_nufft(coord, shape, 4, 2.0)
+    return _nufft._apply_nufft_adj(ksp, plan, None, None, None, 128, deterministic=True)
+
+
 def _noncartesian_acs(kspace, cal_shape, coord, dcf):
     """acs.py:117-152: contrasts folded into views, central samples of the
     first view's radius profile, adjoint NUFFT at oversampling 2, back to
@@ -177,7 +189,7 @@ def _noncartesian_acs(kspace, cal_shape, coord, dcf):
     crd = crd[..., sel, :]
     if dcf is not None:
         ksp = dcf.reshape(1, -1, dcf.shape[-1])[..., sel] * ksp
-    grid = _fft.nufft_adj(ksp, crd, cal_shape, oversamp=2.0).squeeze()
+    grid = _adjoint(ksp, crd, cal_shape).squeeze()
     if grid.ndim != 4:
         grid = grid[None, ...]
     if ndim == 2:

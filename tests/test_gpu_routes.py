@@ -573,3 +573,13 @@ def test_run_time_lengths_3d(shape, os, grid, width):
     ref = R.apply_selfadj(img, R.plan_toeplitz(c, shape, dcf=dcf))
     for k in (1, 9):
         assert rel(F.apply_nufft_selfadj(img[:k].cuda(), T), ref[:k]) < TOL, k
+
+
+def test_calibration_repeats():
+    """Calibrating twice gives the same maps, bit for bit (2D radial, ESPIRiT)."""
+    from deepmr_b200 import calib
+
+    d = np.load(__file__.replace("test_gpu_routes.py", "golden/calib2d.npz"))
+    a = [torch.as_tensor(d[k]).cuda() for k in ("kspace", "coord", "dcf")]
+    maps = [calib.espirit_cal(a[0], coord=a[1], dcf=a[2], shape=int(d["shape"]))[0] for _ in range(20)]
+    assert all(torch.equal(m, maps[0]) for m in maps[1:])
