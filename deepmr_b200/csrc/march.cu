@@ -52,12 +52,12 @@ __host__ __device__ constexpr int march_rec(int W, int ndim = 3) { return (ndim 
 // W 4: 8.1e-7 at 64, 10.2 at 512), and several planes to a warp cost no more in
 // short units (512 and 64: 772 and 790 us; 64^3, 8 coils: 265 and 240). With a
 // plane per warp a unit's flush weighs more (192^3, 32 coils: 12.2 ms at 512, 13.7
-// at 64), so these have lists of both: see launch_planes. At width 6 all are short
+// at 64), so these are long, and short where a call needs it: see launch_planes. At width 6 all are short
 // (144^3, 32 coils: 5.1 and 5.4 ms)
 constexpr int kShortUnit = 64, kLongUnit = 512;
-// unit lists: planes per warp, the last one of short units
-constexpr int kUnitLists = 5;
-constexpr int kUnitPlanes[kUnitLists] = {1, 2, 4, 8, 1};
+// unit lists of a plan: planes per warp
+constexpr int kUnitLists = 4;
+constexpr int kUnitPlanes[kUnitLists] = {1, 2, 4, 8};
 constexpr int unit_visits(int ndim, int W, int list) { return ndim == 3 && W <= 5 && list == 0 ? kLongUnit : kShortUnit; }
 constexpr int kItemSamples = 144;
 constexpr int kItemZ = 8;  // z cells of an interpolation item
@@ -69,6 +69,7 @@ struct MarchGeom {
     int T, nt0, nt1;  // tile extent, tiles along x and y
     int CS;           // coils of the chunk = coil stride of the grid
     int RS;           // coil stride of the rows (CS rounded up to even)
+    bool join;        // gridding: a block's warps add their pieces of a plane first
     int64_t plane;    // G[0] * G[1]
     int64_t gsize;
 };
@@ -552,7 +553,8 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
     // shared memory, `give` to `take`, whose barriers both sides reach). A heavy
     // plane's sum is then a tree over units of a block and a chain over blocks, a
     // quarter as long: it is the chain in the grid that rounds most (64^3, 8 coils:
-    // 8.4e-7 of the result without, see unit_visits)
+    // 8.4e-7 of the result without, see unit_visits). Long units gain nothing from it
+    // (192^3, 32 coils: 1.2e-6 either way, 0.06 of 11.5 ms)
     static_assert(kGridWarps == 4, "pairs of warps");
     auto same = [&](int v) {  // unit v is a piece of the same plane
         if (v < 0 || v >= nunits) return false;
@@ -578,14 +580,14 @@ __global__ void __launch_bounds__(32 * kGridWarps, W <= 4 ? 4 : 3)
             for (int k = 0; k < R; k++) acc[i][k] = __fadd2_rn(acc[i][k], d[(i * R + k) * 32]);
     };
     const int pair = (warp >> 1) * S::PAIR;
-    if (same(warp & 1 ? u - 1 : u + 1)) {
+    if (g.join && same(warp & 1 ? u - 1 : u + 1)) {
         join(1 + (warp >> 1));  // both are done with their rings
         if (warp & 1) give(pair);
         join(1 + (warp >> 1));
         if (warp & 1) return;
         take(pair);
     }
-    if (!(warp & 1) && same(warp ? u - 2 : u + 2)) {  // (the unit between is one of the plane's, too)
+    if (g.join && !(warp & 1) && same(warp ? u - 2 : u + 2)) {  // (the unit between is one of the plane's, too)
         join(3);  // warp 0 has taken what lay in its pair's memory
         if (warp) give(0);
         join(3);
@@ -687,11 +689,18 @@ __global__ void __launch_bounds__(256) grid_planes_gather_kernel(MarchGeom g, in
                 const int dy = cover_at(ycov, ky) & 7;
                 return scratch + ((int64_t)s * (R * R) + dy * R + (vx & 7)) * g.CS + c;
             };
-            auto rest = [&](int2 u, int ky, int vx) {  // a split unit's further pieces, added eight at a time (rounding)
-                for (int s = 1; s < u.y;) {
-                    float2 sum = __ldcs(slot(u.x + s, ky, vx));
-                    for (const int e = min(s + 8, u.y); ++s < e;) sum = __fadd2_rn(sum, __ldcs(slot(u.x + s, ky, vx)));
-                    acc = __fadd2_rn(acc, sum);
+            // a split unit's further pieces; short ones (width 6) eight at a time, the
+            // chain of a heavy plane's pieces rounds most (long ones that way: 1.11e-6
+            // of the result both ways, 64^3, W 4, and 2 % of the call's time)
+            auto rest = [&](int2 u, int ky, int vx) {
+                if constexpr (W < 6) {
+                    for (int s = 1; s < u.y; s++) acc = __fadd2_rn(acc, __ldcs(slot(u.x + s, ky, vx)));
+                } else {
+                    for (int s = 1; s < u.y;) {
+                        float2 sum = __ldcs(slot(u.x + s, ky, vx));
+                        for (const int e = min(s + 8, u.y); ++s < e;) sum = __fadd2_rn(sum, __ldcs(slot(u.x + s, ky, vx)));
+                        acc = __fadd2_rn(acc, sum);
+                    }
                 }
             };
             if (ny <= 2 && cover_at(xc, 2) < 0) {
@@ -1072,26 +1081,32 @@ MarchGeom march_geom(const dmr_plan *p, int CS)
     m.nt1 = p->mp_nt[1];
     m.CS = CS;
     m.RS = (CS + 1) & ~1;
+    m.join = true;
     m.plane = (int64_t)g.G[0] * g.G[1];
     m.gsize = g.gsize;
     return m;
 }
 
 template <int W, int NP, int ND>
-int launch_planes_np(const dmr_plan *p, const MarchGeom &m, int L, const float2 *rows, float2 *grid, float2 *scratch,
-                     cudaStream_t st)
+int launch_planes_np(const dmr_plan *p, const MarchGeom &m, const void *units, int n, const float2 *rows, float2 *grid,
+                     float2 *scratch, cudaStream_t st)
 {
     using S = PlaneShape<W, NP, ND>;
-    const int n = p->mp_nunits[L];
     if (n == 0) return DMR_OK;
     auto kern = grid_planes_kernel<W, NP, ND>;
     DMR_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM));
-    kern<<<(unsigned)ceil_div(n, kGridWarps), 32 * kGridWarps, S::SMEM, st>>>(m, (const int4 *)p->mp_units[L], n,
+    kern<<<(unsigned)ceil_div(n, kGridWarps), 32 * kGridWarps, S::SMEM, st>>>(m, (const int4 *)units, n,
                                                                              p->mp_cstart, p->mp_rec, p->mp_zc, rows,
                                                                              grid, scratch);
     DMR_LAUNCHED("grid_planes_kernel");
     return DMR_OK;
 }
+
+// Single planes come in long units from 20 coils on, where these took the place of
+// tensor-core sums (64^3, W 4: 3.7e-6 of the result, now 1.1e-6); 17 to 19 coils
+// had the sums of the cell-cube kernel (8.0e-7) and get short ones (8.2e-7), built
+// by a plan's first such call
+bool short_planes(const dmr_plan *p, int CS) { return p->g.ndim == 3 && p->mp_W <= 5 && CS > 16 && CS < 20; }
 
 // planes per warp by the coils of the chunk: lanes = coils x planes (96^3, 8
 // coils: 385 us with 4 planes, 760 us with the cell-cube kernel; 1 coil: 227 and
@@ -1100,17 +1115,23 @@ template <int W>
 int launch_planes(const dmr_plan *p, const MarchGeom &m, const float2 *rows, float2 *grid, float2 *scratch,
                   cudaStream_t st)
 {
-    if (p->g.ndim == 2) return launch_planes_np<W, 1, 2>(p, m, 0, rows, grid, scratch, st);
+    const auto units = p->mp_units;
+    const int *n = p->mp_nunits;
+    if (p->g.ndim == 2) return launch_planes_np<W, 1, 2>(p, m, units[0], n[0], rows, grid, scratch, st);
     // deterministic units are always single planes of one list, so that a coil's
     // sums do not depend on how many coils it is gridded with
-    if (scratch) return launch_planes_np<W, 1, 3>(p, m, 0, rows, grid, scratch, st);
-    // single planes in long units from 20 coils on, where these took the place of
-    // tensor-core sums (64^3, W 4: 3.7e-6 of the result, now 1.1e-6); fewer coils
-    // had the sums of the cell-cube kernel (8.0e-7; 8.1e-7 in short units)
-    if (m.CS > 16) return launch_planes_np<W, 1, 3>(p, m, m.CS < 20 && W <= 5 ? 4 : 0, rows, grid, scratch, st);
-    if (m.CS > 8) return launch_planes_np<W, 2, 3>(p, m, 1, rows, grid, scratch, st);
-    if (m.CS > 4) return launch_planes_np<W, 4, 3>(p, m, 2, rows, grid, scratch, st);
-    return launch_planes_np<W, 8, 3>(p, m, 3, rows, grid, scratch, st);
+    if (!scratch && short_planes(p, m.CS)) {
+        const ShortUnits &s = *p->short_ptr.load(std::memory_order_acquire);
+        return launch_planes_np<W, 1, 3>(p, m, s.units, s.n, rows, grid, scratch, st);
+    }
+    if (scratch || m.CS > 16) {
+        MarchGeom long_units = m;
+        long_units.join = W == 6;
+        return launch_planes_np<W, 1, 3>(p, long_units, units[0], n[0], rows, grid, scratch, st);
+    }
+    if (m.CS > 8) return launch_planes_np<W, 2, 3>(p, m, units[1], n[1], rows, grid, scratch, st);
+    if (m.CS > 4) return launch_planes_np<W, 4, 3>(p, m, units[2], n[2], rows, grid, scratch, st);
+    return launch_planes_np<W, 8, 3>(p, m, units[3], n[3], rows, grid, scratch, st);
 }
 
 // dynamic shared memory of a gather block: cover lists of the x positions, unit
@@ -1281,6 +1302,36 @@ int march_build(dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s,
     return DMR_OK;
 }
 
+// the short units of single planes (short_planes), from the plan's cell offsets
+int march_short_build(const dmr_plan *p, ShortUnits &out, cudaStream_t st)
+{
+    const Geom &g = p->g;
+    const int W = p->mp_W, T = march_tile(W), TT = T * T;
+    const int64_t nft = (int64_t)g.nframes * p->mp_nt[0] * p->mp_nt[1], n = nft * g.G[2] + 1;
+    PlanTemp tmp(p->device, st);
+    int32_t *counts = nullptr, *starts = nullptr;
+    char *temp = nullptr;
+    size_t tb = 0;
+    DMR_TRY(tmp.alloc(&counts, n));
+    DMR_TRY(tmp.alloc(&starts, n));
+    DMR_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tb, counts, starts, (int)n, st));
+    DMR_TRY(tmp.alloc(&temp, tb));
+    march_unit_count_kernel<<<march_blocks(n), 256, 0, st>>>(p->mp_cstart, nft, TT, g.G[2], W, 1, g.G[2], kShortUnit,
+                                                            counts);
+    DMR_LAUNCHED("march_unit_count_kernel");
+    DMR_CUDA(cub::DeviceScan::ExclusiveSum(temp, tb, counts, starts, (int)n, st));
+    g_launches.fetch_add(1);
+    DMR_CUDA(cudaMemcpyAsync(&out.n, starts + n - 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    DMR_CUDA(cudaStreamSynchronize(st));
+    int4 *list = nullptr;
+    DMR_TRY(plan_alloc(p->device, &list, out.n, st));
+    out.units = list;
+    march_unit_fill_kernel<<<march_blocks(n), 256, 0, st>>>(starts, nft, g.G[2], kShortUnit, list);
+    DMR_LAUNCHED("march_unit_fill_kernel");
+    DMR_CUDA(cudaStreamSynchronize(st));
+    return DMR_OK;
+}
+
 void march_lists(dmr_plan *p, const MarchTotals &totals)
 {
     for (int l = 0; l < totals.n; l++) (l < kUnitLists ? p->mp_nunits[l] : p->mp_nitems) = totals.v[l];
@@ -1429,6 +1480,7 @@ int march_grid(const dmr_plan *p, const void *ksp, int kreal, float2 *grid, bool
     const size_t chunk_bytes = (size_t)npts * ch.CS * sizeof(float2);
     float2 *scratch = nullptr;
     DMR_CHECK(ch.n < 65536, DMR_ERR_UNSUPPORTED, "batch too large");
+    if (!det && short_planes(p, ch.CS)) DMR_TRY(plan_short(p, st));
     if (!p->mp_W) {
         // 2D, too sparse for tiles
         if (det) return DMR_ERR_UNSUPPORTED;

@@ -14,6 +14,8 @@ struct dmr_plan;
 
 namespace dmr {
 
+struct ShortUnits;
+
 struct MarchChunks {
     int64_t n;
     int CS;
@@ -26,11 +28,12 @@ struct MarchChunks {
 // takes them once the stream has been synchronised
 struct MarchTotals {
     int n = 0;
-    int32_t v[6] = {0};
+    int32_t v[5] = {0};
 };
 int march_build(::dmr_plan *p, float *const rk[3], int32_t *keys, int32_t *keys_s, const int32_t *vals,
                 MarchTotals &totals, cudaStream_t st);
 void march_lists(::dmr_plan *p, const MarchTotals &totals);
+int march_short_build(const ::dmr_plan *p, ShortUnits &out, cudaStream_t st);
 
 // 2D: per-sample records in acquisition order, interpolation, and gridding by
 // direct additions to the (zeroed) grid, for `nch` chunks of CS coils from coil

@@ -665,6 +665,8 @@ static int tg_build(const dmr_plan *p, TgBins &out, cudaStream_t st)
 
 int plan_tg(const dmr_plan *p, cudaStream_t st) { return publish(p, p->tg_ptr, st, tg_build); }
 
+int plan_short(const dmr_plan *p, cudaStream_t st) { return publish(p, p->short_ptr, st, march_short_build); }
+
 }  // namespace dmr
 
 namespace {

@@ -165,6 +165,16 @@ struct TgBins {
 // whether a plan can have them (3D, one width of 2..4 on all axes), and the same for them
 bool tg_geometry_ok(const ::dmr_plan *p);
 int plan_tg(const ::dmr_plan *p, cudaStream_t st);
+// Short gridding units of single planes (march.cu), the same way
+struct ShortUnits {
+    void *units = nullptr;
+    int n = 0;
+    ~ShortUnits()
+    {
+        if (units) cudaFreeAsync(units, cudaStreamPerThread);
+    }
+};
+int plan_short(const ::dmr_plan *p, cudaStream_t st);
 // Register-tile gridding: whether the geometry admits it (3D, grid at least
 // a block region plus the kernel support on every axis); plan the block items after the bin sort (host
 // bin offsets h_start, nframes * nbins + 1 entries); scratch bytes a call of
@@ -239,13 +249,14 @@ struct dmr_plan {
     mutable std::atomic<const dmr::PlanBins *> bins_ptr{nullptr};
     const dmr::PlanBins &bins() const { return *bins_ptr.load(std::memory_order_acquire); }
     mutable std::atomic<const dmr::TgBins *> tg_ptr{nullptr};
+    mutable std::atomic<const dmr::ShortUnits *> short_ptr{nullptr};
     float *apod[3] = {nullptr, nullptr, nullptr};  // per-axis apodisation (image index)
     int64_t *foff_dev = nullptr;        // frame offsets on the device (nframes + 1)
     // march order (march.cu; mp_W == 0: not planned; 3D, and 2D plans dense enough
     // for tiles, which have gridding units only): tiles along x and y,
     // CSR offsets per cell, sorted position -> sample and back, per sorted
     // sample the tap weights and z cell, gridding units for 1, 2, 4 and 8
-    // planes per warp and short ones for 1 (int4), the first unit of each (frame tile, plane), and
+    // planes per warp (int4), the first unit of each (frame tile, plane), and
     // interpolation items (int4)
     int mp_W = 0;
     int mp_nt[2] = {0, 0};
@@ -254,8 +265,8 @@ struct dmr_plan {
     int32_t *mp_inv = nullptr;
     int32_t *mp_zc = nullptr;
     float *mp_rec = nullptr;
-    void *mp_units[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    int mp_nunits[5] = {0, 0, 0, 0, 0};
+    void *mp_units[4] = {nullptr, nullptr, nullptr, nullptr};
+    int mp_nunits[4] = {0, 0, 0, 0};
     int32_t *mp_ustart = nullptr;
     void *mp_items = nullptr;
     int mp_nitems = 0;
@@ -280,6 +291,7 @@ struct dmr_plan {
         drop(tables);
         delete bins_ptr.load();
         delete tg_ptr.load();
+        delete short_ptr.load();
         for (int a = 0; a < 3; a++) drop(rk[a]);
         drop(status);
         drop(mp_cstart);
