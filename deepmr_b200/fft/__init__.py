@@ -81,9 +81,9 @@ def set_deterministic_gridding(flag=True):
 
 
 def release_scratch(device=None):
-    """Give the memory that the library's scratch pool holds beyond what is in
-    use back to the device (default: the current CUDA device). Synchronises
-    the device."""
+    """Give the memory that the library's pools hold beyond what is in use (scratch,
+    and what destroyed plans left) back to the device (default: the current CUDA
+    device). Synchronises the device."""
     import torch
 
     from .. import _lib
