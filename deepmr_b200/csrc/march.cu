@@ -1179,13 +1179,16 @@ template <int W>
 int launch_interp(const dmr_plan *p, const MarchGeom &m, const float2 *grid, float2 *rows, cudaStream_t st)
 {
     // a thread per sample for 1 coil (96^3, 1.8 M samples: W 3, os 1.25, 247 us with
-    // lane groups and 105 with this; W 6, os 2, 1,477 and 535), and for 2 at the
-    // widths whose groups take 3 coils or more at a time (W 2 and 3: 0.95 to 1.8
-    // times the groups' speed, W 6 1.1 to 2.1, W 4 and 5 0.86 to 1.5; 4 coils at W 4
-    // 0.6 to 1.0)
+    // lane groups and 105 with this; W 6, os 2, 1,477 and 535), for 2 at the widths
+    // whose groups take 3 coils or more at a time (W 2 and 3: 0.95 to 1.8 times the
+    // groups' speed, W 6 1.1 to 2.1, W 4 and 5 0.86 to 1.5), and for 3 and 4 at widths
+    // 2 and 3 where items have 16 samples or more (4 coils at 65: 1.2 to 1.4 times, at
+    // 16: 1.0 to 1.1, at 2: 0.9 to 1.0; W 4 0.6 to 1.0)
     if (m.CS == 1) return launch_interp_few<W, 1>(p, m, grid, rows, st);
     if constexpr (W <= 3 || W == 6)
         if (m.CS == 2) return launch_interp_few<W, 2>(p, m, grid, rows, st);
+    if constexpr (W <= 3)
+        if (m.CS <= 4 && p->g.total >= 16 * (int64_t)p->mp_nitems) return launch_interp_few<W, 4>(p, m, grid, rows, st);
     // width 6: 10 coils at a time take 1.7 times as long as 5
     if constexpr (W == 6)
         if (5 * ceil_div(m.CS, 10) < 3 * ceil_div(m.CS, 5)) return launch_interp_n<6, 3, 1>(p, m, grid, rows, st);

@@ -406,9 +406,10 @@ def test_rounding_by_coils_and_mode(width, n, calls):
         assert err(*call) < 1.15 * ref, call
 
 
-@pytest.mark.parametrize("width,coils", [(2, (1, 2, 3)), (3, (1, 2, 3)), (4, (1, 2)), (5, (1, 2)),
+@pytest.mark.parametrize("width,coils", [(2, (1, 2, 3, 4, 5)), (3, (1, 2, 3, 4, 5)), (4, (1, 2)), (5, (1, 2)),
                                          (6, (1, 2, 3, 10, 11, 20, 21, 31))])
-def test_forward_lane_layouts(width, coils):
+@pytest.mark.parametrize("nsamples", [3000, 24000])
+def test_forward_lane_layouts(width, coils, nsamples):
     """Interpolation around the coil counts where its lanes change, items with
     hundreds of samples (parts, more samples than threads), with few and with
     none, and regions that wrap."""
@@ -418,7 +419,7 @@ def test_forward_lane_layouts(width, coils):
 
     shape = (13, 9, 21)
     rng = np.random.default_rng(width)
-    c = rng.uniform(-0.5, 0.5, (1, 3000, 3)) * np.asarray(shape[::-1])
+    c = rng.uniform(-0.5, 0.5, (1, nsamples, 3)) * np.asarray(shape[::-1])
     c[:, :2000] *= 0.02
     c[:, -8:] = np.sign(c[:, -8:]) * np.asarray(shape[::-1]) * 0.4999
     c = torch.as_tensor(c.astype(np.float32))
