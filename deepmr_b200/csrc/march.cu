@@ -52,8 +52,8 @@ __host__ __device__ constexpr int march_rec(int W, int ndim = 3) { return (ndim 
 // W 4: 8.1e-7 at 64, 10.2 at 512), and several planes to a warp cost no more in
 // short units (512 and 64: 772 and 790 us; 64^3, 8 coils: 265 and 240). With a
 // plane per warp a unit's flush weighs more (192^3, 32 coils: 12.2 ms at 512, 13.7
-// at 64), so these are long, and short where a call needs it: see launch_planes. At width 6 all are short
-// (144^3, 32 coils: 5.1 and 5.4 ms)
+// at 64), so these are long, and short where a call needs it: see short_planes. At
+// width 6 all are short (144^3, 32 coils: 5.1 and 5.4 ms)
 constexpr int kShortUnit = 64, kLongUnit = 512;
 // unit lists of a plan: planes per warp
 constexpr int kUnitLists = 4;
